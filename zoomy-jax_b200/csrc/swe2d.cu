@@ -68,6 +68,7 @@ struct SweParams {
   // 1: the strip region is the whole grid (fast_i0 = fast_j0 = 0; the strips
   // reach the boundary and keep the control block; no tile launch)
   int strip_full;
+  int sx, sxc;              // output rows of an interior and of a column-EDGE strip item
   // the bed's interior gradient and limiter value (planes gx, gy, phi of
   // zb_swe2d_bed_prepare), read by the eta / HLL-HR interior strip body;
   // nullptr: evaluated from b like every other variable
@@ -714,7 +715,7 @@ swe2d_stage_kernel(const T* __restrict__ bP, const T* __restrict__ hP,
 // that reach the boundary rows take the EDGE body, items whose rows are inside
 // but whose lanes reach a boundary column the column-EDGE body (strip_item
 // below).
-constexpr int SX = 64;          // output rows per work item
+constexpr int SX = 64;          // output rows per work item at most
 constexpr int SW = 28;          // output columns per strip
 constexpr int STRIP_NT = 128;   // four independent warps per CTA
 constexpr int SXC_MAX = 32;     // output rows of the longest column-EDGE item
@@ -1440,6 +1441,13 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
   }
 }
 
+// The strips of a full-coverage grid whose lanes 28 s - 2 .. 28 s + 29 all lie
+// inside it (strips 1 .. the count).
+__host__ __device__ inline int full_mid_strips(int ny) {
+  const int ns = (ny + SW - 1) / SW, mh = ny >= 30 ? (ny - 30) / SW : 0;
+  return mh > ns - 1 ? ns - 1 : mh;
+}
+
 // Full-coverage item list of a grid with nx, ny >= 4 (strips of SW columns
 // from column 0, rows from 0).  Every strip has two EDGE items for the
 // boundary rows [0, 2) and [nx - 2, nx).  The rows between go in chunks: SX
@@ -1457,6 +1465,7 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
 // longest-first lists one after another and lose less to halo rows with 32
 // (2.094 ms per step; 8: 2.21; 16: 2.127; 64: 2.136).
 constexpr int SXC_GRID = 8;
+constexpr int SXC_GRID_SMALL = 4;
 constexpr int SXC_ENS = 32;
 static_assert(SXC_GRID <= SXC_MAX && SXC_ENS <= SXC_MAX, "column-EDGE pre-pass rows");
 __host__ __device__ inline int full_items(int nx, int ny, int item, int* strip, int* r0,
@@ -1464,9 +1473,7 @@ __host__ __device__ inline int full_items(int nx, int ny, int item, int* strip, 
   const int SXC = sxc;
   const int SX = sx;
   const int ns = (ny + SW - 1) / SW;
-  // middle strips: 1 <= s <= mh
-  int mh = ny >= 30 ? (ny - 30) / SW : 0;
-  if (mh > ns - 1) mh = ns - 1;
+  const int mh = full_mid_strips(ny);   // middle strips: 1 <= s <= mh
   const int nmid = mh, nedge = ns - nmid;
   const int nci = nx > 4 ? (nx - 4 + SX - 1) / SX : 0;
   const int ncc = nx > 4 ? (nx - 4 + SXC - 1) / SXC : 0;
@@ -1500,6 +1507,32 @@ __host__ __device__ inline int full_items(int nx, int ny, int item, int* strip, 
   return total;
 }
 
+// Row-chunk heights of a single grid's interior and column-EDGE items.  An
+// item of S rows marches S + 4 (two halo rows each side), and a row of a warp
+// costs about a + b k, k the warps per scheduler, because a lone warp is bound
+// by its own dependent instructions: short chunks on a small grid spread its
+// rows over more warps, long ones on a large grid save halo rows.  With
+// K = strips x rows / (148 SMs x 4 schedulers), k = K / S and the stage takes
+// (S + 4)(a + b K / S), least at S = sqrt(4 b / a K).  Measured on a B200 (us
+// per step, minmod eta / HLL-HR): float32 a = 0.7, b = 0.6, float64 a = 1.4,
+// b = 2.1, hence S = 2 sqrt(K) for both; from K = 160 (about 1650^2) on the
+// chip is full for several waves and whole 64-row items are as good or better
+// (2048^2 float64: 619 us with 64 rows, 635 with 32).  512^2 float32: 8 rows 28.7, 32 rows
+// 51.2, 64 rows 91.9; 1024^2: 16 rows 65.5, 64 rows 97; 2048^2: 32 rows 196, 64
+// rows 197, 8 rows 230; 512^2 float64: 12 rows 70.6, 64 rows 227.  The
+// column-EDGE items run beside the interior ones: below K = 64 (about 1024^2)
+// 8 rows outlast them (512^2 float32: 4 rows 28.7, 8 rows 40.2), above it the
+// halo rows of 4 cost more.
+static void strip_rows(int nstrips, int rows, int* sx, int* sxc) {
+  const double K = (double)std::max(nstrips, 1) * std::max(rows, 1) / 592.0;
+  int s = K < 160.0 ? (int)(2.0 * std::sqrt(K) + 0.5) : SX;
+  s = std::min(std::max(s, 4), SX);
+  // chunks of equal height
+  const int n = (std::max(rows, 1) + s - 1) / s;
+  *sx = (std::max(rows, 1) + n - 1) / n;
+  *sxc = K < 64.0 ? SXC_GRID_SMALL : SXC_GRID;
+}
+
 // KIND 0: the interior strips of a grid with a periodic side (the tile kernel
 // takes the frame); KIND 1: the boundary items of a full-coverage list
 // (column-EDGE and EDGE); KIND 2: its interior items; KIND 3: its interior
@@ -1519,19 +1552,19 @@ swe2d_strip_kernel(const T* __restrict__ bP, const T* __restrict__ hP,
   int strip, r0, r1, kind = 0;
   if (KIND == 0) {
     const int nstrips = (p.fast_j1 - p.fast_j0) / SW;
-    if (item >= nstrips * ((p.fast_i1 - p.fast_i0 + SX - 1) / SX)) return;   // warp-uniform
+    if (item >= nstrips * ((p.fast_i1 - p.fast_i0 + p.sx - 1) / p.sx)) return;   // warp-uniform
     strip = item % nstrips;
-    r0 = p.fast_i0 + (item / nstrips) * SX;
-    r1 = min(r0 + SX, p.fast_i1);
+    r0 = p.fast_i0 + (item / nstrips) * p.sx;
+    r1 = min(r0 + p.sx, p.fast_i1);
   } else {
-    const int ne = full_items(p.nx, p.ny, -2, nullptr, nullptr, nullptr, nullptr, SXC_GRID);
+    const int ne = full_items(p.nx, p.ny, -2, nullptr, nullptr, nullptr, nullptr, p.sxc, p.sx);
     if (KIND == 1 && item >= ne) return;
     if (KIND >= 2) {
       item += ne;
-      const int n = full_items(p.nx, p.ny, -1, nullptr, nullptr, nullptr, nullptr, SXC_GRID);
+      const int n = full_items(p.nx, p.ny, -1, nullptr, nullptr, nullptr, nullptr, p.sxc, p.sx);
       if (item >= n) return;
     }
-    full_items(p.nx, p.ny, item, &strip, &r0, &r1, &kind, SXC_GRID);
+    full_items(p.nx, p.ny, item, &strip, &r0, &r1, &kind, p.sxc, p.sx);
   }
   if (KIND == 1) {
     // warp-uniform: the item's kind
@@ -2107,12 +2140,14 @@ static int run_step(const zb_swe2d_cfg* c, T* Q, T* ws, zb_ctrl* ctrl, int phase
       pf.fast_j1 = 2 + SW * nstrips;
     }
   }
+  strip_rows(pf.strip_full ? full_mid_strips(c->ny) : nstrips,
+             pf.fast_i1 - pf.fast_i0 - (pf.strip_full ? 4 : 0), &pf.sx, &pf.sxc);
   const bool strips = pf.fast_i1 > pf.fast_i0;
   const bool tiles = !pf.strip_full;
   const int nitems = !strips ? 0
                      : pf.strip_full ? full_items(c->nx, c->ny, -1, nullptr, nullptr, nullptr,
-                                                       nullptr, SXC_GRID)
-                                     : nstrips * ((pf.fast_i1 - pf.fast_i0 + SX - 1) / SX);
+                                                  nullptr, pf.sxc, pf.sx)
+                                     : nstrips * ((pf.fast_i1 - pf.fast_i0 + pf.sx - 1) / pf.sx);
   const int sgrid = (nitems + STRIP_NT / 32 - 1) / (STRIP_NT / 32);
   // full coverage: the boundary items on the side stream, the interior items here
   SideStream* side = nullptr;
@@ -2120,7 +2155,7 @@ static int run_step(const zb_swe2d_cfg* c, T* Q, T* ws, zb_ctrl* ctrl, int phase
   if (pf.strip_full) {
     int rc = side_stream(&side);
     if (rc) return rc;
-    ne = full_items(c->nx, c->ny, -2, nullptr, nullptr, nullptr, nullptr, SXC_GRID);
+    ne = full_items(c->nx, c->ny, -2, nullptr, nullptr, nullptr, nullptr, pf.sxc, pf.sx);
     ni = nitems - ne;
   }
   const int wpb = STRIP_NT / 32;
