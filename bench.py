@@ -24,8 +24,8 @@ workload; rank 0 only.
 At N = 1 the same JSON line also reports the other configurations: "fp64"
 (the same 2048^2 step with a float64 state), "chorin"
 (1024^2 Chorin steps at a 1e-8 pressure residual, plain multigrid FCG against
-the learned U-Net smoother), "ensemble" (512 uneven instances, boundary and
-interior strip launches per stage), "triangles" (about 4M Delaunay triangles,
+the learned U-Net smoother), "ensemble" (512 uneven instances, one strip
+launch per stage), "triangles" (about 4M Delaunay triangles,
 500 steps, with the GPU mesh preparation) and "snapshots" (the 2048^2 march
 with asynchronous snapshot output); --no-extra skips them, --legs picks a
 subset.
@@ -395,10 +395,9 @@ def run_gpu(args, rank, world, local_rank, dtype_key=None, with_e2e=True):
     k0 = args.warmup
 
     # timed region: K steps, L2 flushed before each, events around each stage
-    # (a stage = the interior strip launch and the EDGE strip launch beside it
-    # on the library's second stream, joined back before the stage's end event)
+    # (a stage = one launch of the strip kernel)
     K = args.steps
-    launches_per_step = 4
+    launches_per_step = 2
     ev = [[torch.cuda.Event(enable_timing=True) for _ in range(3)] for _ in range(K)]
     barrier()
     torch.cuda.synchronize(dev)
@@ -435,9 +434,7 @@ def run_gpu(args, rank, world, local_rank, dtype_key=None, with_e2e=True):
     roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm_peak,
             "unit": "GB/s", "frac": round(achieved / hbm_peak, 4),
             "traffic": None,
-            "kernel": ("swe2d_strip_kernel<MODE_STEP2>: the interior launch and the boundary "
-                       "launch (column-EDGE and EDGE items) side by side on two streams, "
-                       "timed together (stage 2)"),
+            "kernel": "swe2d_strip_kernel<MODE_STEP2> (stage 2: interior and boundary items)",
             "algorithmic_bytes_per_launch": bytes2,
             "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
             "stage1": {"ms": round(mean1 * 1e3, 4),
@@ -802,12 +799,10 @@ def run_snapshots(local_rank, n=2048, steps=200, snapshots=5):
 
 def run_ensemble(local_rank, steps=2000):
     """The batched configuration: 512 uneven SWE instances (sides log-uniform
-    in [64, 512]) advanced together: per stage persistent launches over every
-    instance's column-EDGE and EDGE strip items beside one over the interior
-    items, and the tile fallback for grids narrower than four cells (unused
-    here): four launches per stage, replayed from a CUDA graph of 30 steps.
-    The launch shape (strip CTAs per SM, column-EDGE and interior chunk
-    heights per size class of instance) is autotuned first on the ensemble
+    in [64, 512]) advanced together: one launch per stage over every
+    instance's strip items, replayed from a CUDA graph of 30 steps.  The launch
+    shape (boundary-strip and interior chunk heights per size class of
+    instance) is autotuned first on the ensemble
     itself, and the tuned shape is the one timed."""
     import torch
     from zoomy_b200.ensemble import Ensemble
@@ -833,7 +828,7 @@ def run_ensemble(local_rank, steps=2000):
                          "bytes_per_cell_update": 68},
             "ms_per_step": round(ms / chunk, 4),
             "value": cells * chunk / (ms * 1e-3), "unit": "cell-updates/s",
-            "launches_per_step": 8,
+            "launches_per_step": 2,
             "autotune_ms_per_step": {k: round(v, 4) for k, v in tuned.items()},
             "launch_shape": ens.tuned_shape,
             "class_instances_cells": ens.class_sizes(),

@@ -133,12 +133,7 @@ int zb_swe2d_bed_prepare(const zb_swe2d_cfg* cfg, const void* Q, void* bed,
 
 /* Initialise the control block for a march starting at time t0 from state Q:
  * clears status and all slots, sets t[phase] = t0 and amax[phase] = the
- * maximum wave speed of Q.  Also creates, once per device and host thread,
- * the library's second stream that the fused step forks its boundary-strip
- * launch onto (call it outside stream capture, on the thread that will step
- * or capture; the steps themselves capture).  Each host thread has its own
- * second stream and fork / join events, so host threads may step different
- * solvers on one device at once.
+ * maximum wave speed of Q.
  * Replaces the first dt_pass (zoomy_jax/fvm/solver2/blocks.py:36-61). */
 int zb_swe2d_init(const zb_swe2d_cfg* cfg, const void* Q, zb_ctrl* ctrl,
                   int phase, double t0, zb_stream_t stream);
@@ -257,13 +252,14 @@ typedef struct {
  * work list and zb_ens_step_part_tuned launches.  No counterpart in the
  * reference (its ensemble is a Python loop over solvers); the autotuner of
  * the host package picks it by timing candidates on the actual ensemble.
- *   tile_x          tile height of the small-grid fallback (8 or 16)
- *   ctas_per_sm     persistent strip CTAs per SM: 1..4 (float32), 1..2 (float64)
+ *   tile_x          8 or 16 (kept for the ABI: every grid runs on strips)
+ *   ctas_per_sm     1..4 (float32), 1..2 (float64) (kept for the ABI: a launch has
+ *                   a warp per work item, scheduled by the hardware)
  *   n_classes       size classes of instances (1..4); an instance of side
  *                   max(nx, ny) belongs to the first class whose
  *                   class_max_side is >= that side (the last class takes
  *                   every larger one); class_max_side increases
- *   edge_rows       column-EDGE chunk height per class (4..32 rows)
+ *   edge_rows       boundary-strip chunk height per class (4..32 rows)
  *   interior_rows   interior chunk height per class (8..1024 rows) */
 typedef struct {
   int32_t tile_x;
@@ -286,17 +282,16 @@ size_t zb_ens_table_bytes(const zb_swe2d_cfg* common,
  * call waits for all work on the current device before it copies (a table
  * that steps in flight still read is not overwritten under them) and returns
  * once the copy has landed: call at set-up, outside stream capture.  The
- * work list holds every instance's (instance, strip, row chunk) items of the single grid's full-coverage list (interior, boundary-
- * column and boundary-row bodies), and (instance, tile) items for grids
- * narrower than four cells.  *n_items_out receives the work-list length
- * (tiles + strips). */
+ * work list holds every instance's (instance, strip, row chunk) items of the
+ * single grid's list (interior and boundary items).  *n_items_out receives the
+ * work-list length. */
 int zb_ens_prepare(const zb_swe2d_cfg* common, const zb_ens_instance* inst,
                    int n_inst, int tile_x, void* table, size_t table_bytes,
                    int* n_items_out);
 
 /* zb_ens_table_bytes / zb_ens_prepare with an explicit launch shape (the
- * untuned calls use one class with 32-row column-EDGE chunks, 64-row interior
- * chunks and 4 (float32) or 2 (float64) strip CTAs per SM). */
+ * untuned calls use one class with 32-row boundary-strip chunks and 64-row
+ * interior chunks). */
 size_t zb_ens_table_bytes_tuned(const zb_swe2d_cfg* common, const zb_ens_instance* inst,
                                 int n_inst, const zb_ens_tuning* tuning);
 int zb_ens_prepare_tuned(const zb_swe2d_cfg* common, const zb_ens_instance* inst,
@@ -304,19 +299,15 @@ int zb_ens_prepare_tuned(const zb_swe2d_cfg* common, const zb_ens_instance* inst
                          size_t table_bytes, int* n_items_out);
 
 /* Reset the n_inst control blocks ctrls[0..n_inst) and seed each instance's
- * wave-speed maximum from its state (zb_swe2d_init per instance; it also
- * creates the second stream, outside stream capture). */
+ * wave-speed maximum from its state (zb_swe2d_init per instance). */
 int zb_ens_init(const zb_swe2d_cfg* common, const void* table, int n_inst,
                 const void* Q, zb_ctrl* ctrls, int phase, double t0,
                 zb_stream_t stream);
 
 /* One SSP-RK2 step of every instance: part 0 = the first stage, 1 = the
- * second, -1 = both.  Each stage is four persistent kernels: warps walking the
- * boundary-column and then the boundary-row strip items on the library's
- * second stream beside warps walking the interior strip items on `stream`,
- * then CTAs walking the tiles of grids narrower than four cells (grid <= 0
- * picks SMs x occupancy for the latter; with no such grid they exit at
- * once).  Each instance takes its own CFL dt (zb_swe2d_step semantics per
+ * second, -1 = both.  Each stage is one launch of a warp per work item (n_items as
+ * zb_ens_prepare returned it; `grid` is kept for the ABI and not read).  Each
+ * instance takes its own CFL dt (zb_swe2d_step semantics per
  * instance). */
 int zb_ens_step_part(const zb_swe2d_cfg* common, const void* table, int n_inst,
                      int n_items, int tile_x, int grid, void* Q, void* W,

@@ -11,16 +11,14 @@
 //   divergence + cell-edge bed source -> Q_out = a Q0 + (1 - a)(Qk + b dt L).
 //
 // Data layout: SoA planes (the reference's (n_state, n_cells) layout), cell
-// (i, j) at i*ny + j.  Two kernels implement a stage.  The tile kernel
-// (swe2d_stage_kernel): a CTA owns a TX x 32 tile (32 cells along the
-// contiguous y axis = one warp-wide coalesced row) and stages the tile plus a
-// 2-cell halo in shared memory; every face of the tile is evaluated exactly
-// once -- the generic stage API, first order, and the frame of grids with a
-// periodic side.  The strip kernel (swe2d_strip_kernel): one warp marches a
-// 32-column strip down its rows in registers -- the fused step (interior and
-// boundary launches side by side).  The final stage also folds in Manning
-// friction, the troubled-cell flag and the float64 maximum wave speed that
-// sets the next dt, so a step queues with no host synchronisation.
+// (i, j) at i*ny + j.  Order 2: the strip kernel (swe2d_strip_kernel), one
+// launch per stage -- a warp marches a 32-column strip down its rows in
+// registers; interior items run the bare stencil, boundary items the same body
+// with the boundary folded in.  Order 1: the tile kernel (swe2d_stage_kernel),
+// a CTA per TX x 32 tile with its halo in shared memory.  Every face of an
+// item is evaluated once.  The final stage also folds in Manning friction, the
+// troubled-cell flag and the float64 maximum wave speed that sets the next dt,
+// so a step queues with no host synchronisation.
 #include <cstdio>
 #include <cstring>
 #include <cmath>
@@ -61,30 +59,22 @@ struct SweParams {
   double dt_stage;          // generic stage: dt (< 0: read ctrl->dt)
   T inv6dx, inv6dy;         // interior least-squares gradient factors
   T inv4dx, inv4dy;         // 1 / (4 dx), 1 / (4 dy): side-class closed forms
-  // output region of the strip kernel ([fast_i0, fast_i1) x [fast_j0,
-  // fast_j1), empty when fast_i0 >= fast_i1); the tile kernel leaves these
-  // cells alone
-  int fast_i0, fast_i1, fast_j0, fast_j1;
-  // 1: the strip region is the whole grid (fast_i0 = fast_j0 = 0; the strips
-  // reach the boundary and keep the control block; no tile launch)
-  int strip_full;
-  int sx, sxc;              // output rows of an interior and of a column-EDGE strip item
+  T inv5dx, inv5dy;         // 1 / (5 dx), 1 / (5 dy): corner closed forms
+  int sx, sxc;              // output rows of an interior and of a boundary-strip item
+  int single;               // 1: one launch, every item in the general body
   // the bed's interior gradient and limiter value (planes gx, gy, phi of
   // zb_swe2d_bed_prepare), read by the eta / HLL-HR interior strip body;
   // nullptr: evaluated from b like every other variable
   const T* bed;
-  LsqTable<T> lsq;
 };
 
 enum { MODE_STEP1 = 0, MODE_STEP2 = 1, MODE_EULER = 2, MODE_STAGE = 3 };
 
 template <typename T, int TX>
 struct Smem {
-  static constexpr int R2X = TX + 4, R2Y = TY + 4, N2 = R2X * R2Y;
-  static constexpr int R1X = TX + 2, R1Y = TY + 2, N1 = R1X * R1Y;
+  static constexpr int RX = TX + 2, RY = TY + 2, N = RX * RY;   // tile + 1-cell halo
   static constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
-  T b[N2], h[N2], w1[N2], w2[N2], w3[N2], aux[N2];
-  T sx[4][N1], sy[4][N1];
+  T b[N], h[N], qx[N], qy[N], hinv[N];
   T fxh[NFX], fxt[NFX], fxl[NFX], fxr[NFX];
   T fyh[NFY], fyt[NFY], fyl[NFY], fyr[NFY];
 };
@@ -213,30 +203,67 @@ __device__ __forceinline__ void riemann(const Side<T>& L, const Side<T>& R, T sg
   Dp = -(half * g * (R.h * R.h - hRs * hRs));
 }
 
-// ── one tile of one stage ───────────────────────────────────────────────────
-// The body of a stage for the TX x 32 tile at (i0, j0), with the stage dt
-// already decided.  Shared by the single-grid kernel (one tile per CTA) and
-// the ensemble kernel (a persistent CTA walks (instance, tile) work items).
-// p may live in kernel-parameter space or in global memory.
-template <typename T, int TX, int ORDER, int RECON, int RIEMANN, int MODE>
-__device__ __forceinline__ void stage_tile(
-    Smem<T, TX>& s, double* red, const int i0, const int j0,
-    const T* __restrict__ bP, const T* __restrict__ hP, const T* __restrict__ qxP,
-    const T* __restrict__ qyP, const T* h0P, const T* qx0P, const T* qy0P, T* hO, T* qxO,
-    T* qyO, zb_ctrl* ctrl, const int phase, const T* __restrict__ hinv_src,
-    const unsigned char* __restrict__ force_o1, unsigned char* __restrict__ trouble_out,
-    const SweParams<T>& p, const double dtd, const bool lead_block) {
+// ── the first-order stage kernel (one tile per CTA) ─────────────────────────
+// Euler / generic stage without reconstruction for the TX x 32 tile of a CTA:
+// the face traces are the cell states.
+template <typename T, int TX, int RIEMANN, int MODE>
+__global__ void __launch_bounds__(NT)
+swe2d_stage_kernel(const T* __restrict__ bP, const T* __restrict__ hP,
+                   const T* __restrict__ qxP, const T* __restrict__ qyP,
+                   const T* h0P, const T* qx0P, const T* qy0P,
+                   T* hO, T* qxO, T* qyO, zb_ctrl* ctrl, int phase,
+                   const T* __restrict__ hinv_src,
+                   unsigned char* __restrict__ trouble_out,
+                   const SweParams<T> p) {
   using S = Smem<T, TX>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  S& s = *reinterpret_cast<S*>(smem_raw);
+  __shared__ double red[NT / 32];
   const int tid = threadIdx.x;
+  const int i0 = blockIdx.y * TX, j0 = blockIdx.x * TY;
   const int nx = p.nx, ny = p.ny;
+  const bool lead_block = blockIdx.x == 0 && blockIdx.y == 0;
+
+  // dt of this step
+  double dtd;
+  if (MODE == MODE_STAGE) {
+    dtd = p.dt_stage >= 0.0 ? p.dt_stage : ctrl->dt;
+  } else {
+    const int nph = (phase + 1) % 3, nnph = (phase + 2) % 3;
+    const double t = ctrl->t[phase];
+    dtd = dt_from_amax(ctrl->amax[phase], t, p.cfl2r, p.den_fac, p.dt_max, p.t_end);
+    const bool ok = isfinite(dtd) && dtd > 0.0;
+    if (lead_block && tid == 0) {
+      if (!ok && t < p.t_end) atomicOr(&ctrl->status, (unsigned)ZB_ST_DT_INVALID);
+      ctrl->dt = ok ? dtd : 0.0;
+      ctrl->t[nph] = ok ? t + dtd : t;
+      ctrl->amax[nnph] = 0.0;
+      ctrl->troubled = 0u;
+      // no-op step (t_end reached or dt invalid): the state is unchanged, so
+      // the next slot carries this slot's wave-speed maximum forward
+      if (!ok) ctrl->amax[nph] = ctrl->amax[phase];
+    }
+    if (!ok) {
+      // the Euler path writes the workspace that is copied back: keep it equal
+      for (int e = tid; e < TX * TY; e += NT) {
+        const int gi = i0 + e / TY, gj = j0 + e % TY;
+        if (gi < nx && gj < ny) {
+          const size_t k = (size_t)gi * ny + gj;
+          hO[k] = hP[k]; qxO[k] = qxP[k]; qyO[k] = qyP[k];
+        }
+      }
+      return;
+    }
+  }
   const bool per_x = p.bc[0] == ZB_BC_PERIODIC;
   const bool per_y = p.bc[2] == ZB_BC_PERIODIC;
   const T dt = T(dtd);
+  const T g = p.g, half = T(0.5);
 
-  // ── phase A: halo-2 load, W transform ──
-  for (int e = tid; e < S::N2; e += NT) {
-    const int r = e / S::R2Y, c = e - r * S::R2Y;
-    int gi = i0 - 2 + r, gj = j0 - 2 + c;
+  // ── halo load ──
+  for (int e = tid; e < S::N; e += NT) {
+    const int r = e / S::RY, c = e - r * S::RY;
+    int gi = i0 - 1 + r, gj = j0 - 1 + c;
     bool ix = gi >= 0 && gi < nx, iy = gj >= 0 && gj < ny;
     if (!ix && per_x && iy) { gi = (gi + nx) % nx; ix = true; }
     if (!iy && per_y && ix) { gj = (gj + ny) % ny; iy = true; }
@@ -245,316 +272,115 @@ __device__ __forceinline__ void stage_tile(
       const size_t k = (size_t)gi * ny + gj;
       vb = bP[k]; vh = hP[k]; vqx = qxP[k]; vqy = qyP[k];
     }
-    const T hinv = kp_hinv(vh, p.eps_kp);
     s.b[e] = vb;
     s.h[e] = vh;
-    s.aux[e] = hinv;
-    if (RECON == ZB_RECON_ETA) {
-      s.w1[e] = vb + vh;
-      s.w2[e] = vqx * hinv;
-      s.w3[e] = vqy * hinv;
-    } else {
-      s.w1[e] = vh;
-      s.w2[e] = vqx;
-      s.w3[e] = vqy;
-    }
+    s.qx[e] = vqx;
+    s.qy[e] = vqy;
+    s.hinv[e] = kp_hinv(vh, p.eps_kp);
   }
   __syncthreads();
 
-  // ── phase B: gradients, bounds, limiter (halo-1 region) ──
-  if (ORDER >= 2) {
-    for (int e = tid; e < S::N1; e += NT) {
-      const int r = e / S::R1Y, c = e - r * S::R1Y;
-      const int gi = i0 - 1 + r, gj = j0 - 1 + c;
-      if (gi < 0 || gi >= nx || gj < 0 || gj >= ny) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v) { s.sx[v][e] = T(0); s.sy[v][e] = T(0); }
-        continue;
-      }
-      const int e2 = (r + 1) * S::R2Y + (c + 1);
-      const bool bxl = gi == 0, bxh = gi == nx - 1, byl = gj == 0, byh = gj == ny - 1;
-      const bool interior = !(bxl || bxh || byl || byh);
-      const int cls = (bxl ? 0 : (bxh ? 2 : 1)) * 3 + (byl ? 0 : (byh ? 2 : 1));
-      const T* wv[4] = {s.b, s.w1, s.w2, s.w3};
-      T phi[4], gxa[4], gya[4];
-      const T ev2 = p.vk_eps2;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const T* W = wv[v];
-        const T u = W[e2];
-        T gx = T(0), gy = T(0), umax = u, umin = u;
-        if (interior) {
-          // the unweighted 3x3 least-squares gradient of a uniform grid in
-          // closed form: the normal matrix is diag(6 dx^2, 6 dy^2), so
-          // g_x = (sum of the row above - sum of the row below) / (6 dx) and
-          // likewise along y (u itself cancels)
-          const T wmm = W[e2 - S::R2Y - 1], wm0 = W[e2 - S::R2Y], wmp = W[e2 - S::R2Y + 1];
-          const T w0m = W[e2 - 1], w0p = W[e2 + 1];
-          const T wpm = W[e2 + S::R2Y - 1], wp0 = W[e2 + S::R2Y], wpp = W[e2 + S::R2Y + 1];
-          gx = ((wpm + wp0 + wpp) - (wmm + wm0 + wmp)) * p.inv6dx;
-          gy = ((wmp + w0p + wpp) - (wmm + w0m + wpm)) * p.inv6dy;
-          umax = fmx3(umax, wp0, fmx3(wm0, w0p, w0m));
-          umin = fmn3(umin, wp0, fmn3(wm0, w0p, w0m));
-        } else {
-          // ghost values of this cell's boundary faces (BC at the cell state;
-          // a wall negates the normal momentum / velocity; periodic = image)
-          T gxv = u, gyv = u;
-          if (bxl || bxh) {
-            const int side = bxl ? 0 : 1;
-            if (p.bc[side] == ZB_BC_PERIODIC) gxv = W[e2 + (bxl ? -S::R2Y : S::R2Y)];
-            else if (p.bc[side] == ZB_BC_WALL && v == 2) gxv = -u;
-          }
-          if (byl || byh) {
-            const int side = byl ? 2 : 3;
-            if (p.bc[side] == ZB_BC_PERIODIC) gyv = W[e2 + (byl ? -1 : 1)];
-            else if (p.bc[side] == ZB_BC_WALL && v == 3) gyv = -u;
-          }
-          const T* wx = p.lsq.w[cls][0];
-          const T* wy = p.lsq.w[cls][1];
-          int k = 0;
-#pragma unroll
-          for (int a = -1; a <= 1; ++a) {
-#pragma unroll
-            for (int bb = -1; bb <= 1; ++bb) {
-              if (a == 0 && bb == 0) continue;
-              const bool ok = gi + a >= 0 && gi + a < nx && gj + bb >= 0 && gj + bb < ny;
-              const T d = ok ? W[e2 + a * S::R2Y + bb] - u : T(0);
-              gx += wx[k] * d;
-              gy += wy[k] * d;
-              ++k;
-            }
-          }
-          if (bxl || bxh) { const T d = gxv - u; gx += wx[8] * d; gy += wy[8] * d; }
-          if (byl || byh) { const T d = gyv - u; gx += wx[9] * d; gy += wy[9] * d; }
-          // bounds: inside face neighbours + ghost 2 u_bf - u
-          if (!bxh) { umax = fmx(umax, W[e2 + S::R2Y]); umin = fmn(umin, W[e2 + S::R2Y]); }
-          if (!bxl) { umax = fmx(umax, W[e2 - S::R2Y]); umin = fmn(umin, W[e2 - S::R2Y]); }
-          if (!byh) { umax = fmx(umax, W[e2 + 1]); umin = fmn(umin, W[e2 + 1]); }
-          if (!byl) { umax = fmx(umax, W[e2 - 1]); umin = fmn(umin, W[e2 - 1]); }
-          if (bxl || bxh) { const T gg = T(2) * gxv - u; umax = fmx(umax, gg); umin = fmn(umin, gg); }
-          if (byl || byh) { const T gg = T(2) * gyv - u; umax = fmx(umax, gg); umin = fmn(umin, gg); }
-        }
-        gxa[v] = gx;
-        gya[v] = gy;
-        phi[v] = limiter_phi(p.limiter, gx, gy, p.half_dx, p.half_dy,
-                             umax - u, umin - u, ev2);
-      }
-      if (RECON == ZB_RECON_ETA) {
-        if (p.eps_wet >= T(0) && s.h[e2] < p.eps_wet) {
-          phi[0] = phi[1] = phi[2] = phi[3] = T(0);
-        }
-        phi[0] = zmin(phi[0], phi[1]);
-        phi[2] = zmin(phi[2], phi[1]);
-        phi[3] = zmin(phi[3], phi[1]);
-      }
-      if (force_o1 != nullptr && force_o1[(size_t)gi * ny + gj]) {
-        phi[0] = phi[1] = phi[2] = phi[3] = T(0);
-      }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        s.sx[v][e] = phi[v] * gxa[v];
-        s.sy[v][e] = phi[v] * gya[v];
-      }
-    }
-    __syncthreads();
-  }
-
-  // ── phase C: faces ──
-  // side trace of the cell at R2 index e2 / R1 index e1 at offset o along the
-  // face axis (the other offset component is zero: its term is dropped)
-  auto trace = [&](auto axis_tag, int e2, int e1, T o, Side<T>& sd) {
+  // ── faces ──
+  // a cell's state with its velocities from the given hinv (a seam partner
+  // takes the OWNER's: the flux pass hands the inner cell's aux to both sides
+  // of a boundary face, solver_jax.py:827-866)
+  auto side = [&](int e, T hinv, Side<T>& sd) {
+    sd.b = s.b[e];
+    sd.h = s.h[e];
+    sd.qx = s.qx[e];
+    sd.qy = s.qy[e];
+    sd.ux = sd.qx * hinv;
+    sd.uy = sd.qy * hinv;
+  };
+  auto face = [&](auto axis_tag, int eL, int eR, bool lo, bool hi, int kind, T& Fh, T& Ft, T& l,
+                  T& r) {
     constexpr int AX = decltype(axis_tag)::value;
-    T vb = s.b[e2], w1 = s.w1[e2], w2 = s.w2[e2], w3 = s.w3[e2];
-    if (ORDER >= 2) {
-      if (AX == 0) {
-        vb = vb + s.sx[0][e1] * o; w1 = w1 + s.sx[1][e1] * o;
-        w2 = w2 + s.sx[2][e1] * o; w3 = w3 + s.sx[3][e1] * o;
+    Side<T> A, B;
+    T Fx, Fy, Dm, Dp;
+    if (lo || hi) {
+      const int eo = lo ? eR : eL;
+      const T sg = lo ? T(-1) : T(1);
+      side(eo, s.hinv[eo], A);
+      if (kind == ZB_BC_PERIODIC) {
+        side(lo ? eL : eR, s.hinv[eo], B);
       } else {
-        vb = vb + s.sy[0][e1] * o; w1 = w1 + s.sy[1][e1] * o;
-        w2 = w2 + s.sy[2][e1] * o; w3 = w3 + s.sy[3][e1] * o;
+        B = A;
+        if (kind == ZB_BC_WALL) {   // q - 2 (q.n) n
+          if (AX == 0) { B.qx = -A.qx; B.ux = -A.ux; }
+          else { B.qy = -A.qy; B.uy = -A.uy; }
+        }
       }
-    }
-    sd.b = vb;
-    if (RECON == ZB_RECON_ETA) {
-      const T eta = fmx(w1, vb);
-      const T hf = eta - vb;
-      sd.h = hf;
-      sd.ux = w2;
-      sd.uy = w3;
-      sd.qx = w2 * hf;
-      sd.qy = w3 * hf;
+      riemann<T, RIEMANN, AX>(A, B, sg, g, Fh, Fx, Fy, Dm, Dp);
+      const T Fn = AX == 0 ? Fx : Fy, Ftr = AX == 0 ? Fy : Fx;
+      const T own_n = Fn + Dm * sg;
+      Fh = lo ? -Fh : Fh;
+      Ft = lo ? -Ftr : Ftr;
+      r = lo ? own_n : T(0);
+      l = lo ? T(0) : own_n;
     } else {
-      const T hinv = s.aux[e2];
-      sd.h = w1;
-      sd.qx = w2;
-      sd.qy = w3;
-      sd.ux = w2 * hinv;
-      sd.uy = w3 * hinv;
+      side(eL, s.hinv[eL], A);
+      side(eR, s.hinv[eR], B);
+      riemann<T, RIEMANN, AX>(A, B, T(1), g, Fh, Fx, Fy, Dm, Dp);
+      const T Fn = AX == 0 ? Fx : Fy;
+      Ft = AX == 0 ? Fy : Fx;
+      l = Fn + Dm;
+      r = -Fn + Dp;
     }
   };
-  using AxX = std::integral_constant<int, 0>;
-  using AxY = std::integral_constant<int, 1>;
-  // periodic seam: Q_R is the partner cell's (unreconstructed) state; its
-  // velocity is the partner's own W row on the eta path and q times the
-  // OWNER's hinv on the conservative path (the flux pass hands the inner
-  // cell's aux to both sides of a boundary face, solver_jax.py:827-866)
-  auto partner = [&](int e2img, T hinv_owner, Side<T>& sd) {
-    sd.b = s.b[e2img];
-    sd.h = s.h[e2img];
-    if (RECON == ZB_RECON_ETA) {
-      sd.ux = s.w2[e2img];
-      sd.uy = s.w3[e2img];
-      sd.qx = sd.ux * sd.h;   // not read by the hydrostatic-reconstruction fluxes
-      sd.qy = sd.uy * sd.h;
-    } else {
-      sd.qx = s.w2[e2img];
-      sd.qy = s.w3[e2img];
-      sd.ux = sd.qx * hinv_owner;
-      sd.uy = sd.qy * hinv_owner;
-    }
-  };
-  const T g = p.g;
-  const T half = T(0.5);
-  // x-faces
   for (int e = tid; e < S::NFX; e += NT) {
     const int fi = e / TY, fj = e - fi * TY;
     const int gi = i0 + fi, gj = j0 + fj;
     if (gj >= ny || gi > nx) continue;
-    const int e2L = (fi + 1) * S::R2Y + (fj + 2), e2R = e2L + S::R2Y;
-    const int e1L = fi * S::R1Y + (fj + 1), e1R = e1L + S::R1Y;
-    Side<T> A, B;
-    T Fh, Fx, Fy, Dm, Dp;
-    if (gi == 0 || gi == nx) {
-      const bool lo = gi == 0;
-      const int e2o = lo ? e2R : e2L, e1o = lo ? e1R : e1L;
-      const T sg = lo ? T(-1) : T(1);
-      trace(AxX(), e2o, e1o, sg * p.half_dx, A);
-      const int kind = p.bc[lo ? 0 : 1];
-      if (kind == ZB_BC_PERIODIC) {
-        partner(lo ? e2L : e2R, s.aux[e2o], B);
-      } else {
-        B = A;
-        if (kind == ZB_BC_WALL) {   // q - 2 (q.n) n with n = (sg, 0): q_x -> -q_x
-          B.qx = -A.qx;
-          B.ux = -A.ux;
-        }
-      }
-      riemann<T, RIEMANN, 0>(A, B, sg, g, Fh, Fx, Fy, Dm, Dp);
-      T ces = T(0);
-      if (ORDER >= 2) ces = half * g * (s.h[e2o] + A.h) * (A.b - s.b[e2o]);
-      const T own_n = Fx + Dm * sg + ces * sg;
-      if (lo) {
-        s.fxh[e] = -Fh; s.fxt[e] = -Fy; s.fxr[e] = own_n; s.fxl[e] = T(0);
-      } else {
-        s.fxh[e] = Fh; s.fxt[e] = Fy; s.fxl[e] = own_n; s.fxr[e] = T(0);
-      }
-    } else {
-      trace(AxX(), e2L, e1L, p.half_dx, A);
-      trace(AxX(), e2R, e1R, -p.half_dx, B);
-      riemann<T, RIEMANN, 0>(A, B, T(1), g, Fh, Fx, Fy, Dm, Dp);
-      T cesA = T(0), cesB = T(0);
-      if (ORDER >= 2) {
-        cesA = half * g * (s.h[e2L] + A.h) * (A.b - s.b[e2L]);
-        cesB = -(half * g * (s.h[e2R] + B.h) * (B.b - s.b[e2R]));
-      }
-      s.fxh[e] = Fh;
-      s.fxt[e] = Fy;
-      s.fxl[e] = Fx + Dm + cesA;
-      s.fxr[e] = -Fx + Dp + cesB;
-    }
+    const int eL = fi * S::RY + (fj + 1);
+    face(std::integral_constant<int, 0>(), eL, eL + S::RY, gi == 0, gi == nx,
+         p.bc[gi == 0 ? 0 : 1], s.fxh[e], s.fxt[e], s.fxl[e], s.fxr[e]);
   }
-  // y-faces
   for (int e = tid; e < S::NFY; e += NT) {
     const int fi = e / (TY + 1), fj = e - fi * (TY + 1);
     const int gi = i0 + fi, gj = j0 + fj;
     if (gi >= nx || gj > ny) continue;
-    const int e2L = (fi + 2) * S::R2Y + (fj + 1), e2R = e2L + 1;
-    const int e1L = (fi + 1) * S::R1Y + fj, e1R = e1L + 1;
-    Side<T> A, B;
-    T Fh, Fx, Fy, Dm, Dp;
-    if (gj == 0 || gj == ny) {
-      const bool lo = gj == 0;
-      const int e2o = lo ? e2R : e2L, e1o = lo ? e1R : e1L;
-      const T sg = lo ? T(-1) : T(1);
-      trace(AxY(), e2o, e1o, sg * p.half_dy, A);
-      const int kind = p.bc[lo ? 2 : 3];
-      if (kind == ZB_BC_PERIODIC) {
-        partner(lo ? e2L : e2R, s.aux[e2o], B);
-      } else {
-        B = A;
-        if (kind == ZB_BC_WALL) {   // n = (0, sg): q_y -> -q_y
-          B.qy = -A.qy;
-          B.uy = -A.uy;
-        }
-      }
-      riemann<T, RIEMANN, 1>(A, B, sg, g, Fh, Fx, Fy, Dm, Dp);
-      T ces = T(0);
-      if (ORDER >= 2) ces = half * g * (s.h[e2o] + A.h) * (A.b - s.b[e2o]);
-      const T own_n = Fy + Dm * sg + ces * sg;
-      if (lo) {
-        s.fyh[e] = -Fh; s.fyt[e] = -Fx; s.fyr[e] = own_n; s.fyl[e] = T(0);
-      } else {
-        s.fyh[e] = Fh; s.fyt[e] = Fx; s.fyl[e] = own_n; s.fyr[e] = T(0);
-      }
-    } else {
-      trace(AxY(), e2L, e1L, p.half_dy, A);
-      trace(AxY(), e2R, e1R, -p.half_dy, B);
-      riemann<T, RIEMANN, 1>(A, B, T(1), g, Fh, Fx, Fy, Dm, Dp);
-      T cesA = T(0), cesB = T(0);
-      if (ORDER >= 2) {
-        cesA = half * g * (s.h[e2L] + A.h) * (A.b - s.b[e2L]);
-        cesB = -(half * g * (s.h[e2R] + B.h) * (B.b - s.b[e2R]));
-      }
-      s.fyh[e] = Fh;
-      s.fyt[e] = Fx;
-      s.fyl[e] = Fy + Dm + cesA;
-      s.fyr[e] = -Fy + Dp + cesB;
-    }
+    const int eL = (fi + 1) * S::RY + fj;
+    face(std::integral_constant<int, 1>(), eL, eL + 1, gj == 0, gj == ny, p.bc[gj == 0 ? 2 : 3],
+         s.fyh[e], s.fyt[e], s.fyl[e], s.fyr[e]);
   }
   __syncthreads();
 
-  // ── phase D: divergence, stage update, epilogue ──
+  // ── divergence, stage update, epilogue ──
   double amax_loc = 0.0;
   bool bad = false;
   for (int e = tid; e < TX * TY; e += NT) {
     const int ti = e / TY, tj = e - ti * TY;
     const int gi = i0 + ti, gj = j0 + tj;
     if (gi >= nx || gj >= ny) continue;
-    // cells of the interior strip kernel's region are its to write
-    if (gi >= p.fast_i0 && gi < p.fast_i1 && gj >= p.fast_j0 && gj < p.fast_j1) continue;
     const int fl = ti * TY + tj, fr = fl + TY;
     const int fb = ti * (TY + 1) + tj, ft = fb + 1;
     const T kx = p.kx, ky = p.ky;
     const T dh = -(kx * (s.fxh[fr] - s.fxh[fl]) + ky * (s.fyh[ft] - s.fyh[fb]));
     const T dqx = -(kx * (s.fxl[fr] + s.fxr[fl]) + ky * (s.fyt[ft] - s.fyt[fb]));
     const T dqy = -(kx * (s.fxt[fr] - s.fxt[fl]) + ky * (s.fyl[ft] + s.fyr[fb]));
-    const int e2 = (ti + 2) * S::R2Y + (tj + 2);
-    const T hk = s.h[e2];
-    T qxk, qyk;
-    if (RECON == ZB_RECON_ETA) {
-      const size_t k = (size_t)gi * ny + gj;
-      qxk = qxP[k];
-      qyk = qyP[k];
-    } else {
-      qxk = s.w2[e2];
-      qyk = s.w3[e2];
-    }
+    const int e1 = (ti + 1) * S::RY + (tj + 1);
+    const T hk = s.h[e1], qxk = s.qx[e1], qyk = s.qy[e1];
     T hn, qxn, qyn;
     const size_t k = (size_t)gi * ny + gj;
-    if (MODE == MODE_STEP1) {
+    if (MODE == MODE_EULER) {
       hn = hk + dt * dh;
       qxn = qxk + dt * dqx;
       qyn = qyk + dt * dqy;
-    } else if (MODE == MODE_STEP2) {
-      const T h2 = hk + dt * dh, qx2 = qxk + dt * dqx, qy2 = qyk + dt * dqy;
-      const T h0 = h0P[k], qx0 = qx0P[k], qy0 = qy0P[k];
-      hn = half * (h0 + h2);
-      qxn = half * (qx0 + qx2);
-      qyn = half * (qy0 + qy2);
-    } else if (MODE == MODE_EULER) {
-      hn = hk + dt * dh;
-      qxn = qxk + dt * dqx;
-      qyn = qyk + dt * dqy;
+      if (p.manning_n != T(0)) {
+        // source as RK1 after the hyperbolic step with the step's input aux
+        // (zoomy_jax/fvm/solver_jax.py:1129; ode.py:14-18)
+        const T hi0 = kp_hinv(hk, p.eps_kp);
+        const T qn = asqrt(qxn * qxn + qyn * qyn);
+        const T kf = (-p.g) * (p.manning_n * p.manning_n) * qn * (hi0 * hi0) * cbrt(hi0);
+        if (p.implicit_source) {
+          const T den = T(1) + dt * (-kf);
+          qxn = qxn / den;
+          qyn = qyn / den;
+        } else {
+          qxn = qxn + dt * (qxn * kf);
+          qyn = qyn + dt * (qyn * kf);
+        }
+      }
     } else {
       const T a = T(p.alpha), bt = T(p.beta);
       T sqx = dqx, sqy = dqy;
@@ -577,30 +403,14 @@ __device__ __forceinline__ void stage_tile(
         hn = h2; qxn = qx2; qyn = qy2;
       }
     }
-    if ((MODE == MODE_STEP2 || MODE == MODE_EULER) && p.manning_n != T(0)) {
-      // source as RK1 after the hyperbolic step with the step's input aux
-      // (zoomy_jax/fvm/solver_jax.py:1129; ode.py:14-18)
-      const T h0 = (MODE == MODE_STEP2) ? h0P[k] : hk;
-      const T hi0 = kp_hinv(h0, p.eps_kp);
-      const T qn = asqrt(qxn * qxn + qyn * qyn);
-      const T kf = (-p.g) * (p.manning_n * p.manning_n) * qn * (hi0 * hi0) * cbrt(hi0);
-      if (p.implicit_source) {
-        const T den = T(1) + dt * (-kf);
-        qxn = qxn / den;
-        qyn = qyn / den;
-      } else {
-        qxn = qxn + dt * (qxn * kf);
-        qyn = qyn + dt * (qyn * kf);
-      }
-    }
     hO[k] = hn;
     qxO[k] = qxn;
     qyO[k] = qyn;
     const bool tr = (hn < T(0)) || !isfinite(hn) || !isfinite(qxn) || !isfinite(qyn) ||
-                    !isfinite(s.b[e2]);
+                    !isfinite(s.b[e1]);
     bad = bad || tr;
     if (trouble_out != nullptr) trouble_out[k] = tr ? 1 : 0;
-    if (MODE == MODE_STEP2 || MODE == MODE_EULER) {
+    if (MODE == MODE_EULER) {
       const T hi = kp_hinv(hn, p.eps_kp);
       const T c = asqrt(g * fmx(hn, T(0)));
       const T lx = fabs(qxn * hi) + c, ly = fabs(qyn * hi) + c;
@@ -609,7 +419,7 @@ __device__ __forceinline__ void stage_tile(
   }
   const unsigned anybad = __syncthreads_or(bad ? 1 : 0);
   if (anybad && tid == 0) atomicOr(&ctrl->status, (unsigned)ZB_ST_TROUBLED);
-  if (MODE == MODE_STEP2 || MODE == MODE_EULER) {
+  if (MODE == MODE_EULER) {
     const double m = block_max_double(amax_loc, red);
     if (tid == 0) {
       atomic_max_pos_double(&ctrl->amax[(phase + 1) % 3], m);
@@ -618,107 +428,16 @@ __device__ __forceinline__ void stage_tile(
   }
 }
 
-// ── the fused stage kernel (one tile per CTA) ───────────────────────────────
-template <typename T, int TX, int ORDER, int RECON, int RIEMANN, int MODE>
-__global__ void __launch_bounds__(NT)
-swe2d_stage_kernel(const T* __restrict__ bP, const T* __restrict__ hP,
-                   const T* __restrict__ qxP, const T* __restrict__ qyP,
-                   const T* h0P, const T* qx0P, const T* qy0P,
-                   T* hO, T* qxO, T* qyO, zb_ctrl* ctrl, int phase,
-                   const T* __restrict__ hinv_src,
-                   const unsigned char* __restrict__ force_o1,
-                   unsigned char* __restrict__ trouble_out,
-                   const SweParams<T> p) {
-  using S = Smem<T, TX>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  S& s = *reinterpret_cast<S*>(smem_raw);
-  __shared__ double red[NT / 32];
-
-  const int tid = threadIdx.x;
-  int i0 = blockIdx.y * TX, j0 = blockIdx.x * TY;
-  if (p.fast_i1 > p.fast_i0) {
-    // frame launch (1-D grid): enumerate only the tiles that hold cells outside
-    // the strip kernel's region -- whole tile rows above and below it, then
-    // the tile columns left and right of it for the rows in between
-    const int ntc = (p.ny + TY - 1) / TY, ntr = (p.nx + TX - 1) / TX;
-    // (bands never overlap: a region narrower than a tile leaves tcb = tca)
-    const int tra = (p.fast_i0 + TX - 1) / TX, trb = max(tra, p.fast_i1 / TX);
-    const int tca = (p.fast_j0 + TY - 1) / TY, tcb = max(tca, p.fast_j1 / TY);
-    const int nside = tca + (ntc - tcb);
-    int b = blockIdx.x;
-    if (b < tra * ntc) {
-      i0 = (b / ntc) * TX; j0 = (b % ntc) * TY;
-    } else if ((b -= tra * ntc) < (ntr - trb) * ntc) {
-      i0 = (trb + b / ntc) * TX; j0 = (b % ntc) * TY;
-    } else {
-      b -= (ntr - trb) * ntc;
-      const int tr = tra + b / nside, k = b % nside;
-      i0 = tr * TX;
-      j0 = (k < tca ? k : tcb + (k - tca)) * TY;
-    }
-  }
-
-  // dt of this step
-  double dtd;
-  if (MODE == MODE_STAGE) {
-    dtd = p.dt_stage >= 0.0 ? p.dt_stage : ctrl->dt;
-  } else {
-    const int ph = phase;
-    const int nph = (ph + 1) % 3, nnph = (ph + 2) % 3;
-    const double t = ctrl->t[ph];
-    dtd = dt_from_amax(ctrl->amax[ph], t, p.cfl2r, p.den_fac, p.dt_max, p.t_end);
-    const bool ok = isfinite(dtd) && dtd > 0.0;
-    const bool lead = blockIdx.x == 0 && blockIdx.y == 0 && tid == 0;
-    if ((MODE == MODE_STEP1 || MODE == MODE_EULER) && lead) {
-      if (!ok && t < p.t_end) atomicOr(&ctrl->status, (unsigned)ZB_ST_DT_INVALID);
-      ctrl->dt = ok ? dtd : 0.0;
-      ctrl->t[nph] = ok ? t + dtd : t;
-      ctrl->amax[nnph] = 0.0;
-      ctrl->troubled = 0u;
-    }
-    if (!ok) {
-      // no-op step (t_end reached or dt invalid): the state is unchanged, so
-      // the next slot carries this slot's wave-speed maximum forward
-      if ((MODE == MODE_STEP2 || MODE == MODE_EULER) && lead) ctrl->amax[nph] = ctrl->amax[ph];
-      if (MODE == MODE_EULER) {
-        // the Euler path writes the workspace that is copied back: keep it equal
-        const int nx_ = p.nx, ny_ = p.ny;
-        for (int e = tid; e < TX * TY; e += NT) {
-          const int gi = i0 + e / TY, gj = j0 + e % TY;
-          if (gi < nx_ && gj < ny_) {
-            const size_t k = (size_t)gi * ny_ + gj;
-            hO[k] = hP[k]; qxO[k] = qxP[k]; qyO[k] = qyP[k];
-          }
-        }
-      }
-      return;
-    }
-  }
-  // a tile wholly inside the strip kernel's region has nothing to write (the
-  // lead block sits at the corner, outside the region)
-  if (i0 >= p.fast_i0 && i0 + TX <= p.fast_i1 && j0 >= p.fast_j0 && j0 + TY <= p.fast_j1) return;
-  stage_tile<T, TX, ORDER, RECON, RIEMANN, MODE>(
-      s, red, i0, j0, bP, hP, qxP, qyP, h0P, qx0P, qy0P, hO, qxO, qyO, ctrl, phase, hinv_src,
-      force_o1, trouble_out, p, dtd, blockIdx.x == 0 && blockIdx.y == 0);
-}
-
-
 // ── the strip kernel ───────────────────────────────────────────────────────
-// The stage arithmetic of stage_tile organised for registers instead of
-// shared memory: one warp owns a strip of 32 contiguous columns (28 outputs
-// plus two halo columns on each side) and marches down its rows.  Each lane
-// keeps a sliding window of three rows of W, the limited slopes of two rows
-// and the last x-face's fluxes in registers; the column neighbours come from
-// warp shuffles.  Every face is still evaluated once.  Interior items (every
-// cell two cells from every boundary) take the interior body, which for
-// float64 evaluates stage_tile's float expressions (the same bits); items
-// that reach the boundary rows take the EDGE body, items whose rows are inside
-// but whose lanes reach a boundary column the column-EDGE body (strip_item
-// below).
+// The order-2 stage organised for registers: one warp owns a strip of 32
+// contiguous columns (28 outputs plus two halo columns on each side) and
+// marches down its rows.  Each lane keeps a sliding window of three rows of W,
+// the limited slopes of two rows and the last x-face's fluxes in registers; the
+// column neighbours come from warp shuffles.  Every face is evaluated once.
 constexpr int SX = 64;          // output rows per work item at most
 constexpr int SW = 28;          // output columns per strip
 constexpr int STRIP_NT = 128;   // four independent warps per CTA
-constexpr int SXC_MAX = 32;     // output rows of the longest column-EDGE item
+constexpr int SXC_MAX = 32;     // output rows of the ensemble's longest boundary-strip item
 
 template <typename T>
 struct RowW {
@@ -783,27 +502,49 @@ __device__ __forceinline__ NextRow next_row(const RowW<float>& R0, const float* 
   return n;
 }
 
+// The faces of a strip row that lie on the boundary: the x-face (rows r-2 | r-1) where xlo / xhi, the
+// y-face where ylo (this lane is the ghost below column 0) / yhi (column
+// ny - 1).  A boundary face takes the owner's trace on both sides, its normal
+// velocity times sx / sy (-1: a wall mirrors it; +1: extrapolation) on the
+// ghost's; a periodic side passes no flag (its ghost lanes and rows hold the
+// partner cell with zero slopes).
+struct EdgeFaces {
+  bool xlo, xhi, ylo, yhi;
+  float sx, sy;
+};
+
+template <bool EDGE, typename P>
 __device__ __forceinline__ void faces_pair(const RowW<float>& R0, const RowW<float>& R1,
                                            const float* slA, const float* slB,
-                                           const NextRow& nx_, const SweParams<float>& p,
-                                           float& Fh, float& Fy, float& fxl_n, float& fxr_n,
+                                           const NextRow& nx_, const P& p,
+                                           const EdgeFaces& ef, float& Fh, float& Fy, float& fxl_n, float& fxr_n,
                                            float& Gh, float& Gx, float& fyl_t, float& fyr_own) {
   const float g = p.g, hg = 0.5f * g;
   const float nb_b = nx_.b, nb_w1 = nx_.w1, nb_w2 = nx_.w2, nb_w3 = nx_.w3, nb_h = nx_.h;
   const float sn4 = nx_.s4, sn5 = nx_.s5, sn6 = nx_.s6, sn7 = nx_.s7;
-  const float2 o1 = f2(p.half_dx, p.half_dy), o2 = f2(-p.half_dx, -p.half_dy);
+  const float2 o1 = f2(p.half_dx, p.half_dy), o2 = f2(-o1.x, -o1.y);
   // side 1: row r-2 towards +x (x-face) and towards +y (y-face)
-  const float2 b1 = fma2(f2(slA[0], slA[4]), o1, f2(R0.b, R0.b));
+  float2 b1 = fma2(f2(slA[0], slA[4]), o1, f2(R0.b, R0.b));
   const float2 e1 = fma2(f2(slA[1], slA[5]), o1, f2(R0.w1, R0.w1));
-  const float2 un1 = fma2(f2(slA[2], slA[7]), o1, f2(R0.w2, R0.w3));
-  const float2 ut1 = fma2(f2(slA[3], slA[6]), o1, f2(R0.w3, R0.w2));
-  const float2 h1 = sub2(f2(fmaxf(e1.x, b1.x), fmaxf(e1.y, b1.y)), b1);   // Audusse clip
+  float2 un1 = fma2(f2(slA[2], slA[7]), o1, f2(R0.w2, R0.w3));
+  float2 ut1 = fma2(f2(slA[3], slA[6]), o1, f2(R0.w3, R0.w2));
+  float2 h1 = sub2(f2(fmaxf(e1.x, b1.x), fmaxf(e1.y, b1.y)), b1);   // Audusse clip
   // side 2: row r-1 towards -x and the next lane's row r-2 towards -y
-  const float2 b2 = fma2(f2(slB[0], sn4), o2, f2(R1.b, nb_b));
+  float2 b2 = fma2(f2(slB[0], sn4), o2, f2(R1.b, nb_b));
   const float2 e2 = fma2(f2(slB[1], sn5), o2, f2(R1.w1, nb_w1));
-  const float2 un2 = fma2(f2(slB[2], sn7), o2, f2(R1.w2, nb_w3));
-  const float2 ut2 = fma2(f2(slB[3], sn6), o2, f2(R1.w3, nb_w2));
-  const float2 h2 = sub2(f2(fmaxf(e2.x, b2.x), fmaxf(e2.y, b2.y)), b2);
+  float2 un2 = fma2(f2(slB[2], sn7), o2, f2(R1.w2, nb_w3));
+  float2 ut2 = fma2(f2(slB[3], sn6), o2, f2(R1.w3, nb_w2));
+  float2 h2 = sub2(f2(fmaxf(e2.x, b2.x), fmaxf(e2.y, b2.y)), b2);
+  if (EDGE) {
+    // x: uniform over the warp
+    if (ef.xlo) { b1.x = b2.x; h1.x = h2.x; un1.x = ef.sx * un2.x; ut1.x = ut2.x; }
+    if (ef.xhi) { b2.x = b1.x; h2.x = h1.x; un2.x = ef.sx * un1.x; ut2.x = ut1.x; }
+    // y: the lane below column 0 and the lane of column ny - 1
+    b1.y = ef.ylo ? b2.y : b1.y; h1.y = ef.ylo ? h2.y : h1.y;
+    un1.y = ef.ylo ? ef.sy * un2.y : un1.y; ut1.y = ef.ylo ? ut2.y : ut1.y;
+    b2.y = ef.yhi ? b1.y : b2.y; h2.y = ef.yhi ? h1.y : h2.y;
+    un2.y = ef.yhi ? ef.sy * un1.y : un2.y; ut2.y = ef.yhi ? ut1.y : ut2.y;
+  }
   // hydrostatic reconstruction
   const float2 bs = f2(fmaxf(b1.x, b2.x), fmaxf(b1.y, b2.y));
   const float2 t1 = sub2(add2(h1, b1), bs), t2 = sub2(add2(h2, b2), bs);
@@ -842,178 +583,105 @@ __device__ __forceinline__ void faces_pair(const RowW<float>& R0, const RowW<flo
   Gh = Fh2.y; Gx = Ft2.y; fyl_t = fl.y; fyr_own = fr.y;
 }
 
-// Column-EDGE pre-pass for one row: the boundary column's cell (m, c), c = 0
-// (low side) or ny - 1, m two cells or more from the x boundaries.  out[0..8):
-// its limited slopes [sx0..3, sy0..3] (the EDGE body's side-class closed form,
-// limiter, dry demotion and ties); out[8..12): Gh, Gx, fyl_t, fyr_own of its
-// boundary y-face (the owner's trace against its ghost with normal sign sgy),
-// as the EDGE body leaves them on the lane that evaluates that face (cj = -1
-// for the low side, cj = ny - 1 for the high side).
-template <typename T, int RECON, int RIEMANN>
-__device__ __forceinline__ void bcol_row(const T* __restrict__ bP, const T* __restrict__ hP,
-                                         const T* __restrict__ qxP, const T* __restrict__ qyP,
-                                         const SweParams<T>& p, int m, int c, T* out) {
-  const int ny = p.ny;
-  const bool lo = c == 0;
-  const int ci = lo ? 1 : ny - 2;
-  RowW<T> Wc[3], Wi[3];   // rows m - 1, m, m + 1 of column c and of its inner neighbour ci
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const size_t k = (size_t)(m - 1 + a) * ny + (s ? ci : c);
-      const T vb = bP[k], vh = hP[k], vqx = qxP[k], vqy = qyP[k];
-      RowW<T>& w = s ? Wi[a] : Wc[a];
-      const T hinv = kp_hinv(vh, p.eps_kp);
-      w.b = vb;
-      w.h = vh;
-      w.hinv = hinv;
-      if (RECON == ZB_RECON_ETA) {
-        w.w1 = vb + vh; w.w2 = vqx * hinv; w.w3 = vqy * hinv;
-      } else {
-        w.w1 = vh; w.w2 = vqx; w.w3 = vqy;
-      }
-    }
-  }
-  const bool wall = p.bc[lo ? 2 : 3] == ZB_BC_WALL;
-  T gx[4], gy[4], phi[4];
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    const T u = Wc[1].w(v);
-    const T gyv = (wall && v == 3) ? -u : u;
-    const T n0 = Wi[0].w(v), n1 = Wi[1].w(v), n2 = Wi[2].w(v);
-    gx[v] = ((Wc[2].w(v) + n2) - (Wc[0].w(v) + n0)) * p.inv4dx;
-    const T sn = (n0 + n1) + n2;
-    gy[v] = (lo ? (sn - gyv) - T(2) * u : (gyv + T(2) * u) - sn) * p.inv4dy;
-    const T gg = T(2) * gyv - u;
-    const T umax = fmx(fmx(fmx(fmx(u, Wc[2].w(v)), Wc[0].w(v)), n1), gg);
-    const T umin = fmn(fmn(fmn(fmn(u, Wc[2].w(v)), Wc[0].w(v)), n1), gg);
-    phi[v] = limiter_phi(p.limiter, gx[v], gy[v], p.half_dx, p.half_dy, umax - u, umin - u,
-                         p.vk_eps2);
-  }
-  if (RECON == ZB_RECON_ETA) {
-    if (p.eps_wet >= T(0) && Wc[1].h < p.eps_wet) phi[0] = phi[1] = phi[2] = phi[3] = T(0);
-    phi[0] = zmin(phi[0], phi[1]);
-    phi[2] = zmin(phi[2], phi[1]);
-    phi[3] = zmin(phi[3], phi[1]);
-  }
-  T sy[4];
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    out[v] = phi[v] * gx[v];
-    out[4 + v] = sy[v] = phi[v] * gy[v];
-  }
-  Side<T> O;
-  strip_trace<T, RECON>(Wc[1], sy, lo ? -p.half_dy : p.half_dy, O);
-  Side<T> G = O;
-  if (wall) {
-    G.qy = -O.qy;
-    G.uy = -O.uy;
-  }
-  const T sgy = lo ? T(-1) : T(1);
-  T Gh, Gx, Gy, Em, Ep;
-  riemann<T, RIEMANN, 1>(O, G, sgy, p.g, Gh, Gx, Gy, Em, Ep);
-  // the owner's cell-edge bed term: cesC of the high side, -cesD of the low
-  const T ces = T(0.5) * p.g * (Wc[1].h + O.h) * (O.b - Wc[1].b);
-  const T own_n = Gy + Em * sgy + ces * sgy;
-  out[8] = lo ? -Gh : Gh;
-  out[9] = lo ? -Gx : Gx;
-  out[10] = lo ? T(0) : own_n;
-  out[11] = lo ? own_n : T(0);
-}
-
-// One warp's work item: strip `strip` (28 output columns) over the output rows
-// [r0, r1) of the strip region p.fast_*.  EK selects the body:
-//   0  interior: every lane's cell two cells or more from every boundary;
-//   1  EDGE (full-coverage mode, wall / extrapolation sides only): rows and
-//      columns outside the grid are ghosts that load nothing, boundary cells
-//      take the least-squares class weights and the ghost values of their
-//      sides, and the faces on the boundary take the side's ghost state -- the
-//      expressions of stage_tile's boundary branches;
-//   2  column EDGE: the rows [r0 - 2, r1 + 2) lie inside the grid (r0 >= 2,
-//      r1 <= nx - 2) but the strip's lanes reach a boundary column: the
-//      interior body with guarded column loads; the boundary column's slopes
-//      and its boundary y-face by the EDGE expressions, recomputed on the
-//      lanes that hold them, row by row;
-//   3  column EDGE as 2, but for the paired float32 body the boundary
-//      columns' slopes and y-faces of every row of the item come from a
-//      pre-pass that evaluates them one row per lane (bcol_row) into shared
-//      memory: for long items (the ensemble's), whose march it frees of the
-//      one-lane row-by-row work; a short item's pre-pass is latency it cannot
-//      hide (measured on the single grid's 8-row items: 0.189 -> 0.211 ms per
-//      step, where the 32-row ensemble items gain 2.10 -> 1.92 ms).
-// `lead` (one item of the grid in full-coverage mode, where no tile kernel
-// runs) keeps the control block.
-template <typename T, int RECON, int RIEMANN, int MODE, int EK, bool BEDT = false>
+// One warp's work item: strip `strip` (28 output columns from column 28 strip)
+// over the output rows [r0, r1).  EDGE false, the interior body: every lane's
+// cell two cells or more from every boundary.  EDGE true, the general body:
+// any rows and columns of the grid.  It is the interior body with the boundary
+// folded into per-lane and per-row selects, so that no lane runs a branch of
+// its own:
+//   * rows and columns outside the grid load zeros (wall, extrapolation) or
+//     the periodic image;
+//   * least-squares gradient: the 3x3 row and column sums leave out what lies
+//     outside, the cell's own ghost enters as -/+ (ghost + 2 u) along its axis
+//     and the normal matrix is diag(4 dx^2, 4 dy^2) in place of diag(6, 6)
+//     (x of a side column sees five neighbours: 4 dx^2); the four corner cells,
+//     whose matrix is not diagonal, take
+//     g = s (2 d_n + d_diag - 2 d_ghost - d_t) / 5 along each axis, d the
+//     differences to the inner neighbour along the axis, the diagonal one, the
+//     ghost and the inner neighbour across it, s = +1 on the low side;
+//   * bounds: the neighbour beyond a side is 2 ghost - u;
+//   * faces: EdgeFaces.
+// The branchy boundary bodies this replaces cost a column-boundary row 1.7 us
+// of latency (one lane's slopes and face serially, a launch of its own beside
+// the interior): 512^2 float32 27 us per step at best row heights, 64^2 25.
+// `lead` (one item of the grid) keeps the control block.  MODE_STAGE: the
+// generic Shu-Osher stage with a given dt, optional per-cell first-order mask,
+// troubled-mask output and friction inside the stage (hinv_src).
+// P: SweParams<T> in kernel-parameter space, or volatile in shared memory (the
+// ensemble: fields read where they are used instead of held in registers).
+template <typename T, int RECON, int RIEMANN, int MODE, bool EDGE, bool BEDT, typename P>
 __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __restrict__ hP,
                                            const T* __restrict__ qxP, const T* __restrict__ qyP,
                                            const T* __restrict__ h0P,
                                            const T* __restrict__ qx0P,
                                            const T* __restrict__ qy0P, T* __restrict__ hO,
                                            T* __restrict__ qxO, T* __restrict__ qyO,
-                                           zb_ctrl* ctrl, int phase, const SweParams<T>& p,
+                                           zb_ctrl* ctrl, int phase, const P& p,
                                            const int strip, const int r0, const int r1,
-                                           const bool lead) {
-  constexpr bool EDGE = EK == 1;   // row and column guards
-  constexpr bool CG = EK != 0;     // column guards
+                                           const bool lead, const T* __restrict__ hinv_src = nullptr,
+                                           const unsigned char* __restrict__ force_o1 = nullptr,
+                                           unsigned char* __restrict__ trouble_out = nullptr) {
   const int lane = threadIdx.x & 31;
   const int nx = p.nx, ny = p.ny;
-  const int cj = p.fast_j0 - 2 + strip * SW + lane;
-  const bool colv = !CG || (cj >= 0 && cj < ny);
-  const double t = ctrl->t[phase];
-  const double dtd = dt_from_amax(ctrl->amax[phase], t, p.cfl2r, p.den_fac, p.dt_max, p.t_end);
-  const bool ok = isfinite(dtd) && dtd > 0.0;
-  if (lead && lane == 0) {
-    // the duties of the tile kernel's lead block (swe2d_stage_kernel)
-    const int nph = (phase + 1) % 3, nnph = (phase + 2) % 3;
-    if (MODE == MODE_STEP1) {
-      if (!ok && t < p.t_end) atomicOr(&ctrl->status, (unsigned)ZB_ST_DT_INVALID);
-      ctrl->dt = ok ? dtd : 0.0;
-      ctrl->t[nph] = ok ? t + dtd : t;
-      ctrl->amax[nnph] = 0.0;
-      ctrl->troubled = 0u;
-    } else if (!ok) {
-      ctrl->amax[nph] = ctrl->amax[phase];
-    } else {
-      atomicAdd(&ctrl->steps, 1u);
+  const int cj = strip * SW - 2 + lane;
+  const bool cin = !EDGE || (cj >= 0 && cj < ny);
+  double dtd;
+  if (MODE == MODE_STAGE) {
+    dtd = p.dt_stage >= 0.0 ? p.dt_stage : ctrl->dt;
+  } else {
+    const double t = ctrl->t[phase];
+    dtd = dt_from_amax(ctrl->amax[phase], t, p.cfl2r, p.den_fac, p.dt_max, p.t_end);
+    const bool ok = isfinite(dtd) && dtd > 0.0;
+    if (lead && lane == 0) {
+      // the duties of swe2d_stage_kernel's lead block
+      const int nph = (phase + 1) % 3, nnph = (phase + 2) % 3;
+      if (MODE == MODE_STEP1) {
+        if (!ok && t < p.t_end) atomicOr(&ctrl->status, (unsigned)ZB_ST_DT_INVALID);
+        ctrl->dt = ok ? dtd : 0.0;
+        ctrl->t[nph] = ok ? t + dtd : t;
+        ctrl->amax[nnph] = 0.0;
+        ctrl->troubled = 0u;
+      } else if (!ok) {
+        ctrl->amax[nph] = ctrl->amax[phase];
+      } else {
+        atomicAdd(&ctrl->steps, 1u);
+      }
     }
+    if (!ok) return;                    // no-op step (t_end reached or dt invalid)
   }
-  if (!ok) return;                      // no-op step (t_end reached or dt invalid)
   const T dt = T(dtd);
   const T g = p.g, half = T(0.5);
-  const bool out_lane = lane >= 2 && lane < 2 + SW && (!CG || cj < ny);
-  // float32 interior rows of the eta / HLL-HR scheme evaluate their two faces
-  // as paired float32 arithmetic (faces_pair)
+  const bool out_lane = lane >= 2 && lane < 2 + SW && cin;
+  // float32 rows of the eta / HLL-HR scheme evaluate their two faces as paired
+  // float32 arithmetic (faces_pair)
   constexpr bool PAIR = std::is_same<T, float>::value && RECON == ZB_RECON_ETA &&
-                        RIEMANN == ZB_RIEMANN_HLL_HR && !EDGE;
-  // column-EDGE with the paired body: the boundary columns' rows come from
-  // the pre-pass, slots [side][m - (r0 - 1)][12] of this warp (side 0: column
-  // 0, side 1: column ny - 1; rows r0 - 1 .. r1)
-  constexpr bool PRE = EK == 3 && PAIR;
+                        RIEMANN == ZB_RIEMANN_HLL_HR;
   // BEDT: interior items of the eta / HLL-HR scheme read b's gradient and
   // limiter value from the planes swe2d_bed_kernel prepared (b never
   // changes) instead of evaluating them; the planes are laid out like the
   // state's
-  constexpr bool BED = BEDT && EK == 0 && RECON == ZB_RECON_ETA && RIEMANN == ZB_RIEMANN_HLL_HR;
+  constexpr bool BED = BEDT && !EDGE && RECON == ZB_RECON_ETA && RIEMANN == ZB_RIEMANN_HLL_HR;
   const T* __restrict__ bedP = p.bed;
   const size_t bed_plane = (size_t)nx * ny;
-  constexpr int PROWS = SXC_MAX + 2;
-  T* bs = nullptr;
-  if constexpr (PRE) {
-    __shared__ T bsh[STRIP_NT / 32][2 * PROWS * 12];
-    bs = bsh[threadIdx.x >> 5];
-    const int cj0 = p.fast_j0 - 2 + strip * SW;
-    const int nrows = r1 - r0 + 2;   // <= SXC_MAX + 2 (full_items)
-    __syncwarp();                      // the warp's previous item is done with the slots
-    for (int side = 0; side < 2; ++side) {
-      const int c = side ? ny - 1 : 0;
-      if (!(cj0 <= c && c <= cj0 + 31)) continue;   // warp-uniform
-      for (int mm = lane; mm < nrows; mm += 32)
-        bcol_row<T, RECON, RIEMANN>(bP, hP, qxP, qyP, p, r0 - 1 + mm, c,
-                                    bs + (side * PROWS + mm) * 12);
-    }
-    __syncwarp();
+  // EDGE: the lane's column (its periodic image where the sides are periodic)
+  // and what the boundary makes of it
+  const bool per_x = EDGE && p.bc[0] == ZB_BC_PERIODIC, per_y = EDGE && p.bc[2] == ZB_BC_PERIODIC;
+  const bool byl = EDGE && cj == 0, byh = EDGE && cj == ny - 1, by = byl || byh;
+  const bool wall_y = by && p.bc[byl ? 2 : 3] == ZB_BC_WALL;
+  int lc = cj;
+  bool cld = cin;
+  if (EDGE && per_y && !cin) {
+    lc = cj % ny;
+    if (lc < 0) lc += ny;
+    cld = true;
   }
+  // the row the lane loads for row index r (the periodic image), -1: none
+  auto load_row = [&](int r) -> int {
+    if (!EDGE || (r >= 0 && r < nx)) return r;
+    if (!per_x) return -1;
+    const int w = r % nx;
+    return w < 0 ? w + nx : w;
+  };
 
   RowW<T> R0, R1, R2;                 // rows r-2, r-1, r
   T Sx0[4], Sx1[4], Sx2[4];           // (W(j-1) + W(j)) + W(j+1) of those rows
@@ -1023,12 +691,17 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
   T amax_loc = T(0);   // reduced in T; float -> double is exact and monotone
   bool bad = false;
   const int nsteps = (r1 - r0) + 4;
+  const int limiter = p.limiter;
+  const bool clipmin = limiter != ZB_LIM_NONE && limiter != ZB_LIM_VENKATAKRISHNAN;
   // row r + 1 is fetched while row r is processed
   T nbv = T(0), nhv = T(0), nqxv = T(0), nqyv = T(0);
   T nbgx = T(0), nbgy = T(0), nbphi = T(0);   // BED: the next slope row's bed values
-  if (!CG || (colv && (!EDGE || r0 - 2 >= 0))) {
-    const size_t k = (size_t)(r0 - 2) * ny + cj;
-    nbv = bP[k]; nhv = hP[k]; nqxv = qxP[k]; nqyv = qyP[k];
+  {
+    const int lr = load_row(r0 - 2);
+    if (!EDGE || (cld && lr >= 0)) {
+      const size_t k = (size_t)lr * ny + lc;
+      nbv = bP[k]; nhv = hP[k]; nqxv = qxP[k]; nqyv = qyP[k];
+    }
   }
   for (int s = 0; s < nsteps; ++s) {
     const int r = r0 - 2 + s;
@@ -1036,21 +709,27 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
     // the loads now so their latency overlaps the slope and face work
     const int ro = r - 2;
     const bool upd = s >= 4 && out_lane && ro >= r0 && ro < r1;
-    T qxk = T(0), qyk = T(0), h0 = T(0), qx0 = T(0), qy0 = T(0);
+    T qxk = T(0), qyk = T(0), h0 = T(0), qx0 = T(0), qy0 = T(0), hsrc = T(0);
     if (upd) {
       const size_t k = (size_t)ro * ny + cj;
       if (RECON == ZB_RECON_ETA) { qxk = qxP[k]; qyk = qyP[k]; }
-      if (MODE == MODE_STEP2) { h0 = h0P[k]; qx0 = qx0P[k]; qy0 = qy0P[k]; }
+      if (MODE == MODE_STEP2 || (MODE == MODE_STAGE && p.alpha != 0.0)) {
+        h0 = h0P[k]; qx0 = qx0P[k]; qy0 = qy0P[k];
+      }
+      if (MODE == MODE_STAGE && hinv_src != nullptr) hsrc = hinv_src[k];
     }
     // the bed slopes of row r - 1 (the slope block below), fetched in the
     // previous iteration; fetch row r's for the next one
     const T bgx = nbgx, bgy = nbgy, bphi = nbphi;
     if (BED && s >= 1 && r <= r1) {
-      const size_t k = (size_t)r * ny + cj;   // BED: EK == 0, no guards
+      const size_t k = (size_t)r * ny + cj;   // BED: interior items, no guards
       nbgx = __ldg(bedP + k);
       nbgy = __ldg(bedP + bed_plane + k);
       nbphi = __ldg(bedP + 2 * bed_plane + k);
     }
+    bool o1 = false;   // MODE_STAGE: the cell of row r - 1 is demoted to first order
+    if (MODE == MODE_STAGE && force_o1 != nullptr && s >= 2 && cin && r - 1 >= 0 && r - 1 < nx)
+      o1 = force_o1[(size_t)(r - 1) * ny + cj] != 0;
     // shift the windows and take row r
     R0 = R1; R1 = R2;
 #pragma unroll
@@ -1061,8 +740,9 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
     {
       const T vb = nbv, vh = nhv, vqx = nqxv, vqy = nqyv;
       if (s + 1 < nsteps) {
-        if (!CG || (colv && (!EDGE || (r + 1 >= 0 && r + 1 < nx)))) {
-          const size_t k = (size_t)(r + 1) * ny + cj;
+        const int lr = load_row(r + 1);
+        if (!EDGE || (cld && lr >= 0)) {
+          const size_t k = (size_t)lr * ny + lc;
           nbv = bP[k]; nhv = hP[k]; nqxv = qxP[k]; nqyv = qyP[k];
         } else {
           nbv = T(0); nhv = T(0); nqxv = T(0); nqyv = T(0);
@@ -1088,139 +768,85 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
         const T wl = shu(w), wr = shd(w);
         Wm2[v] = wl;
         Wp2[v] = wr;
-        Sx2[v] = (wl + w) + wr;
+        Sx2[v] = EDGE ? ((byl ? T(0) : wl) + w) + (byh ? T(0) : wr) : (wl + w) + wr;
       }
     }
     if (s < 2) continue;
     // limited slopes of row r-1
     {
+      const int m = r - 1;
+      const bool bxl = EDGE && m == 0, bxh = EDGE && m == nx - 1, bx = bxl || bxh;   // uniform
       T phi[4], gxa[4], gya[4];
-      if constexpr (PAIR) {
-        // the x and y components of each variable as the two lanes of
-        // paired float32 arithmetic (gradient, limiter increments, bounds)
-        const bool clipmin = p.limiter != ZB_LIM_NONE && p.limiter != ZB_LIM_VENKATAKRISHNAN;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          if (v == 0 && BED) {
-            gxa[0] = bgx;
-            gya[0] = bgy;
-            phi[0] = bphi;
-            continue;
-          }
-          const float u = R1.w(v);
-          const float tc = (R0.w(v) + R1.w(v)) + R2.w(v);
-          const float tl = shu(tc), tr = shd(tc);
-          const float2 gv = mul2(sub2(f2(Sx2[v], tr), f2(Sx0[v], tl)), f2(p.inv6dx, p.inv6dy));
-          const float wp0 = R2.w(v), wm0 = R0.w(v), w0p = Wp1[v], w0m = Wm1[v];
-          const float umax = fmx3(u, wp0, fmx3(wm0, w0p, w0m));
-          const float umin = fmn3(u, wp0, fmn3(wm0, w0p, w0m));
-          const float2 dd = sub2(f2(umax, umin), f2(u, u));          // (dpos, dneg)
-          gxa[v] = gv.x;
-          gya[v] = gv.y;
-          if (clipmin) {
-            const float2 ac = mul2(gv, f2(p.half_dx, p.half_dy));
-            phi[v] = phi_clipmin(ac.x, ac.y, dd.x, dd.y);
-          } else {
-            phi[v] = limiter_phi(p.limiter, gv.x, gv.y, p.half_dx, p.half_dy, dd.x, dd.y,
-                                 p.vk_eps2);
-          }
-        }
-      } else {
+      // x and y scale of the differences
+      const T ix = (EDGE && (by || bx)) ? p.inv4dx : p.inv6dx;
+      const T iy = (EDGE && (by || bx)) ? p.inv4dy : p.inv6dy;
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        if (v == 0 && BED) {   // float64 interior items: the prepared planes
+        if (v == 0 && BED) {
           gxa[0] = bgx;
           gya[0] = bgy;
           phi[0] = bphi;
           continue;
         }
         const T u = R1.w(v);
-        const T tc = (R0.w(v) + R1.w(v)) + R2.w(v);
-        const T tl = shu(tc), tr = shd(tc);
-        const T gx = (Sx2[v] - Sx0[v]) * p.inv6dx;
-        const T gy = (tr - tl) * p.inv6dy;
-        const T wp0 = R2.w(v), wm0 = R0.w(v), w0p = Wp1[v], w0m = Wm1[v];
+        T wp0 = R2.w(v), wm0 = R0.w(v), w0p = Wp1[v], w0m = Wm1[v];
+        T xhi = Sx2[v], xlo = Sx0[v];       // gx = (xhi - xlo) / ..
+        const T tc = (EDGE && bx) ? (bxl ? u + wp0 : wm0 + u) : (wm0 + u) + wp0;
+        T tl = shu(tc), tr = shd(tc);       // gy = (tr - tl) / ..
+        T cgx = T(0), cgy = T(0);           // corner cells: the gradient itself
+        if (EDGE) {
+          // y: the side's ghost
+          const T gyv = per_y ? (byl ? w0m : w0p) : ((v == 3 && wall_y) ? -u : u);
+          const T cy = gyv + T(2) * u, gg = T(2) * gyv - u;
+          if (bx) {
+            // x: the side's ghost row; the corner cells
+            const T gxv = per_x ? (bxl ? wm0 : wp0)
+                                : ((v == 2 && p.bc[bxl ? 0 : 1] == ZB_BC_WALL) ? -u : u);
+            const T wn = bxl ? wp0 : wm0;                       // inner neighbour along x
+            const T ra = shu(wn), rb = shd(wn);
+            const T wt = byl ? w0p : w0m, wd = byl ? rb : ra;   // across, diagonal
+            const T dn = wn - u, dt_ = wt - u, dd = wd - u;
+            cgx = (T(2) * dn + dd - T(2) * (gxv - u) - dt_) * p.inv5dx;
+            cgy = (T(2) * dt_ + dd - T(2) * (gyv - u) - dn) * p.inv5dy;
+            cgx = bxl ? cgx : -cgx;
+            cgy = byl ? cgy : -cgy;
+            const T cx = gxv + T(2) * u, ggx = T(2) * gxv - u;
+            if (bxl) { xlo = cx; wm0 = ggx; }
+            else { xhi = cx; wp0 = ggx; }
+          }
+          tl = byl ? cy : tl;
+          tr = byh ? cy : tr;
+          w0m = byl ? gg : w0m;
+          w0p = byh ? gg : w0p;
+        }
         const T umax = fmx3(u, wp0, fmx3(wm0, w0p, w0m));
         const T umin = fmn3(u, wp0, fmn3(wm0, w0p, w0m));
+        T gx, gy, dpos, dneg;
+        if constexpr (PAIR) {
+          // the x and y components as the two lanes of paired float32
+          // arithmetic
+          const float2 gv = mul2(sub2(f2(xhi, tr), f2(xlo, tl)), f2(ix, iy));
+          const float2 dd = sub2(f2(umax, umin), f2(u, u));
+          gx = gv.x; gy = gv.y; dpos = dd.x; dneg = dd.y;
+        } else {
+          gx = (xhi - xlo) * ix;
+          gy = (tr - tl) * iy;
+          dpos = umax - u;
+          dneg = umin - u;
+        }
+        if (EDGE && bx) {
+          gx = by ? cgx : gx;
+          gy = by ? cgy : gy;
+        }
         gxa[v] = gx;
         gya[v] = gy;
-        phi[v] = limiter_phi(p.limiter, gx, gy, p.half_dx, p.half_dy, umax - u, umin - u,
-                             p.vk_eps2);
-      }
-      }
-      if (CG) {
-        // row r-1 = m: boundary cells (stage_tile phase B, non-interior
-        // branch) and ghosts (zero slopes); a column-EDGE item's rows are
-        // never boundary rows
-        const int m = r - 1;
-        const bool cellv = colv && (!EDGE || (m >= 0 && m < nx));
-        const bool bxl = EDGE && m == 0, bxh = EDGE && m == nx - 1;
-        const bool byl = cj == 0, byh = cj == ny - 1;
-        const bool bnd = cellv && (bxl || bxh || byl || byh);
-        if (!PRE && __any_sync(0xffffffffu, bnd)) {   // PRE: the pre-pass slots
-          const int cls = (bxl ? 0 : (bxh ? 2 : 1)) * 3 + (byl ? 0 : (byh ? 2 : 1));
-          const T* wx = p.lsq.w[cls][0];
-          const T* wy = p.lsq.w[cls][1];
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const T am = shu(R0.w(v)), ap = shd(R0.w(v));
-            if (bnd) {
-              const T u = R1.w(v);
-              T gx = T(0), gy = T(0), umax = u, umin = u;
-              T gxv = u, gyv = u;
-              if ((bxl || bxh) && p.bc[bxl ? 0 : 1] == ZB_BC_WALL && v == 2) gxv = -u;
-              if ((byl || byh) && p.bc[byl ? 2 : 3] == ZB_BC_WALL && v == 3) gyv = -u;
-              if ((bxl || bxh) && (byl || byh)) {
-                // corner: the class weights (the pseudo-inverse is not diagonal)
-                const T nbr[8] = {am, R0.w(v), ap, Wm1[v], Wp1[v], Wm2[v], R2.w(v), Wp2[v]};
-                int k = 0;
-#pragma unroll
-                for (int a = -1; a <= 1; ++a) {
-#pragma unroll
-                  for (int bb = -1; bb <= 1; ++bb) {
-                    if (a == 0 && bb == 0) continue;
-                    const bool okn = m + a >= 0 && m + a < nx && cj + bb >= 0 && cj + bb < ny;
-                    const T d = okn ? nbr[k] - u : T(0);
-                    gx += wx[k] * d;
-                    gy += wy[k] * d;
-                    ++k;
-                  }
-                }
-                { const T d = gxv - u; gx += wx[8] * d; gy += wy[8] * d; }
-                { const T d = gyv - u; gx += wx[9] * d; gy += wy[9] * d; }
-              } else if (byl || byh) {
-                // side column: the five in-domain neighbours give x the normal
-                // matrix diag(4 dx^2, 3 dy^2); y adds its ghost: diag(4 dx^2,
-                // 4 dy^2) -- the class weights in closed form
-                const T n0 = byl ? ap : am, n1 = byl ? Wp1[v] : Wm1[v];
-                const T n2 = byl ? Wp2[v] : Wm2[v];
-                gx = ((R2.w(v) + n2) - (R0.w(v) + n0)) * p.inv4dx;
-                const T sn = (n0 + n1) + n2;
-                gy = (byl ? (sn - gyv) - T(2) * u : (gyv + T(2) * u) - sn) * p.inv4dy;
-              } else {
-                // side row: the same with the roles of x and y exchanged
-                const T n0 = bxl ? Wm2[v] : am, n1 = bxl ? R2.w(v) : R0.w(v);
-                const T n2 = bxl ? Wp2[v] : ap;
-                gy = ((Wp1[v] + n2) - (Wm1[v] + n0)) * p.inv4dy;
-                const T sn = (n0 + n1) + n2;
-                gx = (bxl ? (sn - gxv) - T(2) * u : (gxv + T(2) * u) - sn) * p.inv4dx;
-              }
-              if (!bxh) { umax = fmx(umax, R2.w(v)); umin = fmn(umin, R2.w(v)); }
-              if (!bxl) { umax = fmx(umax, R0.w(v)); umin = fmn(umin, R0.w(v)); }
-              if (!byh) { umax = fmx(umax, Wp1[v]); umin = fmn(umin, Wp1[v]); }
-              if (!byl) { umax = fmx(umax, Wm1[v]); umin = fmn(umin, Wm1[v]); }
-              if (bxl || bxh) { const T gg = T(2) * gxv - u; umax = fmx(umax, gg); umin = fmn(umin, gg); }
-              if (byl || byh) { const T gg = T(2) * gyv - u; umax = fmx(umax, gg); umin = fmn(umin, gg); }
-              gxa[v] = gx;
-              gya[v] = gy;
-              phi[v] = limiter_phi(p.limiter, gx, gy, p.half_dx, p.half_dy, umax - u, umin - u,
-                                   p.vk_eps2);
-            }
+        if (PAIR && clipmin) {
+          if constexpr (PAIR) {
+            const float2 ac = mul2(f2(gx, gy), f2(p.half_dx, p.half_dy));
+            phi[v] = phi_clipmin(ac.x, ac.y, dpos, dneg);
           }
-        }
-        if (!cellv) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v) { phi[v] = T(0); gxa[v] = T(0); gya[v] = T(0); }
+        } else {
+          phi[v] = limiter_phi<T>(limiter, gx, gy, p.half_dx, p.half_dy, dpos, dneg, p.vk_eps2);
         }
       }
       if (RECON == ZB_RECON_ETA) {
@@ -1230,6 +856,12 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
         phi[0] = zmin(phi[0], phi[1]);
         phi[2] = zmin(phi[2], phi[1]);
         phi[3] = zmin(phi[3], phi[1]);
+      }
+      // ghosts (a periodic partner enters the seam's faces unreconstructed)
+      // and demoted cells have no slopes
+      if ((EDGE && (!cin || m < 0 || m >= nx)) || (MODE == MODE_STAGE && o1)) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) { phi[v] = T(0); gxa[v] = T(0); gya[v] = T(0); }
       }
 #pragma unroll
       for (int v = 0; v < 8; ++v) slA[v] = slB[v];
@@ -1244,140 +876,91 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
           slB[4 + v] = phi[v] * gya[v];
         }
       }
-      if constexpr (PRE) {
-        // the boundary column's cell of row r - 1 (pre-pass slot r - 1 - (r0 - 1))
-        if (cj == 0 || cj == ny - 1) {
-          const T* sl = bs + ((cj == 0 ? 0 : PROWS) + (r - r0)) * 12;
-#pragma unroll
-          for (int v = 0; v < 8; ++v) slB[v] = sl[v];
-        }
-      }
     }
     if (s < 3) continue;
-    // x-face between rows r-2 (A, lower) and r-1 (B, upper)
+    // the x-face between rows r-2 (A, lower) and r-1 (B, upper) and the y-face
+    // of row r-2 above this lane (the lower lane's is the one below)
     T Fh, Fy, fxl_n, fxr_n, Gh, Gx, fyl_t, fyr_own;
     {
+      EdgeFaces ef = {false, false, false, false, 1.0f, 1.0f};
+      if (EDGE) {
+        ef.xlo = !per_x && r - 1 == 0;
+        ef.xhi = !per_x && r - 2 == nx - 1;
+        ef.ylo = !per_y && cj == -1;
+        ef.yhi = !per_y && cj == ny - 1;
+        ef.sx = p.bc[ef.xlo ? 0 : 1] == ZB_BC_WALL ? -1.0f : 1.0f;
+        ef.sy = p.bc[ef.ylo ? 2 : 3] == ZB_BC_WALL ? -1.0f : 1.0f;
+      }
       if constexpr (PAIR) {
         const NextRow nv = next_row(R0, slA);
-        faces_pair(R0, R1, slA, slB, nv, p, Fh, Fy, fxl_n, fxr_n, Gh, Gx, fyl_t, fyr_own);
+        faces_pair<EDGE, P>(R0, R1, slA, slB, nv, p, ef, Fh, Fy, fxl_n, fxr_n, Gh, Gx, fyl_t, fyr_own);
         if (s == 3) {          // face r0 - 1/2: only the next row needs it
           fxh_p = Fh; fxt_p = Fy; fxr_p = fxr_n;
           continue;
         }
-        if constexpr (PRE) {
-          // the y-face on the boundary (the lane below column 0, or column
-          // ny - 1) of row r - 2: pre-pass slot r - 2 - (r0 - 1)
-          if (cj == -1 || cj == ny - 1) {
-            const T* fo = bs + ((cj == -1 ? 0 : PROWS) + (r - 1 - r0)) * 12 + 8;
-            Gh = fo[0]; Gx = fo[1]; fyl_t = fo[2]; fyr_own = fo[3];
-          }
-        } else if (EK >= 2 && (cj == -1 || cj == ny - 1)) {
-          // the y-face on the boundary (the lane below column 0, or column
-          // ny - 1): the owner's trace against its ghost with normal sign sgy,
-          // as the EDGE body evaluates it
-          RowW<T> nb;
-          nb.b = nv.b; nb.w1 = nv.w1; nb.w2 = nv.w2; nb.w3 = nv.w3; nb.h = nv.h; nb.hinv = T(0);
-          const T sln[4] = {nv.s4, nv.s5, nv.s6, nv.s7};
-          Side<T> C, D;
-          strip_trace<T, RECON>(R0, slA + 4, p.half_dy, C);
-          strip_trace<T, RECON>(nb, sln, -p.half_dy, D);
-          const bool ylo = cj == -1;
-          const Side<T> YL = ylo ? D : C;
-          Side<T> YR = YL;
-          if (p.bc[ylo ? 2 : 3] == ZB_BC_WALL) {
-            YR.qy = -YL.qy;
-            YR.uy = -YL.uy;
-          }
-          const T sgy = ylo ? T(-1) : T(1);
-          T Gy, Em, Ep;
-          riemann<T, RIEMANN, 1>(YL, YR, sgy, g, Gh, Gx, Gy, Em, Ep);
-          const T cesC = half * g * (R0.h + C.h) * (C.b - R0.b);
-          const T cesD = -(half * g * (nb.h + D.h) * (D.b - nb.b));
-          const T own_n = Gy + Em * sgy + (ylo ? -cesD : cesC) * sgy;
-          if (ylo) {
-            Gh = -Gh; Gx = -Gx; fyr_own = own_n; fyl_t = T(0);
-          } else {
-            fyl_t = own_n; fyr_own = T(0);
-          }
-        }
       } else {
-      T Fx, Dm, Dp;
-      Side<T> A, B;
-      strip_trace<T, RECON>(R0, slA, p.half_dx, A);
-      strip_trace<T, RECON>(R1, slB, -p.half_dx, B);
-      // EDGE: a face on the x boundary takes the owner's trace (row 0 below
-      // the face, row nx-1 above it) against its ghost with normal sign sg
-      // (stage_tile's x-face boundary branch)
-      const bool xb = EDGE && (r - 1 == 0 || r - 2 == nx - 1);
-      const bool xlo = EDGE && r - 1 == 0;
-      T sgx = T(1);
-      Side<T> L = A, R = B;
-      if (xb) {
-        L = xlo ? B : A;
-        R = L;
-        if (p.bc[xlo ? 0 : 1] == ZB_BC_WALL) {
-          R.qx = -L.qx;
-          R.ux = -L.ux;
+        T Fx, Dm, Dp;
+        RowW<T> LA = R0, LB = R1;
+        if (EDGE && per_x && RECON != ZB_RECON_ETA) {
+          // a seam partner's velocity is its momentum times the owner's hinv
+          if (r - 1 == 0) LA.hinv = R1.hinv;
+          if (r - 2 == nx - 1) LB.hinv = R0.hinv;
         }
-        sgx = xlo ? T(-1) : T(1);
-      }
-      riemann<T, RIEMANN, 0>(L, R, sgx, g, Fh, Fx, Fy, Dm, Dp);
-      const T cesA = half * g * (R0.h + A.h) * (A.b - R0.b);
-      const T cesB = -(half * g * (R1.h + B.h) * (B.b - R1.b));
-      fxl_n = Fx + Dm + cesA;
-      fxr_n = -Fx + Dp + cesB;
-      if (xb) {
-        const T own_n = Fx + Dm * sgx + (xlo ? -cesB : cesA) * sgx;
-        if (xlo) {
-          Fh = -Fh; Fy = -Fy; fxr_n = own_n; fxl_n = T(0);
-        } else {
-          fxl_n = own_n; fxr_n = T(0);
+        Side<T> A, B;
+        strip_trace<T, RECON>(LA, slA, p.half_dx, A);
+        strip_trace<T, RECON>(LB, slB, -p.half_dx, B);
+        if (EDGE && (ef.xlo || ef.xhi)) {   // uniform
+          Side<T> O = ef.xlo ? B : A;
+          O.qx *= T(ef.sx);
+          O.ux *= T(ef.sx);
+          if (ef.xlo) A = O;
+          else B = O;
         }
-      }
-      if (s == 3) {            // face r0 - 1/2: only the next row needs it
-        fxh_p = Fh; fxt_p = Fy; fxr_p = fxr_n;
-        continue;
-      }
-      // y-faces of row r-2: this lane's top face, the lower lane's one below
-      Side<T> C, D;
-      T Gy, Em, Ep;
-      RowW<T> nb;
-      nb.b = shd(R0.b); nb.w1 = shd(R0.w1); nb.w2 = shd(R0.w2); nb.w3 = shd(R0.w3);
-      nb.h = shd(R0.h); nb.hinv = shd(R0.hinv);
-      T sln[8];
+        riemann<T, RIEMANN, 0>(A, B, T(1), g, Fh, Fx, Fy, Dm, Dp);
+        const T cesA = half * g * (R0.h + A.h) * (A.b - R0.b);
+        const T cesB = -(half * g * (R1.h + B.h) * (B.b - R1.b));
+        fxl_n = Fx + Dm + cesA;
+        fxr_n = -Fx + Dp + cesB;
+        if (s == 3) {            // face r0 - 1/2: only the next row needs it
+          fxh_p = Fh; fxt_p = Fy; fxr_p = fxr_n;
+          continue;
+        }
+        // y-face of row r-2: this lane | the next lane
+        Side<T> C, D;
+        T Gy, Em, Ep;
+        RowW<T> nb, own = R0;
+        nb.b = shd(R0.b); nb.w1 = shd(R0.w1); nb.w2 = shd(R0.w2); nb.w3 = shd(R0.w3);
+        nb.h = shd(R0.h); nb.hinv = shd(R0.hinv);
+        if (EDGE && per_y && RECON != ZB_RECON_ETA) {
+          if (cj == -1) own.hinv = nb.hinv;
+          if (cj == ny - 1) nb.hinv = own.hinv;
+        }
+        T sln[8];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) sln[4 + v] = shd(slA[4 + v]);
-      strip_trace<T, RECON>(R0, slA + 4, p.half_dy, C);
-      strip_trace<T, RECON>(nb, sln + 4, -p.half_dy, D);
-      // EDGE: a face on the y boundary takes the owner's trace (the next
-      // lane's cell 0, or this lane's cell ny-1) against its ghost
-      const bool yb = CG && (cj == -1 || cj == ny - 1);
-      const bool ylo = CG && cj == -1;
-      T sgy = T(1);
-      Side<T> YL = C, YR = D;
-      if (CG) {
-        YL.b = ylo ? D.b : C.b; YL.h = ylo ? D.h : C.h; YL.qx = ylo ? D.qx : C.qx;
-        YL.qy = ylo ? D.qy : C.qy; YL.ux = ylo ? D.ux : C.ux; YL.uy = ylo ? D.uy : C.uy;
-        const bool wall = yb && p.bc[ylo ? 2 : 3] == ZB_BC_WALL;
-        YR.b = yb ? YL.b : D.b; YR.h = yb ? YL.h : D.h; YR.qx = yb ? YL.qx : D.qx;
-        YR.ux = yb ? YL.ux : D.ux;
-        YR.qy = yb ? (wall ? -YL.qy : YL.qy) : D.qy;
-        YR.uy = yb ? (wall ? -YL.uy : YL.uy) : D.uy;
-        sgy = ylo ? T(-1) : T(1);
-      }
-      riemann<T, RIEMANN, 1>(YL, YR, sgy, g, Gh, Gx, Gy, Em, Ep);
-      const T cesC = half * g * (R0.h + C.h) * (C.b - R0.b);
-      const T cesD = -(half * g * (nb.h + D.h) * (D.b - nb.b));
-      fyl_t = Gy + Em + cesC;
-      fyr_own = -Gy + Ep + cesD;
-      if (yb) {
-        const T own_n = Gy + Em * sgy + (ylo ? -cesD : cesC) * sgy;
-        if (ylo) {
-          Gh = -Gh; Gx = -Gx; fyr_own = own_n; fyl_t = T(0);
-        } else {
-          fyl_t = own_n; fyr_own = T(0);
+        for (int v = 0; v < 4; ++v) sln[4 + v] = shd(slA[4 + v]);
+        strip_trace<T, RECON>(own, slA + 4, p.half_dy, C);
+        strip_trace<T, RECON>(nb, sln + 4, -p.half_dy, D);
+        if (EDGE) {
+          const T sy = T(ef.sy);
+          const Side<T> O = ef.ylo ? D : C;
+          C.b = ef.ylo ? O.b : C.b;
+          C.h = ef.ylo ? O.h : C.h;
+          C.qx = ef.ylo ? O.qx : C.qx;
+          C.ux = ef.ylo ? O.ux : C.ux;
+          C.qy = ef.ylo ? sy * O.qy : C.qy;
+          C.uy = ef.ylo ? sy * O.uy : C.uy;
+          D.b = ef.yhi ? O.b : D.b;
+          D.h = ef.yhi ? O.h : D.h;
+          D.qx = ef.yhi ? O.qx : D.qx;
+          D.ux = ef.yhi ? O.ux : D.ux;
+          D.qy = ef.yhi ? sy * O.qy : D.qy;
+          D.uy = ef.yhi ? sy * O.uy : D.uy;
         }
-      }
+        riemann<T, RIEMANN, 1>(C, D, T(1), g, Gh, Gx, Gy, Em, Ep);
+        const T cesC = half * g * (R0.h + C.h) * (C.b - R0.b);
+        const T cesD = -(half * g * (nb.h + D.h) * (D.b - nb.b));
+        fyl_t = Gy + Em + cesC;
+        fyr_own = -Gy + Ep + cesD;
       }
       const T fyh_b = shu(Gh), fyt_b = shu(Gx), fyr_b = shu(fyr_own);
       // update of row r-2
@@ -1398,12 +981,33 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
         hn = hk + dt * dh;
         qxn = qxk + dt * dqx;
         qyn = qyk + dt * dqy;
+      } else if (MODE == MODE_STAGE) {
+        const T al = T(p.alpha), bt = T(p.beta);
+        T sqx = dqx, sqy = dqy;
+        if (hinv_src != nullptr && p.manning_n != T(0)) {
+          // solver2 adds the source to the stage residual at Qk with the
+          // step's aux (solver2/blocks.py:241-287, march.py:120-124)
+          const T qn = asqrt(qxk * qxk + qyk * qyk);
+          const T kf = (-p.g) * (p.manning_n * p.manning_n) * qn * (hsrc * hsrc) * cbrt(hsrc);
+          sqx = dqx + qxk * kf;
+          sqy = dqy + qyk * kf;
+        }
+        const T h2 = hk + bt * dt * dh, qx2 = qxk + bt * dt * sqx, qy2 = qyk + bt * dt * sqy;
+        if (p.alpha != 0.0) {
+          hn = al * h0 + (T(1) - al) * h2;
+          qxn = al * qx0 + (T(1) - al) * qx2;
+          qyn = al * qy0 + (T(1) - al) * qy2;
+        } else {
+          hn = h2; qxn = qx2; qyn = qy2;
+        }
       } else {
         const T h2 = hk + dt * dh, qx2 = qxk + dt * dqx, qy2 = qyk + dt * dqy;
         hn = half * (h0 + h2);
         qxn = half * (qx0 + qx2);
         qyn = half * (qy0 + qy2);
         if (p.manning_n != T(0)) {
+          // source as RK1 after the hyperbolic step with the step's input aux
+          // (zoomy_jax/fvm/solver_jax.py:1129; ode.py:14-18)
           const T hi0 = kp_hinv(h0, p.eps_kp);
           const T qn = asqrt(qxn * qxn + qyn * qyn);
           const T kf = (-p.g) * (p.manning_n * p.manning_n) * qn * (hi0 * hi0) * cbrt(hi0);
@@ -1420,11 +1024,18 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
       hO[k] = hn;
       qxO[k] = qxn;
       qyO[k] = qyn;
-      // troubled: h < 0 or a non-finite value (one non-finite term makes
-      // the sum's difference with itself NaN; finite states that overflow
-      // the sum, |q| ~ 1e38, would flag too)
-      const T chk = (hn + qxn) + (qyn + R0.b);
-      bad = bad || !(hn >= T(0)) || !(chk - chk == T(0));
+      if (MODE == MODE_STAGE) {
+        const bool tr = (hn < T(0)) || !isfinite(hn) || !isfinite(qxn) || !isfinite(qyn) ||
+                        !isfinite(R0.b);
+        bad = bad || tr;
+        if (trouble_out != nullptr) trouble_out[k] = tr ? 1 : 0;
+      } else {
+        // troubled: h < 0 or a non-finite value (one non-finite term makes
+        // the sum's difference with itself NaN; finite states that overflow
+        // the sum, |q| ~ 1e38, would flag too)
+        const T chk = (hn + qxn) + (qyn + R0.b);
+        bad = bad || !(hn >= T(0)) || !(chk - chk == T(0));
+      }
       if (MODE == MODE_STEP2) {
         const T hi = kp_hinv(hn, p.eps_kp);
         const T c = asqrt(g * fmx(hn, T(0)));
@@ -1448,173 +1059,140 @@ __host__ __device__ inline int full_mid_strips(int ny) {
   return mh > ns - 1 ? ns - 1 : mh;
 }
 
-// Full-coverage item list of a grid with nx, ny >= 4 (strips of SW columns
-// from column 0, rows from 0).  Every strip has two EDGE items for the
-// boundary rows [0, 2) and [nx - 2, nx).  The rows between go in chunks: SX
-// rows for the middle strips (lanes 28 s - 2 .. 28 s + 29 inside the grid,
-// the interior body), sxc rows for the strips whose lanes reach outside the
-// grid (the first, and the last one or two: the column-EDGE body).  Order:
-// the column-EDGE items, the EDGE items (these two kinds form the boundary
-// launch), then the interior items.  Item 0 keeps the control block.  Returns
-// the item count (item = -1), the count of boundary-launch items (item = -2),
-// or with item >= 0 fills its strip, rows and kind (the strip_item EK).
-// Column-EDGE chunk heights (B200, 2048^2 and the 512-instance ensemble): a
-// single grid's boundary launch shares the SMs with one wave of interior
-// items and fills their tail best with short chunks (8 rows: 0.189 ms per
-// step; 16: 0.213; 32: 0.261); the ensemble's persistent launches walk their
-// longest-first lists one after another and lose less to halo rows with 32
-// (2.094 ms per step; 8: 2.21; 16: 2.127; 64: 2.136).
-constexpr int SXC_GRID = 8;
-constexpr int SXC_GRID_SMALL = 4;
+// Work items of a grid with nx, ny >= 3 (strips of SW columns from column 0).
+// The strips whose lanes reach outside the grid (the first, and the last one
+// or two) go in chunks of sxc rows; every other strip has two items for the
+// rows [0, 2) and [nx - 2, nx) -- these are the boundary items, for the general
+// body -- and sx-row chunks of the rows between for the interior body.  Order:
+// interior items, boundary strips, boundary rows.  Item 0 keeps the control
+// block.  Returns the item count (item = -1), the count of boundary items
+// (item = -2), or with item >= 0 fills its strip, rows and kind (1 boundary, 0
+// interior).
+constexpr int SXC_GRID = 4;
 constexpr int SXC_ENS = 32;
-static_assert(SXC_GRID <= SXC_MAX && SXC_ENS <= SXC_MAX, "column-EDGE pre-pass rows");
 __host__ __device__ inline int full_items(int nx, int ny, int item, int* strip, int* r0,
-                                          int* r1, int* kind, int sxc, int sx = SX) {
-  const int SXC = sxc;
-  const int SX = sx;
+                                          int* r1, int* kind, int sxc, int sx) {
   const int ns = (ny + SW - 1) / SW;
-  const int mh = full_mid_strips(ny);   // middle strips: 1 <= s <= mh
-  const int nmid = mh, nedge = ns - nmid;
-  const int nci = nx > 4 ? (nx - 4 + SX - 1) / SX : 0;
-  const int ncc = nx > 4 ? (nx - 4 + SXC - 1) / SXC : 0;
-  const int nside = nedge * ncc + 2 * ns;
-  const int total = nside + nmid * nci;
+  const int nmid = full_mid_strips(ny);   // middle strips: 1 <= s <= nmid
+  const int nedge = ns - nmid;
+  const int nint = nx > 4 ? nmid * ((nx - 4 + sx - 1) / sx) : 0;
+  const int ncc = (nx + sxc - 1) / sxc;
+  const int nside = nedge * ncc + 2 * nmid;
   if (item == -2) return nside;
-  if (item < 0) return total;
-  int st, a, b, k;
-  if (item < nedge * ncc) {
-    const int e = item / ncc;                // edge strips: 0, mh + 1, ..., ns - 1
-    st = e == 0 ? 0 : mh + e;
-    a = 2 + (item % ncc) * SXC;
-    b = a + SXC < nx - 2 ? a + SXC : nx - 2;
-    k = 2;
-  } else if ((item -= nedge * ncc) < 2 * ns) {
-    st = item >> 1;
-    a = (item & 1) ? nx - 2 : 0;
-    b = a + 2;
-    k = 1;
-  } else {
-    item -= 2 * ns;
+  if (item < 0) return nint + nside;
+  int st, a, b, k = 1;
+  if (item < nint) {
     st = 1 + item % nmid;
-    a = 2 + (item / nmid) * SX;
-    b = a + SX < nx - 2 ? a + SX : nx - 2;
+    a = 2 + (item / nmid) * sx;
+    b = a + sx < nx - 2 ? a + sx : nx - 2;
     k = 0;
+  } else if ((item -= nint) < nedge * ncc) {
+    const int e = item / ncc;                // boundary strips: 0, nmid + 1, ..., ns - 1
+    st = e == 0 ? 0 : nmid + e;
+    a = (item % ncc) * sxc;
+    b = a + sxc < nx ? a + sxc : nx;
+  } else {
+    item -= nedge * ncc;
+    st = 1 + (item >> 1);
+    a = (item & 1) ? (nx - 2 > 2 ? nx - 2 : 2) : 0;
+    b = (item & 1) ? nx : 2;
   }
   *strip = st;
   *r0 = a;
   *r1 = b;
   *kind = k;
-  return total;
+  return nint + nside;
 }
 
-// Row-chunk heights of a single grid's interior and column-EDGE items.  An
-// item of S rows marches S + 4 (two halo rows each side), and a row of a warp
-// costs about a + b k, k the warps per scheduler, because a lone warp is bound
-// by its own dependent instructions: short chunks on a small grid spread its
-// rows over more warps, long ones on a large grid save halo rows.  With
-// K = strips x rows / (148 SMs x 4 schedulers), k = K / S and the stage takes
-// (S + 4)(a + b K / S), least at S = sqrt(4 b / a K).  Measured on a B200 (us
-// per step, minmod eta / HLL-HR): float32 a = 0.7, b = 0.6, float64 a = 1.4,
-// b = 2.1, hence S = 2 sqrt(K) for both; from K = 160 (about 1650^2) on the
-// chip is full for several waves and whole 64-row items are as good or better
-// (2048^2 float64: 619 us with 64 rows, 635 with 32).  512^2 float32: 8 rows 28.7, 32 rows
-// 51.2, 64 rows 91.9; 1024^2: 16 rows 65.5, 64 rows 97; 2048^2: 32 rows 196, 64
-// rows 197, 8 rows 230; 512^2 float64: 12 rows 70.6, 64 rows 227.  The
-// column-EDGE items run beside the interior ones: below K = 64 (about 1024^2)
-// 8 rows outlast them (512^2 float32: 4 rows 28.7, 8 rows 40.2), above it the
-// halo rows of 4 cost more.
-static void strip_rows(int nstrips, int rows, int* sx, int* sxc) {
-  const double K = (double)std::max(nstrips, 1) * std::max(rows, 1) / 592.0;
-  int s = K < 160.0 ? (int)(2.0 * std::sqrt(K) + 0.5) : SX;
-  s = std::min(std::max(s, 4), SX);
-  // chunks of equal height
-  const int n = (std::max(rows, 1) + s - 1) / s;
-  *sx = (std::max(rows, 1) + n - 1) / n;
-  *sxc = K < 64.0 ? SXC_GRID_SMALL : SXC_GRID;
+// Row-chunk heights of a single grid's items.  An item of S rows marches S + 4
+// (two halo rows each side): long chunks save halo rows, short ones spread a
+// small grid over more warps.  A row of a CTA (four items) takes about a + b k,
+// k the CTAs on its SM -- a lone warp is bound by its own dependent
+// instructions, so the first CTA costs most (float32 1 + 0.3 k us for the two
+// stages, k <= 4; float64 2.6 + 0.7 k, k <= 2; fitted to 250 timings of 15 grid
+// sizes, mean error 5 %).  The height is the least modelled time over the
+// candidates: whole waves of interior CTAs, the last wave with the boundary
+// CTAs beside it, and a tail where those do not fit.  Measured on a B200 (us per
+// step, minmod eta / HLL-HR; 64 rows everywhere after it): float32 512^2 25 / 94,
+// 1024^2 59 / 97, 1448^2 93 / 137, 2048^2 174 / 174; float64 512^2 62 / 230,
+// 1024^2 177 / 245, 2048^2 571 / 571; over the 15 sizes within 0.5 % (float64
+// 2 %) of the best of ten fixed heights on average.
+// A grid of fewer than 6 x 592 strip rows (about 300^2) takes the general body
+// everywhere in one uniform list: its two-row boundary items and four-row
+// boundary chunks would outlast the rest (256^2 float32 17.6 against 20.5,
+// 64^2 14 against 20; 400^2 24 against 22.6).
+template <typename T>
+static void strip_rows(int nx, int ny, SweParams<T>* p) {
+  constexpr bool F32 = sizeof(T) == 4;
+  constexpr double A = F32 ? 1.0 : 2.6, B = F32 ? 0.3 : 0.7, CPS = F32 ? 4 : 2;
+  constexpr double EDGE_ROWS = 8.0 * (F32 ? 1.3 : 1.1);   // a boundary item, in interior rows
+  constexpr double SLOTS = 148.0 * CPS, FULL = A + B * CPS;
+  const int ns = (ny + SW - 1) / SW, nmid = full_mid_strips(ny);
+  p->single = (double)ns * nx < 6.0 * 592.0 ? 1 : 0;
+  p->sxc = SXC_GRID;
+  const int strips = p->single ? ns : nmid, rows = p->single ? nx : std::max(nx - 4, 1);
+  const double ne =
+      p->single ? 0.0 : ((ns - nmid) * ((nx + SXC_GRID - 1) / SXC_GRID) + 2.0 * nmid) / 4.0;
+  double best = 1e300;
+  for (int s : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64}) {
+    const int n = (rows + s - 1) / s, h = (rows + n - 1) / n;   // chunks of equal height
+    const double L = h + 4, ctas = strips * (double)n / 4.0;
+    const double q = std::floor(ctas / SLOTS), r = ctas - q * SLOTS, last = r + ne;
+    const double own = r > 0.0 ? L : 0.0;
+    double cost = L * q * FULL;
+    if (last <= SLOTS)
+      cost += std::max(own, ne > 0.0 ? EDGE_ROWS : 0.0) *
+              (A + B * (F32 ? std::max(1.0, last / 148.0) : std::ceil(last / 148.0)));
+    else
+      cost += (own + EDGE_ROWS * std::max(0.5, (last - SLOTS) / SLOTS)) * FULL;
+    if (cost < best) {
+      best = cost;
+      p->sx = h;
+    }
+  }
 }
 
-// KIND 0: the interior strips of a grid with a periodic side (the tile kernel
-// takes the frame); KIND 1: the boundary items of a full-coverage list
-// (column-EDGE and EDGE); KIND 2: its interior items; KIND 3: its interior
-// items reading the prepared bed planes (p.bed).  Kinds 1 and 2 are
-// separate launches (they run side by side on two streams) so that the
-// boundary bodies never raise the interior body's register allocation.
-// float32: 4 CTAs of 4 warps per SM (128 registers; the paired-face interior
-// body spills at 96).
-template <typename T, int RECON, int RIEMANN, int MODE, int KIND>
+// One stage of a grid: a warp per item, the interior or the general body by
+// the item's kind (p.single: the general body for all), both bodies in one
+// launch.  BED: the interior items read the prepared bed planes (p.bed).
+// float32: 4 CTAs of 4 warps per SM (128 registers; the bodies spill at 96).
+template <typename T, int RECON, int RIEMANN, int MODE, bool BED>
 __global__ void __launch_bounds__(STRIP_NT, sizeof(T) == 4 ? 4 : 2)
 swe2d_strip_kernel(const T* __restrict__ bP, const T* __restrict__ hP,
                    const T* __restrict__ qxP, const T* __restrict__ qyP,
                    const T* __restrict__ h0P, const T* __restrict__ qx0P,
                    const T* __restrict__ qy0P, T* __restrict__ hO, T* __restrict__ qxO,
-                   T* __restrict__ qyO, zb_ctrl* ctrl, int phase, const SweParams<T> p) {
-  int item = blockIdx.x * (STRIP_NT / 32) + (threadIdx.x >> 5);
-  int strip, r0, r1, kind = 0;
-  if (KIND == 0) {
-    const int nstrips = (p.fast_j1 - p.fast_j0) / SW;
-    if (item >= nstrips * ((p.fast_i1 - p.fast_i0 + p.sx - 1) / p.sx)) return;   // warp-uniform
-    strip = item % nstrips;
-    r0 = p.fast_i0 + (item / nstrips) * p.sx;
-    r1 = min(r0 + p.sx, p.fast_i1);
+                   T* __restrict__ qyO, zb_ctrl* ctrl, int phase,
+                   const T* __restrict__ hinv_src, const unsigned char* __restrict__ force_o1,
+                   unsigned char* __restrict__ trouble_out, const SweParams<T> p) {
+  const int item = blockIdx.x * (STRIP_NT / 32) + (threadIdx.x >> 5);
+  const bool lead = item == 0;
+  int strip, r0, r1, kind = 1;
+  if (p.single) {
+    const int ns = (p.ny + SW - 1) / SW;
+    strip = item % ns;
+    r0 = (item / ns) * p.sx;
+    r1 = min(r0 + p.sx, p.nx);
+    if (r0 >= p.nx) return;   // warp-uniform
   } else {
-    const int ne = full_items(p.nx, p.ny, -2, nullptr, nullptr, nullptr, nullptr, p.sxc, p.sx);
-    if (KIND == 1 && item >= ne) return;
-    if (KIND >= 2) {
-      item += ne;
-      const int n = full_items(p.nx, p.ny, -1, nullptr, nullptr, nullptr, nullptr, p.sxc, p.sx);
-      if (item >= n) return;
-    }
+    if (item >= full_items(p.nx, p.ny, -1, nullptr, nullptr, nullptr, nullptr, p.sxc, p.sx))
+      return;
     full_items(p.nx, p.ny, item, &strip, &r0, &r1, &kind, p.sxc, p.sx);
   }
-  if (KIND == 1) {
-    // warp-uniform: the item's kind
-    if (kind == 2)
-      strip_item<T, RECON, RIEMANN, MODE, 2>(bP, hP, qxP, qyP, h0P, qx0P, qy0P, hO, qxO, qyO,
-                                             ctrl, phase, p, strip, r0, r1, item == 0);
-    else
-      strip_item<T, RECON, RIEMANN, MODE, 1>(bP, hP, qxP, qyP, h0P, qx0P, qy0P, hO, qxO, qyO,
-                                             ctrl, phase, p, strip, r0, r1, item == 0);
-  } else {
-    strip_item<T, RECON, RIEMANN, MODE, 0, KIND == 3>(bP, hP, qxP, qyP, h0P, qx0P, qy0P, hO,
-                                                      qxO, qyO, ctrl, phase, p, strip, r0, r1,
-                                                      false);
-  }
+  if (kind)
+    strip_item<T, RECON, RIEMANN, MODE, true, false>(
+        bP, hP, qxP, qyP, h0P, qx0P, qy0P, hO, qxO, qyO, ctrl, phase, p, strip, r0, r1, lead,
+        hinv_src, force_o1, trouble_out);
+  else
+    strip_item<T, RECON, RIEMANN, MODE, false, BED>(
+        bP, hP, qxP, qyP, h0P, qx0P, qy0P, hO, qxO, qyO, ctrl, phase, p, strip, r0, r1, lead,
+        hinv_src, force_o1, trouble_out);
 }
 
-// A second stream per device with a fork and a join event: the EDGE launch of
-// a full-coverage stage runs on it beside the interior launch.  Each host
-// thread has its own (thread_local), so the fork / join records of calls from
-// different threads never interleave and a stream capture on one thread never
-// pulls in another thread's launches.  Calls from one thread are ordered by
-// the host; on the side stream they run in call order, whatever the caller's
-// stream.
-struct SideStream {
-  cudaStream_t s;
-  cudaEvent_t fork, join;
-};
-static int side_stream(SideStream** out) {
-  thread_local SideStream ss[32];
-  thread_local unsigned made = 0u;
-  int dev = 0;
-  ZB_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 32) return ZB_E_UNSUPPORTED;
-  if (!(made & (1u << dev))) {
-    ZB_CUDA_TRY(cudaStreamCreateWithFlags(&ss[dev].s, cudaStreamNonBlocking));
-    ZB_CUDA_TRY(cudaEventCreateWithFlags(&ss[dev].fork, cudaEventDisableTiming));
-    ZB_CUDA_TRY(cudaEventCreateWithFlags(&ss[dev].join, cudaEventDisableTiming));
-    made |= 1u << dev;
-  }
-  *out = &ss[dev];
-  return ZB_OK;
-}
-
-// ── batched ensemble: one persistent launch per stage over all instances ────
+// ── batched ensemble: one launch per stage over all instances ───────────────
 // Each instance is an independent Cartesian grid with its own size, spacing,
-// Manning coefficient, dt and control block.  The work list holds one item
-// per (instance, tile): {instance, i0, j0, first-tile flag}.  A persistent CTA
-// walks items with a grid stride; every item is one stage_tile() call with its
-// instance's own dt (read from the instance's control slots), so the whole
-// ensemble advances one stage per launch.
+// Manning coefficient, dt and control block; the work list holds the strip
+// items of every instance, so the whole ensemble advances one stage per launch.
 template <typename T>
 struct EnsDesc {
   SweParams<T> p;
@@ -1622,126 +1200,92 @@ struct EnsDesc {
   long long ws_off;  // element offset of its (3, C) stage buffer
 };
 
-template <typename T, int TX, int ORDER, int RECON, int RIEMANN, int MODE>
-__global__ void __launch_bounds__(NT)
-ens_stage_kernel(const EnsDesc<T>* __restrict__ desc, const int4* __restrict__ items,
-                 T* Q, T* W, zb_ctrl* ctrls, int phase) {
-  using S = Smem<T, TX>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  S& s = *reinterpret_cast<S*>(smem_raw);
-  __shared__ double red[NT / 32];
-  const int tid = threadIdx.x;
-  // items[0].x = the tile item count; the tile items follow the header
-  const int n_items = items[0].x;
-  items += 1;
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const int4 w = items[it];
-    const EnsDesc<T>* d = desc + w.x;
-    const SweParams<T>& p = d->p;
-    zb_ctrl* ctrl = ctrls + w.x;
-    const size_t C = (size_t)p.nx * p.ny;
-    T* q = Q + d->q_off;
-    T* ws = W + d->ws_off;
-    const int ph = phase, nph = (ph + 1) % 3, nnph = (ph + 2) % 3;
-    const double t = ctrl->t[ph];
-    double dtd = dt_from_amax(ctrl->amax[ph], t, p.cfl2r, p.den_fac, p.dt_max, p.t_end);
-    const bool ok = isfinite(dtd) && dtd > 0.0;
-    const bool lead = w.w != 0 && tid == 0;
-    __syncthreads();   // the previous item is done with shared memory
-    if (MODE == MODE_STEP1 && lead) {
-      if (!ok && t < p.t_end) atomicOr(&ctrl->status, (unsigned)ZB_ST_DT_INVALID);
-      ctrl->dt = ok ? dtd : 0.0;
-      ctrl->t[nph] = ok ? t + dtd : t;
-      ctrl->amax[nnph] = 0.0;
-    }
-    if (!ok) {
-      if (MODE == MODE_STEP2 && lead) ctrl->amax[nph] = ctrl->amax[ph];
-      continue;   // block-uniform: every thread of the CTA skips this item
-    }
-    if (MODE == MODE_STEP1) {
-      stage_tile<T, TX, ORDER, RECON, RIEMANN, MODE_STEP1>(
-          s, red, w.y, w.z, q, q + C, q + 2 * C, q + 3 * C, nullptr, nullptr, nullptr, ws,
-          ws + C, ws + 2 * C, ctrl, ph, nullptr, nullptr, nullptr, p, dtd, w.w != 0);
-    } else {
-      stage_tile<T, TX, ORDER, RECON, RIEMANN, MODE_STEP2>(
-          s, red, w.y, w.z, q, ws, ws + C, ws + 2 * C, q + C, q + 2 * C, q + 3 * C, q + C,
-          q + 2 * C, q + 3 * C, ctrl, ph, nullptr, nullptr, nullptr, p, dtd, w.w != 0);
-    }
-  }
-}
-
 // One strip item of an instance: stage 1 reads Q and writes the stage buffer,
 // stage 2 reads the stage buffer and Q0 = Q and writes Q.
-template <typename T, int MODE, int EK>
-__device__ __forceinline__ void ens_item(const EnsDesc<T>* d, T* Q, T* W, zb_ctrl* ctrl,
-                                         int phase, int strip, int r0, int r1, bool lead) {
-  const SweParams<T>& p = d->p;
+template <typename T, int MODE, bool EDGE>
+__device__ __forceinline__ void ens_item(const volatile SweParams<T>& p, T* q, T* ws,
+                                         zb_ctrl* ctrl, int phase, int strip, int r0, int r1,
+                                         bool lead) {
   const size_t C = (size_t)p.nx * p.ny;
-  T* q = Q + d->q_off;
-  T* ws = W + d->ws_off;
   if (MODE == MODE_STEP1)
-    strip_item<T, ZB_RECON_ETA, ZB_RIEMANN_HLL_HR, MODE_STEP1, EK>(
+    strip_item<T, ZB_RECON_ETA, ZB_RIEMANN_HLL_HR, MODE_STEP1, EDGE, false>(
         q, q + C, q + 2 * C, q + 3 * C, nullptr, nullptr, nullptr, ws, ws + C, ws + 2 * C,
         ctrl, phase, p, strip, r0, r1, lead);
   else
-    strip_item<T, ZB_RECON_ETA, ZB_RIEMANN_HLL_HR, MODE_STEP2, EK>(
+    strip_item<T, ZB_RECON_ETA, ZB_RIEMANN_HLL_HR, MODE_STEP2, EDGE, false>(
         q, ws, ws + C, ws + 2 * C, q + C, q + 2 * C, q + 3 * C, q + C, q + 2 * C, q + 3 * C,
         ctrl, phase, p, strip, r0, r1, lead);
 }
 
-// All instances' strip items of one body (EK, as strip_item: 0 interior, 1
-// EDGE, 3 column EDGE with its pre-pass): persistent warps walk them.  The
-// work list's header items[0] = {tile items, interior strip items, EDGE strip
-// items, column-EDGE strip items}; the lists follow it in that order.  Each
-// body is a launch of its own, so that the boundary bodies' extra live values
-// never raise another body's register allocation.
-template <typename T, int MODE, int EK>
+// All instances' strip items, a warp per item: the interior items, then the
+// boundary items, each list longest item first (the block scheduler fills the
+// tail of the long ones with the short ones).  The work list's header items[0] =
+// {interior items, boundary items}; the lists follow it.  A warp's instance
+// parameters sit in shared memory: read from global memory they were held in
+// registers and spilled (408 bytes a thread with both bodies in one kernel,
+// 222 us a stage of 64 instances).
+template <typename T, int MODE>
 __global__ void __launch_bounds__(STRIP_NT, sizeof(T) == 4 ? 4 : 2)
 ens_strip_kernel(const EnsDesc<T>* __restrict__ desc, const int4* __restrict__ items, T* Q,
                  T* W, zb_ctrl* ctrls, int phase) {
-  static_assert(EK == 0 || EK == 1 || EK == 3, "ensemble bodies");
+  __shared__ SweParams<T> par[STRIP_NT / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int4 hd = items[0];
-  const int4* list = items + 1 + hd.x + (EK >= 1 ? hd.y : 0) + (EK == 3 ? hd.z : 0);
-  const int n = EK == 0 ? hd.y : (EK == 1 ? hd.z : hd.w);
-  const int nw = gridDim.x * (STRIP_NT / 32);
-  for (int it = blockIdx.x * (STRIP_NT / 32) + (threadIdx.x >> 5); it < n; it += nw) {
-    // w = {instance, strip, r0, flags | r1 << 3}; flags bit 1 = the item keeps
-    // the instance's control block
-    const int4 w = list[it];
-    ens_item<T, MODE, EK>(desc + w.x, Q, W, ctrls + w.x, phase, w.y, w.z, w.w >> 3,
-                          (w.w & 2) != 0);
-  }
+  const int it = blockIdx.x * (STRIP_NT / 32) + warp;
+  if (it >= hd.x + hd.y) return;
+  // w = {instance, strip, r0, flags | r1 << 1}; flag bit 0 = the item keeps the
+  // instance's control block
+  const int4 w = items[1 + it];
+  const EnsDesc<T>* d = desc + w.x;
+  static_assert(sizeof(SweParams<T>) % 4 == 0, "copied by words");
+  for (int k = lane; k < (int)(sizeof(SweParams<T>) / 4); k += 32)
+    ((int*)&par[warp])[k] = ((const int*)&d->p)[k];
+  __syncwarp();
+  const volatile SweParams<T>& p = par[warp];
+  T* q = Q + d->q_off;
+  T* ws = W + d->ws_off;
+  if (it < hd.x)
+    ens_item<T, MODE, false>(p, q, ws, ctrls + w.x, phase, w.y, w.z, w.w >> 1, (w.w & 1) != 0);
+  else
+    ens_item<T, MODE, true>(p, q, ws, ctrls + w.x, phase, w.y, w.z, w.w >> 1, (w.w & 1) != 0);
+}
+
+// A march's start: the control blocks, then the wave-speed maximum of every
+// instance by AMAX_PARTS CTAs (one CTA per instance left the largest ones to a
+// single SM: 64 instances of 64^2 .. 512^2 475 us, now 16).
+constexpr int AMAX_PARTS = 16;
+
+__global__ void ens_ctrl_init_kernel(zb_ctrl* ctrls, int n_inst, int phase, double t0) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_inst) return;
+  zb_ctrl* ctrl = ctrls + i;
+  for (int j = 0; j < 3; ++j) { ctrl->amax[j] = 0.0; ctrl->t[j] = 0.0; }
+  ctrl->t[phase] = t0;
+  ctrl->dt = 0.0;
+  ctrl->status = 0u;
+  ctrl->steps = 0u;
+  ctrl->troubled = 0u;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(NT)
 ens_amax_kernel(const EnsDesc<T>* __restrict__ desc, const T* __restrict__ Q, zb_ctrl* ctrls,
-                int n_inst, int phase, double t0, T g, T eps) {
+                int n_inst, int phase, T g, T eps) {
   __shared__ double red[NT / 32];
-  for (int i = blockIdx.x; i < n_inst; i += gridDim.x) {
-    const EnsDesc<T>* d = desc + i;
-    const size_t C = (size_t)d->p.nx * d->p.ny;
-    const T* q = Q + d->q_off;
-    double m = 0.0;
-    for (size_t k = threadIdx.x; k < C; k += NT) {
-      const T h = q[C + k];
-      const T hi = kp_hinv(h, eps);
-      const T c = asqrt(g * nmax(h, T(0)));
-      m = nmax(m, (double)nmax(fabs(q[2 * C + k] * hi) + c, fabs(q[3 * C + k] * hi) + c));
-    }
-    __syncthreads();
-    m = block_max_double(m, red);
-    if (threadIdx.x == 0) {
-      zb_ctrl* ctrl = ctrls + i;
-      for (int j = 0; j < 3; ++j) { ctrl->amax[j] = 0.0; ctrl->t[j] = 0.0; }
-      ctrl->amax[phase] = m;
-      ctrl->t[phase] = t0;
-      ctrl->dt = 0.0;
-      ctrl->status = 0u;
-      ctrl->steps = 0u;
-      ctrl->troubled = 0u;
-    }
+  const int i = blockIdx.x / AMAX_PARTS, part = blockIdx.x % AMAX_PARTS;
+  if (i >= n_inst) return;
+  const EnsDesc<T>* d = desc + i;
+  const size_t C = (size_t)d->p.nx * d->p.ny;
+  const T* q = Q + d->q_off;
+  double m = 0.0;
+  for (size_t k = (size_t)part * NT + threadIdx.x; k < C; k += (size_t)AMAX_PARTS * NT) {
+    const T h = q[C + k];
+    const T hi = kp_hinv(h, eps);
+    const T c = asqrt(g * nmax(h, T(0)));
+    m = nmax(m, (double)nmax(fabs(q[2 * C + k] * hi) + c, fabs(q[3 * C + k] * hi) + c));
   }
+  m = block_max_double(m, red);
+  if (threadIdx.x == 0) atomic_max_pos_double(&ctrls[i].amax[phase], m);
 }
 
 // ── wave-speed max / aux / mass kernels ─────────────────────────────────────
@@ -2045,13 +1589,14 @@ static SweParams<T> make_params(const zb_swe2d_cfg* c, double alpha, double beta
   p.alpha = alpha;
   p.beta = beta;
   p.dt_stage = dt_stage;
-  p.lsq = make_lsq<T>(c->dx, c->dy);
   p.inv6dx = (T)(1.0 / (6.0 * c->dx));
   p.inv6dy = (T)(1.0 / (6.0 * c->dy));
   p.inv4dx = (T)(1.0 / (4.0 * c->dx));
   p.inv4dy = (T)(1.0 / (4.0 * c->dy));
-  p.fast_i0 = p.fast_i1 = p.fast_j0 = p.fast_j1 = 0;
-  p.strip_full = 0;
+  p.inv5dx = (T)(1.0 / (5.0 * c->dx));
+  p.inv5dy = (T)(1.0 / (5.0 * c->dy));
+  p.sx = p.sxc = SX;
+  p.single = 0;
   p.bed = (bed_scheme(c) && (c->dtype == ZB_F64) == std::is_same<T, double>::value)
               ? (const T*)c->bed : nullptr;
   return p;
@@ -2060,25 +1605,13 @@ static SweParams<T> make_params(const zb_swe2d_cfg* c, double alpha, double beta
 template <typename T>
 constexpr int tile_x() { return sizeof(T) == 4 ? 16 : 8; }
 
-// number of frame tiles the tile kernel enumerates when the strip kernel
-// owns the interior (see swe2d_stage_kernel)
-template <int TX>
-static int frame_tiles(int nx, int ny, int fi0, int fi1, int fj0, int fj1) {
-  const int ntc = (ny + TY - 1) / TY, ntr = (nx + TX - 1) / TX;
-  const int tra = (fi0 + TX - 1) / TX, trb = std::max(tra, fi1 / TX);
-  const int tca = (fj0 + TY - 1) / TY, tcb = std::max(tca, fj1 / TY);
-  return tra * ntc + (ntr - trb) * ntc + (trb - tra) * (tca + ntc - tcb);
-}
-
-template <typename T, int ORDER, int RECON, int RIEMANN, int MODE, int TX = tile_x<T>()>
+template <typename T, int RIEMANN, int MODE, int TX = tile_x<T>()>
 static int launch_stage(const zb_swe2d_cfg* c, const T* b, const T* h, const T* qx,
                         const T* qy, const T* h0, const T* qx0, const T* qy0,
                         T* ho, T* qxo, T* qyo, zb_ctrl* ctrl, int phase,
-                        const SweParams<T>& p, cudaStream_t st,
-                        const T* hinv_src = nullptr,
-                        const unsigned char* force_o1 = nullptr,
+                        const SweParams<T>& p, cudaStream_t st, const T* hinv_src = nullptr,
                         unsigned char* trouble_out = nullptr) {
-  auto kern = swe2d_stage_kernel<T, TX, ORDER, RECON, RIEMANN, MODE>;
+  auto kern = swe2d_stage_kernel<T, TX, RIEMANN, MODE>;
   const size_t sm = sizeof(Smem<T, TX>);
   static std::atomic<unsigned> attr_mask{0u};   // per instantiation, one bit per device
   int dev = 0;
@@ -2088,12 +1621,33 @@ static int launch_stage(const zb_swe2d_cfg* c, const T* b, const T* h, const T* 
     ZB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     attr_mask.fetch_or(1u << dev);
   }
-  dim3 grid((c->ny + TY - 1) / TY, (c->nx + TX - 1) / TX);
-  if (p.fast_i1 > p.fast_i0)
-    grid = dim3(frame_tiles<TX>(c->nx, c->ny, p.fast_i0, p.fast_i1, p.fast_j0, p.fast_j1), 1);
+  const dim3 grid((c->ny + TY - 1) / TY, (c->nx + TX - 1) / TX);
   kern<<<grid, NT, sm, st>>>(b, h, qx, qy, h0, qx0, qy0, ho, qxo, qyo, ctrl, phase,
-                             hinv_src, force_o1, trouble_out, p);
+                             hinv_src, trouble_out, p);
   return zb_launch_check();
+}
+
+// One order-2 stage of a single grid: one launch of the strip kernel.
+template <typename T, int RECON, int RIEMANN, int MODE>
+static int launch_strips(const zb_swe2d_cfg* c, const T* b, const T* h, const T* qx, const T* qy,
+                         const T* h0, const T* qx0, const T* qy0, T* ho, T* qxo, T* qyo,
+                         zb_ctrl* ctrl, int phase, SweParams<T> p, cudaStream_t st,
+                         const T* hinv_src = nullptr, const unsigned char* force_o1 = nullptr,
+                         unsigned char* trouble_out = nullptr) {
+  strip_rows(c->nx, c->ny, &p);
+  const int n = p.single ? ((c->ny + SW - 1) / SW) * ((c->nx + p.sx - 1) / p.sx)
+                         : full_items(c->nx, c->ny, -1, nullptr, nullptr, nullptr, nullptr, p.sxc,
+                                      p.sx);
+  const int wpb = STRIP_NT / 32;
+  auto go = [&](auto bed) -> int {
+    swe2d_strip_kernel<T, RECON, RIEMANN, MODE, decltype(bed)::value>
+        <<<(n + wpb - 1) / wpb, STRIP_NT, 0, st>>>(b, h, qx, qy, h0, qx0, qy0, ho, qxo, qyo, ctrl,
+                                                   phase, hinv_src, force_o1, trouble_out, p);
+    return zb_launch_check();
+  };
+  if constexpr (RECON == ZB_RECON_ETA && RIEMANN == ZB_RIEMANN_HLL_HR && MODE != MODE_STAGE)
+    if (p.bed && !p.single) return go(std::true_type());
+  return go(std::false_type());
 }
 
 // part: -1 = the whole step, 0 = first launch only, 1 = second launch only
@@ -2104,11 +1658,11 @@ static int run_step(const zb_swe2d_cfg* c, T* Q, T* ws, zb_ctrl* ctrl, int phase
   T *b = Q, *h = Q + C, *qx = Q + 2 * C, *qy = Q + 3 * C;
   const SweParams<T> p = make_params<T>(c, 0.0, 1.0);
   T *h1 = ws, *qx1 = ws + C, *qy1 = ws + 2 * C;
-  if (ORDER == 1) {
+  if constexpr (ORDER == 1) {
     // Euler reads the stencil of Q and cannot write Q in place: write the
     // workspace (launch 0), then copy the three evolving planes back (part 1)
     if (part != 1) {
-      int rc = launch_stage<T, ORDER, RECON, RIEMANN, MODE_EULER>(
+      int rc = launch_stage<T, RIEMANN, MODE_EULER>(
           c, b, h, qx, qy, nullptr, nullptr, nullptr, h1, qx1, qy1, ctrl, phase, p, st);
       if (rc) return rc;
     }
@@ -2116,107 +1670,17 @@ static int run_step(const zb_swe2d_cfg* c, T* Q, T* ws, zb_ctrl* ctrl, int phase
       ZB_CUDA_TRY(cudaMemcpyAsync(h, h1, 3 * C * sizeof(T), cudaMemcpyDeviceToDevice, st));
     return ZB_OK;
   }
-  // Without a periodic side the strip kernel covers the whole grid (strips
-  // and row chunks that reach the boundary take its EDGE body) and keeps the
-  // control block.  With one, the interior (two cells in from every side)
-  // goes to the strip kernel and the boundary frame to the tile kernel.
-  SweParams<T> pf = p;
-  int nstrips = 0;
-  if (ORDER == 2) {
-    bool periodic = false;
-    for (int sd = 0; sd < 4; ++sd) periodic = periodic || c->bc[sd] == ZB_BC_PERIODIC;
-    if (!periodic && c->nx >= 4 && c->ny >= 4) {
-      nstrips = (c->ny + SW - 1) / SW;
-      pf.fast_i0 = 0;
-      pf.fast_i1 = c->nx;
-      pf.fast_j0 = 0;
-      pf.fast_j1 = SW * nstrips;
-      pf.strip_full = 1;
-    } else if (c->ny >= 32 && c->nx >= 8) {
-      nstrips = (c->ny - 32) / SW + 1;
-      pf.fast_i0 = 2;
-      pf.fast_i1 = c->nx - 2;
-      pf.fast_j0 = 2;
-      pf.fast_j1 = 2 + SW * nstrips;
-    }
-  }
-  strip_rows(pf.strip_full ? full_mid_strips(c->ny) : nstrips,
-             pf.fast_i1 - pf.fast_i0 - (pf.strip_full ? 4 : 0), &pf.sx, &pf.sxc);
-  const bool strips = pf.fast_i1 > pf.fast_i0;
-  const bool tiles = !pf.strip_full;
-  const int nitems = !strips ? 0
-                     : pf.strip_full ? full_items(c->nx, c->ny, -1, nullptr, nullptr, nullptr,
-                                                  nullptr, pf.sxc, pf.sx)
-                                     : nstrips * ((pf.fast_i1 - pf.fast_i0 + pf.sx - 1) / pf.sx);
-  const int sgrid = (nitems + STRIP_NT / 32 - 1) / (STRIP_NT / 32);
-  // full coverage: the boundary items on the side stream, the interior items here
-  SideStream* side = nullptr;
-  int ne = 0, ni = 0;
-  if (pf.strip_full) {
-    int rc = side_stream(&side);
-    if (rc) return rc;
-    ne = full_items(c->nx, c->ny, -2, nullptr, nullptr, nullptr, nullptr, pf.sxc, pf.sx);
-    ni = nitems - ne;
-  }
-  const int wpb = STRIP_NT / 32;
-  auto launch_strips = [&](auto mode, const T* h_, const T* qx_, const T* qy_, const T* h0_,
-                           const T* qx0_, const T* qy0_, T* ho_, T* qxo_, T* qyo_) -> int {
-    constexpr int M = decltype(mode)::value;
-    if (!pf.strip_full) {
-      swe2d_strip_kernel<T, RECON, RIEMANN, M, 0><<<sgrid, STRIP_NT, 0, st>>>(
-          b, h_, qx_, qy_, h0_, qx0_, qy0_, ho_, qxo_, qyo_, ctrl, phase, pf);
-      return zb_launch_check();
-    }
-    ZB_CUDA_TRY(cudaEventRecord(side->fork, st));
-    ZB_CUDA_TRY(cudaStreamWaitEvent(side->s, side->fork, 0));
-    swe2d_strip_kernel<T, RECON, RIEMANN, M, 1><<<(ne + wpb - 1) / wpb, STRIP_NT, 0, side->s>>>(
-        b, h_, qx_, qy_, h0_, qx0_, qy0_, ho_, qxo_, qyo_, ctrl, phase, pf);
-    ZB_CUDA_TRY(cudaGetLastError());
-    if (ni > 0) {
-      // the interior items read the prepared bed planes when there are some
-      constexpr bool BEDK = RECON == ZB_RECON_ETA &&
-                            RIEMANN == ZB_RIEMANN_HLL_HR;
-      bool done = false;
-      if constexpr (BEDK) {
-        if (pf.bed) {
-          swe2d_strip_kernel<T, RECON, RIEMANN, M, 3><<<(ni + wpb - 1) / wpb, STRIP_NT, 0, st>>>(
-              b, h_, qx_, qy_, h0_, qx0_, qy0_, ho_, qxo_, qyo_, ctrl, phase, pf);
-          ZB_CUDA_TRY(cudaGetLastError());
-          done = true;
-        }
-      }
-      if (!done) {
-        swe2d_strip_kernel<T, RECON, RIEMANN, M, 2><<<(ni + wpb - 1) / wpb, STRIP_NT, 0, st>>>(
-            b, h_, qx_, qy_, h0_, qx0_, qy0_, ho_, qxo_, qyo_, ctrl, phase, pf);
-        ZB_CUDA_TRY(cudaGetLastError());
-      }
-    }
-    ZB_CUDA_TRY(cudaEventRecord(side->join, side->s));
-    ZB_CUDA_TRY(cudaStreamWaitEvent(st, side->join, 0));
-    return ZB_OK;
-  };
-  using M1 = std::integral_constant<int, MODE_STEP1>;
-  using M2 = std::integral_constant<int, MODE_STEP2>;
-  if (part != 1) {
-    if (strips) {
-      int rc = launch_strips(M1(), h, qx, qy, nullptr, nullptr, nullptr, h1, qx1, qy1);
+  if constexpr (ORDER == 2) {
+    if (part != 1) {
+      const int rc = launch_strips<T, RECON, RIEMANN, MODE_STEP1>(
+          c, b, h, qx, qy, nullptr, nullptr, nullptr, h1, qx1, qy1, ctrl, phase, p, st);
       if (rc) return rc;
     }
-    if (tiles) {
-      // the frame is thin: 8-row tiles waste less of their work on it
-      int rc = launch_stage<T, ORDER, RECON, RIEMANN, MODE_STEP1, 8>(
-          c, b, h, qx, qy, nullptr, nullptr, nullptr, h1, qx1, qy1, ctrl, phase, pf, st);
-      if (rc) return rc;
-    }
+    if (part == 0) return ZB_OK;
+    return launch_strips<T, RECON, RIEMANN, MODE_STEP2>(c, b, h1, qx1, qy1, h, qx, qy, h, qx, qy,
+                                                        ctrl, phase, p, st);
   }
-  if (part == 0) return ZB_OK;
-  if (strips) {
-    int rc = launch_strips(M2(), h1, qx1, qy1, h, qx, qy, h, qx, qy);
-    if (rc) return rc;
-  }
-  if (!tiles) return ZB_OK;
-  return launch_stage<T, ORDER, RECON, RIEMANN, MODE_STEP2, 8>(
-      c, b, h1, qx1, qy1, h, qx, qy, h, qx, qy, ctrl, phase, pf, st);
+  return ZB_OK;
 }
 
 template <typename T, int ORDER, int RECON, int RIEMANN>
@@ -2227,10 +1691,16 @@ static int run_generic_stage(const zb_swe2d_cfg* c, const T* Qk, const T* Q0, T*
   const size_t C = (size_t)c->nx * c->ny;
   const SweParams<T> p = make_params<T>(c, alpha, beta, dt);
   const T* b0 = Q0 ? Q0 : Qk;
-  return launch_stage<T, ORDER, RECON, RIEMANN, MODE_STAGE>(
-      c, b0, Qk + C, Qk + 2 * C, Qk + 3 * C, Q0 ? Q0 + C : nullptr,
-      Q0 ? Q0 + 2 * C : nullptr, Q0 ? Q0 + 3 * C : nullptr, Qo + C, Qo + 2 * C,
-      Qo + 3 * C, ctrl, 0, p, st, hinv_src, force_o1, trouble_out);
+  if constexpr (ORDER == 2)
+    return launch_strips<T, RECON, RIEMANN, MODE_STAGE>(
+        c, b0, Qk + C, Qk + 2 * C, Qk + 3 * C, Q0 ? Q0 + C : nullptr, Q0 ? Q0 + 2 * C : nullptr,
+        Q0 ? Q0 + 3 * C : nullptr, Qo + C, Qo + 2 * C, Qo + 3 * C, ctrl, 0, p, st, hinv_src,
+        force_o1, trouble_out);
+  else   // first order already: force_o1 changes nothing
+    return launch_stage<T, RIEMANN, MODE_STAGE>(
+        c, b0, Qk + C, Qk + 2 * C, Qk + 3 * C, Q0 ? Q0 + C : nullptr, Q0 ? Q0 + 2 * C : nullptr,
+        Q0 ? Q0 + 3 * C : nullptr, Qo + C, Qo + 2 * C, Qo + 3 * C, ctrl, 0, p, st, hinv_src,
+        trouble_out);
 }
 
 // dispatch over (order, recon, riemann)
@@ -2269,22 +1739,8 @@ static size_t ens_desc_bytes(int n_inst) {
   return ((size_t)n_inst * sizeof(EnsDesc<T>) + 255) / 256 * 256;
 }
 
-// strip region of an instance: the whole grid (every instance has wall or
-// extrapolation sides), or empty for a grid too small for strips (all tiles)
-struct Fast { int i0, i1, j0, j1, nstrips, nchunks; };
-static Fast fast_region(int nx, int ny) {
-  Fast f{0, 0, 0, 0, 0, 0};
-  if (nx >= 4 && ny >= 4) {
-    f.nstrips = (ny + SW - 1) / SW;
-    f.nchunks = (nx + SX - 1) / SX;
-    f.i1 = nx; f.j1 = SW * f.nstrips;
-  }
-  return f;
-}
-
-// strip items of an instance (the single grid's full-coverage list):
-// {strip, r0, r1, flags}; flags bit 0 = a boundary-launch item, bit 1 = it
-// keeps the control block, bit 2 = a column-EDGE item (else EDGE, when bit 0)
+// strip items of an instance (the single grid's list): {strip, r0, r1, kind,
+// first item}
 // the chunk heights of an instance's size class (zb_ens_tuning)
 static void ens_class_rows(const zb_ens_tuning& t, const zb_ens_instance& in, int* sxc,
                            int* sx) {
@@ -2297,42 +1753,29 @@ static void ens_class_rows(const zb_ens_tuning& t, const zb_ens_instance& in, in
 
 template <typename F>
 static void ens_strip_items(const zb_ens_instance& in, const zb_ens_tuning& t, F&& visit) {
-  if (fast_region(in.nx, in.ny).nstrips == 0) return;
   int sxc, sx;
   ens_class_rows(t, in, &sxc, &sx);
   const int n = full_items(in.nx, in.ny, -1, nullptr, nullptr, nullptr, nullptr, sxc, sx);
   for (int it = 0; it < n; ++it) {
     int st, r0, r1, kind;
     full_items(in.nx, in.ny, it, &st, &r0, &r1, &kind, sxc, sx);
-    visit(st, r0, r1, (kind != 0 ? 1 : 0) | (it == 0 ? 2 : 0) | (kind == 2 ? 4 : 0));
+    visit(st, r0, r1, kind, it == 0);
   }
 }
 
-// tiles of an instance that the strips do not cover (all of a small grid's)
-template <typename F>
-static void ens_frame_tiles(const zb_ens_instance& in, int tile_x, F&& visit) {
-  if (fast_region(in.nx, in.ny).nstrips > 0) return;
-  for (int i0 = 0; i0 < in.nx; i0 += tile_x)
-    for (int j0 = 0; j0 < in.ny; j0 += TY) visit(i0, j0);
-}
-
-static void ens_counts(const zb_ens_instance* inst, int n, const zb_ens_tuning& t,
-                       size_t* tiles, size_t* strips) {
-  *tiles = 0;
-  *strips = 0;
+static size_t ens_count(const zb_ens_instance* inst, int n, const zb_ens_tuning& t) {
+  size_t strips = 0;
   for (int i = 0; i < n; ++i) {
-    ens_frame_tiles(inst[i], t.tile_x, [&](int, int) { ++*tiles; });
-    if (fast_region(inst[i].nx, inst[i].ny).nstrips > 0) {
-      int sxc, sx;
-      ens_class_rows(t, inst[i], &sxc, &sx);
-      *strips += (size_t)full_items(inst[i].nx, inst[i].ny, -1, nullptr, nullptr, nullptr,
-                                    nullptr, sxc, sx);
-    }
+    int sxc, sx;
+    ens_class_rows(t, inst[i], &sxc, &sx);
+    strips += (size_t)full_items(inst[i].nx, inst[i].ny, -1, nullptr, nullptr, nullptr, nullptr,
+                                 sxc, sx);
   }
+  return strips;
 }
 
 // the launch shape of the untuned entry points: one size class, 32-row
-// column-EDGE chunks, 64-row interior chunks, 4 (float) or 2 (double) strip
+// boundary-strip chunks, 64-row interior chunks, 4 (float) or 2 (double) strip
 // CTAs per SM
 static zb_ens_tuning ens_default_tuning(const zb_swe2d_cfg* c, int tile_x) {
   zb_ens_tuning t;
@@ -2371,75 +1814,18 @@ static bool ens_valid(const zb_swe2d_cfg* c, const zb_ens_instance* inst, int n,
   return true;
 }
 
-template <typename T, int TX>
-static int ens_launch(int part, const void* table, int n_inst, int n_items, int grid,
-                      int ctas_per_sm, void* Q, void* W, zb_ctrl* ctrls, int phase,
-                      cudaStream_t st) {
+template <typename T>
+static int ens_launch(int part, const void* table, int n_inst, int n_items, void* Q, void* W,
+                      zb_ctrl* ctrls, int phase, cudaStream_t st) {
   const EnsDesc<T>* desc = (const EnsDesc<T>*)table;
   const int4* items = (const int4*)((const char*)table + ens_desc_bytes<T>(n_inst));
-  const size_t sm = sizeof(Smem<T, TX>);
-  int dev = 0;
-  ZB_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 32) return ZB_E_UNSUPPORTED;
-  static std::atomic<int> sms_cache[32];
-  if (!sms_cache[dev].load()) {
-    int v = 0;
-    ZB_CUDA_TRY(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
-    sms_cache[dev].store(v);
-  }
-  // boundary strips, interior strips (persistent warps over their items; a
-  // grid that finds none exits at once), then the tiles of grids too small
-  // for strips
-  const int sgrid_e = sms_cache[dev].load() * ctas_per_sm;
-  const int sgrid_i = sgrid_e;
-  // the boundary items on the library's second stream, beside the interior ones
-  SideStream* side = nullptr;
-  {
-    const int rc = side_stream(&side);
-    if (rc) return rc;
-  }
-  ZB_CUDA_TRY(cudaEventRecord(side->fork, st));
-  ZB_CUDA_TRY(cudaStreamWaitEvent(side->s, side->fork, 0));
-  // the column-EDGE items (longer) before the EDGE items on the second stream
-  if (part == 0) {
-    ens_strip_kernel<T, MODE_STEP1, 3><<<sgrid_e, STRIP_NT, 0, side->s>>>(
-        desc, items, (T*)Q, (T*)W, ctrls, phase);
-    ens_strip_kernel<T, MODE_STEP1, 1><<<sgrid_e, STRIP_NT, 0, side->s>>>(
-        desc, items, (T*)Q, (T*)W, ctrls, phase);
-    ens_strip_kernel<T, MODE_STEP1, 0><<<sgrid_i, STRIP_NT, 0, st>>>(desc, items, (T*)Q,
-                                                                    (T*)W, ctrls, phase);
-  } else {
-    ens_strip_kernel<T, MODE_STEP2, 3><<<sgrid_e, STRIP_NT, 0, side->s>>>(
-        desc, items, (T*)Q, (T*)W, ctrls, phase);
-    ens_strip_kernel<T, MODE_STEP2, 1><<<sgrid_e, STRIP_NT, 0, side->s>>>(
-        desc, items, (T*)Q, (T*)W, ctrls, phase);
-    ens_strip_kernel<T, MODE_STEP2, 0><<<sgrid_i, STRIP_NT, 0, st>>>(desc, items, (T*)Q,
-                                                                    (T*)W, ctrls, phase);
-  }
-  ZB_CUDA_TRY(cudaGetLastError());
-  ZB_CUDA_TRY(cudaEventRecord(side->join, side->s));
-  ZB_CUDA_TRY(cudaStreamWaitEvent(st, side->join, 0));
-  // the tile fallback (grids narrower than four cells; its CTAs exit at once
-  // when the work list holds no tile items)
-  static std::atomic<unsigned> mask1{0u};
-  auto k1 = ens_stage_kernel<T, TX, 2, ZB_RECON_ETA, ZB_RIEMANN_HLL_HR, MODE_STEP1>;
-  auto k2 = ens_stage_kernel<T, TX, 2, ZB_RECON_ETA, ZB_RIEMANN_HLL_HR, MODE_STEP2>;
-  if (!(mask1.load() & (1u << dev))) {
-    ZB_CUDA_TRY(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    ZB_CUDA_TRY(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    mask1.fetch_or(1u << dev);
-  }
-  if (grid <= 0) {
-    int per_sm = 0, sms = 0;
-    ZB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k1, NT, sm));
-    ZB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    grid = std::max(1, per_sm) * sms;
-  }
-  grid = std::min(grid, n_items);
+  const int sgrid = (n_items + STRIP_NT / 32 - 1) / (STRIP_NT / 32);
   if (part == 0)
-    k1<<<grid, NT, sm, st>>>(desc, items, (T*)Q, (T*)W, ctrls, phase);
+    ens_strip_kernel<T, MODE_STEP1><<<sgrid, STRIP_NT, 0, st>>>(desc, items, (T*)Q, (T*)W, ctrls,
+                                                               phase);
   else
-    k2<<<grid, NT, sm, st>>>(desc, items, (T*)Q, (T*)W, ctrls, phase);
+    ens_strip_kernel<T, MODE_STEP2><<<sgrid, STRIP_NT, 0, st>>>(desc, items, (T*)Q, (T*)W, ctrls,
+                                                               phase);
   return zb_launch_check();
 }
 
@@ -2484,12 +1870,6 @@ int zb_swe2d_init(const zb_swe2d_cfg* cfg, const void* Q, zb_ctrl* ctrl, int pha
                   double t0, zb_stream_t stream) {
   if (!valid_cfg(cfg) || !Q || !ctrl || phase < 0 || phase > 2) return ZB_E_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  {
-    // the second stream of the fused step is created here, outside any capture
-    SideStream* side = nullptr;
-    const int rc = side_stream(&side);
-    if (rc) return rc;
-  }
   swe2d_ctrl_init_kernel<<<1, 32, 0, st>>>(ctrl, phase, t0);
   if (cfg->dtype == ZB_F32) return amax_into<float>(cfg, (const float*)Q, &ctrl->amax[phase], st);
   return amax_into<double>(cfg, (const double*)Q, &ctrl->amax[phase], st);
@@ -2668,11 +2048,10 @@ size_t zb_ens_table_bytes_tuned(const zb_swe2d_cfg* common, const zb_ens_instanc
                                 int n_inst, const zb_ens_tuning* tuning) {
   if (!ens_tuning_valid(common, tuning)) return 0;
   if (!ens_valid(common, inst, n_inst, tuning->tile_x)) return 0;
-  size_t tiles = 0, strips = 0;
-  ens_counts(inst, n_inst, *tuning, &tiles, &strips);
+  const size_t strips = ens_count(inst, n_inst, *tuning);
   const size_t d = common->dtype == ZB_F64 ? ens_desc_bytes<double>(n_inst)
                                            : ens_desc_bytes<float>(n_inst);
-  return d + (1 + tiles + strips) * sizeof(int4);
+  return d + (1 + strips) * sizeof(int4);
 }
 
 size_t zb_ens_table_bytes(const zb_swe2d_cfg* common, const zb_ens_instance* inst, int n_inst,
@@ -2699,9 +2078,8 @@ int zb_ens_prepare_tuned(const zb_swe2d_cfg* common, const zb_ens_instance* inst
   auto build = [&](auto tag) -> int {
     using T = decltype(tag);
     std::vector<EnsDesc<T>> desc(n_inst);
-    // items[0]: {tile items, interior strip items, EDGE strip items,
-    // column-EDGE strip items}
-    std::vector<int4> items(1), strips, estrips, cstrips;
+    // items[0]: {interior items, boundary items}
+    std::vector<int4> items(1), strips, estrips;
     for (int i = 0; i < n_inst; ++i) {
       zb_swe2d_cfg c = *common;
       c.bed = nullptr;   // instances read their own b; no prepared bed planes
@@ -2715,34 +2093,22 @@ int zb_ens_prepare_tuned(const zb_swe2d_cfg* common, const zb_ens_instance* inst
       desc[i].p = make_params<T>(&c, 0.0, 1.0);
       desc[i].q_off = inst[i].q_offset;
       desc[i].ws_off = inst[i].ws_offset;
-      const Fast f = fast_region(c.nx, c.ny);
-      desc[i].p.fast_i0 = f.i0; desc[i].p.fast_i1 = f.i1;
-      desc[i].p.fast_j0 = f.j0; desc[i].p.fast_j1 = f.j1;
-      desc[i].p.strip_full = f.nstrips > 0 ? 1 : 0;
-      // tile (0, 0) or strip item (0, 0) keeps the lead duties
-      ens_frame_tiles(inst[i], tile_x, [&](int i0, int j0) {
-        items.push_back(make_int4(i, i0, j0, i0 == 0 && j0 == 0));
-      });
-      ens_strip_items(inst[i], *tuning, [&](int st, int r0, int r1, int fl) {
-        std::vector<int4>& to = (fl & 4) ? cstrips : ((fl & 1) ? estrips : strips);
-        to.push_back(make_int4(i, st, r0, fl | (r1 << 3)));
+      ens_strip_items(inst[i], *tuning, [&](int st, int r0, int r1, int kind, bool lead) {
+        (kind ? estrips : strips).push_back(make_int4(i, st, r0, (lead ? 1 : 0) | (r1 << 1)));
       });
     }
     // longest items first: the persistent warps take items round-robin, so
     // each warp's k-th item is about as long as every other warp's k-th
     auto longest_first = [](std::vector<int4>& v) {
       std::stable_sort(v.begin(), v.end(), [](const int4& a, const int4& b) {
-        return (a.w >> 3) - a.z > (b.w >> 3) - b.z;
+        return (a.w >> 1) - a.z > (b.w >> 1) - b.z;
       });
     };
     longest_first(strips);
     longest_first(estrips);
-    longest_first(cstrips);
-    items[0] = make_int4((int)(items.size() - 1), (int)strips.size(), (int)estrips.size(),
-                         (int)cstrips.size());
+    items[0] = make_int4((int)strips.size(), (int)estrips.size(), 0, 0);
     items.insert(items.end(), strips.begin(), strips.end());
     items.insert(items.end(), estrips.begin(), estrips.end());
-    items.insert(items.end(), cstrips.begin(), cstrips.end());
     const size_t db = ens_desc_bytes<T>(n_inst);
     // the table may still be read by steps in flight on any stream: wait for
     // the device, copy, and return only once the copy has landed
@@ -2762,19 +2128,15 @@ int zb_ens_init(const zb_swe2d_cfg* common, const void* table, int n_inst, const
                 zb_ctrl* ctrls, int phase, double t0, zb_stream_t stream) {
   if (!common || !table || !Q || !ctrls || n_inst < 1 || phase < 0 || phase > 2) return ZB_E_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  {
-    SideStream* side = nullptr;   // created here, outside any capture
-    const int rc = side_stream(&side);
-    if (rc) return rc;
-  }
-  const int grid = std::min(n_inst, 148 * 8);
+  ens_ctrl_init_kernel<<<(n_inst + NT - 1) / NT, NT, 0, st>>>(ctrls, n_inst, phase, t0);
+  const int grid = n_inst * AMAX_PARTS;
   if (common->dtype == ZB_F64)
     ens_amax_kernel<double><<<grid, NT, 0, st>>>((const EnsDesc<double>*)table, (const double*)Q,
-                                                 ctrls, n_inst, phase, t0, common->g,
+                                                 ctrls, n_inst, phase, common->g,
                                                  common->wet_dry_eps);
   else
     ens_amax_kernel<float><<<grid, NT, 0, st>>>((const EnsDesc<float>*)table, (const float*)Q,
-                                                ctrls, n_inst, phase, t0, (float)common->g,
+                                                ctrls, n_inst, phase, (float)common->g,
                                                 (float)common->wet_dry_eps);
   return zb_launch_check();
 }
@@ -2785,18 +2147,12 @@ int zb_ens_step_part_tuned(const zb_swe2d_cfg* common, const void* table, int n_
   if (!common || !table || !Q || !W || !ctrls || n_inst < 1 || n_items < 1) return ZB_E_ARG;
   if (phase < 0 || phase > 2 || part < -1 || part > 1) return ZB_E_ARG;
   if (!ens_tuning_valid(common, tuning)) return ZB_E_ARG;
-  const int tile_x = tuning->tile_x, cps = tuning->ctas_per_sm;
+  (void)grid;
   cudaStream_t st = (cudaStream_t)stream;
   for (int pt = (part == 1 ? 1 : 0); pt <= (part == 0 ? 0 : 1); ++pt) {
-    int rc;
-    if (common->dtype == ZB_F64)
-      rc = tile_x == 8
-               ? ens_launch<double, 8>(pt, table, n_inst, n_items, grid, cps, Q, W, ctrls, phase, st)
-               : ens_launch<double, 16>(pt, table, n_inst, n_items, grid, cps, Q, W, ctrls, phase, st);
-    else
-      rc = tile_x == 8
-               ? ens_launch<float, 8>(pt, table, n_inst, n_items, grid, cps, Q, W, ctrls, phase, st)
-               : ens_launch<float, 16>(pt, table, n_inst, n_items, grid, cps, Q, W, ctrls, phase, st);
+    const int rc = common->dtype == ZB_F64
+                       ? ens_launch<double>(pt, table, n_inst, n_items, Q, W, ctrls, phase, st)
+                       : ens_launch<float>(pt, table, n_inst, n_items, Q, W, ctrls, phase, st);
     if (rc) return rc;
   }
   return ZB_OK;
