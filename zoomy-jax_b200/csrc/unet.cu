@@ -99,57 +99,245 @@ conv3x3_fwd(const float* __restrict__ inA, int cin_a, const float* __restrict__ 
   }
 }
 
-// dW[co][ci][tap] += sum_p dout[co](p) in[ci](p + tap); dbias[co] += sum_p dout
-// one CTA per (16x16 tile, image); each thread owns weight entries and walks
-// the tile's pixels from shared memory
-__global__ void __launch_bounds__(NTT)
+// Weight and bias gradients of one layer,
+//   dW[co][ci][tap] = sum_p dout[co](p) in[ci](p + tap),  dbias[co] = sum_p dout[co](p),
+// in float32 on the FMA pipe.  A thread owns one input channel and WG_COT output
+// channels with all nine taps in registers and walks the pixels of a WG_TY x
+// WG_TX tile: per pixel three new input values (the 3 x 3 window slides along x)
+// and one 16-byte load of output gradients (the same address for a warp's
+// lanes) feed 9 WG_COT FMAs.  The bias is one more input channel that holds
+// ones.  Where a layer has few (channel, channel group) pairs the threads also
+// split the tile's row segments (nsl slices) and add their sums in a fixed
+// order.  Tiles arrive by cp.async into two buffers.  A CTA keeps its
+// accumulators over all its tiles and writes one partial set; wgrad_reduce adds
+// the partial sets in order, so the gradients are deterministic.  One thread per
+// weight walking the pixels in shared memory with a float atomic per tile, as
+// before, was bound by its two shared loads per FMA: the six layers of a
+// 64 x 32^2 batch (24, 48) took 1234 us, now 285 and 15 for the reduction (the
+// FMA pipe's floor is 50; the copies of the halo tiles are the rest).
+constexpr int WG_TX = 16, WG_TY = 4, WG_SEG = 8;          // tile, pixels per row segment
+constexpr int WG_HX = WG_TX + 2, WG_HY = WG_TY + 2;
+constexpr int WG_PLANE = WG_HX * WG_HY + 1;               // odd: lanes of a warp hit 32 banks
+constexpr int WG_UNITS = WG_TY * (WG_TX / WG_SEG);        // row segments of a tile
+constexpr int WG_MAX_THREADS = 448;                       // two CTAs of 72 registers a thread
+constexpr int WG_COT = 4;                                 // output channels of a thread
+constexpr int WG_SLOTS = 296;                             // partial sets: two CTAs per SM
+
+struct WgShape {
+  int ncog, cic, nchunk, nsl, threads, slots;
+  size_t smem, part;   // bytes of shared memory; floats of one partial set
+};
+
+// channel groups, input channels per chunk (the ones channel included), slices
+// and threads of a layer's CTAs
+static WgShape wg_shape(int cin, int cout, int B, int H, int W) {
+  WgShape g;
+  const int cot = cout % WG_COT == 0 ? WG_COT : 1;
+  g.ncog = cout / cot;
+  const int planes = cin + 1, cmax = WG_MAX_THREADS / g.ncog;
+  g.nchunk = (planes + cmax - 1) / cmax;
+  g.cic = (planes + g.nchunk - 1) / g.nchunk;
+  const int pairs = g.cic * g.ncog;
+  g.nsl = std::max(1, std::min(WG_UNITS, WG_MAX_THREADS / pairs));
+  g.threads = (pairs * g.nsl + 31) / 32 * 32;
+  const long long ntiles = (long long)((W + WG_TX - 1) / WG_TX) * ((H + WG_TY - 1) / WG_TY) * B;
+  g.slots = (int)std::min<long long>(ntiles, WG_SLOTS);
+  const size_t stage =
+      2 * ((((size_t)g.cic * WG_PLANE + 3) & ~(size_t)3) +
+           (size_t)WG_TX * WG_TY * (cot > 1 ? cout + 4 : 1));
+  const size_t red = g.nsl > 1 ? (size_t)pairs * g.nsl * 9 * cot : 0;
+  g.smem = std::max(stage, red) * sizeof(float);
+  g.part = (size_t)cout * cin * 9 + cout;
+  return g;
+}
+
+__device__ __forceinline__ void cp_async4z(float* dst, const float* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
+               "r"(valid ? 4 : 0)
+               : "memory");
+}
+
+template <int COT>
+__global__ void __launch_bounds__(WG_MAX_THREADS, 2)
 conv3x3_wgrad(const float* __restrict__ inA, int cin_a, const float* __restrict__ inB, int cin,
-              const float* __restrict__ dout, int cout, float* __restrict__ dw,
-              float* __restrict__ dbias, int B, int H, int W, int mode_a) {
-  __shared__ float sin_[CCH][TS + 2][TS + 2];
-  __shared__ float sd[8][TS * TS];
-  const int x0 = blockIdx.x * TS, y0 = blockIdx.y * TS, b = blockIdx.z;
+              const float* __restrict__ dout, int cout, float* __restrict__ part, int B, int H,
+              int W, int mode_a, int ncog, int cic, int nsl) {
+  extern __shared__ __align__(16) float wsm[];
+  const int nt = blockDim.x, tid = threadIdx.x;
+  const int c_lo = blockIdx.y * cic, c_n = min(cic, cin + 1 - c_lo);
+  const int c_real = min(c_n, cin - c_lo);   // input channels of this chunk without the ones
+  // a staging buffer: input planes, then the output gradients [pixel][dstr]
+  // (16-byte rows); two of them, so that a tile's copies land while the one
+  // before it is worked on
+  const int dstr = COT > 1 ? cout + 4 : 1;
+  const int sd_off = (cic * WG_PLANE + 3) & ~3, buf = sd_off + WG_TX * WG_TY * dstr;
+  const int pairs = cic * ncog;
+  const int sl = tid / pairs, pr = tid - sl * pairs;
+  const int cog = pr / cic, ci = pr - cog * cic;
+  const bool work = sl < nsl && ci < c_n;
   const size_t plane = (size_t)B * H * W;
-  const size_t img = (size_t)b * H * W;
-  for (int co0 = 0; co0 < cout; co0 += 8) {
-    const int nco = min(8, cout - co0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < 8 * TS * TS; e += NTT) {
-      const int c = e / (TS * TS), pp = e - c * TS * TS;
-      const int yy = y0 + pp / TS, xx = x0 + pp % TS;
-      sd[c][pp] = (c < nco && yy < H && xx < W)
-                      ? dout[(size_t)(co0 + c) * plane + img + (size_t)yy * W + xx] : 0.0f;
+  const int tx = (W + WG_TX - 1) / WG_TX, ty = (H + WG_TY - 1) / WG_TY;
+  const int ntiles = tx * ty * B;
+  if (c_real < c_n)
+    for (int e = tid; e < 2 * WG_HX * WG_HY; e += nt) {
+      const int k = e / (WG_HX * WG_HY);
+      wsm[k * buf + c_real * WG_PLANE + (e - k * (WG_HX * WG_HY))] = 1.0f;
     }
-    __syncthreads();
-    if (dbias != nullptr && threadIdx.x < nco) {
-      float s = 0.0f;
-      for (int pp = 0; pp < TS * TS; ++pp) s += sd[threadIdx.x][pp];
-      atomicAdd(&dbias[co0 + threadIdx.x], s);
-    }
-    for (int c0 = 0; c0 < cin; c0 += CCH) {
-      const int nc = min(CCH, cin - c0);
-      __syncthreads();
-      for (int e = threadIdx.x; e < CCH * (TS + 2) * (TS + 2); e += NTT) {
-        const int cc = e / ((TS + 2) * (TS + 2));
-        const int rr = e - cc * (TS + 2) * (TS + 2);
-        const int yy = y0 - 1 + rr / (TS + 2), xx = x0 - 1 + rr % (TS + 2);
-        float v = 0.0f;
-        if (cc < nc && yy >= 0 && yy < H && xx >= 0 && xx < W)
-          v = src_at(inA, cin_a, inB, mode_a, c0 + cc, b, B, H, W, yy, xx);
-        sin_[cc][rr / (TS + 2)][rr % (TS + 2)] = v;
+  const int hl = tid & 15, hw = tid >> 4, nhw = nt >> 4;
+  auto stage = [&](int t, int k) {
+    float* sin_ = wsm + k * buf;
+    float* sd = sin_ + sd_off;
+    const int b = t / (tx * ty), rt = t - b * (tx * ty);
+    const int x0 = (rt % tx) * WG_TX, y0 = (rt / tx) * WG_TY;
+    const size_t img = (size_t)b * H * W;
+    // a half-warp per row of 16 pixels: the lane's column, plus the two halo
+    // columns on lanes 0 and 1
+    const int xx = x0 + hl, xh = hl == 0 ? x0 - 1 : x0 + WG_TX;
+    const bool xin = xx < W, hin = hl < 2 && xh >= 0 && xh < W;
+    const int hcol = hl == 0 ? 0 : WG_HX - 1;
+    for (int e = hw; e < c_real * WG_HY; e += nhw) {
+      const int cc = e / WG_HY, r = e - cc * WG_HY;
+      const int yy = y0 - 1 + r, c = c_lo + cc;
+      const bool yin = yy >= 0 && yy < H;
+      float* dst = sin_ + cc * WG_PLANE + r * WG_HX;
+      if (mode_a == SRC_POOL && c < cin_a) {   // the average is formed, not copied
+        dst[1 + hl] = (yin && xin) ? src_at(inA, cin_a, inB, mode_a, c, b, B, H, W, yy, xx) : 0.0f;
+        if (hl < 2)
+          dst[hcol] = (yin && hin) ? src_at(inA, cin_a, inB, mode_a, c, b, B, H, W, yy, xh) : 0.0f;
+        continue;
       }
-      __syncthreads();
-      // entries: nco x nc x 9 <= 8 * 8 * 9 = 576 over 256 threads
-      for (int e = threadIdx.x; e < nco * nc * 9; e += NTT) {
-        const int c = e / (nc * 9), rem = e - c * nc * 9;
-        const int cc = rem / 9, tap = rem - cc * 9;
-        const int dy = tap / 3, dx = tap % 3;
-        float s = 0.0f;
-        for (int pp = 0; pp < TS * TS; ++pp) s += sd[c][pp] * sin_[cc][pp / TS + dy][pp % TS + dx];
-        atomicAdd(&dw[((size_t)(co0 + c) * cin + c0 + cc) * 9 + tap], s);
+      const bool up = mode_a == SRC_UP && c < cin_a;
+      const float* row = inA;
+      if (yin)
+        row = c >= cin_a ? inB + (size_t)(c - cin_a) * plane + img + yy * W
+              : up ? inA + ((size_t)c * B + b) * (H >> 1) * (W >> 1) + (yy >> 1) * (W >> 1)
+                   : inA + (size_t)c * plane + img + yy * W;
+      cp_async4z(dst + 1 + hl, row + (yin && xin ? (up ? xx >> 1 : xx) : 0), yin && xin);
+      if (hl < 2) cp_async4z(dst + hcol, row + (yin && hin ? (up ? xh >> 1 : xh) : 0), yin && hin);
+    }
+    for (int e = hw; e < cout * WG_TY; e += nhw) {
+      const int c = e / WG_TY, r = e - c * WG_TY;
+      const bool in = y0 + r < H && xin;
+      cp_async4z(sd + (r * WG_TX + hl) * dstr + c,
+                 in ? dout + (size_t)c * plane + img + (y0 + r) * W + xx : dout, in);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[COT][9];
+#pragma unroll
+  for (int c = 0; c < COT; ++c)
+#pragma unroll
+    for (int k = 0; k < 9; ++k) acc[c][k] = 0.0f;
+  stage(blockIdx.x, 0);   // gridDim.x <= ntiles
+  int k = 0;
+#pragma unroll 1
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x, k ^= 1) {
+    // the other buffer was read in the previous round, which every thread has
+    // left: the barrier below
+    if (t + (int)gridDim.x < ntiles) {
+      stage(t + gridDim.x, k ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    if (work) {
+      const float* ip = wsm + k * buf + ci * WG_PLANE;
+      const float* dp = wsm + k * buf + sd_off + cog * COT;
+#pragma unroll 1
+      for (int u = sl; u < WG_UNITS; u += nsl) {
+        const int yy = u / (WG_TX / WG_SEG), xs = (u % (WG_TX / WG_SEG)) * WG_SEG;
+        const float* r0 = ip + yy * WG_HX + xs;
+        const float* q = dp + (yy * WG_TX + xs) * dstr;
+        float w[9];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          w[3 * a + 1] = r0[a * WG_HX];
+          w[3 * a + 2] = r0[a * WG_HX + 1];
+        }
+#pragma unroll
+        for (int x = 0; x < WG_SEG; ++x) {
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            w[3 * a] = w[3 * a + 1];
+            w[3 * a + 1] = w[3 * a + 2];
+            w[3 * a + 2] = r0[a * WG_HX + x + 2];
+          }
+          float d[COT];
+          if constexpr (COT == 4) {
+            const float4 v = *(const float4*)(q + x * dstr);
+            d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+          } else {
+            d[0] = q[x * dstr];
+          }
+#pragma unroll
+          for (int c = 0; c < COT; ++c)
+#pragma unroll
+            for (int j = 0; j < 9; ++j) acc[c][j] = fmaf(d[c], w[j], acc[c][j]);
+        }
       }
     }
+    __syncthreads();
   }
+  // slices in order through shared memory: slot [sl][9 COT values][pair]
+  if (nsl > 1) {
+    __syncthreads();
+    if (work)
+#pragma unroll
+      for (int c = 0; c < COT; ++c)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) wsm[((size_t)sl * 9 * COT + c * 9 + k) * pairs + pr] = acc[c][k];
+    __syncthreads();
+    if (!work || sl > 0) return;
+    for (int s2 = 1; s2 < nsl; ++s2)
+#pragma unroll
+      for (int c = 0; c < COT; ++c)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) acc[c][k] += wsm[((size_t)s2 * 9 * COT + c * 9 + k) * pairs + pr];
+  }
+  if (!work) return;
+  const int gci = c_lo + ci;
+  float* out = part + (size_t)blockIdx.x * ((size_t)cout * cin * 9 + cout);
+  if (gci < cin) {
+#pragma unroll
+    for (int c = 0; c < COT; ++c)
+#pragma unroll
+      for (int k = 0; k < 9; ++k) out[((size_t)(cog * COT + c) * cin + gci) * 9 + k] = acc[c][k];
+  } else {
+#pragma unroll
+    for (int c = 0; c < COT; ++c) out[(size_t)cout * cin * 9 + cog * COT + c] = acc[c][4];
+  }
+}
+
+// the partial sets of all six layers added in order
+struct WgReduce {
+  const float* part[6];
+  int slots[6], nw[6], nb[6], off_w[6], off_b[6], first[7];   // first: entry offsets
+};
+
+// A CTA adds 32 entries: warp w takes the sets w, w + 8, ... and the eight sums
+// are added in order.
+__global__ void __launch_bounds__(NT)
+wgrad_reduce(const WgReduce R, float* __restrict__ dw, float* __restrict__ db) {
+  __shared__ float sh[NT / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e = blockIdx.x * 32 + lane;
+  int l = 0;
+  while (l < 5 && e >= R.first[l + 1]) ++l;
+  const int k = e - R.first[l], n = R.nw[l] + R.nb[l];
+  float s = 0.0f;
+  if (e < R.first[6]) {
+    const float* q = R.part[l] + k;
+#pragma unroll 8
+    for (int i = warp; i < R.slots[l]; i += NT / 32) s += q[(size_t)i * n];
+  }
+  sh[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0 || e >= R.first[6]) return;
+#pragma unroll
+  for (int w = 1; w < NT / 32; ++w) s += sh[w][lane];
+  if (k < R.nw[l]) dw[R.off_w[l] + k] = s;
+  else db[R.off_b[l] + k - R.nw[l]] = s;
 }
 
 // transposed, flipped weights for the data gradient: wt[ci][co][8 - tap]
@@ -649,15 +837,36 @@ static int conv(const float* inA, int cin_a, const float* inB, int cin,
   return zb_launch_check();
 }
 
+// one layer's partial weight and bias gradients
 static int wgrad(const float* inA, int cin_a, const float* inB, int cin, const float* dout,
-                 int cout, float* dw, float* db, int B, int H, int W, cudaStream_t st,
+                 int cout, float* part, int B, int H, int W, cudaStream_t st,
                  int mode_a = SRC_DIRECT) {
-  dim3 grid((W + TS - 1) / TS, (H + TS - 1) / TS, B);
-  conv3x3_wgrad<<<grid, NTT, 0, st>>>(inA, cin_a, inB, cin, dout, cout, dw, db, B, H, W, mode_a);
+  const WgShape g = wg_shape(cin, cout, B, H, W);
+  static std::atomic<unsigned> attr{0u};
+  int dev = 0;
+  ZB_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 32 || g.smem > 227 * 1024) return ZB_E_UNSUPPORTED;
+  if (!(attr.load() & (1u << dev))) {
+    ZB_CUDA_TRY(cudaFuncSetAttribute(conv3x3_wgrad<WG_COT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     227 * 1024));
+    ZB_CUDA_TRY(cudaFuncSetAttribute(conv3x3_wgrad<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     227 * 1024));
+    attr.fetch_or(1u << dev);
+  }
+  const dim3 grid(g.slots, g.nchunk);
+  if (cout % WG_COT == 0)
+    conv3x3_wgrad<WG_COT><<<grid, g.threads, g.smem, st>>>(inA, cin_a, inB, cin, dout, cout, part, B, H,
+                                                      W, mode_a, g.ncog, g.cic, g.nsl);
+  else
+    conv3x3_wgrad<1><<<grid, g.threads, g.smem, st>>>(inA, cin_a, inB, cin, dout, cout, part, B, H,
+                                                      W, mode_a, g.ncog, g.cic, g.nsl);
   return zb_launch_check();
 }
 
 static int gridn(size_t n) { return (int)std::max<size_t>(1, std::min<size_t>((n + NT - 1) / NT, 148 * 16)); }
+
+// m1 and m2 run at half resolution
+static bool layer_half(int l) { return l == 2 || l == 3; }
 
 // activation buffers (floats) for a batch of B images H x W
 struct Acts {
@@ -665,6 +874,7 @@ struct Acts {
   // training: gradients and scratch
   float *d_e1, *d_e2, *d_p, *d_m1, *d_m2, *d_cat, *d_o1, *d_out, *res, *lnum, *lden, *tmp;
   __nv_bfloat16* wflip;
+  float* wpart[6];   // partial weight gradients of each layer
 };
 
 static size_t acts_floats(const Net& n, int B, int H, int W, bool train) {
@@ -676,6 +886,12 @@ static size_t acts_floats(const Net& n, int B, int H, int W, bool train) {
     f += 2 * (size_t)n.c1 * N0 + (size_t)n.c1 * N1 + 2 * (size_t)n.c2 * N1 +
          (size_t)(n.c1 + n.c2) * N0 + (size_t)n.c1 * N0 + N0 + N0 + 1024 +
          (size_t)n.c1 * N0 + (n.nw + 64);   // tmp + flipped weights (bf16 fits in floats)
+  if (train)
+    for (int l = 0; l < 6; ++l) {
+      const WgShape g = wg_shape(n.cin[l], n.cout[l], B, layer_half(l) ? H / 2 : H,
+                                 layer_half(l) ? W / 2 : W);
+      f += (size_t)g.slots * g.part;
+    }
   return f;
 }
 
@@ -707,6 +923,13 @@ static Acts acts_split(const Net& n, void* base, int B, int H, int W, bool train
     a.lden = f; f += 512;
     a.tmp = f; f += (size_t)n.c1 * N0;
     a.wflip = (__nv_bfloat16*)f;
+    f += n.nw + 64;
+    for (int l = 0; l < 6; ++l) {
+      const WgShape g = wg_shape(n.cin[l], n.cout[l], B, layer_half(l) ? H / 2 : H,
+                                 layer_half(l) ? W / 2 : W);
+      a.wpart[l] = f;
+      f += (size_t)g.slots * g.part;
+    }
   }
   return a;
 }
@@ -899,33 +1122,43 @@ int zb_unet_backward(const zb_unet_trainer* t, const float* r, const float* targ
     loss_grad_kernel<<<gridn(N0), NT, 0, st>>>(a.res, nullptr, cx, cy, a.lden, a.s, B, H, W, idx2,
                                                dx2, a.d_out);
   }
-  cudaMemsetAsync(t->g_w, 0, n.nw * sizeof(float), st);
-  cudaMemsetAsync(t->g_b, 0, n.nb * sizeof(float), st);
-  float* gw = t->g_w;
-  float* gb = t->g_b;
   // out = conv(o1)
-  if ((rc = wgrad(a.o1, n.c1, nullptr, n.c1, a.d_out, 1, gw + n.off_w[5], gb + n.off_b[5], B, H, W, st))) return rc;
+  if ((rc = wgrad(a.o1, n.c1, nullptr, n.c1, a.d_out, 1, a.wpart[5], B, H, W, st))) return rc;
   if ((rc = data_grad(n, 5, w, a.wflip, a.d_out, a.d_o1, B, H, W, st))) return rc;
   tanh_back<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_o1, a.o1, (size_t)n.c1 * N0);
   // o1 = tanh(conv([u, e2]))
-  if ((rc = wgrad(a.m2, n.c2, a.e2, n.c2 + n.c1, a.d_o1, n.c1, gw + n.off_w[4], gb + n.off_b[4], B, H, W, st, SRC_UP))) return rc;
+  if ((rc = wgrad(a.m2, n.c2, a.e2, n.c2 + n.c1, a.d_o1, n.c1, a.wpart[4], B, H, W, st, SRC_UP))) return rc;
   if ((rc = data_grad(n, 4, w, a.wflip, a.d_o1, a.d_cat, B, H, W, st))) return rc;
   // d_cat = [du (c2), de2_b (c1)]
   upsample2_back<<<gridn((size_t)n.c2 * N1), NT, 0, st>>>(a.d_cat, a.d_m2, n.c2, B, H, W);
   tanh_back<<<gridn((size_t)n.c2 * N1), NT, 0, st>>>(a.d_m2, a.m2, (size_t)n.c2 * N1);
-  if ((rc = wgrad(a.m1, n.c2, nullptr, n.c2, a.d_m2, n.c2, gw + n.off_w[3], gb + n.off_b[3], B, H1, W1, st))) return rc;
+  if ((rc = wgrad(a.m1, n.c2, nullptr, n.c2, a.d_m2, n.c2, a.wpart[3], B, H1, W1, st))) return rc;
   if ((rc = data_grad(n, 3, w, a.wflip, a.d_m2, a.d_m1, B, H1, W1, st))) return rc;
   tanh_back<<<gridn((size_t)n.c2 * N1), NT, 0, st>>>(a.d_m1, a.m1, (size_t)n.c2 * N1);
-  if ((rc = wgrad(a.e2, n.c1, nullptr, n.c1, a.d_m1, n.c2, gw + n.off_w[2], gb + n.off_b[2], B, H1, W1, st, SRC_POOL))) return rc;
+  if ((rc = wgrad(a.e2, n.c1, nullptr, n.c1, a.d_m1, n.c2, a.wpart[2], B, H1, W1, st, SRC_POOL))) return rc;
   if ((rc = data_grad(n, 2, w, a.wflip, a.d_m1, a.d_p, B, H1, W1, st))) return rc;
   avgpool2_back<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_p, a.d_e2, n.c1, B, H, W);
   add_inplace<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_e2, a.d_cat + (size_t)n.c2 * N0,
                                                        (size_t)n.c1 * N0);
   tanh_back<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_e2, a.e2, (size_t)n.c1 * N0);
-  if ((rc = wgrad(a.e1, n.c1, nullptr, n.c1, a.d_e2, n.c1, gw + n.off_w[1], gb + n.off_b[1], B, H, W, st))) return rc;
+  if ((rc = wgrad(a.e1, n.c1, nullptr, n.c1, a.d_e2, n.c1, a.wpart[1], B, H, W, st))) return rc;
   if ((rc = data_grad(n, 1, w, a.wflip, a.d_e2, a.d_e1, B, H, W, st))) return rc;
   tanh_back<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_e1, a.e1, (size_t)n.c1 * N0);
-  if ((rc = wgrad(a.in, 2, nullptr, 2, a.d_e1, n.c1, gw + n.off_w[0], gb + n.off_b[0], B, H, W, st))) return rc;
+  if ((rc = wgrad(a.in, 2, nullptr, 2, a.d_e1, n.c1, a.wpart[0], B, H, W, st))) return rc;
+  WgReduce R;
+  R.first[0] = 0;
+  for (int l = 0; l < 6; ++l) {
+    const WgShape g = wg_shape(n.cin[l], n.cout[l], B, layer_half(l) ? H1 : H,
+                               layer_half(l) ? W1 : W);
+    R.part[l] = a.wpart[l];
+    R.slots[l] = g.slots;
+    R.nb[l] = n.cout[l];
+    R.nw[l] = n.cout[l] * n.cin[l] * 9;
+    R.off_w[l] = (int)n.off_w[l];
+    R.off_b[l] = (int)n.off_b[l];
+    R.first[l + 1] = R.first[l] + R.nw[l] + R.nb[l];
+  }
+  wgrad_reduce<<<(R.first[6] + 31) / 32, NT, 0, st>>>(R, t->g_w, t->g_b);
   return zb_launch_check();
 }
 
