@@ -11,7 +11,7 @@
 //                     of both sides with the Audusse clip, hydrostatic-
 //                     reconstruction HLL / Rusanov, the cell-edge bed term;
 //                     writes the owner's and the neighbour's contribution
-//                     (6 planes over faces).  On the first stage it also
+//                     (5 planes over faces).  On the first stage it also
 //                     reduces the CFL dt over faces in float64.
 //   tri_update_kernel one thread per cell: gathers its three faces in a fixed
 //                     order (deterministic, no atomics, exactly conservative
@@ -19,6 +19,17 @@
 //                     applies the Shu-Osher update; the last stage adds
 //                     Manning friction and the troubled-cell flag.
 // Connectivity is int32 (C, F < 2^31); geometry SoA in the state precision.
+// What bounds it: memory, each pass moving 1.0-1.3x its own minimum (about 310
+// bytes per cell and stage over the three).  Slopes and momentum contributions
+// are stored as pairs (a scattered neighbour's 8 bytes fill its 32-byte sector
+// better than two 4-byte planes), the mesh arrays are read with the streaming
+// hint, so that what one pass hands the next stays in the L2, and every
+// neighbour gather of a thread is issued before the first is used.  980k cells,
+// float32, us per step: branches around the gathers, six contribution planes, b
+// copied per stage 176; gathers together 149; streaming hint 140; pairs 135.
+// One pass per stage with the slopes in shared memory moves half the bytes but
+// evaluates every face twice and waits on its block's outer neighbours: 180 us
+// a stage.
 #include <cstring>
 #include <algorithm>
 #include <type_traits>
@@ -30,6 +41,20 @@ namespace tri {
 
 constexpr int NT = 256;
 enum { MODE_STEP1 = 0, MODE_STEP2 = 1, MODE_EULER = 2, MODE_STAGE = 3 };
+
+// pairs: the two slope components of a variable, the two momentum
+// contributions of a face side
+template <typename T> struct Pair;
+template <> struct Pair<float> { using type = float2; };
+template <> struct Pair<double> { using type = double2; };
+template <typename T> using T2 = typename Pair<T>::type;
+template <typename T>
+__device__ __forceinline__ T2<T> pair(T x, T y) {
+  T2<T> r;
+  r.x = x;
+  r.y = y;
+  return r;
+}
 
 template <typename T>
 struct Geo {
@@ -83,15 +108,38 @@ __device__ __forceinline__ void to_w(T b, T h, T qx, T qy, T eps, T w[4], T& hin
 }
 
 // ── gradient + limiter ──────────────────────────────────────────────────────
+// The three neighbours' states are gathered together (a boundary side gathers
+// the cell itself and is mended after): with a branch around each gather they
+// came one after another, three memory latencies in a row.
 template <typename T, int RECON>
 __global__ void __launch_bounds__(NT)
-tri_grad_kernel(const T* __restrict__ Q, T* __restrict__ S, const Geo<T> geo,
-                const Prm<T> p, const unsigned char* __restrict__ force_o1) {
+tri_grad_kernel(const T* __restrict__ bP, const T* __restrict__ Q, T2<T>* __restrict__ S,
+                const Geo<T> geo, const Prm<T> p, const unsigned char* __restrict__ force_o1) {
   const int C = geo.C;
   const int c = blockIdx.x * NT + threadIdx.x;
   if (c >= C) return;
   const size_t Cs = (size_t)C;
-  const T bc_ = Q[c], hc = Q[Cs + c], qxc = Q[2 * Cs + c], qyc = Q[3 * Cs + c];
+  int idx[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) idx[k] = __ldcs(geo.lsq_idx + k * Cs + c);
+  const T bc_ = bP[c], hc = Q[Cs + c], qxc = Q[2 * Cs + c], qyc = Q[3 * Cs + c];
+  T qn[3][4];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int j = idx[k] >= 0 ? idx[k] : c;
+    qn[k][0] = bP[j];
+    qn[k][1] = Q[Cs + j];
+    qn[k][2] = Q[2 * Cs + j];
+    qn[k][3] = Q[3 * Cs + j];
+  }
+  T lx[3], ly[3], rx[3], ry[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    lx[k] = __ldcs(geo.lsq_wx + k * Cs + c);
+    ly[k] = __ldcs(geo.lsq_wy + k * Cs + c);
+    rx[k] = __ldcs(geo.cf_rx + k * Cs + c);
+    ry[k] = __ldcs(geo.cf_ry + k * Cs + c);
+  }
   T wc[4], hic;
   to_w<T, RECON>(bc_, hc, qxc, qyc, p.eps_kp, wc, hic);
   T d[3][4], gx[4], gy[4], umax[4], umin[4];
@@ -99,49 +147,33 @@ tri_grad_kernel(const T* __restrict__ Q, T* __restrict__ S, const Geo<T> geo,
   for (int v = 0; v < 4; ++v) { gx[v] = T(0); gy[v] = T(0); umax[v] = wc[v]; umin[v] = wc[v]; }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const int idx = geo.lsq_idx[k * Cs + c];
-    T wn[4];
-    T gb[4];   // value entering the bounds
-    if (idx >= 0) {
-      T hin;
-      to_w<T, RECON>(Q[idx], Q[Cs + idx], Q[2 * Cs + idx], Q[3 * Cs + idx], p.eps_kp, wn, hin);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) gb[v] = wn[v];
-    } else {
+    if (idx[k] < 0) {
       // boundary ghost: BC at the cell state (solver2/blocks.py:129-157); a
       // wall mirrors the normal momentum q - 2 (q.n) n
-      const int bf = -1 - idx;
-      const int kind = geo.bf_kind[bf];
-      T gqx = qxc, gqy = qyc;
-      if (kind == ZB_BC_WALL) {
+      const int bf = -1 - idx[k];
+      if (geo.bf_kind[bf] == ZB_BC_WALL) {
         const T nx = geo.bf_nx[bf], ny = geo.bf_ny[bf];
-        const T qn = qxc * nx + qyc * ny;
-        gqx = qxc - T(2) * qn * nx;
-        gqy = qyc - T(2) * qn * ny;
+        const T qd = qxc * nx + qyc * ny;
+        qn[k][2] = qxc - T(2) * qd * nx;
+        qn[k][3] = qyc - T(2) * qd * ny;
       }
-      T hg;
-      to_w<T, RECON>(bc_, hc, gqx, gqy, p.eps_kp, wn, hg);
-      // bounds see the ghost at 2 u_bf - u (reconstruction_jax.py:535-579)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) gb[v] = T(2) * wn[v] - wc[v];
     }
+    T wn[4], hin;
+    to_w<T, RECON>(qn[k][0], qn[k][1], qn[k][2], qn[k][3], p.eps_kp, wn, hin);
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
+      // the bounds see a ghost at 2 u_bf - u (reconstruction_jax.py:535-579)
+      const T gb = idx[k] >= 0 ? wn[v] : T(2) * wn[v] - wc[v];
       d[k][v] = wn[v] - wc[v];
-      umax[v] = fmx(umax[v], gb[v]);
-      umin[v] = fmn(umin[v], gb[v]);
+      umax[v] = fmx(umax[v], gb);
+      umin[v] = fmn(umin[v], gb);
     }
   }
   // gradient: weights are zero for a ghost not counted in a direction
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const T wx = geo.lsq_wx[k * Cs + c], wy = geo.lsq_wy[k * Cs + c];
+  for (int k = 0; k < 3; ++k)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) { gx[v] += wx * d[k][v]; gy[v] += wy * d[k][v]; }
-  }
-  T rx[3], ry[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) { rx[k] = geo.cf_rx[k * Cs + c]; ry[k] = geo.cf_ry[k * Cs + c]; }
+    for (int v = 0; v < 4; ++v) { gx[v] += lx[k] * d[k][v]; gy[v] += ly[k] * d[k][v]; }
   T phi[4];
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
@@ -172,10 +204,7 @@ tri_grad_kernel(const T* __restrict__ Q, T* __restrict__ S, const Geo<T> geo,
   }
   if (force_o1 != nullptr && force_o1[c]) phi[0] = phi[1] = phi[2] = phi[3] = T(0);
 #pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    S[(2 * v) * Cs + c] = phi[v] * gx[v];
-    S[(2 * v + 1) * Cs + c] = phi[v] * gy[v];
-  }
+  for (int v = 0; v < 4; ++v) S[v * Cs + c] = pair<T>(phi[v] * gx[v], phi[v] * gy[v]);
 }
 
 // ── face kernel ─────────────────────────────────────────────────────────────
@@ -185,18 +214,21 @@ struct Side {
 };
 
 template <typename T, int ORDER, int RECON>
-__device__ __forceinline__ void face_trace(const T* __restrict__ Q, const T* __restrict__ S,
+__device__ __forceinline__ void face_trace(const T* __restrict__ bP, const T* __restrict__ Q,
+                                           const T2<T>* __restrict__ S,
                                            int c, size_t Cs, T rx, T ry, T eps,
                                            Side<T>& sd, T& hc, T& bcell) {
-  const T b = Q[c], h = Q[Cs + c], qx = Q[2 * Cs + c], qy = Q[3 * Cs + c];
+  const T b = bP[c], h = Q[Cs + c], qx = Q[2 * Cs + c], qy = Q[3 * Cs + c];
   hc = h;
   bcell = b;
   T w[4], hinv;
   to_w<T, RECON>(b, h, qx, qy, eps, w, hinv);
   if (ORDER >= 2) {
 #pragma unroll
-    for (int v = 0; v < 4; ++v)
-      w[v] = w[v] + (S[(2 * v) * Cs + c] * rx + S[(2 * v + 1) * Cs + c] * ry);
+    for (int v = 0; v < 4; ++v) {
+      const T2<T> g = S[v * Cs + c];
+      w[v] = w[v] + (g.x * rx + g.y * ry);
+    }
   }
   sd.b = w[0];
   if (RECON == ZB_RECON_ETA) {
@@ -264,9 +296,13 @@ __device__ __forceinline__ void riemann_n(const Side<T>& L, const Side<T>& R, T 
   Dp = -(half * g * (R.h * R.h - hRs * hRs));
 }
 
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 template <typename T, int ORDER, int RECON, int RIEMANN, bool DT>
 __global__ void __launch_bounds__(NT)
-tri_face_kernel(const T* __restrict__ Q, const T* __restrict__ S, T* __restrict__ Fc,
+tri_face_kernel(const T* __restrict__ bP, const T* __restrict__ Q,
+                const T2<T>* __restrict__ S, T2<T>* __restrict__ Fc, T* __restrict__ Fm,
                 const Geo<T> geo, const Prm<T> p, double* dt_slot, unsigned* status) {
   __shared__ double red[NT / 32];
   const int F = geo.F;
@@ -274,15 +310,18 @@ tri_face_kernel(const T* __restrict__ Q, const T* __restrict__ S, T* __restrict_
   const int f = blockIdx.x * NT + threadIdx.x;
   double loc = INFINITY;
   if (f < F) {
-    const int a = geo.face_a[f], bcode = geo.face_b[f];
-    const T nx = geo.face_nx[f], ny = geo.face_ny[f];
+    const int a = __ldcs(geo.face_a + f), bcode = __ldcs(geo.face_b + f);
+    const T nx = __ldcs(geo.face_nx + f), ny = __ldcs(geo.face_ny + f);
+    // both sides' gathers together: a boundary face gathers its owner twice and
+    // takes the boundary state after
+    const int nb = bcode >= 0 ? bcode : a;
     Side<T> A, B;
     T hA, bA, hB, bB;
-    face_trace<T, ORDER, RECON>(Q, S, a, Cs, geo.face_rax[f], geo.face_ray[f], p.eps_kp, A, hA, bA);
-    if (bcode >= 0) {
-      face_trace<T, ORDER, RECON>(Q, S, bcode, Cs, geo.face_rbx[f], geo.face_rby[f], p.eps_kp, B,
-                                  hB, bB);
-    } else {
+    const T rax = __ldcs(geo.face_rax + f), ray = __ldcs(geo.face_ray + f);
+    const T rbx = __ldcs(geo.face_rbx + f), rby = __ldcs(geo.face_rby + f);
+    face_trace<T, ORDER, RECON>(bP, Q, S, a, Cs, rax, ray, p.eps_kp, A, hA, bA);
+    face_trace<T, ORDER, RECON>(bP, Q, S, nb, Cs, rbx, rby, p.eps_kp, B, hB, bB);
+    if (bcode < 0) {
       // boundary: Q_R = BC(Q_L) at the reconstructed face state
       // (solver_jax.py:827-858)
       B = A;
@@ -305,24 +344,23 @@ tri_face_kernel(const T* __restrict__ Q, const T* __restrict__ S, T* __restrict_
       gA = T(0.5) * p.g * (hA + A.h) * (A.b - bA);
       gB = T(0.5) * p.g * (hB + B.h) * (B.b - bB);
     }
-    // owner: F + (Dm + gA) n ; neighbour: -F + (Dp - gB) n
-    Fc[0 * Fs + f] = Fh;
-    Fc[1 * Fs + f] = Fx + (Dm + gA) * nx;
-    Fc[2 * Fs + f] = Fy + (Dm + gA) * ny;
-    Fc[3 * Fs + f] = -Fh;
-    Fc[4 * Fs + f] = -Fx + (Dp - gB) * nx;
-    Fc[5 * Fs + f] = -Fy + (Dp - gB) * ny;
+    // owner: F + (Dm + gA) n ; neighbour: -F + (Dp - gB) n; the mass flux is
+    // one plane for both
+    Fm[f] = Fh;
+    Fc[f] = pair<T>(Fx + (Dm + gA) * nx, Fy + (Dm + gA) * ny);
+    Fc[Fs + f] = pair<T>(-Fx + (Dp - gB) * nx, -Fy + (Dp - gB) * ny);
     if (DT) {
       // CFL law over faces at the CELL states, owner on both sides of a
       // boundary face (solver2/blocks.py:36-95, context.py:111-117)
-      const int bc2 = bcode >= 0 ? bcode : a;
-      const T hia = kp_hinv(Q[Cs + a], p.eps_kp), hib = kp_hinv(Q[Cs + bc2], p.eps_kp);
+      const T hia = kp_hinv(Q[Cs + a], p.eps_kp), hib = kp_hinv(Q[Cs + nb], p.eps_kp);
       const T lA = fabs(Q[2 * Cs + a] * hia * nx + Q[3 * Cs + a] * hia * ny) +
                    sqrt(p.g * fmx(Q[Cs + a], T(0)));
-      const T lB = fabs(Q[2 * Cs + bc2] * hib * nx + Q[3 * Cs + bc2] * hib * ny) +
-                   sqrt(p.g * fmx(Q[Cs + bc2], T(0)));
+      // (the neighbour's products rounded on their own: shared with its trace
+      // they would take that one's fused multiply-adds apart)
+      const T lB = fabs(mul_rn(Q[2 * Cs + nb], hib) * nx + mul_rn(Q[3 * Cs + nb], hib) * ny) +
+                   sqrt(p.g * fmx(Q[Cs + nb], T(0)));
       const double am = (double)nmax(lA, lB);
-      loc = (p.cfl2 * geo.face_inr[f]) / (p.den_fac * am);
+      loc = (p.cfl2 * __ldcs(geo.face_inr + f)) / (p.den_fac * am);
       if (loc != loc) loc = -1.0;   // non-finite state: poison the minimum
     }
   }
@@ -350,8 +388,8 @@ tri_face_kernel(const T* __restrict__ Q, const T* __restrict__ S, T* __restrict_
 // ── cell update ─────────────────────────────────────────────────────────────
 template <typename T, int MODE>
 __global__ void __launch_bounds__(NT)
-tri_update_kernel(const T* __restrict__ Qk, const T* Q0, T* Qo, const T* __restrict__ Fc,
-                  const Geo<T> geo, const Prm<T> p, zb_ctrl* ctrl, int phase,
+tri_update_kernel(const T* __restrict__ Qk, const T* Q0, T* Qo, const T2<T>* __restrict__ Fc,
+                  const T* __restrict__ Fm, const Geo<T> geo, const Prm<T> p, zb_ctrl* ctrl, int phase,
                   const T* __restrict__ hinv_src, unsigned char* __restrict__ trouble_out) {
   const int C = geo.C;
   const size_t Cs = (size_t)C, Fs = (size_t)geo.F;
@@ -376,14 +414,17 @@ tri_update_kernel(const T* __restrict__ Qk, const T* Q0, T* Qo, const T* __restr
   if (c >= C) return;
   const T dtT = T(dtd);
   T dq[3] = {T(0), T(0), T(0)};
-  const T ia = geo.cell_inv_area[c];
+  const T ia = __ldcs(geo.cell_inv_area + c);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const int code = geo.cell_face[k * Cs + c];
+    const int code = __ldcs(geo.cell_face + k * Cs + c);
     const int f = code >> 1, side = code & 1;
     const T lw = geo.face_len[f] * ia;
-#pragma unroll
-    for (int v = 0; v < 3; ++v) dq[v] -= lw * Fc[(3 * side + v) * Fs + f];
+    const T fh = Fm[f];
+    const T2<T> fq = Fc[side * Fs + f];
+    dq[0] -= lw * (side ? -fh : fh);
+    dq[1] -= lw * fq.x;
+    dq[2] -= lw * fq.y;
   }
   const T hk = Qk[Cs + c], qxk = Qk[2 * Cs + c], qyk = Qk[3 * Cs + c];
   T hn, qxn, qyn;
@@ -528,9 +569,9 @@ tri_aux_kernel(const T* __restrict__ Q, T* __restrict__ A, const Geo<T> geo, T e
   T g[4][2] = {{T(0), T(0)}, {T(0), T(0)}, {T(0), T(0)}, {T(0), T(0)}};
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const int idx = geo.lsq_idx[k * Cs + c];
+    const int idx = __ldcs(geo.lsq_idx + k * Cs + c);
     if (idx < 0) continue;
-    const T wx = geo.lsq_wx[k * Cs + c], wy = geo.lsq_wy[k * Cs + c];
+    const T wx = __ldcs(geo.lsq_wx + k * Cs + c), wy = __ldcs(geo.lsq_wy + k * Cs + c);
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       const T d = Q[v * Cs + idx] - Q[v * Cs + c];
@@ -622,35 +663,35 @@ static Prm<T> make_prm(const zb_tri_cfg* c, double alpha, double beta, double dt
 }
 
 template <typename T, int ORDER, int RECON, int RIEMANN>
-static int stage(const zb_tri_cfg* cfg, const Geo<T>& geo, const Prm<T>& p, const T* Qk,
-                 const T* Q0, T* Qo, T* S, T* Fc, zb_ctrl* ctrl, int phase, int mode,
+static int stage(const Geo<T>& geo, const Prm<T>& p, const T* bP, const T* Qk,
+                 const T* Q0, T* Qo, T2<T>* S, T2<T>* Fc, T* Fm, zb_ctrl* ctrl, int phase, int mode,
                  const T* hinv_src, const unsigned char* force_o1, unsigned char* trouble,
                  cudaStream_t st) {
   const int gc = (geo.C + NT - 1) / NT, gf = (geo.F + NT - 1) / NT;
-  if (ORDER >= 2) tri_grad_kernel<T, RECON><<<gc, NT, 0, st>>>(Qk, S, geo, p, force_o1);
+  if (ORDER >= 2) tri_grad_kernel<T, RECON><<<gc, NT, 0, st>>>(bP, Qk, S, geo, p, force_o1);
   const bool dt = mode == MODE_STEP1 || mode == MODE_EULER;
   double* slot = &ctrl->amax[phase < 3 ? phase : 0];
   if (dt)
     tri_face_kernel<T, ORDER, RECON, RIEMANN, true>
-        <<<gf, NT, 0, st>>>(Qk, S, Fc, geo, p, slot, &ctrl->status);
+        <<<gf, NT, 0, st>>>(bP, Qk, S, Fc, Fm, geo, p, slot, &ctrl->status);
   else
     tri_face_kernel<T, ORDER, RECON, RIEMANN, false>
-        <<<gf, NT, 0, st>>>(Qk, S, Fc, geo, p, slot, &ctrl->status);
+        <<<gf, NT, 0, st>>>(bP, Qk, S, Fc, Fm, geo, p, slot, &ctrl->status);
   switch (mode) {
     case MODE_STEP1:
-      tri_update_kernel<T, MODE_STEP1><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, geo, p, ctrl, phase,
+      tri_update_kernel<T, MODE_STEP1><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, Fm, geo, p, ctrl, phase,
                                                            hinv_src, trouble);
       break;
     case MODE_STEP2:
-      tri_update_kernel<T, MODE_STEP2><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, geo, p, ctrl, phase,
+      tri_update_kernel<T, MODE_STEP2><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, Fm, geo, p, ctrl, phase,
                                                            hinv_src, trouble);
       break;
     case MODE_EULER:
-      tri_update_kernel<T, MODE_EULER><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, geo, p, ctrl, phase,
+      tri_update_kernel<T, MODE_EULER><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, Fm, geo, p, ctrl, phase,
                                                            hinv_src, trouble);
       break;
     default:
-      tri_update_kernel<T, MODE_STAGE><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, geo, p, ctrl, phase,
+      tri_update_kernel<T, MODE_STAGE><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, Fm, geo, p, ctrl, phase,
                                                            hinv_src, trouble);
   }
   return zb_launch_check();
@@ -673,40 +714,42 @@ static int dispatch(const zb_tri_cfg* c, Fn&& f) {
   return ZB_E_UNSUPPORTED;
 }
 
-// workspace layout (elements of T): Q1 (4 planes, b unused), slopes (8
-// planes over cells), face contributions (6 planes over faces)
+// workspace (from its first 16-byte boundary): Q1 (4 planes, b unused), slopes
+// (4 planes of pairs over cells), face contributions (2 planes of pairs and one
+// plane over faces)
 template <typename T>
-static void ws_split(const zb_tri_mesh* m, void* ws, T** Q1, T** S, T** Fc) {
-  T* base = (T*)ws;
-  const size_t C = (size_t)m->n_cells, F = (size_t)m->n_faces;
-  *Q1 = base;
-  *S = base + 4 * C;
-  *Fc = base + 12 * C;
-  (void)F;
-}
+struct Work {
+  T *Q1, *Fm;
+  T2<T> *S, *Fc;
+  Work(const zb_tri_mesh* m, void* ws) {
+    T* base = (T*)(((uintptr_t)ws + 15u) & ~(uintptr_t)15u);
+    const size_t C = (size_t)m->n_cells, F = (size_t)m->n_faces;
+    Q1 = base;
+    S = (T2<T>*)(base + 4 * C);
+    Fc = (T2<T>*)(base + 12 * C);
+    Fm = base + 12 * C + 4 * F;
+  }
+};
 
 template <typename T, int ORDER, int RECON, int RIEMANN>
 static int run_step(const zb_tri_cfg* cfg, const zb_tri_mesh* m, T* Q, void* ws,
                     zb_ctrl* ctrl, int phase, cudaStream_t st) {
   const Geo<T> geo = make_geo<T>(m);
   const Prm<T> p = make_prm<T>(cfg, 0.0, 1.0, -1.0);
-  T *Q1, *S, *Fc;
-  ws_split<T>(m, ws, &Q1, &S, &Fc);
+  const Work<T> w(m, ws);
   const size_t C = (size_t)m->n_cells;
   if constexpr (ORDER == 1) {
-    int rc = stage<T, ORDER, RECON, RIEMANN>(cfg, geo, p, Q, Q, Q1, S, Fc, ctrl, phase,
+    int rc = stage<T, ORDER, RECON, RIEMANN>(geo, p, Q, Q, Q, w.Q1, w.S, w.Fc, w.Fm, ctrl, phase,
                                              MODE_EULER, nullptr, nullptr, nullptr, st);
     if (rc) return rc;
-    ZB_CUDA_TRY(cudaMemcpyAsync(Q + C, Q1 + C, 3 * C * sizeof(T), cudaMemcpyDeviceToDevice, st));
+    ZB_CUDA_TRY(cudaMemcpyAsync(Q + C, w.Q1 + C, 3 * C * sizeof(T), cudaMemcpyDeviceToDevice, st));
     return ZB_OK;
   } else {
-    // stage 1 reads the b plane of Q through Qk = Q; the stage-1 state Q1
-    // holds h, qx, qy in planes 1..3 and Q's b plane is copied once per step
-    ZB_CUDA_TRY(cudaMemcpyAsync(Q1, Q, C * sizeof(T), cudaMemcpyDeviceToDevice, st));
-    int rc = stage<T, ORDER, RECON, RIEMANN>(cfg, geo, p, Q, Q, Q1, S, Fc, ctrl, phase,
+    // both stages read b from Q; the stage-1 state Q1 holds h, qx, qy in planes 1..3
+    int rc = stage<T, ORDER, RECON, RIEMANN>(geo, p, Q, Q, Q, w.Q1, w.S, w.Fc, w.Fm, ctrl, phase,
                                              MODE_STEP1, nullptr, nullptr, nullptr, st);
     if (rc) return rc;
-    return stage<T, ORDER, RECON, RIEMANN>(cfg, geo, p, Q1, Q, Q, S, Fc, ctrl, phase, MODE_STEP2,
+    return stage<T, ORDER, RECON, RIEMANN>(geo, p, Q, w.Q1, Q, Q, w.S, w.Fc, w.Fm, ctrl, phase, MODE_STEP2,
                                            nullptr, nullptr, nullptr, st);
   }
 }
@@ -760,10 +803,9 @@ int zb_tri_stage(const zb_tri_cfg* cfg, const zb_tri_mesh* mesh, const void* Qk,
     using T = decltype(tag);
     const Geo<T> geo = make_geo<T>(mesh);
     const Prm<T> p = make_prm<T>(cfg, alpha, beta, dt);
-    T *Q1, *S, *Fc;
-    ws_split<T>(mesh, workspace, &Q1, &S, &Fc);
+    const Work<T> w(mesh, workspace);
     return stage<T, decltype(O)::value, decltype(R)::value, decltype(M)::value>(
-        cfg, geo, p, (const T*)Qk, (const T*)Q0, (T*)Q_out, S, Fc, ctrl, 0, MODE_STAGE,
+        geo, p, (const T*)Qk, (const T*)Qk, (const T*)Q0, (T*)Q_out, w.S, w.Fc, w.Fm, ctrl, 0, MODE_STAGE,
         (const T*)hinv_src, force_o1, trouble_out, st);
   };
   if (cfg->dtype == ZB_F32)
@@ -783,11 +825,11 @@ int zb_tri_dt(const zb_tri_cfg* cfg, const zb_tri_mesh* mesh, const void* Q, voi
     using T = decltype(tag);
     const Geo<T> geo = make_geo<T>(mesh);
     Prm<T> p = make_prm<T>(cfg, 0.0, 1.0, -1.0);
-    T *Q1, *S, *Fc;
-    ws_split<T>(mesh, workspace, &Q1, &S, &Fc);
+    const Work<T> w(mesh, workspace);
     const int gf = (geo.F + NT - 1) / NT;
     tri_face_kernel<T, 1, ZB_RECON_CONSTANT, ZB_RIEMANN_RUSANOV_HR, true>
-        <<<gf, NT, 0, st>>>((const T*)Q, S, Fc, geo, p, &ctrl->reserved[0], &ctrl->status);
+        <<<gf, NT, 0, st>>>((const T*)Q, (const T*)Q, w.S, w.Fc, w.Fm, geo, p, &ctrl->reserved[0],
+                            &ctrl->status);
     return zb_launch_check();
   };
   int rc = cfg->dtype == ZB_F32 ? go(float()) : go(double());
