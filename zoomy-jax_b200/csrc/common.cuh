@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
+#include <utility>
 
 #include "zb.h"
 
@@ -145,6 +146,38 @@ __device__ __forceinline__ double block_max_double(double v, double* sh) {
     v = w;
   }
   return v;  // valid in thread 0
+}
+
+// Programmatic dependent launch: the kernels of a step, of a solve iteration and
+// of the V-cycle are launched with programmatic stream serialisation, so the next
+// kernel's launch overlaps the tail of this one.  Each of them first waits for
+// its predecessor's completion and memory (griddepcontrol.wait, before any
+// global read or write), then lets its own successor launch; launched without
+// the attribute, both instructions are no-ops.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... KArgs, typename... Args>
+static inline cudaError_t pdl_launch(void (*k)(KArgs...), dim3 g, dim3 b, size_t sm, cudaStream_t st,
+                              Args&&... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = g;
+  c.blockDim = b;
+  c.dynamicSmemBytes = sm;
+  c.stream = st;
+  cudaLaunchAttribute a[1];
+  a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = a;
+  // only on launches outside stream capture: inside the FCG graph's
+  // conditional body the programmatic edges measured slower than plain ones
+  // (1024^2 pressure solve, 8 iterations: 1.655 ms against 1.628 ms)
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusNone;
+  c.numAttrs = cs == cudaStreamCaptureStatusNone ? 1 : 0;
+  return cudaLaunchKernelEx(&c, k, std::forward<Args>(args)...);
 }
 
 }  // namespace zb

@@ -1179,6 +1179,7 @@ swe2d_strip_kernel(const T* __restrict__ bP, const T* __restrict__ hP,
       return;
     full_items(p.nx, p.ny, item, &strip, &r0, &r1, &kind, p.sxc, p.sx);
   }
+  pdl_enter();
   if (kind)
     strip_item<T, RECON, RIEMANN, MODE, true, false>(
         bP, hP, qxP, qyP, h0P, qx0P, qy0P, hO, qxO, qyO, ctrl, phase, p, strip, r0, r1, lead,
@@ -1241,6 +1242,7 @@ ens_strip_kernel(const EnsDesc<T>* __restrict__ desc, const int4* __restrict__ i
   for (int k = lane; k < (int)(sizeof(SweParams<T>) / 4); k += 32)
     ((int*)&par[warp])[k] = ((const int*)&d->p)[k];
   __syncwarp();
+  pdl_enter();
   const volatile SweParams<T>& p = par[warp];
   T* q = Q + d->q_off;
   T* ws = W + d->ws_off;
@@ -1640,9 +1642,9 @@ static int launch_strips(const zb_swe2d_cfg* c, const T* b, const T* h, const T*
                                       p.sx);
   const int wpb = STRIP_NT / 32;
   auto go = [&](auto bed) -> int {
-    swe2d_strip_kernel<T, RECON, RIEMANN, MODE, decltype(bed)::value>
-        <<<(n + wpb - 1) / wpb, STRIP_NT, 0, st>>>(b, h, qx, qy, h0, qx0, qy0, ho, qxo, qyo, ctrl,
-                                                   phase, hinv_src, force_o1, trouble_out, p);
+    ZB_CUDA_TRY(pdl_launch(swe2d_strip_kernel<T, RECON, RIEMANN, MODE, decltype(bed)::value>,
+                           dim3((n + wpb - 1) / wpb), dim3(STRIP_NT), 0, st, b, h, qx, qy, h0, qx0,
+                           qy0, ho, qxo, qyo, ctrl, phase, hinv_src, force_o1, trouble_out, p));
     return zb_launch_check();
   };
   if constexpr (RECON == ZB_RECON_ETA && RIEMANN == ZB_RIEMANN_HLL_HR && MODE != MODE_STAGE)
@@ -1821,11 +1823,11 @@ static int ens_launch(int part, const void* table, int n_inst, int n_items, void
   const int4* items = (const int4*)((const char*)table + ens_desc_bytes<T>(n_inst));
   const int sgrid = (n_items + STRIP_NT / 32 - 1) / (STRIP_NT / 32);
   if (part == 0)
-    ens_strip_kernel<T, MODE_STEP1><<<sgrid, STRIP_NT, 0, st>>>(desc, items, (T*)Q, (T*)W, ctrls,
-                                                               phase);
+    ZB_CUDA_TRY(pdl_launch(ens_strip_kernel<T, MODE_STEP1>, dim3(sgrid), dim3(STRIP_NT), 0, st, desc,
+                           items, (T*)Q, (T*)W, ctrls, phase));
   else
-    ens_strip_kernel<T, MODE_STEP2><<<sgrid, STRIP_NT, 0, st>>>(desc, items, (T*)Q, (T*)W, ctrls,
-                                                               phase);
+    ZB_CUDA_TRY(pdl_launch(ens_strip_kernel<T, MODE_STEP2>, dim3(sgrid), dim3(STRIP_NT), 0, st, desc,
+                           items, (T*)Q, (T*)W, ctrls, phase));
   return zb_launch_check();
 }
 

@@ -115,6 +115,7 @@ template <typename T, int RECON>
 __global__ void __launch_bounds__(NT)
 tri_grad_kernel(const T* __restrict__ bP, const T* __restrict__ Q, T2<T>* __restrict__ S,
                 const Geo<T> geo, const Prm<T> p, const unsigned char* __restrict__ force_o1) {
+  pdl_enter();
   const int C = geo.C;
   const int c = blockIdx.x * NT + threadIdx.x;
   if (c >= C) return;
@@ -304,6 +305,7 @@ __global__ void __launch_bounds__(NT)
 tri_face_kernel(const T* __restrict__ bP, const T* __restrict__ Q,
                 const T2<T>* __restrict__ S, T2<T>* __restrict__ Fc, T* __restrict__ Fm,
                 const Geo<T> geo, const Prm<T> p, double* dt_slot, unsigned* status) {
+  pdl_enter();
   __shared__ double red[NT / 32];
   const int F = geo.F;
   const size_t Cs = (size_t)geo.C, Fs = (size_t)F;
@@ -391,6 +393,7 @@ __global__ void __launch_bounds__(NT)
 tri_update_kernel(const T* __restrict__ Qk, const T* Q0, T* Qo, const T2<T>* __restrict__ Fc,
                   const T* __restrict__ Fm, const Geo<T> geo, const Prm<T> p, zb_ctrl* ctrl, int phase,
                   const T* __restrict__ hinv_src, unsigned char* __restrict__ trouble_out) {
+  pdl_enter();
   const int C = geo.C;
   const size_t Cs = (size_t)C, Fs = (size_t)geo.F;
   const int c = blockIdx.x * NT + threadIdx.x;
@@ -668,31 +671,37 @@ static int stage(const Geo<T>& geo, const Prm<T>& p, const T* bP, const T* Qk,
                  const T* hinv_src, const unsigned char* force_o1, unsigned char* trouble,
                  cudaStream_t st) {
   const int gc = (geo.C + NT - 1) / NT, gf = (geo.F + NT - 1) / NT;
-  if (ORDER >= 2) tri_grad_kernel<T, RECON><<<gc, NT, 0, st>>>(bP, Qk, S, geo, p, force_o1);
+  const dim3 bc(gc), bf(gf), nt(NT);
+  if (ORDER >= 2)
+    ZB_CUDA_TRY(pdl_launch(tri_grad_kernel<T, RECON>, bc, nt, 0, st, bP, Qk, S, geo, p, force_o1));
   const bool dt = mode == MODE_STEP1 || mode == MODE_EULER;
   double* slot = &ctrl->amax[phase < 3 ? phase : 0];
   if (dt)
-    tri_face_kernel<T, ORDER, RECON, RIEMANN, true>
-        <<<gf, NT, 0, st>>>(bP, Qk, S, Fc, Fm, geo, p, slot, &ctrl->status);
+    ZB_CUDA_TRY(pdl_launch(tri_face_kernel<T, ORDER, RECON, RIEMANN, true>, bf, nt, 0, st, bP, Qk,
+                           (const T2<T>*)S, Fc, Fm, geo, p, slot, &ctrl->status));
   else
-    tri_face_kernel<T, ORDER, RECON, RIEMANN, false>
-        <<<gf, NT, 0, st>>>(bP, Qk, S, Fc, Fm, geo, p, slot, &ctrl->status);
+    ZB_CUDA_TRY(pdl_launch(tri_face_kernel<T, ORDER, RECON, RIEMANN, false>, bf, nt, 0, st, bP, Qk,
+                           (const T2<T>*)S, Fc, Fm, geo, p, slot, &ctrl->status));
   switch (mode) {
     case MODE_STEP1:
-      tri_update_kernel<T, MODE_STEP1><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, Fm, geo, p, ctrl, phase,
-                                                           hinv_src, trouble);
+      ZB_CUDA_TRY(pdl_launch(tri_update_kernel<T, MODE_STEP1>, bc, nt, 0, st, Qk, Q0, Qo,
+                             (const T2<T>*)Fc, (const T*)Fm, geo, p, ctrl, phase, hinv_src,
+                             trouble));
       break;
     case MODE_STEP2:
-      tri_update_kernel<T, MODE_STEP2><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, Fm, geo, p, ctrl, phase,
-                                                           hinv_src, trouble);
+      ZB_CUDA_TRY(pdl_launch(tri_update_kernel<T, MODE_STEP2>, bc, nt, 0, st, Qk, Q0, Qo,
+                             (const T2<T>*)Fc, (const T*)Fm, geo, p, ctrl, phase, hinv_src,
+                             trouble));
       break;
     case MODE_EULER:
-      tri_update_kernel<T, MODE_EULER><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, Fm, geo, p, ctrl, phase,
-                                                           hinv_src, trouble);
+      ZB_CUDA_TRY(pdl_launch(tri_update_kernel<T, MODE_EULER>, bc, nt, 0, st, Qk, Q0, Qo,
+                             (const T2<T>*)Fc, (const T*)Fm, geo, p, ctrl, phase, hinv_src,
+                             trouble));
       break;
     default:
-      tri_update_kernel<T, MODE_STAGE><<<gc, NT, 0, st>>>(Qk, Q0, Qo, Fc, Fm, geo, p, ctrl, phase,
-                                                           hinv_src, trouble);
+      ZB_CUDA_TRY(pdl_launch(tri_update_kernel<T, MODE_STAGE>, bc, nt, 0, st, Qk, Q0, Qo,
+                             (const T2<T>*)Fc, (const T*)Fm, geo, p, ctrl, phase, hinv_src,
+                             trouble));
   }
   return zb_launch_check();
 }
