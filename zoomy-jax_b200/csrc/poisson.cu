@@ -37,6 +37,7 @@ constexpr int NT = 256;
 constexpr int MAXL = 16;
 constexpr int SMALL = 32;        // levels with nx, ny <= SMALL go to the one-CTA kernel
 constexpr int RED_BLOCKS = 592;  // 148 SMs x 4
+constexpr int MG_PARTS = 4096;   // partials of z.q that a level-0 launch on strips may leave
 constexpr int DENSE_MAX_CELLS = 64;   // coarsest levels this small are solved exactly
 
 struct Level {
@@ -117,7 +118,7 @@ static Plan make_plan(const zb_poisson_cfg* c) {
   P.vr = d; d += C;
   P.vp = d; d += C;
   P.vq = d; d += C;
-  P.part = d; d += 4 * RED_BLOCKS;
+  P.part = d; d += 3 * RED_BLOCKS + std::max(RED_BLOCKS, MG_PARTS);   // p.q, p.r, r.r; z.q
   P.scal = d; d += S_COUNT;
   P.fbase = ((d * 8 + 255) / 256) * 256;
   P.bytes = P.fbase + f * 4 + 256;
@@ -167,6 +168,7 @@ setup0_kernel(const T* __restrict__ h, int nx, int ny, double cmin, double cmax,
               float idx2f, double* __restrict__ cx64, double* __restrict__ cy64,
               double* __restrict__ dg64, float* __restrict__ cx32, float* __restrict__ cy32,
               float* __restrict__ idg32) {
+  pdl_enter();
   for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < (long long)nx * ny;
        k += (long long)gridDim.x * NT) {
     const int i = (int)(k / ny), j = (int)(k - (long long)i * ny);
@@ -211,6 +213,7 @@ __global__ void __launch_bounds__(NT)
 coarsen_kernel(const float* __restrict__ cxf, const float* __restrict__ cyf, int nxc, int nyc,
                float idx2, float* __restrict__ cxc, float* __restrict__ cyc,
                float* __restrict__ idg) {
+  pdl_enter();
   for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < (long long)nxc * nyc;
        k += (long long)gridDim.x * NT) {
     const int I = (int)(k / nyc), J = (int)(k - (long long)I * nyc);
@@ -235,114 +238,143 @@ __device__ __forceinline__ void block_sum(double v, double* red, double* out) {
   }
 }
 
-// Grid-wide finish of a two-stage reduction without another launch: every
-// block has stored its partial sums; the last block to arrive (a counter in
-// the workspace) adds the partials in a fixed order -- the same order and
-// arithmetic as a separate reduction kernel, so the result is deterministic --
-// derives the FCG scalar and re-arms the counter.  No block waits on another.
-enum { FIN_NONE = 0, FIN_REL = 1, FIN_ALPHA = 2, FIN_BETA = 3 };
-
-__device__ void finish_scalars(const double* part_a, const double* part_b, unsigned* counter,
-                               double* scal, int dst_a, int dst_b, int what, double* red) {
-  __shared__ bool last;
-  __threadfence();
+// Two-stage reductions without a launch or a tail of their own: a kernel leaves
+// one partial sum per block, and every block of the kernel that needs the scalar
+// adds them itself, all in the same fixed order, so all get the same bits.  (A
+// last block adding them at the producer's end cost each kernel of an iteration
+// 3 us.)  These kernels are bound by the latency of their loads (1024^2 vectors
+// sit in L2), so a thread has two to four cells' loads in flight.  1024^2, us:
+// A p 17 -> 13, x and r 15 -> 12.9, z.q 9.4 -> in the V-cycle's last launch,
+// p 5.8 -> 8.2 (it adds the partials now); the four 47 -> 40.
+__device__ __forceinline__ double sum_parts(const double* part, int n, double* red) {
+  double s = 0.0;
+  for (int k = threadIdx.x; k < n; k += NT) s += __ldcg(part + k);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __syncthreads();   // red is free
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double sa = 0.0, sb = 0.0;
-  for (int k = threadIdx.x; k < (int)gridDim.x; k += NT) {
-    sa += __ldcg(part_a + k);
-    if (part_b) sb += __ldcg(part_b + k);
-  }
-  block_sum(sa, red, &scal[dst_a]);
-  __syncthreads();
-  if (part_b) block_sum(sb, red, &scal[dst_b]);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (what == FIN_REL) {
-      scal[S_REL] = sqrt(scal[S_RR] / scal[S_BB]);
-    } else if (what == FIN_ALPHA) {
-      const double pq = scal[S_PQ];
-      scal[S_ALPHA] = pq != 0.0 ? scal[S_PR] / pq : 0.0;
-    } else if (what == FIN_BETA) {
-      const double pq = scal[S_PQ];
-      scal[S_BETA] = pq != 0.0 ? scal[S_ZQ] / pq : 0.0;
-    }
-    *counter = 0u;
-  }
+  double t = red[0];
+#pragma unroll
+  for (int w = 1; w < NT / 32; ++w) t += red[w];
+  return t;          // in every thread
 }
+
+// (A p)_k of the float64 operator; the four neighbours are loaded before any is
+// used (beyond a wall the cell itself, whose Dirichlet ghost is -p_k)
+__device__ __forceinline__ double apply64(const double* __restrict__ cx,
+                                          const double* __restrict__ cy,
+                                          const double* __restrict__ p, unsigned nx, unsigned ny,
+                                          unsigned k, double pc, double idx2) {
+  const unsigned i = k / ny, j = k - i * ny;
+  const bool e = i + 1 < nx, w = i > 0, n = j + 1 < ny, s = j > 0;
+  const double pe = p[e ? k + ny : k], pw = p[w ? k - ny : k];
+  const double pn = p[n ? k + 1 : k], ps = p[s ? k - 1 : k];
+  const double ce = cx[(size_t)k + ny], cw = cx[k];
+  const double cn = cy[(size_t)k + i + 1], cs = cy[(size_t)k + i];
+  return (ce * (pc - (e ? pe : -pc)) + cw * (pc - (w ? pw : -pc)) + cn * (pc - (n ? pn : -pc)) +
+          cs * (pc - (s ? ps : -pc))) *
+         idx2;
+}
+
+constexpr int KU = 4;   // cells of a thread in flight in the vector kernels
 
 // q = A p; partial[b] = sum p.q ; partial2[b] = sum p.r
 __global__ void __launch_bounds__(NT)
 apply_dot_kernel(const double* __restrict__ cx, const double* __restrict__ cy,
                  const double* __restrict__ p, const double* __restrict__ r,
-                 double* __restrict__ q, int nx, int ny, double idx2, double* part_pq,
-                 double* part_pr, unsigned* counter, double* scal) {
+                 double* __restrict__ q, unsigned nx, unsigned ny, double idx2, double* part_pq,
+                 double* part_pr) {
   pdl_enter();
   __shared__ double red[NT / 32];
+  const unsigned n = nx * ny;
   double spq = 0.0, spr = 0.0;
-  for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < (long long)nx * ny;
-       k += (long long)gridDim.x * NT) {
-    const int i = (int)(k / ny), j = (int)(k - (long long)i * ny);
-    const double pc = p[k];
-    const double v = (cx[(long long)(i + 1) * ny + j] * (pc - ghost_or(p, nx, ny, i + 1, j, pc)) +
-                      cx[(long long)i * ny + j] * (pc - ghost_or(p, nx, ny, i - 1, j, pc)) +
-                      cy[(long long)i * (ny + 1) + j + 1] * (pc - ghost_or(p, nx, ny, i, j + 1, pc)) +
-                      cy[(long long)i * (ny + 1) + j] * (pc - ghost_or(p, nx, ny, i, j - 1, pc))) *
-                     idx2;
-    if (q) q[k] = v;
-    spq += pc * v;
-    if (r) spr += pc * r[k];
+  for (unsigned k0 = blockIdx.x * (2 * NT) + threadIdx.x; k0 < n; k0 += gridDim.x * (2 * NT)) {
+    double pc[2], rk[2], v[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const unsigned k = k0 + u * NT;
+      pc[u] = k < n ? p[k] : 0.0;
+      rk[u] = r && k < n ? r[k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const unsigned k = k0 + u * NT;
+      v[u] = k < n ? apply64(cx, cy, p, nx, ny, k, pc[u], idx2) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const unsigned k = k0 + u * NT;
+      if (k < n) q[k] = v[u];
+      spq += pc[u] * v[u];
+      spr += pc[u] * rk[u];
+    }
   }
   block_sum(spq, red, &part_pq[blockIdx.x]);
   __syncthreads();
   if (part_pr) block_sum(spr, red, &part_pr[blockIdx.x]);
-  if (counter) finish_scalars(part_pq, part_pr, counter, scal, S_PQ, S_PR, FIN_ALPHA, red);
 }
 
-// x += alpha p ; r -= alpha q ; partial r.r ; r32 = (float) r
+// alpha = p.r / p.q ; x += alpha p ; r -= alpha q ; partial r.r ; r32 = (float) r
 __global__ void __launch_bounds__(NT)
 update_xr_kernel(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
-                 const double* __restrict__ q, double* scal, long long n,
-                 double* part_rr, float* __restrict__ r32, unsigned* counter) {
+                 const double* __restrict__ q, double* scal, unsigned n, const double* part_pq,
+                 const double* part_pr, int nparts, double* part_rr, float* __restrict__ r32) {
   pdl_enter();
   __shared__ double red[NT / 32];
-  const double a = scal[S_ALPHA];
-  double s = 0.0;
-  for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < n; k += (long long)gridDim.x * NT) {
-    x[k] += a * p[k];
-    const double rk = r[k] - a * q[k];
-    r[k] = rk;
-    s += rk * rk;
-    if (r32) r32[k] = (float)rk;
+  const double pq = sum_parts(part_pq, nparts, red), pr = sum_parts(part_pr, nparts, red);
+  const double a = pq != 0.0 ? pr / pq : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    scal[S_PQ] = pq;
+    scal[S_PR] = pr;
+    scal[S_ALPHA] = a;
   }
+  double s = 0.0;
+  for (unsigned k0 = blockIdx.x * (KU * NT) + threadIdx.x; k0 < n; k0 += gridDim.x * (KU * NT)) {
+    double xv[KU], rv[KU], pv[KU], qv[KU];
+#pragma unroll
+    for (int u = 0; u < KU; ++u) {
+      const unsigned k = k0 + u * NT;
+      const bool in = k < n;
+      xv[u] = in ? x[k] : 0.0;
+      rv[u] = in ? r[k] : 0.0;
+      pv[u] = in ? p[k] : 0.0;
+      qv[u] = in ? q[k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < KU; ++u) {
+      const unsigned k = k0 + u * NT;
+      if (k >= n) continue;
+      x[k] = xv[u] + a * pv[u];
+      const double rk = rv[u] - a * qv[u];
+      r[k] = rk;
+      s += rk * rk;
+      r32[k] = (float)rk;
+    }
+  }
+  __syncthreads();
   block_sum(s, red, &part_rr[blockIdx.x]);
-  finish_scalars(part_rr, nullptr, counter, scal, S_RR, 0, FIN_REL, red);
 }
 
 // partial z.q with z = (double) z32, the V-cycle's float32 result (the
 // conversion is exact, so z is never stored in float64)
 __global__ void __launch_bounds__(NT)
-zq_kernel(const float* __restrict__ z32, const double* __restrict__ q, long long n,
-          double* part_zq, unsigned* counter, double* scal) {
+zq_kernel(const float* __restrict__ z32, const double* __restrict__ q, unsigned n,
+          double* part_zq) {
   pdl_enter();
   __shared__ double red[NT / 32];
   double s = 0.0;
-  for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < n; k += (long long)gridDim.x * NT)
-    s += (double)z32[k] * q[k];
+  for (unsigned k0 = blockIdx.x * (KU * NT) + threadIdx.x; k0 < n; k0 += gridDim.x * (KU * NT)) {
+    double zv[KU], qv[KU];
+#pragma unroll
+    for (int u = 0; u < KU; ++u) {
+      const unsigned k = k0 + u * NT;
+      zv[u] = k < n ? (double)z32[k] : 0.0;
+      qv[u] = k < n ? q[k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < KU; ++u) s += zv[u] * qv[u];
+  }
   block_sum(s, red, &part_zq[blockIdx.x]);
-  finish_scalars(part_zq, nullptr, counter, scal, S_ZQ, 0, FIN_BETA, red);
-}
-
-// p = z - beta p, z = (double) z32
-__global__ void p_update_kernel(double* __restrict__ p, const float* __restrict__ z32,
-                                const double* scal, long long n, int first) {
-  pdl_enter();
-  const double b = first ? 0.0 : scal[S_BETA];
-  for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < n; k += (long long)gridDim.x * NT)
-    p[k] = first ? (double)z32[k] : (double)z32[k] - b * p[k];
 }
 
 // loop control of the graph solve: counts the iteration and keeps the WHILE
@@ -356,47 +388,74 @@ __device__ __forceinline__ void fcg_loop_control(double* scal, cudaGraphConditio
   cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
-// p_update with the graph solve's loop control folded in (block 0, thread 0;
-// it reads S_REL, set by update_xr before the V-cycle, and writes S_ITER,
-// which p_update does not touch): one launch fewer per iteration
-__global__ void p_update_cond_kernel(double* __restrict__ p, const float* __restrict__ z32,
-                                     double* scal, long long n, int first,
-                                     cudaGraphConditionalHandle h, double tol, int maxit) {
+// p = z - beta p, z = (double) z32, beta = z.q / p.q (first: p = z).  The
+// residual norms of the iteration (first: r.r and b.b of the start) become
+// scalars here, and in the graph solve block 0 keeps the loop (COND): one launch
+// fewer per iteration.
+template <bool COND>
+__global__ void __launch_bounds__(NT)
+p_update_kernel(double* __restrict__ p, const float* __restrict__ z32, double* scal, unsigned n,
+                int first, const double* part_rr, const double* part_bb, int nparts,
+                const double* part_zq, int nzq, cudaGraphConditionalHandle h, double tol,
+                int maxit) {
   pdl_enter();
-  const double b = first ? 0.0 : scal[S_BETA];
-  for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < n; k += (long long)gridDim.x * NT)
-    p[k] = first ? (double)z32[k] : (double)z32[k] - b * p[k];
-  if (blockIdx.x == 0 && threadIdx.x == 0) fcg_loop_control(scal, h, tol, maxit, first);
+  __shared__ double red[NT / 32];
+  double b = 0.0;
+  if (!first) {
+    const double zq = sum_parts(part_zq, nzq, red), pq = scal[S_PQ];
+    b = pq != 0.0 ? zq / pq : 0.0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      scal[S_ZQ] = zq;
+      scal[S_BETA] = b;
+    }
+  }
+  if (blockIdx.x == 0) {
+    const double rr = sum_parts(part_rr, nparts, red);
+    const double bb = first ? sum_parts(part_bb, nparts, red) : scal[S_BB];
+    if (threadIdx.x == 0) {
+      scal[S_RR] = rr;
+      if (first) scal[S_BB] = bb;
+      scal[S_REL] = sqrt(rr / bb);
+      if (COND) fcg_loop_control(scal, h, tol, maxit, first);
+    }
+  }
+  for (unsigned k0 = blockIdx.x * (KU * NT) + threadIdx.x; k0 < n; k0 += gridDim.x * (KU * NT)) {
+    double zv[KU], pv[KU];
+#pragma unroll
+    for (int u = 0; u < KU; ++u) {
+      const unsigned k = k0 + u * NT;
+      zv[u] = k < n ? (double)z32[k] : 0.0;
+      pv[u] = !first && k < n ? p[k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < KU; ++u) {
+      const unsigned k = k0 + u * NT;
+      if (k < n) p[k] = first ? zv[u] : zv[u] - b * pv[u];
+    }
+  }
 }
 
 // r = b - A x ; partial r.r and b.b ; r32
 __global__ void __launch_bounds__(NT)
 residual64_kernel(const double* __restrict__ cx, const double* __restrict__ cy,
                   const double* __restrict__ x, const double* __restrict__ b,
-                  double* __restrict__ r, int nx, int ny, double idx2, double* part_rr,
-                  double* part_bb, float* __restrict__ r32, unsigned* counter, double* scal) {
+                  double* __restrict__ r, unsigned nx, unsigned ny, double idx2, double* part_rr,
+                  double* part_bb, float* __restrict__ r32) {
   pdl_enter();
   __shared__ double red[NT / 32];
+  const unsigned n = nx * ny;
   double srr = 0.0, sbb = 0.0;
-  for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < (long long)nx * ny;
-       k += (long long)gridDim.x * NT) {
-    const int i = (int)(k / ny), j = (int)(k - (long long)i * ny);
-    const double pc = x[k];
-    const double ax = (cx[(long long)(i + 1) * ny + j] * (pc - ghost_or(x, nx, ny, i + 1, j, pc)) +
-                       cx[(long long)i * ny + j] * (pc - ghost_or(x, nx, ny, i - 1, j, pc)) +
-                       cy[(long long)i * (ny + 1) + j + 1] * (pc - ghost_or(x, nx, ny, i, j + 1, pc)) +
-                       cy[(long long)i * (ny + 1) + j] * (pc - ghost_or(x, nx, ny, i, j - 1, pc))) *
-                      idx2;
-    const double rk = b[k] - ax;
+  for (unsigned k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
+    const double bk = b[k];
+    const double rk = bk - apply64(cx, cy, x, nx, ny, k, x[k], idx2);
     r[k] = rk;
     srr += rk * rk;
-    sbb += b[k] * b[k];
-    if (r32) r32[k] = (float)rk;
+    sbb += bk * bk;
+    r32[k] = (float)rk;
   }
   block_sum(srr, red, &part_rr[blockIdx.x]);
   __syncthreads();
   block_sum(sbb, red, &part_bb[blockIdx.x]);
-  finish_scalars(part_rr, part_bb, counter, scal, S_RR, S_BB, FIN_REL, red);
 }
 
 // ── float32 multigrid kernels ───────────────────────────────────────────────
@@ -946,6 +1005,342 @@ mg_up_kernel(const float* __restrict__ f, const float* __restrict__ cx,
   }
 }
 
+// ── strip kernels: the same two launches of a large level ───────────────────
+// A warp owns a strip of 64 columns (a lane holds an even column and the odd one
+// after it) and marches down its rows with a sliding window of rows in
+// registers.  The half-sweeps run as a pipeline: at the step that takes in row
+// r, half-sweep k updates row r - k (each needs the rows around it to have had
+// the half-sweep before), then the residual and the restriction follow.  Of a
+// row and colour every lane holds exactly one cell, so no lane idles; the column
+// neighbours come from shuffles, everything else is in the lane's own registers.
+// Columns and rows outside the level hold zeros (x stays zero there: the inverse
+// diagonal is zero), the residual's Dirichlet ghosts and the restriction's and
+// prolongation's wall weights are per-lane and per-row selects.  The loop is
+// unrolled over the window, so that the window rotates by name and the colours
+// are static.  The same float expressions in the same order as the tiles (the
+// solves end on the same residual bits) without their shared-memory traffic and
+// barriers, which bound them.  Bound by the issue of a warp's dependent row
+// steps: two warps per scheduler; 1024^2, nu = 2: down 14.0 us (tiles 19.8), up
+// 14.6 us (18.2), 21 with z.q formed on the way (a separate pass took 9.4).
+// Updates two rows apart instead of one (independent half-sweeps in a step) lost:
+// down 14.4, up 15.7 us.
+constexpr int MW = 64;            // columns of a strip
+constexpr int MG_NT = 128;        // four independent warps per CTA
+
+// halo rows of an item, halo columns of a strip (each half-sweep, the residual,
+// the restriction and the prolongation's coarse neighbour take one column)
+__host__ __device__ constexpr int mg_halo(bool down, int nu) { return down ? 2 * nu + 2 : 2 * nu; }
+__host__ __device__ constexpr int mg_chalo(int nu) { return 2 * nu + 2; }
+__host__ __device__ constexpr int mg_cols(int nu) { return MW - 2 * mg_chalo(nu); }
+
+__device__ __forceinline__ float sh_up(float v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ float sh_dn(float v) { return __shfl_down_sync(0xffffffffu, v, 1); }
+
+// the window of rows: row slot s holds x, f, idg and the west face cx of both
+// columns, and the faces cy south of the even column, between the two and north
+// of the odd one
+template <int WN>
+struct MgRows {
+  float x[WN][2], f[WN][2], g[WN][2], w[WN][2], ys[WN], ym[WN], yn[WN];
+};
+
+struct MgGrid {
+  const float *f, *cx, *cy, *idg;
+  int nx, ny, j;        // j: the lane's even column
+  bool in, ine, ino;    // columns j, j + 1 in the level; face j; face j + 1
+};
+
+// A warp's rows on their way in: MG_DEPTH of them as asynchronous copies in its
+// part of shared memory (f, idg, cx, cy south and north of the even column, on
+// the way up x and the coarse row; 32 float2 or 32 floats each), because a load
+// takes far longer than the step that uses it (loads two steps ahead into
+// registers: 1300 cycles a step, 64^2 12 us a launch).  A lane reads only what
+// it copied itself, so its own wait is the only synchronisation.
+constexpr int MG_DEPTH = 6;
+__host__ __device__ constexpr int mg_row_floats(bool down) { return down ? 256 : 352; }
+__host__ __device__ constexpr size_t mg_smem(bool down) {
+  return (size_t)(MG_NT / 32) * MG_DEPTH * mg_row_floats(down) * sizeof(float);
+}
+
+__device__ __forceinline__ void cp_async8(float* dst, const float* src, bool valid) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
+               "r"(valid ? 8 : 0)
+               : "memory");
+}
+// issue row r's copies (zeros outside the level)
+__device__ __forceinline__ void mg_issue(float* buf, int lane, const MgGrid& G, int r) {
+  const bool rin = r >= 0 && r < G.nx, a = G.in && rin, w = G.in && r >= 0 && r <= G.nx;
+  const long long k = (long long)r * G.ny + G.j, ky = k + r;
+  cp_async8(buf + 2 * lane, G.f + (a ? k : 0), a);
+  cp_async8(buf + 64 + 2 * lane, G.idg + (a ? k : 0), a);
+  cp_async8(buf + 128 + 2 * lane, G.cx + (w ? k : 0), w);
+  const bool e = rin && G.ine, o = rin && G.ino;
+  cp_async4(buf + 192 + lane, G.cy + (e ? ky : 0), e);
+  cp_async4(buf + 224 + lane, G.cy + (o ? ky + 1 : 0), o);
+}
+
+// take the row in: window slot s
+template <int WN>
+__device__ __forceinline__ void mg_take(MgRows<WN>& R, int s, const float* buf, int lane) {
+  const float2 f = *(const float2*)(buf + 2 * lane), g = *(const float2*)(buf + 64 + 2 * lane);
+  const float2 w = *(const float2*)(buf + 128 + 2 * lane);
+  R.f[s][0] = f.x; R.f[s][1] = f.y;
+  R.g[s][0] = g.x; R.g[s][1] = g.y;
+  R.w[s][0] = w.x; R.w[s][1] = w.y;
+  R.ys[s] = buf[192 + lane];
+  R.ym[s] = buf[224 + lane];
+  R.yn[s] = sh_dn(R.ys[s]);
+}
+
+// red-black update of the cells of one colour of the row in slot s (sm, sp: the
+// rows before and after); ODD: they sit in the odd columns
+template <int WN, bool ODD>
+__device__ __forceinline__ void mg_sweep(MgRows<WN>& R, int sm, int s, int sp, float idx2) {
+  constexpr int c = ODD ? 1 : 0;
+  const float xs = ODD ? R.x[s][0] : sh_up(R.x[s][1]);
+  const float xn = ODD ? sh_dn(R.x[s][0]) : R.x[s][1];
+  const float nb = ODD ? R.yn[s] : R.ym[s], sb = ODD ? R.ym[s] : R.ys[s];
+  const float sum = (R.w[sp][c] * R.x[sp][c] + R.w[s][c] * R.x[sm][c]) + (nb * xn + sb * xs);
+  R.x[s][c] = (R.f[s][c] + sum * idx2) * R.g[s][c];
+}
+
+// pre-smoothing from x = 0 (NU red/black pairs), residual, restriction: writes
+// the level's x and the coarse right-hand side
+template <int NU>
+__global__ void __launch_bounds__(MG_NT)
+mg_down_strip(const float* __restrict__ f, const float* __restrict__ cx,
+               const float* __restrict__ cy, const float* __restrict__ idg, float* __restrict__ x,
+               float* __restrict__ fc, int nx, int ny, float idx2, int nstrips, int rows) {
+  constexpr int HALO = mg_halo(true, NU), CH = mg_chalo(NU), WN = 2 * NU + 2, NS = 2 * NU;
+  const int item = blockIdx.x * (MG_NT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int strip = item % nstrips, i0 = (item / nstrips) * rows;
+  pdl_enter();
+  if (i0 >= nx) return;   // warp-uniform
+  const int i1 = min(i0 + rows, nx);
+  MgGrid G = {f, cx, cy, idg, nx, ny, strip * mg_cols(NU) - CH + 2 * lane, false, false,
+              false};
+  const int j = G.j;
+  G.in = j >= 0 && j < ny;
+  G.ine = j >= 0 && j <= ny;
+  G.ino = j + 1 >= 0 && j + 1 <= ny;
+  const bool out = lane >= CH / 2 && lane < 32 - CH / 2 && j < ny;
+  const bool lo = j == 0, hi = j + 2 == ny;
+  // restriction weights along the row (w1d): fine columns j - 1 .. j + 2
+  const float v0 = lo ? 0.f : 0.25f, v1 = lo ? 0.5f : 0.75f;
+  const float v2 = hi ? 0.5f : 0.75f, v3 = hi ? 0.f : 0.25f;
+  const int nyc = ny / 2, nxc = nx / 2;
+  MgRows<WN> R;
+#pragma unroll
+  for (int s = 0; s < WN; ++s) {
+    R.x[s][0] = R.x[s][1] = R.f[s][0] = R.f[s][1] = R.g[s][0] = R.g[s][1] = 0.f;
+    R.w[s][0] = R.w[s][1] = R.ys[s] = R.ym[s] = R.yn[s] = 0.f;
+  }
+  float t0 = 0.f, t1 = 0.f, t2 = 0.f;
+  const int rs = i0 - HALO, re = i1 + NS;   // rs even
+  extern __shared__ float mg_sm[];
+  constexpr int RF = mg_row_floats(true);
+  float* ring = mg_sm + (threadIdx.x >> 5) * MG_DEPTH * RF;
+#pragma unroll 1
+  for (int t = 0; t < MG_DEPTH - 1; ++t) {
+    mg_issue(ring + t * RF, lane, G, rs + t);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  int in = (MG_DEPTH - 1) * RF, at = 0;   // ring offsets of the row issued, the row taken in
+#pragma unroll 1
+  for (int rb = rs; rb <= re; rb += WN) {
+#pragma unroll
+    for (int ph = 0; ph < WN; ++ph) {
+      const int r = rb + ph;
+      if (r > re) break;
+      auto sl = [](int p, int k) { return (p - k + 4 * WN) % WN; };   // slot of row r - k
+      if (r + MG_DEPTH - 1 <= re) mg_issue(ring + in, lane, G, r + MG_DEPTH - 1);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group %0;" ::"n"(MG_DEPTH - 1) : "memory");
+      {
+        const int s = sl(ph, 0);
+        mg_take<WN>(R, s, ring + at, lane);
+        in = in == (MG_DEPTH - 1) * RF ? 0 : in + RF;
+        at = at == (MG_DEPTH - 1) * RF ? 0 : at + RF;
+        // half-sweep 0 starts from x = 0: x = f / d on its colour (even
+        // columns of even rows)
+        const float e = R.f[s][0] * R.g[s][0], o = R.f[s][1] * R.g[s][1];
+        R.x[s][0] = (NU == 0 || (ph & 1)) ? 0.f : e;
+        R.x[s][1] = (NU == 0 || !(ph & 1)) ? 0.f : o;
+      }
+#pragma unroll
+      for (int k = 1; k < NS; ++k) {
+        // row r - k, colour k & 1: the odd columns where row and colour differ
+        if (((ph + 4 * WN - k) & 1) != (k & 1))
+          mg_sweep<WN, true>(R, sl(ph, k + 1), sl(ph, k), sl(ph, k - 1), idx2);
+        else
+          mg_sweep<WN, false>(R, sl(ph, k + 1), sl(ph, k), sl(ph, k - 1), idx2);
+      }
+      {   // the row of the last half-sweep is final
+        constexpr int FIN = NS > 0 ? NS - 1 : 0;
+        const int i = r - FIN, s = sl(ph, FIN);
+        if (out && i >= i0 && i < i1)
+          *(float2*)(x + (long long)i * ny + j) = make_float2(R.x[s][0], R.x[s][1]);
+      }
+      // residual of row i = r - NS and its restriction along the row
+      const int i = r - NS;
+      if (i < i0 - 1) continue;   // uniform
+      float res[2];
+      {
+        const int sm = sl(ph, NS + 1), s = sl(ph, NS), sp = sl(ph, NS - 1);
+        const float xl = sh_up(R.x[s][1]), xr = sh_dn(R.x[s][0]);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const float xc = R.x[s][c];
+          const float xe = i == nx - 1 ? -xc : R.x[sp][c], xw = i == 0 ? -xc : R.x[sm][c];
+          const float xn = c ? (hi ? -xc : xr) : R.x[s][1], xs = c ? R.x[s][0] : (lo ? -xc : xl);
+          const float nb = c ? R.yn[s] : R.ym[s], sb = c ? R.ym[s] : R.ys[s];
+          const float ax = (R.w[sp][c] * (xc - xe) + R.w[s][c] * (xc - xw) + nb * (xc - xn) +
+                            sb * (xc - xs)) * idx2;
+          res[c] = R.f[s][c] - ax;
+        }
+      }
+      const float rl = sh_up(res[1]), rr = sh_dn(res[0]);
+      const float t3 = fmaf(v3, rr, fmaf(v2, res[1], fmaf(v1, res[0], v0 * rl)));
+      if (!(ph & 1)) {   // i even (NS even): coarse row I = i / 2 - 1 from rows 2 I - 1 .. 2 I + 2
+        const int I = (i >> 1) - 1;
+        if (out && 2 * I >= i0 && 2 * I < i1) {
+          const float u0 = I == 0 ? 0.f : 0.25f, u1 = I == 0 ? 0.5f : 0.75f;
+          const float u2 = I == nxc - 1 ? 0.5f : 0.75f, u3 = I == nxc - 1 ? 0.f : 0.25f;
+          fc[(long long)I * nyc + (j >> 1)] =
+              0.25f * fmaf(u3, t3, fmaf(u2, t2, fmaf(u1, t1, u0 * t0)));
+        }
+      }
+      t0 = t1;
+      t1 = t2;
+      t2 = t3;
+    }
+  }
+}
+
+// x += P e (coarse correction), post-smoothing (NU black/red pairs); the
+// level's result goes to the separate `xo` (a strip reads its halo from `x`,
+// which a neighbouring strip must not have overwritten).  q (level 0 of the
+// flexible CG, else null): part[block] receives the block's part of z.q.
+template <int NU>
+__global__ void __launch_bounds__(MG_NT)
+mg_up_strip(const float* __restrict__ f, const float* __restrict__ cx,
+             const float* __restrict__ cy, const float* __restrict__ idg,
+             const float* __restrict__ x, const float* __restrict__ ec, float* __restrict__ xo,
+             int nx, int ny, float idx2, int nstrips, int rows, const double* __restrict__ q,
+             double* __restrict__ part) {
+  constexpr int HALO = mg_halo(false, NU), CH = mg_chalo(NU), WN = 2 * NU + 2, NS = 2 * NU;
+  __shared__ double red[MG_NT / 32];
+  const int item = blockIdx.x * (MG_NT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int strip = item % nstrips, i0 = (item / nstrips) * rows;
+  pdl_enter();
+  double zq = 0.0;
+  if (i0 < nx) {   // warp-uniform
+    const int i1 = min(i0 + rows, nx);
+    MgGrid G = {f, cx, cy, idg, nx, ny, strip * mg_cols(NU) - CH + 2 * lane, false, false,
+                false};
+    const int j = G.j;
+    G.in = j >= 0 && j < ny;
+    G.ine = j >= 0 && j <= ny;
+    G.ino = j + 1 >= 0 && j + 1 <= ny;
+    const bool out = lane >= CH / 2 && lane < 32 - CH / 2 && j < ny;
+    const int nyc = ny / 2, nxc = nx / 2;
+    // the lane's coarse column (clamped) and the sign of the odd reflection
+    const int J = j >> 1, Jc = min(max(J, 0), nyc - 1);
+    const float sgj = (J < 0 || J >= nyc) ? -1.f : 1.f;
+    extern __shared__ float mg_sm[];
+    constexpr int RF = mg_row_floats(false);
+    float* ring = mg_sm + (threadIdx.x >> 5) * MG_DEPTH * RF;
+    // row r's copies: the level's operands, x, and with an even row the coarse
+    // row r / 2 + 1 (clamped; its reflection's sign comes when it is taken in)
+    auto issue = [&](float* buf, int r) {
+      mg_issue(buf, lane, G, r);
+      const bool a = G.in && r >= 0 && r < nx;
+      cp_async8(buf + 256 + 2 * lane, x + (a ? (long long)r * ny + j : 0), a);
+      if (!(r & 1)) {
+        const int Ic = min(max((r >> 1) + 1, 0), nxc - 1);
+        cp_async4(buf + 320 + lane, ec + (long long)Ic * nyc + Jc, true);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto coarse = [&](int I, float v) { return (I < 0 || I >= nxc) ? -sgj * v : sgj * v; };
+    MgRows<WN> R;
+#pragma unroll
+    for (int s = 0; s < WN; ++s) {
+      R.x[s][0] = R.x[s][1] = R.f[s][0] = R.f[s][1] = R.g[s][0] = R.g[s][1] = 0.f;
+      R.w[s][0] = R.w[s][1] = R.ys[s] = R.ym[s] = R.yn[s] = 0.f;
+    }
+    const int rs = i0 - HALO, re = i1 - 1 + NS;   // rs even
+#pragma unroll 1
+    for (int t = 0; t < MG_DEPTH - 1; ++t) issue(ring + t * RF, rs + t);
+    // the first two coarse rows (I - 1 and I of the first row)
+    const int If = rs >> 1;
+    float ca = 0.f;
+    float cb = coarse(If - 1, ec[(long long)min(max(If - 1, 0), nxc - 1) * nyc + Jc]);
+    float cc = coarse(If, ec[(long long)min(max(If, 0), nxc - 1) * nyc + Jc]);
+    int in = (MG_DEPTH - 1) * RF, at = 0;   // ring offsets of the row issued, the row taken in
+#pragma unroll 1
+    for (int rb = rs; rb <= re; rb += WN) {
+#pragma unroll
+      for (int ph = 0; ph < WN; ++ph) {
+        const int r = rb + ph;
+        if (r > re) break;
+        auto sl = [](int p, int k) { return (p - k + 4 * WN) % WN; };   // slot of row r - k
+        if (r + MG_DEPTH - 1 <= re) issue(ring + in, r + MG_DEPTH - 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(MG_DEPTH - 1) : "memory");
+        const float* buf = ring + at;
+        in = in == (MG_DEPTH - 1) * RF ? 0 : in + RF;
+        at = at == (MG_DEPTH - 1) * RF ? 0 : at + RF;
+        if (!(ph & 1)) {   // ca, cb, cc = coarse rows I - 1, I, I + 1, I = r / 2
+          ca = cb;
+          cb = cc;
+          cc = coarse((r >> 1) + 1, buf[320 + lane]);
+        }
+        {
+          const int s = sl(ph, 0);
+          mg_take<WN>(R, s, buf, lane);
+          const float2 xv = *(const float2*)(buf + 256 + 2 * lane);
+          // prolong_at's weights in its order; outside the level x stays zero
+          const float ex = (ph & 1) ? cc : ca;
+          const float bl = sh_up(cb), br = sh_dn(cb), el = sh_up(ex), er = sh_dn(ex);
+          const float b9 = (9.0f / 16.0f) * cb, e3 = fmaf(3.0f / 16.0f, ex, b9);
+          const float ve = fmaf(1.0f / 16.0f, el, fmaf(3.0f / 16.0f, bl, e3));
+          const float vo = fmaf(1.0f / 16.0f, er, fmaf(3.0f / 16.0f, br, e3));
+          const bool inr = G.in && r >= 0 && r < nx;
+          R.x[s][0] = inr ? xv.x + ve : 0.f;
+          R.x[s][1] = inr ? xv.y + vo : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+          // row r - 1 - k, colour 1 - (k & 1)
+          if (((ph + 4 * WN - 1 - k) & 1) != (1 - (k & 1)))
+            mg_sweep<WN, true>(R, sl(ph, k + 2), sl(ph, k + 1), sl(ph, k), idx2);
+          else
+            mg_sweep<WN, false>(R, sl(ph, k + 2), sl(ph, k + 1), sl(ph, k), idx2);
+        }
+        const int i = r - NS, s = sl(ph, NS);   // final
+        if (out && i >= i0 && i < i1) {
+          const long long k = (long long)i * ny + j;
+          *(float2*)(xo + k) = make_float2(R.x[s][0], R.x[s][1]);
+          if (q) {
+            zq += (double)R.x[s][0] * q[k] + (double)R.x[s][1] * q[k + 1];
+          }
+        }
+      }
+    }
+  }
+  if (!q) return;
+  for (int o = 16; o > 0; o >>= 1) zq += __shfl_xor_sync(0xffffffffu, zq, o);
+  if (lane == 0) red[threadIdx.x >> 5] = zq;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = red[0];
+    for (int w = 1; w < MG_NT / 32; ++w) t += red[w];
+    part[blockIdx.x] = t;
+  }
+}
+
 __global__ void zero32_kernel(float* x, long long n) {
   for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < n; k += (long long)gridDim.x * NT)
     x[k] = 0.0f;
@@ -1197,6 +1592,7 @@ __global__ void __launch_bounds__(ST) small_setup_kernel(const Plan P, float* ws
   __shared__ double a[DENSE_MAX_CELLS][DENSE_MAX_CELLS];
   __shared__ double fcol[DENSE_MAX_CELLS];
   __shared__ double prow[DENSE_MAX_CELLS];
+  pdl_enter();
   for (int l = l_first; l < P.nlev; ++l) {
     const Level& L = P.L[l];
     const Level& Lf = P.L[l - 1];
@@ -1290,6 +1686,14 @@ static int enable_coarse_smem() {
     ZB_SMEM_ATTR((mg_up_kernel<1, FTS>)); ZB_SMEM_ATTR((mg_up_kernel<2, FTS>));
     ZB_SMEM_ATTR((mg_up_kernel<3, FTS>)); ZB_SMEM_ATTR((mg_up_kernel<4, FTS>));
 #undef ZB_SMEM_ATTR
+#define ZB_SMEM_ATTR(NU)                                                                      \
+  ZB_CUDA_TRY(cudaFuncSetAttribute(mg_down_strip<NU>,                                         \
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,               \
+                                   (int)mg_smem(true)));                                      \
+  ZB_CUDA_TRY(cudaFuncSetAttribute(                                                           \
+      mg_up_strip<NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg_smem(false)))
+    ZB_SMEM_ATTR(1); ZB_SMEM_ATTR(2); ZB_SMEM_ATTR(3); ZB_SMEM_ATTR(4);
+#undef ZB_SMEM_ATTR
     set_mask.fetch_or(1u << dev);
   }
   return ZB_OK;
@@ -1302,10 +1706,6 @@ struct LoopCtl {
   double tol;
   int maxit;
 };
-
-// reduction counters of finish_scalars: four unsigned slots in the last
-// doubles of the scalar block (zeroed at set-up, re-armed by every use)
-static unsigned* counters(double* scal) { return (unsigned*)(scal + 12); }
 
 static int grid_for(long long n) {
   return (int)std::max<long long>(1, std::min<long long>((n + NT - 1) / NT, 148 * 8));
@@ -1321,6 +1721,7 @@ namespace pois {
 template <typename T>
 __global__ void rhs_kernel(const T* __restrict__ qx, const T* __restrict__ qy, int nx, int ny,
                            double inv_dt_dx, double* __restrict__ b) {
+  pdl_enter();
   for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < (long long)nx * ny;
        k += (long long)gridDim.x * NT) {
     const int i = (int)(k / ny), j = (int)(k - (long long)i * ny);
@@ -1338,6 +1739,7 @@ __global__ void correct_kernel(T* __restrict__ qx, T* __restrict__ qy,
                                const double* __restrict__ cx, const double* __restrict__ cy,
                                const double* __restrict__ p, int nx, int ny, double dt,
                                double inv_dx) {
+  pdl_enter();
   for (long long k = blockIdx.x * (long long)NT + threadIdx.x; k < (long long)nx * ny;
        k += (long long)gridDim.x * NT) {
     const int i = (int)(k / ny), j = (int)(k - (long long)i * ny);
@@ -1404,19 +1806,66 @@ static int fused_level(bool down, int nu, const Level& L, float* fw, float* to, 
   return e == cudaSuccess ? ZB_OK : ZB_E_CUDA;
 }
 
-// 32 x 32 tiles with 256 threads when the level has a tile for every SM; else
-// 16 x 16 tiles with 512 threads (four times the CTAs, two threads per staged
-// cell), so that the few CTAs of a small level finish their serial phases
-// sooner.  At 512^2 (256 tiles of 32^2) the large tiles win: a
-// 16^2 tile stages 28^2 cells for nu = 2, three times its own
+// A large level's launch on strips (on level 0 of the flexible CG the way up also
+// leaves the partial sums of z.q).  The rows of an item spread the level over two
+// warps per scheduler (1184), four rows at least, 64 at most; an item marches its
+// rows plus the pipeline's 4 nu + 3 (down) or 4 nu (up).
+// Returns the number of CTAs through *blocks.
+static int fused_strip(bool down, int nu, const Level& L, float* fw, float* to, float idx2,
+                 cudaStream_t st, const double* q = nullptr, double* part = nullptr,
+                 int* blocks = nullptr) {
+  const int strips = (L.ny + mg_cols(nu) - 1) / mg_cols(nu);
+  int rows = std::max(4, (int)((long long)strips * L.nx / 1184 + 1) & ~1);
+  rows = std::min(rows, 64);
+  const int wpb = MG_NT / 32;
+  auto ctas = [&](int rw) {
+    return (int)(((long long)strips * ((L.nx + rw - 1) / rw) + wpb - 1) / wpb);
+  };
+  while (q && ctas(rows) > MG_PARTS) rows *= 2;
+  const int n = ctas(rows);
+  if (blocks) *blocks = n;
+  const float *a0 = fw + L.f, *a1 = fw + L.cx, *a2 = fw + L.cy, *a3 = fw + L.idg;
+  float *a4 = fw + L.x, *a5 = fw + L.xo;
+  cudaError_t e = cudaSuccess;
+#define ZB_STRIP(NU) \
+  e = down ? pdl_launch(mg_down_strip<NU>, dim3(n), dim3(MG_NT), mg_smem(true), st, a0, a1,    \
+                        a2, a3, a4, to, L.nx, L.ny, idx2, strips, rows)                       \
+           : pdl_launch(mg_up_strip<NU>, dim3(n), dim3(MG_NT), mg_smem(false), st, a0, a1, a2, \
+                        a3, (const float*)a4, (const float*)to, a5, L.nx, L.ny, idx2, strips, \
+                        rows, q, part)
+  switch (nu) {
+    case 1: ZB_STRIP(1); break;
+    case 2: ZB_STRIP(2); break;
+    case 3: ZB_STRIP(3); break;
+    default: ZB_STRIP(4); break;
+  }
+#undef ZB_STRIP
+  return e == cudaSuccess ? ZB_OK : ZB_E_CUDA;
+}
+
+// Levels of 800^2 cells and more go on strips: a warp takes some 500 cycles a
+// row whatever the level, so strips need rows enough to fill the chip (down + up
+// of a V-cycle, us: 2048^2 on strips 80 against 130 on tiles, 1024^2 28.6 against
+// 38.0, 512^2 18.9 against 17.7, 256^2 13.8 against 11.0).  Smaller levels go on
+// tiles: 32 x 32 tiles with 256 threads when the level has a tile for every SM;
+// else 16 x 16 tiles with 512 threads (four times the CTAs, two threads per
+// staged cell), so that the few CTAs of a small level finish their serial phases
+// sooner.  At 512^2 (256 tiles of 32^2) the large tiles win: a 16^2 tile stages
+// 28^2 cells for nu = 2, three times its own.
 static int fused(bool down, int nu, const Level& L, float* fw, float* to, float idx2,
-                 cudaStream_t st) {
+                 cudaStream_t st, const double* q = nullptr, double* part = nullptr,
+                 int* blocks = nullptr) {
+  if ((long long)L.nx * L.ny >= 800LL * 800LL)
+    return fused_strip(down, nu, L, fw, to, idx2, st, q, part, blocks);
   const bool big = ((L.ny + FT - 1) / FT) * ((L.nx + FT - 1) / FT) >= 148;
   if (big) return fused_level<FT>(down, nu, L, fw, to, idx2, dim3(fused_threads(FT)), st);
   return fused_level<FTS>(down, nu, L, fw, to, idx2, dim3(fused_threads(FTS)), st);
 }
 
-static int vcycle(const Plan& P, void* ws, int precond, const zb_smoother* smo, cudaStream_t st) {
+// q, part, nzq (the flexible CG): where level 0's way up forms the partial sums of
+// z.q with q itself, they land in part and *nzq is their count, else 0
+static int vcycle(const Plan& P, void* ws, int precond, const zb_smoother* smo, cudaStream_t st,
+                  const double* q = nullptr, double* part = nullptr, int* nzq = nullptr) {
   float* fw = (float*)((char*)ws + P.fbase);
   const Level& L0 = P.L[0];
   const long long n0 = (long long)L0.nx * L0.ny;
@@ -1479,7 +1928,12 @@ static int vcycle(const Plan& P, void* ws, int precond, const zb_smoother* smo, 
                                  fw + L.r, L.nx, L.ny, (double)L.dx, 0, (void*)st);
       if (rc) return rc;
     } else {
-      if (const int rc = fused(false, P.nu, L, fw, result(l + 1), idx2, st)) return rc;
+      const bool dot = l == 0 && precond == 1 && q && nzq;
+      int n = 0;
+      if (const int rc = fused(false, P.nu, L, fw, result(l + 1), idx2, st, dot ? q : nullptr, part,
+                               &n))
+        return rc;
+      if (dot) *nzq = n;
     }
   }
   if (result(0) != fw + L0.xo)   // a single level swept in place
@@ -1542,24 +1996,25 @@ int zb_poisson_setup(const zb_poisson_cfg* cfg, const void* h, int dtype, void* 
   const double idx2 = 1.0 / (cfg->dx * cfg->dx);
   const float idx2f = 1.0f / (L0.dx * L0.dx);
   if (dtype == ZB_F64)
-    setup0_kernel<double><<<grid_for(n0), NT, 0, st>>>(
+    ZB_CUDA_TRY(pdl_launch(setup0_kernel<double>, dim3(grid_for(n0)), dim3(NT), 0, st,
         (const double*)h, L0.nx, L0.ny, cfg->cmin, cfg->cmax, idx2, idx2f, dw + P.cx64,
-        dw + P.cy64, dw + P.dg64, fw + L0.cx, fw + L0.cy, fw + L0.idg);
+        dw + P.cy64, dw + P.dg64, fw + L0.cx, fw + L0.cy, fw + L0.idg));
   else
-    setup0_kernel<float><<<grid_for(n0), NT, 0, st>>>(
+    ZB_CUDA_TRY(pdl_launch(setup0_kernel<float>, dim3(grid_for(n0)), dim3(NT), 0, st,
         (const float*)h, L0.nx, L0.ny, cfg->cmin, cfg->cmax, idx2, idx2f, dw + P.cx64,
-        dw + P.cy64, dw + P.dg64, fw + L0.cx, fw + L0.cy, fw + L0.idg);
+        dw + P.cy64, dw + P.dg64, fw + L0.cx, fw + L0.cy, fw + L0.idg));
   // levels above the one-CTA part: one launch each; the rest and the
   // coarsest inverse: one CTA
   const int l_small = std::max(1, std::min(P.small0, P.nlev));
   for (int l = 1; l < l_small; ++l) {
     const Level& L = P.L[l];
     const Level& Lf = P.L[l - 1];
-    coarsen_kernel<<<grid_for((long long)L.nx * L.ny), NT, 0, st>>>(
-        fw + Lf.cx, fw + Lf.cy, L.nx, L.ny, 1.0f / (L.dx * L.dx), fw + L.cx, fw + L.cy,
-        fw + L.idg);
+    ZB_CUDA_TRY(pdl_launch(coarsen_kernel, dim3(grid_for((long long)L.nx * L.ny)), dim3(NT), 0,
+                           st, (const float*)(fw + Lf.cx), (const float*)(fw + Lf.cy), L.nx, L.ny,
+                           1.0f / (L.dx * L.dx), fw + L.cx, fw + L.cy, fw + L.idg));
   }
-  if (l_small < P.nlev || P.cinv >= 0) small_setup_kernel<<<1, ST, 0, st>>>(P, fw, l_small);
+  if (l_small < P.nlev || P.cinv >= 0)
+    ZB_CUDA_TRY(pdl_launch(small_setup_kernel, dim3(1), dim3(ST), 0, st, P, fw, l_small));
   ZB_CUDA_TRY(cudaMemsetAsync(dw + P.scal, 0, S_COUNT * sizeof(double), st));
   return zb_launch_check();
 }
@@ -1570,9 +2025,9 @@ int zb_poisson_apply(const zb_poisson_cfg* cfg, void* ws, const double* p, doubl
   const Plan P = make_plan(cfg);
   cudaStream_t st = (cudaStream_t)stream;
   double* dw = (double*)ws;
-  apply_dot_kernel<<<RED_BLOCKS, NT, 0, st>>>(dw + P.cx64, dw + P.cy64, p, nullptr, q, cfg->nx,
-                                              cfg->ny, 1.0 / (cfg->dx * cfg->dx), dw + P.part,
-                                              nullptr, nullptr, nullptr);
+  apply_dot_kernel<<<RED_BLOCKS, NT, 0, st>>>(dw + P.cx64, dw + P.cy64, p, nullptr, q,
+                                              (unsigned)cfg->nx, (unsigned)cfg->ny,
+                                              1.0 / (cfg->dx * cfg->dx), dw + P.part, nullptr);
   return zb_launch_check();
 }
 
@@ -1598,11 +2053,13 @@ int zb_poisson_rhs(const zb_poisson_cfg* cfg, const void* Q, int dtype, double d
   const long long n = (long long)cfg->nx * cfg->ny;
   const double s = 1.0 / (dt * cfg->dx);
   if (dtype == ZB_F64)
-    rhs_kernel<double><<<grid_for(n), NT, 0, st>>>((const double*)Q + 2 * n,
-                                                   (const double*)Q + 3 * n, cfg->nx, cfg->ny, s, b);
+    ZB_CUDA_TRY(pdl_launch(rhs_kernel<double>, dim3(grid_for(n)), dim3(NT), 0, st,
+                           (const double*)Q + 2 * n, (const double*)Q + 3 * n, cfg->nx, cfg->ny, s,
+                           b));
   else if (dtype == ZB_F32)
-    rhs_kernel<float><<<grid_for(n), NT, 0, st>>>((const float*)Q + 2 * n, (const float*)Q + 3 * n,
-                                                  cfg->nx, cfg->ny, s, b);
+    ZB_CUDA_TRY(pdl_launch(rhs_kernel<float>, dim3(grid_for(n)), dim3(NT), 0, st,
+                           (const float*)Q + 2 * n, (const float*)Q + 3 * n, cfg->nx, cfg->ny, s,
+                           b));
   else
     return ZB_E_ARG;
   return zb_launch_check();
@@ -1616,15 +2073,30 @@ int zb_poisson_correct(const zb_poisson_cfg* cfg, void* ws, void* Q, int dtype, 
   double* dw = (double*)ws;
   const long long n = (long long)cfg->nx * cfg->ny;
   if (dtype == ZB_F64)
-    correct_kernel<double><<<grid_for(n), NT, 0, st>>>((double*)Q + 2 * n, (double*)Q + 3 * n,
-                                                       dw + P.cx64, dw + P.cy64, p, cfg->nx,
-                                                       cfg->ny, dt, 1.0 / cfg->dx);
+    ZB_CUDA_TRY(pdl_launch(correct_kernel<double>, dim3(grid_for(n)), dim3(NT), 0, st,
+                           (double*)Q + 2 * n, (double*)Q + 3 * n, (const double*)(dw + P.cx64),
+                           (const double*)(dw + P.cy64), p, cfg->nx, cfg->ny, dt,
+                           1.0 / cfg->dx));
   else if (dtype == ZB_F32)
-    correct_kernel<float><<<grid_for(n), NT, 0, st>>>((float*)Q + 2 * n, (float*)Q + 3 * n,
-                                                      dw + P.cx64, dw + P.cy64, p, cfg->nx,
-                                                      cfg->ny, dt, 1.0 / cfg->dx);
+    ZB_CUDA_TRY(pdl_launch(correct_kernel<float>, dim3(grid_for(n)), dim3(NT), 0, st,
+                           (float*)Q + 2 * n, (float*)Q + 3 * n, (const double*)(dw + P.cx64),
+                           (const double*)(dw + P.cy64), p, cfg->nx, cfg->ny, dt,
+                           1.0 / cfg->dx));
   else
     return ZB_E_ARG;
+  return zb_launch_check();
+}
+
+static int p_update(const Plan& P, void* ws, long long n, int first, const double* rr,
+                    const double* bb, const double* zq, int nzq, const LoopCtl* lc,
+                    cudaStream_t st) {
+  double* dw = (double*)ws;
+  const float* z32 = (const float*)((const char*)ws + P.fbase) + P.L[0].xo;
+  const LoopCtl none = {};
+  const LoopCtl& c = lc ? *lc : none;
+  ZB_CUDA_TRY(pdl_launch(lc ? p_update_kernel<true> : p_update_kernel<false>, dim3(RED_BLOCKS),
+                         dim3(NT), 0, st, dw + P.vp, z32, dw + P.scal, (unsigned)n, first, rr, bb,
+                         RED_BLOCKS, zq, nzq, c.h, c.tol, c.maxit));
   return zb_launch_check();
 }
 
@@ -1640,22 +2112,13 @@ static int fcg_start_impl(const zb_poisson_cfg* cfg, void* ws, const double* b, 
   const long long n = (long long)cfg->nx * cfg->ny;
   double* part = dw + P.part;
   double* scal = dw + P.scal;
-  unsigned* ctr = counters(scal);
   ZB_CUDA_TRY(pdl_launch(residual64_kernel, dim3(RED_BLOCKS), dim3(NT), 0, st,
                          (const double*)(dw + P.cx64), (const double*)(dw + P.cy64),
-                         (const double*)x, b, dw + P.vr, cfg->nx, cfg->ny,
-                         1.0 / (cfg->dx * cfg->dx), part, part + RED_BLOCKS, fw + P.L[0].f, ctr,
-                         scal));
+                         (const double*)x, b, dw + P.vr, (unsigned)cfg->nx, (unsigned)cfg->ny,
+                         1.0 / (cfg->dx * cfg->dx), part, part + RED_BLOCKS, fw + P.L[0].f));
   int rc = vcycle(P, ws, precond, smo, st);
   if (rc) return rc;
-  const float* z32 = fw + P.L[0].xo;
-  if (lc)
-    ZB_CUDA_TRY(pdl_launch(p_update_cond_kernel, dim3(grid_for(n)), dim3(NT), 0, st, dw + P.vp,
-                           z32, scal, n, 1, lc->h, lc->tol, lc->maxit));
-  else
-    ZB_CUDA_TRY(pdl_launch(p_update_kernel, dim3(grid_for(n)), dim3(NT), 0, st, dw + P.vp, z32,
-                           (const double*)scal, n, 1));
-  return zb_launch_check();
+  return p_update(P, ws, n, 1, part, part + RED_BLOCKS, nullptr, 0, lc, st);
 }
 
 int zb_fcg_start(const zb_poisson_cfg* cfg, void* ws, const double* b, double* x, int precond,
@@ -1674,27 +2137,25 @@ static int fcg_iterate_impl(const zb_poisson_cfg* cfg, void* ws, double* x, int 
   const long long n = (long long)cfg->nx * cfg->ny;
   double* part = dw + P.part;
   double* scal = dw + P.scal;
-  unsigned* ctr = counters(scal);
+  double *pq = part, *pr = part + RED_BLOCKS, *rr = part + 2 * RED_BLOCKS,
+         *zq = part + 3 * RED_BLOCKS;
   ZB_CUDA_TRY(pdl_launch(apply_dot_kernel, dim3(RED_BLOCKS), dim3(NT), 0, st,
                          (const double*)(dw + P.cx64), (const double*)(dw + P.cy64),
-                         (const double*)(dw + P.vp), (const double*)(dw + P.vr), dw + P.vq, cfg->nx,
-                         cfg->ny, 1.0 / (cfg->dx * cfg->dx), part, part + RED_BLOCKS, ctr + 1,
-                         scal));
+                         (const double*)(dw + P.vp), (const double*)(dw + P.vr), dw + P.vq,
+                         (unsigned)cfg->nx, (unsigned)cfg->ny, 1.0 / (cfg->dx * cfg->dx), pq, pr));
   ZB_CUDA_TRY(pdl_launch(update_xr_kernel, dim3(RED_BLOCKS), dim3(NT), 0, st, x, dw + P.vr,
-                         (const double*)(dw + P.vp), (const double*)(dw + P.vq), scal, n,
-                         part + 2 * RED_BLOCKS, fw + P.L[0].f, ctr + 2));
-  int rc = vcycle(P, ws, precond, smo, st);
+                         (const double*)(dw + P.vp), (const double*)(dw + P.vq), scal, (unsigned)n,
+                         (const double*)pq, (const double*)pr, RED_BLOCKS, rr, fw + P.L[0].f));
+  int nzq = 0;
+  int rc = vcycle(P, ws, precond, smo, st, dw + P.vq, zq, &nzq);
   if (rc) return rc;
-  const float* z32 = fw + P.L[0].xo;
-  ZB_CUDA_TRY(pdl_launch(zq_kernel, dim3(RED_BLOCKS), dim3(NT), 0, st, z32,
-                         (const double*)(dw + P.vq), n, part + 3 * RED_BLOCKS, ctr + 3, scal));
-  if (lc)
-    ZB_CUDA_TRY(pdl_launch(p_update_cond_kernel, dim3(grid_for(n)), dim3(NT), 0, st, dw + P.vp,
-                           z32, scal, n, 0, lc->h, lc->tol, lc->maxit));
-  else
-    ZB_CUDA_TRY(pdl_launch(p_update_kernel, dim3(grid_for(n)), dim3(NT), 0, st, dw + P.vp, z32,
-                           (const double*)scal, n, 0));
-  return zb_launch_check();
+  if (nzq == 0) {
+    nzq = RED_BLOCKS;
+    ZB_CUDA_TRY(pdl_launch(zq_kernel, dim3(RED_BLOCKS), dim3(NT), 0, st,
+                           (const float*)(fw + P.L[0].xo), (const double*)(dw + P.vq), (unsigned)n,
+                           zq));
+  }
+  return p_update(P, ws, n, 0, rr, nullptr, zq, nzq, lc, st);
 }
 
 int zb_fcg_iterate(const zb_poisson_cfg* cfg, void* ws, double* x, int precond,
