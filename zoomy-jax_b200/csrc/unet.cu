@@ -708,14 +708,17 @@ static int conv_tc_launch(const float* inA, int cin_a, const float* inB, int cin
     sms[dev].store(v);
   }
   if (!attr[dev].load()) {
-    ZB_CUDA_TRY(cudaFuncSetAttribute(conv3x3_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     227 * 1024));
+#define ZB_SMEM_ATTR(G)                                                                       \
+  ZB_CUDA_TRY(                                                                                 \
+      cudaFuncSetAttribute(conv3x3_tc<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024))
+    ZB_SMEM_ATTR(1); ZB_SMEM_ATTR(2); ZB_SMEM_ATTR(3); ZB_SMEM_ATTR(5);
+#undef ZB_SMEM_ATTR
     attr[dev].store(true);
   }
   // resident CTAs of one SM must never ask for more than its 512 TMEM
   // columns: pad the shared memory so that at most 512 / cols fit
   const int smem_sm = 228 * 1024, per_cta_reserved = 1024;
-  const int by_tmem = 512 / cols, by_threads = 2048 / TC_THREADS;
+  const int by_tmem = 512 / cols, by_threads = TC_PER_SM;
   size_t smem = tc_smem_bytes(cinp, coutp);
   if (by_tmem < by_threads) {
     const size_t floor_bytes = (size_t)(smem_sm / (by_tmem + 1) - per_cta_reserved + 16);
@@ -726,8 +729,17 @@ static int conv_tc_launch(const float* inA, int cin_a, const float* inB, int cin
   const long long ntiles =
       (long long)((W + TCX - 1) / TCX) * ((H + TCY - 1) / TCY) * B;
   const int grid = (int)std::max<long long>(1, std::min<long long>(ntiles, (long long)sms[dev] * std::max(1, fit)));
-  conv3x3_tc<<<grid, TC_THREADS, smem, st>>>(inA, cin_a, inB, cin, w, bias, out, cout, B, H, W,
-                                             act, mode_a, cols, unet_err_word());
+  // channel groups of 16 of the networks' layers (valid_channels)
+  switch (cinp / 16) {
+#define ZB_TC(G)                                                                               \
+  case G:                                                                                      \
+    conv3x3_tc<G><<<grid, TC_THREADS, smem, st>>>(inA, cin_a, inB, cin, w, bias, out, cout, B, H, \
+                                                  W, act, mode_a, cols, unet_err_word());      \
+    break
+    ZB_TC(1); ZB_TC(2); ZB_TC(3); ZB_TC(5);
+#undef ZB_TC
+    default: return ZB_E_UNSUPPORTED;
+  }
   return zb_launch_check();
 }
 
@@ -771,9 +783,9 @@ static int conv_cb8_launch(const uint4* inA, int chA, int mode_a, const uint4* i
                            uint4* pool, int cout, int out_form, int B, int H, int W, int act,
                            cudaStream_t st) {
   const int cinp = pad16(cin), coutp = pad16(cout);
-  if (2 * coutp > 256 || cinp > 256 || chA + chB > cinp / 8) return ZB_E_UNSUPPORTED;
+  if (4 * coutp > 512 || cinp > 256 || chA + chB > cinp / 8) return ZB_E_UNSUPPORTED;
   int cols = 32;
-  while (cols < 2 * coutp) cols *= 2;
+  while (cols < 4 * coutp) cols *= 2;   // two buffers of two M tiles
   static std::atomic<int> sms[64];
   static std::atomic<bool> attr[64];
   int dev = 0;
@@ -785,25 +797,36 @@ static int conv_cb8_launch(const uint4* inA, int chA, int mode_a, const uint4* i
     sms[dev].store(v);
   }
   if (!attr[dev].load()) {
-    ZB_CUDA_TRY(cudaFuncSetAttribute(conv3x3_cb8<128>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    ZB_CUDA_TRY(cudaFuncSetAttribute(conv3x3_cb8<256>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+#define ZB_SMEM_ATTR(G)                                                                        \
+  ZB_CUDA_TRY(cudaFuncSetAttribute(conv3x3_cb8<G, CB_NTH>,                                     \
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)); \
+  ZB_CUDA_TRY(cudaFuncSetAttribute(conv3x3_cb8<G, CB_NTH_UP>,                                  \
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024))
+    ZB_SMEM_ATTR(1); ZB_SMEM_ATTR(2); ZB_SMEM_ATTR(3); ZB_SMEM_ATTR(5);
+#undef ZB_SMEM_ATTR
     attr[dev].store(true);
   }
-  const int nth = cinp / 8 >= CB_WIDE_CHUNKS ? 256 : 128;
+  const bool up = mode_a == SRC_UP && chA > 0;
+  const int nth = up ? CB_NTH_UP : CB_NTH, stages = cb_stages(up);
   const int smem_sm = 228 * 1024, per_cta_reserved = 1024;
-  const int by_tmem = 512 / cols, by_threads = 2048 / nth;
-  size_t smem = cb8_smem_bytes(cinp, coutp);
+  const int by_tmem = 512 / cols, by_threads = cb_per_sm(nth);
+  size_t smem = cb8_smem_bytes(cinp, coutp, stages);
   if (by_tmem < by_threads) {
     const size_t floor_bytes = (size_t)(smem_sm / (by_tmem + 1) - per_cta_reserved + 16);
     smem = std::max(smem, floor_bytes);
   }
   if (smem > 227 * 1024) return ZB_E_UNSUPPORTED;
-  const int fit = std::min(by_threads, (int)(smem_sm / (smem + per_cta_reserved)));
+  const int fit = std::max(1, std::min(by_threads, (int)(smem_sm / (smem + per_cta_reserved))));
   const long long nreg = (long long)((W + CBX - 1) / CBX) * ((H + CBY - 1) / CBY) * B;
-  const int grid = (int)std::max<long long>(
-      1, std::min<long long>(nreg, (long long)sms[dev] * std::max(1, fit)));
+  // CTAs per SM: the most that leave no SM waiting on a last round
+  int per_sm = 1;
+  auto rounds = [&](int k) {
+    const long long g = (long long)sms[dev] * k;
+    return (nreg + g - 1) / g * k;
+  };
+  for (int k = 2; k <= fit; ++k)
+    if (rounds(k) <= rounds(per_sm)) per_sm = k;
+  const int grid = (int)std::max<long long>(1, std::min<long long>(nreg, (long long)sms[dev] * per_sm));
   // tensor maps of the sources read as stored (the upsampled source, and one
   // whose map cannot be encoded, stay on the cp.async copies)
   CUtensorMap tm_a, tm_b;
@@ -811,14 +834,17 @@ static int conv_cb8_launch(const uint4* inA, int chA, int mode_a, const uint4* i
   std::memset(&tm_b, 0, sizeof(tm_b));
   const int tma_a = (mode_a == SRC_DIRECT && chA > 0 && cb8_map(&tm_a, inA, chA, B, H, W)) ? 1 : 0;
   const int tma_b = (chB > 0 && cb8_map(&tm_b, inB, chB, B, H, W)) ? 1 : 0;
-  if (nth == 256)
-    conv3x3_cb8<256><<<grid, 256, smem, st>>>(inA, chA, mode_a, inB, chB, cin, w, bias, out,
-                                              pool, cout, out_form, B, H, W, act, cols,
-                                              unet_err_word(), tm_a, tm_b, tma_a, tma_b);
-  else
-    conv3x3_cb8<128><<<grid, 128, smem, st>>>(inA, chA, mode_a, inB, chB, cin, w, bias, out,
-                                              pool, cout, out_form, B, H, W, act, cols,
-                                              unet_err_word(), tm_a, tm_b, tma_a, tma_b);
+  switch (cinp / 16) {
+#define ZB_CB8(G)                                                                              \
+  case G:                                                                                      \
+    ZB_CUDA_TRY(pdl_launch(up ? conv3x3_cb8<G, CB_NTH_UP> : conv3x3_cb8<G, CB_NTH>, dim3(grid), dim3(nth), smem, st, inA, chA, mode_a, inB, \
+                           chB, cin, w, bias, out, pool, cout, out_form, B, H, W, act, cols,   \
+                           stages, unet_err_word(), tm_a, tm_b, tma_a, tma_b));                \
+    break
+    ZB_CB8(1); ZB_CB8(2); ZB_CB8(3); ZB_CB8(5);
+#undef ZB_CB8
+    default: return ZB_E_UNSUPPORTED;
+  }
   return zb_launch_check();
 }
 
