@@ -29,6 +29,8 @@ from ..trimesh import DeviceTriangleMesh, TriangleMesh
 class _CartBackend:
     """libzb calls of the Cartesian path (``zb_swe2d_*``)."""
 
+    stage_b_from_q0 = True    # a stage with Q0 never reads Qk's b row
+
     def __init__(self, lib, cfg):
         self.lib, self.cfg = lib, cfg
         self.ref = C.byref(cfg)
@@ -63,6 +65,8 @@ class _CartBackend:
 
 class _TriBackend:
     """libzb calls of the triangle path (``zb_tri_*``)."""
+
+    stage_b_from_q0 = False
 
     def __init__(self, lib, cfg, mesh_struct):
         self.lib, self.cfg, self.mesh = lib, cfg, mesh_struct
@@ -249,6 +253,7 @@ class HyperbolicSolver:
         self._ws_bytes = self.be.workspace_bytes()
         self._ws = torch.empty(self._ws_bytes, dtype=torch.uint8, device=dev)
         self._ctrl = torch.zeros(L.CTRL_BYTES, dtype=torch.uint8, device=dev)
+        self._probe = torch.zeros_like(self._ctrl)    # zero between steps
         self._mass_part = torch.zeros(self.be.mass_partials(), dtype=torch.float64, device=dev)
         self._n = 0
         self._bed, self._bed_key = None, None
@@ -307,29 +312,44 @@ class HyperbolicSolver:
                            self._s()), "dt")
         return float(self.read_ctrl().dt)
 
-    def _stage(self, cfg, Qk, Q0, Qo, alpha, beta, dt, hinv=None, fo=None, tr=None):
+    def _stage(self, cfg, Qk, Q0, Qo, alpha, beta, dt, hinv=None, fo=None, tr=None,
+               ctrl=None):
         L.check(self.be.stage(
             C.byref(cfg), L.ptr(Qk), L.ptr(Q0) if Q0 is not None else None, L.ptr(Qo),
             float(alpha), float(beta), float(dt),
             L.ptr(hinv) if hinv is not None else None,
             L.ptr(fo) if fo is not None else None, L.ptr(tr) if tr is not None else None,
-            L.ptr(self._ws), C.c_size_t(self._ws_bytes), L.ptr(self._ctrl), self._s()),
-            "stage")
+            L.ptr(self._ws), C.c_size_t(self._ws_bytes),
+            L.ptr(self._ctrl if ctrl is None else ctrl), self._s()), "stage")
 
-    def _advance(self, Q, dt, force_o1=None, trouble=None):
+    def _probe_troubled(self):
+        """Whether the stage that ran with the probe control block flagged a cell
+        (synchronises).  Its status word replaces a reduction over the mask (18 us
+        at 320 x 200, and the fill before it); a set status moves to the solver's
+        block, and the probe is zero again."""
+        import torch
+        i = L.ZbCtrl.status.offset // 4
+        status = int(self._probe.view(torch.int32)[i].item())
+        if status:
+            self._ctrl.view(torch.int32)[i].bitwise_or_(status)
+            self._probe.zero_()
+        return bool(status & L.ZB_ST_TROUBLED)
+
+    def _advance(self, Q, dt, force_o1=None, trouble=None, ctrl=None):
         """Hyperbolic sub-step with a host dt: SSP-RK2 in Shu-Osher form
         (alpha = 0.5 is exact: scaling by 1/2 commutes with rounding, so it is
-        bit-identical to 0.5 (Q0 + Q2)) or Euler.  Optional per-cell MOOD mask
-        and troubled-mask output (C bytes)."""
+        bit-identical to 0.5 (Q0 + Q2)) or Euler.  Optional per-cell MOOD mask,
+        troubled-mask output (C bytes) and control block of the last stage."""
         import torch
         Qn = Q.clone()
         if self.cfg.order >= 2:
             Q1 = torch.empty_like(Q)
-            Q1[0].copy_(Q[0])
+            if not self.be.stage_b_from_q0:
+                Q1[0].copy_(Q[0])
             self._stage(self.cfg, Q, None, Q1, 0.0, 1.0, dt, fo=force_o1)
-            self._stage(self.cfg, Q1, Q, Qn, 0.5, 1.0, dt, fo=force_o1, tr=trouble)
+            self._stage(self.cfg, Q1, Q, Qn, 0.5, 1.0, dt, fo=force_o1, tr=trouble, ctrl=ctrl)
         else:
-            self._stage(self.cfg, Q, None, Qn, 0.0, 1.0, dt, fo=force_o1, tr=trouble)
+            self._stage(self.cfg, Q, None, Qn, 0.0, 1.0, dt, fo=force_o1, tr=trouble, ctrl=ctrl)
         return Qn
 
     def step(self, dt, time, Q, Qaux, parameters=None):
@@ -341,9 +361,12 @@ class HyperbolicSolver:
         import torch
         dt = float(dt)
         if self.mood:
-            mask = torch.zeros(Q.shape[1], dtype=torch.uint8, device=Q.device)
-            Qn = self._advance(Q, dt, trouble=mask)
-            if bool(mask.any()):
+            # the last stage writes every byte of the mask; a negative dt is the
+            # solver's control block's, so that block goes to the stage
+            mask = torch.empty(Q.shape[1], dtype=torch.uint8, device=Q.device)
+            probe = dt >= 0.0
+            Qn = self._advance(Q, dt, trouble=mask, ctrl=self._probe if probe else None)
+            if self._probe_troubled() if probe else bool(mask.any()):
                 Qn = self._advance(Q, dt, force_o1=mask)
         else:
             Qn = self._advance(Q, dt)
