@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(TC_THREADS, TC_PER_SM)
 conv3x3_tc(const float* __restrict__ inA, int cin_a, const float* __restrict__ inB, int cin,
            const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
            float* __restrict__ out, int cout, int B, int H, int W, int act, int mode_a,
-           int tmem_cols, unsigned* err) {
+           const float* __restrict__ ytanh, int tmem_cols, unsigned* err) {
   extern __shared__ __align__(128) unsigned char tc_sm[];
   const int cinp = pad16(cin), coutp = pad16(cout);
   const int nch = cinp / 8;
@@ -280,6 +280,7 @@ conv3x3_tc(const float* __restrict__ inA, int cin_a, const float* __restrict__ i
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_enter();   // the weights do not come from the preceding launch
   const uint32_t tmem = *tmem_slot;
   const uint32_t mbar_a = smem_u32(mbar);
   const uint32_t sA_a = smem_u32(sA), sB_a = smem_u32(sB);
@@ -317,6 +318,19 @@ conv3x3_tc(const float* __restrict__ inA, int cin_a, const float* __restrict__ i
       tc_issue_tile<G, THP * 16, THX>(tmem, sA_a, sB_a, coutp, idesc);
       tc_commit(mbar_a);
     }
+    // the activations that a data gradient is multiplied with, on their way while
+    // the MMAs run (read in the epilogue one by one they doubled the launch)
+    const int m = (warp & 3) * 32 + lane;
+    const int x = x0 + (m % TCX), y = y0 + (m / TCX);
+    const bool store = x < W && y < H;
+    const size_t pix = img + (size_t)y * W + x;
+    float yv[16];
+    auto load_y = [&](int c0) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        yv[i] = store && c0 + i < cout ? ytanh[(size_t)(c0 + i) * plane + pix] : 0.0f;
+    };
+    if (ytanh) load_y((warp >> 2) * 16);
     // wait for the tile's MMAs (bounded); the CTA agrees on the outcome so
     // every warp takes the same path through the collective TMEM loads
     bool done = false;
@@ -332,9 +346,6 @@ conv3x3_tc(const float* __restrict__ inA, int cin_a, const float* __restrict__ i
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // epilogue: warps w and w + 4 own accumulator rows (pixels) 32w .. 32w+31 and
     // take every second group of 16 channels
-    const int m = (warp & 3) * 32 + lane;
-    const int x = x0 + (m % TCX), y = y0 + (m / TCX);
-    const bool store = x < W && y < H;
     for (int c0 = (warp >> 2) * 16; c0 < coutp; c0 += 32) {
       float v[16];
       __syncwarp();
@@ -346,9 +357,11 @@ conv3x3_tc(const float* __restrict__ inA, int cin_a, const float* __restrict__ i
           float s = v[i] + (bias ? bias[co] : 0.0f);
           if (act == 1) s = tanhf(s);
           else if (act == 2) s = tanh_sfu(s);
-          out[(size_t)co * plane + img + (size_t)y * W + x] = s;
+          if (ytanh) s *= 1.0f - yv[i] * yv[i];   // a data gradient into a tanh
+          out[(size_t)co * plane + pix] = s;
         }
       }
+      if (ytanh && c0 + 32 < coutp) load_y(c0 + 32);
     }
     // TMEM reads and smem reads of this tile complete before the next tile
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

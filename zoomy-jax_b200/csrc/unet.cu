@@ -47,12 +47,14 @@ enum { ACT_NONE = 0, ACT_TANH = 1, ACT_TANH_SFU = 2 };   // see conv_tc.cuh
 
 // out[co][b][y][x] = act(bias[co] + sum_ci sum_tap w[co][ci][tap] in[ci][b][y+dy][x+dx])
 // input channels may come from two planes sets (the concatenation): channels
-// [0, cin_a) from inA, [cin_a, cin) from inB
+// [0, cin_a) from inA, [cin_a, cin) from inB; ytanh (a data gradient): the result
+// times 1 - ytanh^2
 template <int COUT>
 __global__ void __launch_bounds__(NTT)
 conv3x3_fwd(const float* __restrict__ inA, int cin_a, const float* __restrict__ inB, int cin,
             const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
-            float* __restrict__ out, int B, int H, int W, int act, int mode_a) {
+            float* __restrict__ out, int B, int H, int W, int act, int mode_a,
+            const float* __restrict__ ytanh) {
   __shared__ float sin_[CCH][TS + 2][TS + 2];
   __shared__ float sw[COUT][CCH][9];
   const int tx = threadIdx.x % TS, ty = threadIdx.x / TS;
@@ -93,8 +95,10 @@ conv3x3_fwd(const float* __restrict__ inA, int cin_a, const float* __restrict__ 
   if (x < W && y < H) {
 #pragma unroll
     for (int co = 0; co < COUT; ++co) {
-      const float v = act != ACT_NONE ? tanhf(acc[co]) : acc[co];   // exact reference
-      out[(size_t)co * plane + img + (size_t)y * W + x] = v;
+      float v = act != ACT_NONE ? tanhf(acc[co]) : acc[co];   // exact reference
+      const size_t k = (size_t)co * plane + img + (size_t)y * W + x;
+      if (ytanh) v *= 1.0f - ytanh[k] * ytanh[k];
+      out[k] = v;
     }
   }
 }
@@ -162,6 +166,7 @@ __global__ void __launch_bounds__(WG_MAX_THREADS, 2)
 conv3x3_wgrad(const float* __restrict__ inA, int cin_a, const float* __restrict__ inB, int cin,
               const float* __restrict__ dout, int cout, float* __restrict__ part, int B, int H,
               int W, int mode_a, int ncog, int cic, int nsl) {
+  pdl_enter();
   extern __shared__ __align__(16) float wsm[];
   const int nt = blockDim.x, tid = threadIdx.x;
   const int c_lo = blockIdx.y * cic, c_n = min(cic, cin + 1 - c_lo);
@@ -319,6 +324,7 @@ struct WgReduce {
 // are added in order.
 __global__ void __launch_bounds__(NT)
 wgrad_reduce(const WgReduce R, float* __restrict__ dw, float* __restrict__ db) {
+  pdl_enter();
   __shared__ float sh[NT / 32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int e = blockIdx.x * 32 + lane;
@@ -340,68 +346,82 @@ wgrad_reduce(const WgReduce R, float* __restrict__ dw, float* __restrict__ db) {
   else db[R.off_b[l] + k - R.nw[l]] = s;
 }
 
-// transposed, flipped weights for the data gradient: wt[ci][co][8 - tap]
+// transposed, flipped weights for the data gradients, wt[ci][co][8 - tap], of
+// layers 1 .. 5 (each at its own offset)
+struct FlipTab {
+  int off[6], cin[6], cout[6];
+};
+
 __global__ void flip_weights(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt,
-                             int cout, int cin) {
-  for (int e = blockIdx.x * NT + threadIdx.x; e < cout * cin * 9; e += gridDim.x * NT) {
-    const int co = e / (cin * 9), rem = e - co * cin * 9;
+                             const FlipTab f, int n) {
+  pdl_enter();
+  for (int e = f.off[1] + blockIdx.x * NT + threadIdx.x; e < n; e += gridDim.x * NT) {
+    int l = 1;
+    while (l < 5 && e >= f.off[l + 1]) ++l;
+    const int k = e - f.off[l], cin = f.cin[l];
+    const int co = k / (cin * 9), rem = k - co * cin * 9;
     const int ci = rem / 9, tap = rem - ci * 9;
-    wt[((size_t)ci * cout + co) * 9 + (8 - tap)] = w[e];
+    wt[f.off[l] + (ci * f.cout[l] + co) * 9 + (8 - tap)] = w[e];
   }
 }
 
-// g *= (1 - y^2) (tanh derivative), in place on the gradient
-__global__ void tanh_back(float* __restrict__ g, const float* __restrict__ y, size_t n) {
-  for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT)
-    g[k] *= 1.0f - y[k] * y[k];
-}
+// The backward of the layer inputs, each with the tanh derivative 1 - y^2 of the
+// activation it reaches (in the convolution's epilogue where the data gradient is
+// that input itself).  Separate passes for the pooling, the sum and the derivative
+// took 22 us of a 64 x 32^2 batch's step, the upsampling 12.
 
-__global__ void avgpool2_back(const float* __restrict__ gout, float* __restrict__ gin, int C,
-                              int B, int H, int W) {
-  const int Wo = W / 2, Ho = H / 2;
-  const size_t n = (size_t)C * B * H * W;
-  for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT) {
-    const int xx = (int)(k % W);
-    const size_t t = k / W;
-    const int yy = (int)(t % H);
-    const size_t cb = t / H;
-    gin[k] = 0.25f * gout[cb * (size_t)Ho * Wo + (size_t)(yy / 2) * Wo + xx / 2];
+// gradient of e2: the average pool's (g1 / 4, half resolution) plus the
+// concatenation's, then the derivative
+__global__ void pool_add_tanh_back(const float* __restrict__ g1, const float* __restrict__ g2,
+                                   const float* __restrict__ y, float* __restrict__ gin, int C,
+                                   int B, int H, int W) {
+  pdl_enter();
+  const unsigned n = (unsigned)C * B * H * W, uW = W, uH = H;
+  for (unsigned k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
+    const unsigned t = k / uW, xx = k - t * uW;
+    const unsigned cb = t / uH, yy = t - cb * uH;
+    const float yk = y[k];
+    gin[k] = (0.25f * g1[((size_t)cb * (uH / 2) + yy / 2) * (uW / 2) + xx / 2] + g2[k]) *
+             (1.0f - yk * yk);
   }
 }
 
-__global__ void upsample2_back(const float* __restrict__ gout, float* __restrict__ gin, int C,
-                               int B, int H, int W) {
-  const int Ho = H / 2, Wo = W / 2;
-  const size_t n = (size_t)C * B * Ho * Wo;
-  for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT) {
-    const int xo = (int)(k % Wo);
-    const size_t t = k / Wo;
-    const int yo = (int)(t % Ho);
-    const size_t cb = t / Ho;
-    const float* src = gout + cb * (size_t)H * W;
-    gin[k] = src[(size_t)(2 * yo) * W + 2 * xo] + src[(size_t)(2 * yo) * W + 2 * xo + 1] +
-             src[(size_t)(2 * yo + 1) * W + 2 * xo] + src[(size_t)(2 * yo + 1) * W + 2 * xo + 1];
+// gradient of m2 through the nearest upsampling: the 2x2 sum, then the derivative
+__global__ void upsample2_tanh_back(const float* __restrict__ gout, const float* __restrict__ y,
+                                    float* __restrict__ gin, int C, int B, int H, int W) {
+  pdl_enter();
+  const unsigned Ho = H / 2, Wo = W / 2, n = (unsigned)C * B * Ho * Wo;
+  for (unsigned k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
+    const unsigned t = k / Wo, xo = k - t * Wo;
+    const unsigned cb = t / Ho, yo = t - cb * Ho;
+    const float* q = gout + (size_t)cb * H * W + (size_t)(2 * yo) * W + 2 * xo;
+    const float yk = y[k];
+    gin[k] = (q[0] + q[1] + q[W] + q[W + 1]) * (1.0f - yk * yk);
   }
 }
 
-__global__ void add_inplace(float* __restrict__ a, const float* __restrict__ b, size_t n) {
-  for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT)
-    a[k] += b[k];
-}
+// one Adam step of the weights (the first n entries) and the biases
+struct AdamSet {
+  float *w, *m, *v;
+  const float* g;
+  __nv_bfloat16* wb;
+};
 
-__global__ void adam_kernel(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                            const float* __restrict__ g, __nv_bfloat16* __restrict__ wb, int n,
-                            float lr, float b1, float b2, float eps, float c1, float c2) {
-  for (int k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
-    const float g0 = g[k];
+__global__ void adam_kernel(const AdamSet W, const AdamSet Bi, int n, int nb, float lr, float b1,
+                            float b2, float eps, float c1, float c2) {
+  pdl_enter();
+  for (int e = blockIdx.x * NT + threadIdx.x; e < n + nb; e += gridDim.x * NT) {
+    const AdamSet& S = e < n ? W : Bi;
+    const int k = e < n ? e : e - n;
+    const float g0 = S.g[k];
     const float gk = isfinite(g0) ? g0 : 0.0f;   // a non-finite entry is skipped
-    const float mk = b1 * m[k] + (1.0f - b1) * gk;
-    const float vk = b2 * v[k] + (1.0f - b2) * gk * gk;
-    m[k] = mk;
-    v[k] = vk;
-    const float wk = w[k] - lr * (mk / c1) / (sqrtf(vk / c2) + eps);
-    w[k] = wk;
-    wb[k] = __float2bfloat16(wk);
+    const float mk = b1 * S.m[k] + (1.0f - b1) * gk;
+    const float vk = b2 * S.v[k] + (1.0f - b2) * gk * gk;
+    S.m[k] = mk;
+    S.v[k] = vk;
+    const float wk = S.w[k] - lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+    S.w[k] = wk;
+    S.wb[k] = __float2bfloat16(wk);
   }
 }
 
@@ -417,39 +437,58 @@ namespace unet {
 // (grid (P, B)), then one warp per image adds them in a fixed order
 constexpr int RMS_PARTS = 1024;   // partial-sum slots in the workspace
 
-__global__ void rms_part_kernel(const float* __restrict__ r, size_t npix, int P,
-                                float* __restrict__ part) {
+// part p of P of image b's sum of squares: a fixed set of cells in a fixed order (the
+// first NT threads' sums)
+__device__ __forceinline__ void rms_store_part(float acc, float* part, int slot) {
   __shared__ float red[NT / 32];
-  const int b = blockIdx.y, p = blockIdx.x;
-  float acc = 0.0f;
-  for (size_t k = (size_t)p * NT + threadIdx.x; k < npix; k += (size_t)P * NT) {
-    const float v = r[(size_t)b * npix + k];
-    acc += v * v;
-  }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  if ((threadIdx.x & 31) == 0 && threadIdx.x < NT) red[threadIdx.x >> 5] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
     float t = 0.0f;
     for (int i = 0; i < NT / 32; ++i) t += red[i];
-    part[b * P + p] = t;
+    part[slot] = t;
   }
+}
+
+__global__ void rms_part_kernel(const float* __restrict__ r, size_t npix, int P,
+                                float* __restrict__ part) {
+  pdl_enter();
+  const int b = blockIdx.y, p = blockIdx.x;
+  float acc = 0.0f;
+#pragma unroll 4
+  for (size_t k = (size_t)p * NT + threadIdx.x; k < npix; k += (size_t)P * NT) {
+    const float v = r[(size_t)b * npix + k];
+    acc += v * v;
+  }
+  rms_store_part(acc, part, b * P + p);
+}
+
+// s of image b from its parts, by a whole warp
+__device__ __forceinline__ float rms_of(const float* part, int P, int b, size_t npix) {
+  float t = 0.0f;
+  for (int p = threadIdx.x & 31; p < P; p += 32) t += part[b * P + p];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return fmaxf(sqrtf(t / (float)npix), 1e-30f);
 }
 
 __global__ void rms_final_kernel(const float* __restrict__ part, int P, size_t npix,
                                  float* __restrict__ s) {
-  const int b = blockIdx.x;
-  float t = 0.0f;
-  for (int p = threadIdx.x; p < P; p += 32) t += part[b * P + p];
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (threadIdx.x == 0) s[b] = fmaxf(sqrtf(t / (float)npix), 1e-30f);
+  pdl_enter();
+  const float v = rms_of(part, P, blockIdx.x, npix);
+  if (threadIdx.x == 0) s[blockIdx.x] = v;
 }
 
-static void rms(const float* r, int B, size_t npix, float* part, float* s, cudaStream_t st) {
-  int P = (int)std::min<size_t>(256, std::max<size_t>(1, npix / (NT * 16)));
-  P = std::max(1, std::min(P, RMS_PARTS / std::max(1, B)));
-  rms_part_kernel<<<dim3(P, B), NT, 0, st>>>(r, npix, P, part);
-  rms_final_kernel<<<B, 32, 0, st>>>(part, P, npix, s);
+static int rms_parts(int B, size_t npix) {
+  const int P = (int)std::min<size_t>(256, std::max<size_t>(1, npix / (NT * 16)));
+  return std::max(1, std::min(P, RMS_PARTS / std::max(1, B)));
+}
+
+static int rms(const float* r, int B, size_t npix, float* part, float* s, cudaStream_t st) {
+  const int P = rms_parts(B, npix);
+  ZB_CUDA_TRY(pdl_launch(rms_part_kernel, dim3(P, B), dim3(NT), 0, st, r, npix, P, part));
+  ZB_CUDA_TRY(pdl_launch(rms_final_kernel, dim3(B), dim3(32), 0, st, (const float*)part, P, npix, s));
+  return ZB_OK;
 }
 
 // cell coefficient of image b's cell (i, j) from its faces: cx (B, H+1, W),
@@ -465,6 +504,7 @@ __device__ __forceinline__ float cell_c(const float* cx, const float* cy, int b,
 __global__ void features_kernel(const float* __restrict__ r, const float* __restrict__ s,
                                 const float* __restrict__ cx, const float* __restrict__ cy,
                                 int B, int H, int W, float inv_cmax, float* __restrict__ in) {
+  pdl_enter();
   const size_t npix = (size_t)H * W, n = (size_t)B * npix;
   for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT) {
     const int b = (int)(k / npix);
@@ -475,19 +515,32 @@ __global__ void features_kernel(const float* __restrict__ r, const float* __rest
   }
 }
 
-// the same two input channels as one chunk of the chunked bf16 layout
-// (channels 2..7 zero), each rounded as the planar kernel rounds them
-__global__ void features_cb8_kernel(const float* __restrict__ r, const float* __restrict__ s,
-                                    const float* __restrict__ cx, const float* __restrict__ cy,
-                                    int B, int H, int W, float inv_cmax, uint4* __restrict__ in) {
-  const size_t npix = (size_t)H * W, n = (size_t)B * npix;
-  for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT) {
-    const int b = (int)(k / npix);
-    const size_t p = k - (size_t)b * npix;
-    const int i = (int)(p / W), j = (int)(p - (size_t)i * W);
+// the same two input channels of one image as one chunk of the chunked bf16 layout
+// (channels 2..7 zero), each rounded as the planar kernel rounds them.  Every block
+// adds the P parts of s itself (in rms_final_kernel's order); block 0 stores it.
+__global__ void __launch_bounds__(NT)
+features_cb8_kernel(const float* __restrict__ r, const float* __restrict__ part, int P,
+                    float* __restrict__ s_out, const float* __restrict__ cx,
+                    const float* __restrict__ cy, int H, int W, float inv_cmax,
+                    uint4* __restrict__ in) {
+  pdl_enter();
+  __shared__ float sh;
+  const unsigned n = (unsigned)H * W, uW = W;
+  if (threadIdx.x < 32) {
+    const float v = rms_of(part, P, 0, n);
+    if (threadIdx.x == 0) {
+      sh = v;
+      if (blockIdx.x == 0) s_out[0] = v;
+    }
+  }
+  __syncthreads();
+  const float s = sh;
+#pragma unroll 2
+  for (unsigned k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
+    const unsigned i = k / uW, j = k - i * uW;
     __align__(16) __nv_bfloat16 v[8];
-    v[0] = __float2bfloat16_rn(r[k] / s[b]);
-    v[1] = __float2bfloat16_rn(cell_c(cx, cy, b, H, W, i, j) * inv_cmax);
+    v[0] = __float2bfloat16_rn(r[k] / s);
+    v[1] = __float2bfloat16_rn(cell_c(cx, cy, 0, H, W, i, j) * inv_cmax);
 #pragma unroll
     for (int c = 2; c < 8; ++c) v[c] = __float2bfloat16_rn(0.0f);
     in[k] = *(const uint4*)v;
@@ -498,11 +551,11 @@ __global__ void features_cb8_kernel(const float* __restrict__ r, const float* __
 __global__ void scale_out_kernel(const float* __restrict__ out, const float* __restrict__ s,
                                  const float* __restrict__ cx, const float* __restrict__ cy,
                                  int B, int H, int W, float dx2, const float* x_in, float* y) {
-  const size_t npix = (size_t)H * W, n = (size_t)B * npix;
-  for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT) {
-    const int b = (int)(k / npix);
-    const size_t p = k - (size_t)b * npix;
-    const int i = (int)(p / W), j = (int)(p - (size_t)i * W);
+  pdl_enter();
+  const unsigned npix = (unsigned)H * W, n = B * npix, uW = W;
+  for (unsigned k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
+    const unsigned b = k / npix, p = k - b * npix;
+    const int i = (int)(p / uW), j = (int)(p - i * uW);
     const float v = s[b] * dx2 / cell_c(cx, cy, b, H, W, i, j) * out[k];
     y[k] = x_in ? x_in[k] + v : v;
   }
@@ -512,28 +565,77 @@ __device__ __forceinline__ float xg(const float* x, int H, int W, int i, int j, 
   return (i < 0 || i >= H || j < 0 || j >= W) ? -self : x[(size_t)i * W + j];
 }
 
-// res = f - A x per image (Dirichlet ghost -x), with x null meaning zero
+// f - A x at cell (i, j) of an image whose arrays start at x, ax, ay (Dirichlet
+// ghost -x; x null means zero)
+__device__ __forceinline__ float residual_at(float f, const float* x, const float* ax_,
+                                             const float* ay_, int H, int W, int i, int j,
+                                             float idx2) {
+  float ax = 0.0f;
+  if (x) {
+    const float xc = x[(size_t)i * W + j];
+    ax = (ax_[(size_t)(i + 1) * W + j] * (xc - xg(x, H, W, i + 1, j, xc)) +
+          ax_[(size_t)i * W + j] * (xc - xg(x, H, W, i - 1, j, xc)) +
+          ay_[(size_t)i * (W + 1) + j + 1] * (xc - xg(x, H, W, i, j + 1, xc)) +
+          ay_[(size_t)i * (W + 1) + j] * (xc - xg(x, H, W, i, j - 1, xc))) * idx2;
+  }
+  return f - ax;
+}
+
+// res = f - A x per image
 __global__ void patch_residual(const float* __restrict__ f, const float* __restrict__ x,
                                const float* __restrict__ cx, const float* __restrict__ cy,
                                int B, int H, int W, float idx2, float* __restrict__ res) {
-  const size_t npix = (size_t)H * W, n = (size_t)B * npix;
-  for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT) {
-    const int b = (int)(k / npix);
-    const size_t p = k - (size_t)b * npix;
-    const int i = (int)(p / W), j = (int)(p - (size_t)i * W);
-    float ax = 0.0f;
-    if (x) {
-      const float* xb = x + (size_t)b * npix;
-      const float* ax_ = cx + (size_t)b * (H + 1) * W;
-      const float* ay_ = cy + (size_t)b * H * (W + 1);
-      const float xc = xb[p];
-      ax = (ax_[(size_t)(i + 1) * W + j] * (xc - xg(xb, H, W, i + 1, j, xc)) +
-            ax_[(size_t)i * W + j] * (xc - xg(xb, H, W, i - 1, j, xc)) +
-            ay_[(size_t)i * (W + 1) + j + 1] * (xc - xg(xb, H, W, i, j + 1, xc)) +
-            ay_[(size_t)i * (W + 1) + j] * (xc - xg(xb, H, W, i, j - 1, xc))) * idx2;
-    }
-    res[k] = f[k] - ax;
+  pdl_enter();
+  const unsigned npix = (unsigned)H * W, n = B * npix, uW = W;
+  for (unsigned k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
+    const unsigned b = k / npix, p = k - b * npix;
+    const int i = (int)(p / uW), j = (int)(p - i * uW);
+    res[k] = residual_at(f[k], x ? x + (size_t)b * npix : nullptr, cx + (size_t)b * (H + 1) * W,
+                         cy + (size_t)b * H * (W + 1), H, W, i, j, idx2);
   }
+}
+
+// res = f - A x of one image and the parts of its sum of squares.  The parts are
+// rms_part_kernel's, cell for cell and in its order (the same bits), but four
+// threads share one of its threads' cells: they leave them in shared memory, 16 at
+// a time, and one adds them in order.  Bound by the latency of its loads; 1024^2: 11 us
+// and 10 for the separate sum, now 10.7 (one thread per sum: 17.6).
+constexpr int RR_SPLIT = 4, RR_CELLS = 16;
+
+__global__ void __launch_bounds__(NT * RR_SPLIT)
+residual_rms_kernel(const float* __restrict__ f, const float* __restrict__ x,
+                    const float* __restrict__ cx, const float* __restrict__ cy, int H, int W,
+                    float idx2, float* __restrict__ res, int P, float* __restrict__ part) {
+  pdl_enter();
+  __shared__ float sv[RR_CELLS][NT];
+  const unsigned n = (unsigned)H * W, uW = W, stride = (unsigned)P * NT;
+  const unsigned t = threadIdx.x % NT, q = threadIdx.x / NT;
+  float acc = 0.0f;
+  for (unsigned k0 = blockIdx.x * NT; k0 < n; k0 += RR_CELLS * stride) {
+    float v[RR_CELLS / RR_SPLIT];
+#pragma unroll
+    for (int u = 0; u < RR_CELLS / RR_SPLIT; ++u) {
+      const unsigned k = k0 + t + (RR_SPLIT * u + q) * stride;
+      v[u] = 0.0f;   // adds nothing to the sum
+      if (k < n) {
+        const unsigned i = k / uW;
+        v[u] = residual_at(f[k], x, cx, cy, H, W, (int)i, (int)(k - i * uW), idx2);
+      }
+    }
+    __syncthreads();   // the sum of the cells before
+#pragma unroll
+    for (int u = 0; u < RR_CELLS / RR_SPLIT; ++u) {
+      const unsigned k = k0 + t + (RR_SPLIT * u + q) * stride;
+      if (k < n) res[k] = v[u];
+      sv[RR_SPLIT * u + q][t] = v[u];
+    }
+    __syncthreads();
+    if (q == 0) {
+#pragma unroll
+      for (int c = 0; c < RR_CELLS; ++c) acc += sv[c][t] * sv[c][t];
+    }
+  }
+  rms_store_part(acc, part, blockIdx.x);
 }
 
 // loss terms per image: lnum[b] = a_b . b_b, lden[b] = c_b . d_b (residual
@@ -543,6 +645,7 @@ __global__ void patch_residual(const float* __restrict__ f, const float* __restr
 __global__ void loss_kernel(const float* __restrict__ a_, const float* __restrict__ b_,
                             const float* __restrict__ c_, const float* __restrict__ d_, int B,
                             size_t npix, float* __restrict__ lnum, float* __restrict__ lden) {
+  pdl_enter();
   __shared__ float red[2][NT / 32];
   const int b = blockIdx.x;
   float a = 0.0f, c = 0.0f;
@@ -567,24 +670,25 @@ __global__ void loss_kernel(const float* __restrict__ a_, const float* __restric
 
 __device__ __forceinline__ bool loss_counts(float den) { return den > 1e-30f && den < 3e38f; }
 
+// one warp, its lanes' sums added in a fixed order
 __global__ void loss_total(const float* lnum, const float* lden, int B, double* out) {
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int b = 0; b < B; ++b)
-      if (loss_counts(lden[b])) t += (double)lnum[b] / (double)lden[b];
-    *out = t / B;
-  }
+  pdl_enter();
+  double t = 0.0;
+  for (int b = threadIdx.x; b < B; b += 32)
+    if (loss_counts(lden[b])) t += (double)lnum[b] / (double)lden[b];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (threadIdx.x == 0) *out = t / B;
 }
 
 // A x per image (Dirichlet ghost -x)
 __global__ void patch_apply(const float* __restrict__ x, const float* __restrict__ cx,
                             const float* __restrict__ cy, int B, int H, int W, float idx2,
                             float* __restrict__ out) {
-  const size_t npix = (size_t)H * W, n = (size_t)B * npix;
-  for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT) {
-    const int b = (int)(k / npix);
-    const size_t p = k - (size_t)b * npix;
-    const int i = (int)(p / W), j = (int)(p - (size_t)i * W);
+  pdl_enter();
+  const unsigned npix = (unsigned)H * W, n = B * npix, uW = W;
+  for (unsigned k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
+    const unsigned b = k / npix, p = k - b * npix;
+    const int i = (int)(p / uW), j = (int)(p - i * uW);
     const float* xb = x + (size_t)b * npix;
     const float* ax_ = cx + (size_t)b * (H + 1) * W;
     const float* ay_ = cy + (size_t)b * H * (W + 1);
@@ -598,6 +702,7 @@ __global__ void patch_apply(const float* __restrict__ x, const float* __restrict
 
 __global__ void sub_kernel(const float* __restrict__ a, const float* __restrict__ b, size_t n,
                            float* __restrict__ out) {
+  pdl_enter();
   for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT)
     out[k] = a[k] - b[k];
 }
@@ -609,11 +714,11 @@ __global__ void loss_grad_kernel(const float* __restrict__ res, const float* __r
                                  const float* __restrict__ lden, const float* __restrict__ s,
                                  int B, int H, int W, float idx2, float dx2,
                                  float* __restrict__ dout) {
-  const size_t npix = (size_t)H * W, n = (size_t)B * npix;
-  for (size_t k = blockIdx.x * (size_t)NT + threadIdx.x; k < n; k += (size_t)gridDim.x * NT) {
-    const int b = (int)(k / npix);
-    const size_t p = k - (size_t)b * npix;
-    const int i = (int)(p / W), j = (int)(p - (size_t)i * W);
+  pdl_enter();
+  const unsigned npix = (unsigned)H * W, n = B * npix, uW = W;
+  for (unsigned k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
+    const unsigned b = k / npix, p = k - b * npix;
+    const int i = (int)(p / uW), j = (int)(p - i * uW);
     float ar;
     if (ar_in) {
       ar = ar_in[k];
@@ -692,7 +797,8 @@ static unsigned* unet_err_word() {
 
 static int conv_tc_launch(const float* inA, int cin_a, const float* inB, int cin,
                           const __nv_bfloat16* w, const float* bias, float* out, int cout, int B,
-                          int H, int W, int act, int mode_a, cudaStream_t st) {
+                          int H, int W, int act, int mode_a, const float* ytanh,
+                          cudaStream_t st) {
   const int cinp = pad16(cin), coutp = pad16(cout);
   if (coutp > 256 || cinp > 256) return ZB_E_UNSUPPORTED;
   int cols = 32;
@@ -733,8 +839,9 @@ static int conv_tc_launch(const float* inA, int cin_a, const float* inB, int cin
   switch (cinp / 16) {
 #define ZB_TC(G)                                                                               \
   case G:                                                                                      \
-    conv3x3_tc<G><<<grid, TC_THREADS, smem, st>>>(inA, cin_a, inB, cin, w, bias, out, cout, B, H, \
-                                                  W, act, mode_a, cols, unet_err_word());      \
+    ZB_CUDA_TRY(pdl_launch(conv3x3_tc<G>, dim3(grid), dim3(TC_THREADS), smem, st, inA, cin_a,  \
+                           inB, cin, w, bias, out, cout, B, H, W, act, mode_a, ytanh, cols,    \
+                           unet_err_word()));                                                  \
     break
     ZB_TC(1); ZB_TC(2); ZB_TC(3); ZB_TC(5);
 #undef ZB_TC
@@ -850,12 +957,14 @@ static int conv_cb8_launch(const uint4* inA, int chA, int mode_a, const uint4* i
 
 static int conv(const float* inA, int cin_a, const float* inB, int cin,
                 const __nv_bfloat16* w, const float* bias, float* out, int cout, int B, int H,
-                int W, int act, cudaStream_t st, int mode_a = SRC_DIRECT) {
+                int W, int act, cudaStream_t st, int mode_a = SRC_DIRECT,
+                const float* ytanh = nullptr) {
   if (g_conv_impl >= 1)
-    return conv_tc_launch(inA, cin_a, inB, cin, w, bias, out, cout, B, H, W, act, mode_a, st);
+    return conv_tc_launch(inA, cin_a, inB, cin, w, bias, out, cout, B, H, W, act, mode_a, ytanh,
+                          st);
   dim3 grid((W + TS - 1) / TS, (H + TS - 1) / TS, B);
   switch (cout) {
-#define ZB_CONV(N) case N: conv3x3_fwd<N><<<grid, NTT, 0, st>>>(inA, cin_a, inB, cin, w, bias, out, B, H, W, act, mode_a); break;
+#define ZB_CONV(N) case N: conv3x3_fwd<N><<<grid, NTT, 0, st>>>(inA, cin_a, inB, cin, w, bias, out, B, H, W, act, mode_a, ytanh); break;
     ZB_CONV(1) ZB_CONV(8) ZB_CONV(16) ZB_CONV(24) ZB_CONV(32) ZB_CONV(48) ZB_CONV(72)
 #undef ZB_CONV
     default: return ZB_E_UNSUPPORTED;
@@ -880,12 +989,9 @@ static int wgrad(const float* inA, int cin_a, const float* inB, int cin, const f
     attr.fetch_or(1u << dev);
   }
   const dim3 grid(g.slots, g.nchunk);
-  if (cout % WG_COT == 0)
-    conv3x3_wgrad<WG_COT><<<grid, g.threads, g.smem, st>>>(inA, cin_a, inB, cin, dout, cout, part, B, H,
-                                                      W, mode_a, g.ncog, g.cic, g.nsl);
-  else
-    conv3x3_wgrad<1><<<grid, g.threads, g.smem, st>>>(inA, cin_a, inB, cin, dout, cout, part, B, H,
-                                                      W, mode_a, g.ncog, g.cic, g.nsl);
+  ZB_CUDA_TRY(pdl_launch(cout % WG_COT == 0 ? conv3x3_wgrad<WG_COT> : conv3x3_wgrad<1>, grid,
+                         dim3(g.threads), g.smem, st, inA, cin_a, inB, cin, dout, cout, part, B, H,
+                         W, mode_a, g.ncog, g.cic, g.nsl));
   return zb_launch_check();
 }
 
@@ -1015,12 +1121,13 @@ static int forward_cb8(const Net& n, const Acts& a, const ActsCB8& c, const __nv
   return zb_launch_check();
 }
 
-// data gradient through conv layer l: din (cin channels) from dout (cout)
-static int data_grad(const Net& n, int l, const __nv_bfloat16* w, __nv_bfloat16* wflip,
-                     const float* dout, float* din, int B, int H, int W, cudaStream_t st) {
+// data gradient through conv layer l: din (cin channels) from dout (cout) with the
+// flipped weights, times 1 - y^2 where y is given
+static int data_grad(const Net& n, int l, const __nv_bfloat16* wflip, const float* dout, float* din,
+                     int B, int H, int W, cudaStream_t st, const float* y = nullptr) {
   const int ci = n.cin[l], co = n.cout[l];
-  flip_weights<<<gridn((size_t)ci * co * 9), NT, 0, st>>>(w + n.off_w[l], wflip, co, ci);
-  return conv(dout, co, nullptr, co, wflip, nullptr, din, ci, B, H, W, ACT_NONE, st);
+  return conv(dout, co, nullptr, co, wflip + n.off_w[l], nullptr, din, ci, B, H, W, ACT_NONE, st,
+              SRC_DIRECT, y);
 }
 
 }  // namespace unet
@@ -1076,22 +1183,27 @@ int zb_smoother_apply(const zb_smoother* smo, const float* f, const float* x_in,
   const Acts a = acts_split(n, smo->act, 1, nx, ny, false);
   const float idx2 = (float)(1.0 / (dx * dx));
   const size_t N0 = (size_t)nx * ny;
-  patch_residual<<<gridn(N0), NT, 0, st>>>(f, x_in, cx, cy, 1, nx, ny, idx2, r_scratch);
-  rms(r_scratch, 1, N0, a.part, a.s, st);
+  const int P = rms_parts(1, N0);
+  ZB_CUDA_TRY(pdl_launch(residual_rms_kernel, dim3(P), dim3(NT * RR_SPLIT), 0, st, f, x_in, cx, cy, nx, ny,
+                         idx2, r_scratch, P, a.part));
   int rc;
   ActsCB8 c;
   if (g_conv_impl == 1 && acts_cb8(n, a, 1, nx, ny, &c)) {
-    features_cb8_kernel<<<gridn(N0), NT, 0, st>>>(r_scratch, a.s, cx, cy, 1, nx, ny,
-                                                  1.0f / smo->cmax, c.in);
+    ZB_CUDA_TRY(pdl_launch(features_cb8_kernel, dim3(std::min(gridn(N0), 148 * 8)), dim3(NT), 0, st,
+                           (const float*)r_scratch, (const float*)a.part, P, a.s, cx, cy, nx, ny,
+                           1.0f / smo->cmax, c.in));
     rc = forward_cb8(n, a, c, (const __nv_bfloat16*)smo->w, smo->b, 1, nx, ny, st);
   } else {
-    features_kernel<<<gridn(N0), NT, 0, st>>>(r_scratch, a.s, cx, cy, 1, nx, ny,
-                                              1.0f / smo->cmax, a.in);
+    ZB_CUDA_TRY(pdl_launch(rms_final_kernel, dim3(1), dim3(32), 0, st, (const float*)a.part, P, N0,
+                           a.s));
+    ZB_CUDA_TRY(pdl_launch(features_kernel, dim3(gridn(N0)), dim3(NT), 0, st,
+                           (const float*)r_scratch, (const float*)a.s, cx, cy, 1, nx, ny,
+                           1.0f / smo->cmax, a.in));
     rc = forward(n, a, (const __nv_bfloat16*)smo->w, smo->b, 1, nx, ny, st, ACT_TANH_SFU);
   }
   if (rc) return rc;
-  scale_out_kernel<<<gridn(N0), NT, 0, st>>>(a.out, a.s, cx, cy, 1, nx, ny, (float)(dx * dx),
-                                             x_in, x_out);
+  ZB_CUDA_TRY(pdl_launch(scale_out_kernel, dim3(gridn(N0)), dim3(NT), 0, st, (const float*)a.out,
+                         (const float*)a.s, cx, cy, 1, nx, ny, (float)(dx * dx), x_in, x_out));
   return zb_launch_check();
 }
 
@@ -1108,12 +1220,15 @@ int zb_unet_forward(const zb_unet_trainer* t, const float* r, const float* cx, c
   const Acts a = acts_split(n, t->act, t->batch, t->n, t->n, true);
   const int B = t->batch, H = t->n, W = t->n;
   const size_t N0 = (size_t)B * H * W;
-  rms(r, B, (size_t)H * W, a.part, a.s, st);
-  features_kernel<<<gridn(N0), NT, 0, st>>>(r, a.s, cx, cy, B, H, W, 1.0f / t->cmax, a.in);
-  int rc = forward(n, a, (const __nv_bfloat16*)t->w_bf16, t->b_master, B, H, W, st);
+  int rc = rms(r, B, (size_t)H * W, a.part, a.s, st);
   if (rc) return rc;
-  scale_out_kernel<<<gridn(N0), NT, 0, st>>>(a.out, a.s, cx, cy, B, H, W, (float)(dx * dx),
-                                             nullptr, y);
+  ZB_CUDA_TRY(pdl_launch(features_kernel, dim3(gridn(N0)), dim3(NT), 0, st, r, (const float*)a.s,
+                         cx, cy, B, H, W, 1.0f / t->cmax, a.in));
+  rc = forward(n, a, (const __nv_bfloat16*)t->w_bf16, t->b_master, B, H, W, st);
+  if (rc) return rc;
+  ZB_CUDA_TRY(pdl_launch(scale_out_kernel, dim3(gridn(N0)), dim3(NT), 0, st, (const float*)a.out,
+                         (const float*)a.s, cx, cy, B, H, W, (float)(dx * dx),
+                         (const float*)nullptr, y));
   return zb_launch_check();
 }
 
@@ -1131,45 +1246,54 @@ int zb_unet_backward(const zb_unet_trainer* t, const float* r, const float* targ
   int rc;
   // forward (keeps activations), y into a.tmp
   if ((rc = zb_unet_forward(t, r, cx, cy, dx, a.tmp, stream))) return rc;
+  const dim3 g0(gridn(N0)), nt(NT);
+  FlipTab ft;
+  for (int l = 0; l < 6; ++l) {
+    ft.off[l] = (int)n.off_w[l];
+    ft.cin[l] = n.cin[l];
+    ft.cout[l] = n.cout[l];
+  }
+  ZB_CUDA_TRY(pdl_launch(flip_weights, dim3(gridn(n.nw)), nt, 0, st, w, a.wflip, ft, (int)n.nw));
   if (target) {
     // energy loss: res = e - y, (res . A res) / (e . A e); A res -> d_out,
     // A e -> tmp (y is no longer needed once res is formed)
-    sub_kernel<<<gridn(N0), NT, 0, st>>>(target, a.tmp, N0, a.res);
-    patch_apply<<<gridn(N0), NT, 0, st>>>(a.res, cx, cy, B, H, W, idx2, a.d_out);
-    patch_apply<<<gridn(N0), NT, 0, st>>>(target, cx, cy, B, H, W, idx2, a.tmp);
-    loss_kernel<<<B, NT, 0, st>>>(a.res, a.d_out, target, a.tmp, B, (size_t)H * W, a.lnum, a.lden);
-    if (loss_out) loss_total<<<1, 32, 0, st>>>(a.lnum, a.lden, B, loss_out);
-    loss_grad_kernel<<<gridn(N0), NT, 0, st>>>(a.res, a.d_out, cx, cy, a.lden, a.s, B, H, W, idx2,
-                                               dx2, a.d_out);
+    ZB_CUDA_TRY(pdl_launch(sub_kernel, g0, nt, 0, st, target, (const float*)a.tmp, N0, a.res));
+    ZB_CUDA_TRY(pdl_launch(patch_apply, g0, nt, 0, st, (const float*)a.res, cx, cy, B, H, W, idx2,
+                           a.d_out));
+    ZB_CUDA_TRY(pdl_launch(patch_apply, g0, nt, 0, st, target, cx, cy, B, H, W, idx2, a.tmp));
+    ZB_CUDA_TRY(pdl_launch(loss_kernel, dim3(B), nt, 0, st, (const float*)a.res,
+                           (const float*)a.d_out, target, (const float*)a.tmp, B, (size_t)H * W,
+                           a.lnum, a.lden));
   } else {
-    patch_residual<<<gridn(N0), NT, 0, st>>>(r, a.tmp, cx, cy, B, H, W, idx2, a.res);
-    loss_kernel<<<B, NT, 0, st>>>(a.res, a.res, r, r, B, (size_t)H * W, a.lnum, a.lden);
-    if (loss_out) loss_total<<<1, 32, 0, st>>>(a.lnum, a.lden, B, loss_out);
-    loss_grad_kernel<<<gridn(N0), NT, 0, st>>>(a.res, nullptr, cx, cy, a.lden, a.s, B, H, W, idx2,
-                                               dx2, a.d_out);
+    ZB_CUDA_TRY(pdl_launch(patch_residual, g0, nt, 0, st, r, (const float*)a.tmp, cx, cy, B, H, W,
+                           idx2, a.res));
+    ZB_CUDA_TRY(pdl_launch(loss_kernel, dim3(B), nt, 0, st, (const float*)a.res,
+                           (const float*)a.res, r, r, B, (size_t)H * W, a.lnum, a.lden));
   }
+  if (loss_out)
+    ZB_CUDA_TRY(pdl_launch(loss_total, dim3(1), dim3(32), 0, st, (const float*)a.lnum,
+                           (const float*)a.lden, B, loss_out));
+  ZB_CUDA_TRY(pdl_launch(loss_grad_kernel, g0, nt, 0, st, (const float*)a.res,
+                         (const float*)(target ? a.d_out : nullptr), cx, cy, (const float*)a.lden,
+                         (const float*)a.s, B, H, W, idx2, dx2, a.d_out));
   // out = conv(o1)
   if ((rc = wgrad(a.o1, n.c1, nullptr, n.c1, a.d_out, 1, a.wpart[5], B, H, W, st))) return rc;
-  if ((rc = data_grad(n, 5, w, a.wflip, a.d_out, a.d_o1, B, H, W, st))) return rc;
-  tanh_back<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_o1, a.o1, (size_t)n.c1 * N0);
+  if ((rc = data_grad(n, 5, a.wflip, a.d_out, a.d_o1, B, H, W, st, a.o1))) return rc;
   // o1 = tanh(conv([u, e2]))
   if ((rc = wgrad(a.m2, n.c2, a.e2, n.c2 + n.c1, a.d_o1, n.c1, a.wpart[4], B, H, W, st, SRC_UP))) return rc;
-  if ((rc = data_grad(n, 4, w, a.wflip, a.d_o1, a.d_cat, B, H, W, st))) return rc;
+  if ((rc = data_grad(n, 4, a.wflip, a.d_o1, a.d_cat, B, H, W, st))) return rc;
   // d_cat = [du (c2), de2_b (c1)]
-  upsample2_back<<<gridn((size_t)n.c2 * N1), NT, 0, st>>>(a.d_cat, a.d_m2, n.c2, B, H, W);
-  tanh_back<<<gridn((size_t)n.c2 * N1), NT, 0, st>>>(a.d_m2, a.m2, (size_t)n.c2 * N1);
+  ZB_CUDA_TRY(pdl_launch(upsample2_tanh_back, dim3(gridn((size_t)n.c2 * N1)), nt, 0, st,
+                         (const float*)a.d_cat, (const float*)a.m2, a.d_m2, n.c2, B, H, W));
   if ((rc = wgrad(a.m1, n.c2, nullptr, n.c2, a.d_m2, n.c2, a.wpart[3], B, H1, W1, st))) return rc;
-  if ((rc = data_grad(n, 3, w, a.wflip, a.d_m2, a.d_m1, B, H1, W1, st))) return rc;
-  tanh_back<<<gridn((size_t)n.c2 * N1), NT, 0, st>>>(a.d_m1, a.m1, (size_t)n.c2 * N1);
+  if ((rc = data_grad(n, 3, a.wflip, a.d_m2, a.d_m1, B, H1, W1, st, a.m1))) return rc;
   if ((rc = wgrad(a.e2, n.c1, nullptr, n.c1, a.d_m1, n.c2, a.wpart[2], B, H1, W1, st, SRC_POOL))) return rc;
-  if ((rc = data_grad(n, 2, w, a.wflip, a.d_m1, a.d_p, B, H1, W1, st))) return rc;
-  avgpool2_back<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_p, a.d_e2, n.c1, B, H, W);
-  add_inplace<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_e2, a.d_cat + (size_t)n.c2 * N0,
-                                                       (size_t)n.c1 * N0);
-  tanh_back<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_e2, a.e2, (size_t)n.c1 * N0);
+  if ((rc = data_grad(n, 2, a.wflip, a.d_m1, a.d_p, B, H1, W1, st))) return rc;
+  ZB_CUDA_TRY(pdl_launch(pool_add_tanh_back, dim3(gridn((size_t)n.c1 * N0)), nt, 0, st,
+                         (const float*)a.d_p, (const float*)(a.d_cat + (size_t)n.c2 * N0),
+                         (const float*)a.e2, a.d_e2, n.c1, B, H, W));
   if ((rc = wgrad(a.e1, n.c1, nullptr, n.c1, a.d_e2, n.c1, a.wpart[1], B, H, W, st))) return rc;
-  if ((rc = data_grad(n, 1, w, a.wflip, a.d_e2, a.d_e1, B, H, W, st))) return rc;
-  tanh_back<<<gridn((size_t)n.c1 * N0), NT, 0, st>>>(a.d_e1, a.e1, (size_t)n.c1 * N0);
+  if ((rc = data_grad(n, 1, a.wflip, a.d_e2, a.d_e1, B, H, W, st, a.e1))) return rc;
   if ((rc = wgrad(a.in, 2, nullptr, 2, a.d_e1, n.c1, a.wpart[0], B, H, W, st))) return rc;
   WgReduce R;
   R.first[0] = 0;
@@ -1184,7 +1308,7 @@ int zb_unet_backward(const zb_unet_trainer* t, const float* r, const float* targ
     R.off_b[l] = (int)n.off_b[l];
     R.first[l + 1] = R.first[l] + R.nw[l] + R.nb[l];
   }
-  wgrad_reduce<<<(R.first[6] + 31) / 32, NT, 0, st>>>(R, t->g_w, t->g_b);
+  ZB_CUDA_TRY(pdl_launch(wgrad_reduce, dim3((R.first[6] + 31) / 32), nt, 0, st, R, t->g_w, t->g_b));
   return zb_launch_check();
 }
 
@@ -1194,13 +1318,11 @@ int zb_unet_adam(const zb_unet_trainer* t, float lr, int step, zb_stream_t strea
   const Net n = net_layout(t->c1, t->c2);
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
-  adam_kernel<<<gridn(n.nw), NT, 0, st>>>(t->w_master, t->m_w, t->v_w, t->g_w,
-                                          (__nv_bfloat16*)t->w_bf16, (int)n.nw, lr, b1, b2, eps,
-                                          c1, c2);
   // biases stay float32: the bf16 shadow is only written for the weights
-  adam_kernel<<<gridn(n.nb), NT, 0, st>>>(t->b_master, t->m_b, t->v_b, t->g_b,
-                                          (__nv_bfloat16*)t->b_shadow, (int)n.nb, lr, b1, b2,
-                                          eps, c1, c2);
+  const AdamSet W = {t->w_master, t->m_w, t->v_w, t->g_w, (__nv_bfloat16*)t->w_bf16};
+  const AdamSet Bi = {t->b_master, t->m_b, t->v_b, t->g_b, (__nv_bfloat16*)t->b_shadow};
+  ZB_CUDA_TRY(pdl_launch(adam_kernel, dim3(gridn(n.nw + n.nb)), dim3(NT), 0, st, W, Bi, (int)n.nw,
+                         (int)n.nb, lr, b1, b2, eps, c1, c2));
   return zb_launch_check();
 }
 
