@@ -473,9 +473,12 @@ enum { CB_OUT_CHUNKED = 0, CB_OUT_F32 = 1 };
 // free, its tensor copies landed, its cp.async copies landed; acc_full /
 // acc_free[k]: accumulator buffer k.  With all warps in step (stage, MMA,
 // epilogue) and several CTAs per SM to overlap, one application on 1024^2 (24, 48)
-// took 429 us, now 242: the wide layer (o1) 143 -> 83, at the 32 cycles that an MMA
-// takes to read its A operand from shared memory (180 a region), e1 44 -> 27, e2 68
-// -> 41, m1 35 -> 19, m2 63 -> 22, out 47 -> 34.
+// took 429 us, now 242 (convolutions 415 -> 226): the wide layer (o1) 143 -> 83, which
+// is the 32 cycles that each of a region's 180 MMAs (M = 128, N = 32) takes, e1 44 ->
+// 27, e2 68 -> 41, m1 35 -> 19, m2 63 -> 22, out 47 -> 34.  Lines of 128 pixels as
+// tiles, the three rows of taps in one MMA (N = 96, a third of the MMAs), gave 218 us
+// for the application: an MMA takes about N cycles in every form, and as an output's
+// accumulator then moves from line to line, the lines wait for one another.
 //
 // Every wait is bounded: on a timeout the role raises the CTA's failure flag (which
 // ends every other wait) and the error word, waits, bounded, for its own copies or
