@@ -117,13 +117,13 @@ conv3x3_fwd(const float* __restrict__ inA, int cin_a, const float* __restrict__ 
 // the partial sets in order, so the gradients are deterministic.  One thread per
 // weight walking the pixels in shared memory with a float atomic per tile, as
 // before, was bound by its two shared loads per FMA: the six layers of a
-// 64 x 32^2 batch (24, 48) took 1234 us, now 285 and 15 for the reduction (the
-// FMA pipe's floor is 50; the copies of the halo tiles are the rest).
+// 64 x 32^2 batch (24, 48) took 1234 us, now 201 and 13 for the reduction (the
+// FMA pipe's floor is 35; the copies of the halo tiles are the rest).
 constexpr int WG_TX = 16, WG_TY = 4, WG_SEG = 8;          // tile, pixels per row segment
 constexpr int WG_HX = WG_TX + 2, WG_HY = WG_TY + 2;
 constexpr int WG_PLANE = WG_HX * WG_HY + 1;               // odd: lanes of a warp hit 32 banks
 constexpr int WG_UNITS = WG_TY * (WG_TX / WG_SEG);        // row segments of a tile
-constexpr int WG_MAX_THREADS = 448;                       // two CTAs of 72 registers a thread
+constexpr int WG_MAX_THREADS = 320;                       // two CTAs of 96 registers a thread
 constexpr int WG_COT = 4;                                 // output channels of a thread
 constexpr int WG_SLOTS = 296;                             // partial sets: two CTAs per SM
 
@@ -132,9 +132,16 @@ struct WgShape {
   size_t smem, part;   // bytes of shared memory; floats of one partial set
 };
 
+// the upsampled source of the concatenation layer: tiles of UG_Y x UG_X of its pixels
+// and the output gradients around them
+constexpr int UG_X = 8, UG_Y = 4, UG_P = UG_X * UG_Y;
+constexpr int UG_FX = 2 * UG_X + 2, UG_FY = 2 * UG_Y + 2, UG_FS = UG_FX * UG_FY + 1;
+constexpr int UG_THREADS = 288;
+
 // channel groups, input channels per chunk (the ones channel included), slices
-// and threads of a layer's CTAs
-static WgShape wg_shape(int cin, int cout, int B, int H, int W) {
+// and threads of a layer's CTAs; up: the input channels in front of these that are
+// upsampled (conv3x3_wgrad_up's, which fills the same partial sets)
+static WgShape wg_shape(int cin, int cout, int B, int H, int W, int up) {
   WgShape g;
   const int cot = cout % WG_COT == 0 ? WG_COT : 1;
   g.ncog = cout / cot;
@@ -145,13 +152,17 @@ static WgShape wg_shape(int cin, int cout, int B, int H, int W) {
   g.nsl = std::max(1, std::min(WG_UNITS, WG_MAX_THREADS / pairs));
   g.threads = (pairs * g.nsl + 31) / 32 * 32;
   const long long ntiles = (long long)((W + WG_TX - 1) / WG_TX) * ((H + WG_TY - 1) / WG_TY) * B;
-  g.slots = (int)std::min<long long>(ntiles, WG_SLOTS);
+  const long long utiles =
+      (long long)((W / 2 + UG_X - 1) / UG_X) * ((H / 2 + UG_Y - 1) / UG_Y) * B;
+  // as few partial sets as take the same number of rounds
+  const long long nt = up ? utiles : ntiles, rounds = (nt + WG_SLOTS - 1) / WG_SLOTS;
+  g.slots = (int)((nt + rounds - 1) / rounds);
   const size_t stage =
       2 * ((((size_t)g.cic * WG_PLANE + 3) & ~(size_t)3) +
            (size_t)WG_TX * WG_TY * (cot > 1 ? cout + 4 : 1));
   const size_t red = g.nsl > 1 ? (size_t)pairs * g.nsl * 9 * cot : 0;
   g.smem = std::max(stage, red) * sizeof(float);
-  g.part = (size_t)cout * cin * 9 + cout;
+  g.part = (size_t)cout * (up + cin) * 9 + cout;
   return g;
 }
 
@@ -163,9 +174,9 @@ __device__ __forceinline__ void cp_async4z(float* dst, const float* src, bool va
 
 template <int COT>
 __global__ void __launch_bounds__(WG_MAX_THREADS, 2)
-conv3x3_wgrad(const float* __restrict__ inA, int cin_a, const float* __restrict__ inB, int cin,
-              const float* __restrict__ dout, int cout, float* __restrict__ part, int B, int H,
-              int W, int mode_a, int ncog, int cic, int nsl) {
+conv3x3_wgrad(const float* __restrict__ in, int cin, const float* __restrict__ dout, int cout,
+              float* __restrict__ part, int up, int B, int H, int W, int mode, int ncog, int cic,
+              int nsl) {
   pdl_enter();
   extern __shared__ __align__(16) float wsm[];
   const int nt = blockDim.x, tid = threadIdx.x;
@@ -205,20 +216,17 @@ conv3x3_wgrad(const float* __restrict__ inA, int cin_a, const float* __restrict_
       const int yy = y0 - 1 + r, c = c_lo + cc;
       const bool yin = yy >= 0 && yy < H;
       float* dst = sin_ + cc * WG_PLANE + r * WG_HX;
-      if (mode_a == SRC_POOL && c < cin_a) {   // the average is formed, not copied
-        dst[1 + hl] = (yin && xin) ? src_at(inA, cin_a, inB, mode_a, c, b, B, H, W, yy, xx) : 0.0f;
+      if (mode == SRC_POOL) {   // the average is formed, not copied
+        dst[1 + hl] =
+            (yin && xin) ? src_at(in, cin, nullptr, SRC_POOL, c, b, B, H, W, yy, xx) : 0.0f;
         if (hl < 2)
-          dst[hcol] = (yin && hin) ? src_at(inA, cin_a, inB, mode_a, c, b, B, H, W, yy, xh) : 0.0f;
+          dst[hcol] =
+              (yin && hin) ? src_at(in, cin, nullptr, SRC_POOL, c, b, B, H, W, yy, xh) : 0.0f;
         continue;
       }
-      const bool up = mode_a == SRC_UP && c < cin_a;
-      const float* row = inA;
-      if (yin)
-        row = c >= cin_a ? inB + (size_t)(c - cin_a) * plane + img + yy * W
-              : up ? inA + ((size_t)c * B + b) * (H >> 1) * (W >> 1) + (yy >> 1) * (W >> 1)
-                   : inA + (size_t)c * plane + img + yy * W;
-      cp_async4z(dst + 1 + hl, row + (yin && xin ? (up ? xx >> 1 : xx) : 0), yin && xin);
-      if (hl < 2) cp_async4z(dst + hcol, row + (yin && hin ? (up ? xh >> 1 : xh) : 0), yin && hin);
+      const float* row = in + (yin ? (size_t)c * plane + img + yy * W : 0);
+      cp_async4z(dst + 1 + hl, row + (yin && xin ? xx : 0), yin && xin);
+      if (hl < 2) cp_async4z(dst + hcol, row + (yin && hin ? xh : 0), yin && hin);
     }
     for (int e = hw; e < cout * WG_TY; e += nhw) {
       const int c = e / WG_TY, r = e - c * WG_TY;
@@ -302,22 +310,132 @@ conv3x3_wgrad(const float* __restrict__ inA, int cin_a, const float* __restrict_
   }
   if (!work) return;
   const int gci = c_lo + ci;
-  float* out = part + (size_t)blockIdx.x * ((size_t)cout * cin * 9 + cout);
+  const int ct = up + cin;   // the layer's input channels
+  float* out = part + (size_t)blockIdx.x * ((size_t)cout * ct * 9 + cout);
   if (gci < cin) {
 #pragma unroll
     for (int c = 0; c < COT; ++c)
 #pragma unroll
-      for (int k = 0; k < 9; ++k) out[((size_t)(cog * COT + c) * cin + gci) * 9 + k] = acc[c][k];
+      for (int k = 0; k < 9; ++k)
+        out[(size_t)((cog * COT + c) * 9 + k) * ct + up + gci] = acc[c][k];
   } else {
 #pragma unroll
-    for (int c = 0; c < COT; ++c) out[(size_t)cout * cin * 9 + cog * COT + c] = acc[c][4];
+    for (int c = 0; c < COT; ++c) out[(size_t)cout * ct * 9 + cog * COT + c] = acc[c][4];
   }
 }
 
-// the partial sets of all six layers added in order
+// Weight gradients of the upsampled channels of the concatenation layer (the first cin
+// of its cin + direct inputs), at the source's resolution.  in(p + tap - 1) is the
+// source's pixel P for p in a 2 x 2 block that depends on the tap, so
+//   dW[co][ci][tap] = sum_P in[ci](P) S[co][tap](P),  S = the block's sum of dout:
+// a quarter of the products.  A CTA forms S of a tile (32 source pixels) once in shared
+// memory; a thread owns one input and four output channels with all nine taps, and per
+// pixel one value and nine 16-byte loads (the same address for most of a warp) feed 36
+// FMAs.  64 x 32^2, 48 + 24 -> 24 channels: all 72 channels at full resolution 116 us,
+// now 30 here and 41 for the other 24.
+__global__ void __launch_bounds__(UG_THREADS, 2)
+conv3x3_wgrad_up(const float* __restrict__ in, int cin, const float* __restrict__ dout, int cout,
+                 float* __restrict__ part, int direct, int B, int H, int W, int nsl) {
+  pdl_enter();
+  extern __shared__ __align__(16) float wsm[];
+  float* S = wsm;                                 // [pixel][tap][cout]
+  float* sin_ = S + UG_P * 9 * cout;              // [cin][pixel], odd stride
+  float* sd = sin_ + cin * (UG_P + 1);            // [cout][fine pixel], odd stride
+  const int tid = threadIdx.x;
+  const int h = H / 2, w = W / 2, pairs = cin * (cout / WG_COT);
+  const int sl = tid / pairs, pr = tid - sl * pairs;
+  const int cog = pr / cin, ci = pr - cog * cin;
+  const bool work = sl < nsl;
+  const int tx = (w + UG_X - 1) / UG_X, ty = (h + UG_Y - 1) / UG_Y, ntiles = tx * ty * B;
+  float acc[WG_COT][9];
+#pragma unroll
+  for (int c = 0; c < WG_COT; ++c)
+#pragma unroll
+    for (int k = 0; k < 9; ++k) acc[c][k] = 0.0f;
+#pragma unroll 1
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const int b = t / (tx * ty), rt = t - b * (tx * ty);
+    const int x0 = (rt % tx) * UG_X, y0 = (rt / tx) * UG_Y;
+    for (int e = tid; e < cout * UG_FX * UG_FY; e += UG_THREADS) {
+      const int c = e / (UG_FX * UG_FY), q = e - c * (UG_FX * UG_FY);
+      const int fy = q / UG_FX, yy = 2 * y0 - 1 + fy, xx = 2 * x0 - 1 + q - fy * UG_FX;
+      const bool ok = yy >= 0 && yy < H && xx >= 0 && xx < W;
+      cp_async4z(sd + c * UG_FS + q,
+                 ok ? dout + (((size_t)c * B + b) * H + yy) * W + xx : dout, ok);
+    }
+    for (int e = tid; e < cin * UG_P; e += UG_THREADS) {
+      const int c = e / UG_P, q = e % UG_P, yy = y0 + q / UG_X, xx = x0 + q % UG_X;
+      const bool ok = yy < h && xx < w;
+      cp_async4z(sin_ + c * (UG_P + 1) + q,
+                 ok ? in + (((size_t)c * B + b) * h + yy) * w + xx : in, ok);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int e = tid; e < UG_P * cout; e += UG_THREADS) {
+      const int P = e / cout, c = e - P * cout;
+      const float* q = sd + c * UG_FS + 2 * (P / UG_X) * UG_FX + 2 * (P % UG_X);
+      float r[3][4];   // sums of neighbouring rows
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const float a0 = q[x], a1 = q[UG_FX + x], a2 = q[2 * UG_FX + x], a3 = q[3 * UG_FX + x];
+        r[0][x] = a0 + a1;
+        r[1][x] = a1 + a2;
+        r[2][x] = a2 + a3;
+      }
+#pragma unroll
+      for (int k = 0; k < 9; ++k)   // tap (dy, dx): rows and columns 2 - dy, 2 - dx on
+        S[(P * 9 + k) * cout + c] = r[2 - k / 3][2 - k % 3] + r[2 - k / 3][3 - k % 3];
+    }
+    __syncthreads();
+    if (work) {
+#pragma unroll 1
+      for (int P = sl; P < UG_P; P += nsl) {
+        const float v = sin_[ci * (UG_P + 1) + P];
+        const float* q = S + P * 9 * cout + cog * WG_COT;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+          const float4 d = *(const float4*)(q + k * cout);
+          acc[0][k] = fmaf(d.x, v, acc[0][k]);
+          acc[1][k] = fmaf(d.y, v, acc[1][k]);
+          acc[2][k] = fmaf(d.z, v, acc[2][k]);
+          acc[3][k] = fmaf(d.w, v, acc[3][k]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // slices in order through shared memory
+  if (nsl > 1) {
+    if (work)
+#pragma unroll
+      for (int c = 0; c < WG_COT; ++c)
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+          wsm[((size_t)sl * 9 * WG_COT + c * 9 + k) * pairs + pr] = acc[c][k];
+    __syncthreads();
+    if (!work || sl > 0) return;
+    for (int s2 = 1; s2 < nsl; ++s2)
+#pragma unroll
+      for (int c = 0; c < WG_COT; ++c)
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+          acc[c][k] += wsm[((size_t)s2 * 9 * WG_COT + c * 9 + k) * pairs + pr];
+  }
+  if (!work) return;
+  const int ct = cin + direct;
+  float* out = part + (size_t)blockIdx.x * ((size_t)cout * ct * 9 + cout);
+#pragma unroll
+  for (int c = 0; c < WG_COT; ++c)
+#pragma unroll
+    for (int k = 0; k < 9; ++k) out[(size_t)((cog * WG_COT + c) * 9 + k) * ct + ci] = acc[c][k];
+}
+
+// the partial sets of all six layers added in order; a set is [cout][tap][cin], then
+// the biases (as [cout][cin][tap] its stores were nine times as many sectors)
 struct WgReduce {
   const float* part[6];
-  int slots[6], nw[6], nb[6], off_w[6], off_b[6], first[7];   // first: entry offsets
+  int slots[6], cin[6], nw[6], nb[6], off_w[6], off_b[6], first[7];   // first: entry offsets
 };
 
 // A CTA adds 32 entries: warp w takes the sets w, w + 8, ... and the eight sums
@@ -342,8 +460,12 @@ wgrad_reduce(const WgReduce R, float* __restrict__ dw, float* __restrict__ db) {
   if (warp != 0 || e >= R.first[6]) return;
 #pragma unroll
   for (int w = 1; w < NT / 32; ++w) s += sh[w][lane];
-  if (k < R.nw[l]) dw[R.off_w[l] + k] = s;
-  else db[R.off_b[l] + k - R.nw[l]] = s;
+  if (k < R.nw[l]) {
+    const int row = k / R.cin[l], ci = k - row * R.cin[l], co = row / 9, tap = row - co * 9;
+    dw[R.off_w[l] + (co * R.cin[l] + ci) * 9 + tap] = s;
+  } else {
+    db[R.off_b[l] + k - R.nw[l]] = s;
+  }
 }
 
 // transposed, flipped weights for the data gradients, wt[ci][co][8 - tap], of
@@ -972,11 +1094,12 @@ static int conv(const float* inA, int cin_a, const float* inB, int cin,
   return zb_launch_check();
 }
 
-// one layer's partial weight and bias gradients
-static int wgrad(const float* inA, int cin_a, const float* inB, int cin, const float* dout,
-                 int cout, float* part, int B, int H, int W, cudaStream_t st,
-                 int mode_a = SRC_DIRECT) {
-  const WgShape g = wg_shape(cin, cout, B, H, W);
+// one layer's partial weight and bias gradients: `up` input channels of the half
+// resolution inUp (may be 0), then cin from `in`
+static int wgrad(const float* in, int cin, const float* dout, int cout, float* part, int B, int H,
+                 int W, cudaStream_t st, int mode = SRC_DIRECT, const float* inUp = nullptr,
+                 int up = 0) {
+  const WgShape g = wg_shape(cin, cout, B, H, W, up);
   static std::atomic<unsigned> attr{0u};
   int dev = 0;
   ZB_CUDA_TRY(cudaGetDevice(&dev));
@@ -986,12 +1109,23 @@ static int wgrad(const float* inA, int cin_a, const float* inB, int cin, const f
                                      227 * 1024));
     ZB_CUDA_TRY(cudaFuncSetAttribute(conv3x3_wgrad<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      227 * 1024));
+    ZB_CUDA_TRY(cudaFuncSetAttribute(conv3x3_wgrad_up, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     227 * 1024));
     attr.fetch_or(1u << dev);
   }
-  const dim3 grid(g.slots, g.nchunk);
-  ZB_CUDA_TRY(pdl_launch(cout % WG_COT == 0 ? conv3x3_wgrad<WG_COT> : conv3x3_wgrad<1>, grid,
-                         dim3(g.threads), g.smem, st, inA, cin_a, inB, cin, dout, cout, part, B, H,
-                         W, mode_a, g.ncog, g.cic, g.nsl));
+  if (up) {
+    const int pairs = up * (cout / WG_COT);
+    if (cout % WG_COT != 0 || pairs > UG_THREADS) return ZB_E_UNSUPPORTED;
+    const int nsl = std::max(1, std::min(8, UG_THREADS / pairs));
+    const size_t stage = (size_t)UG_P * 9 * cout + (size_t)up * (UG_P + 1) + (size_t)cout * UG_FS;
+    const size_t red = nsl > 1 ? (size_t)pairs * nsl * 9 * WG_COT : 0;
+    ZB_CUDA_TRY(pdl_launch(conv3x3_wgrad_up, dim3(g.slots), dim3(UG_THREADS),
+                           std::max(stage, red) * sizeof(float), st, inUp, up, dout, cout, part,
+                           cin, B, H, W, nsl));
+  }
+  ZB_CUDA_TRY(pdl_launch(cout % WG_COT == 0 ? conv3x3_wgrad<WG_COT> : conv3x3_wgrad<1>,
+                         dim3(g.slots, g.nchunk), dim3(g.threads), g.smem, st, in, cin, dout, cout,
+                         part, up, B, H, W, mode, g.ncog, g.cic, g.nsl));
   return zb_launch_check();
 }
 
@@ -999,6 +1133,13 @@ static int gridn(size_t n) { return (int)std::max<size_t>(1, std::min<size_t>((n
 
 // m1 and m2 run at half resolution
 static bool layer_half(int l) { return l == 2 || l == 3; }
+
+// the gradient partials' shape of layer l on images H x W (the network's)
+static WgShape wg_layer(const Net& n, int l, int B, int H, int W) {
+  const int up = l == 4 ? n.c2 : 0;
+  return wg_shape(n.cin[l] - up, n.cout[l], B, layer_half(l) ? H / 2 : H,
+                  layer_half(l) ? W / 2 : W, up);
+}
 
 // activation buffers (floats) for a batch of B images H x W
 struct Acts {
@@ -1020,8 +1161,7 @@ static size_t acts_floats(const Net& n, int B, int H, int W, bool train) {
          (size_t)n.c1 * N0 + (n.nw + 64);   // tmp + flipped weights (bf16 fits in floats)
   if (train)
     for (int l = 0; l < 6; ++l) {
-      const WgShape g = wg_shape(n.cin[l], n.cout[l], B, layer_half(l) ? H / 2 : H,
-                                 layer_half(l) ? W / 2 : W);
+      const WgShape g = wg_layer(n, l, B, H, W);
       f += (size_t)g.slots * g.part;
     }
   return f;
@@ -1057,8 +1197,7 @@ static Acts acts_split(const Net& n, void* base, int B, int H, int W, bool train
     a.wflip = (__nv_bfloat16*)f;
     f += n.nw + 64;
     for (int l = 0; l < 6; ++l) {
-      const WgShape g = wg_shape(n.cin[l], n.cout[l], B, layer_half(l) ? H / 2 : H,
-                                 layer_half(l) ? W / 2 : W);
+      const WgShape g = wg_layer(n, l, B, H, W);
       a.wpart[l] = f;
       f += (size_t)g.slots * g.part;
     }
@@ -1277,31 +1416,31 @@ int zb_unet_backward(const zb_unet_trainer* t, const float* r, const float* targ
                          (const float*)(target ? a.d_out : nullptr), cx, cy, (const float*)a.lden,
                          (const float*)a.s, B, H, W, idx2, dx2, a.d_out));
   // out = conv(o1)
-  if ((rc = wgrad(a.o1, n.c1, nullptr, n.c1, a.d_out, 1, a.wpart[5], B, H, W, st))) return rc;
+  if ((rc = wgrad(a.o1, n.c1, a.d_out, 1, a.wpart[5], B, H, W, st))) return rc;
   if ((rc = data_grad(n, 5, a.wflip, a.d_out, a.d_o1, B, H, W, st, a.o1))) return rc;
   // o1 = tanh(conv([u, e2]))
-  if ((rc = wgrad(a.m2, n.c2, a.e2, n.c2 + n.c1, a.d_o1, n.c1, a.wpart[4], B, H, W, st, SRC_UP))) return rc;
+  if ((rc = wgrad(a.e2, n.c1, a.d_o1, n.c1, a.wpart[4], B, H, W, st, SRC_DIRECT, a.m2, n.c2))) return rc;
   if ((rc = data_grad(n, 4, a.wflip, a.d_o1, a.d_cat, B, H, W, st))) return rc;
   // d_cat = [du (c2), de2_b (c1)]
   ZB_CUDA_TRY(pdl_launch(upsample2_tanh_back, dim3(gridn((size_t)n.c2 * N1)), nt, 0, st,
                          (const float*)a.d_cat, (const float*)a.m2, a.d_m2, n.c2, B, H, W));
-  if ((rc = wgrad(a.m1, n.c2, nullptr, n.c2, a.d_m2, n.c2, a.wpart[3], B, H1, W1, st))) return rc;
+  if ((rc = wgrad(a.m1, n.c2, a.d_m2, n.c2, a.wpart[3], B, H1, W1, st))) return rc;
   if ((rc = data_grad(n, 3, a.wflip, a.d_m2, a.d_m1, B, H1, W1, st, a.m1))) return rc;
-  if ((rc = wgrad(a.e2, n.c1, nullptr, n.c1, a.d_m1, n.c2, a.wpart[2], B, H1, W1, st, SRC_POOL))) return rc;
+  if ((rc = wgrad(a.e2, n.c1, a.d_m1, n.c2, a.wpart[2], B, H1, W1, st, SRC_POOL))) return rc;
   if ((rc = data_grad(n, 2, a.wflip, a.d_m1, a.d_p, B, H1, W1, st))) return rc;
   ZB_CUDA_TRY(pdl_launch(pool_add_tanh_back, dim3(gridn((size_t)n.c1 * N0)), nt, 0, st,
                          (const float*)a.d_p, (const float*)(a.d_cat + (size_t)n.c2 * N0),
                          (const float*)a.e2, a.d_e2, n.c1, B, H, W));
-  if ((rc = wgrad(a.e1, n.c1, nullptr, n.c1, a.d_e2, n.c1, a.wpart[1], B, H, W, st))) return rc;
+  if ((rc = wgrad(a.e1, n.c1, a.d_e2, n.c1, a.wpart[1], B, H, W, st))) return rc;
   if ((rc = data_grad(n, 1, a.wflip, a.d_e2, a.d_e1, B, H, W, st, a.e1))) return rc;
-  if ((rc = wgrad(a.in, 2, nullptr, 2, a.d_e1, n.c1, a.wpart[0], B, H, W, st))) return rc;
+  if ((rc = wgrad(a.in, 2, a.d_e1, n.c1, a.wpart[0], B, H, W, st))) return rc;
   WgReduce R;
   R.first[0] = 0;
   for (int l = 0; l < 6; ++l) {
-    const WgShape g = wg_shape(n.cin[l], n.cout[l], B, layer_half(l) ? H1 : H,
-                               layer_half(l) ? W1 : W);
+    const WgShape g = wg_layer(n, l, B, H, W);
     R.part[l] = a.wpart[l];
     R.slots[l] = g.slots;
+    R.cin[l] = n.cin[l];
     R.nb[l] = n.cout[l];
     R.nw[l] = n.cout[l] * n.cin[l] * 9;
     R.off_w[l] = (int)n.off_w[l];
