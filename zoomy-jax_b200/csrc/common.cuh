@@ -69,14 +69,13 @@ __device__ __forceinline__ double nrsqrt(double x) {
   t = fma(-hx * y, y, 0.5);
   return fma(y, t, y);
 }
-// x >= 0; a negative or NaN x gives NaN, as sqrt does
+// x >= 0; a negative or NaN x gives NaN, as sqrt does.  Selects, not a branch, so that the
+// roots of a row step run side by side (2048^2 float64, three steps: 1827 -> 1723 us).
 __device__ __forceinline__ double nsqrt(double x) {
-  if (x > 0.0) {
-    const double y = nrsqrt(x);
-    const double s = x * y;
-    return fma(fma(-s, s, x), 0.5 * y, s);
-  }
-  return x == 0.0 ? x : __longlong_as_double(0x7ff8000000000000LL);
+  const double y = nrsqrt(x);
+  const double s = x * y;
+  const double r = fma(fma(-s, s, x), 0.5 * y, s);
+  return x > 0.0 ? r : x == 0.0 ? x : __longlong_as_double(0x7ff8000000000000LL);
 }
 
 // Division of the shallow-water limiter and flux path.  float: __fdividef

@@ -110,16 +110,14 @@ __device__ __forceinline__ T phi_clipmin(T a, T c, T dpos, T dneg) {
 template <typename T>
 __device__ __forceinline__ T vk_cand(T delta, T dpos, T dneg, T ev2) {
   const T eps = T(1e-30);
-  if (delta > eps) {
-    T num = dpos * dpos + ev2 + T(2) * delta * dpos;
-    T den = dpos * dpos + T(2) * delta * delta + delta * dpos + ev2;
-    return clip01(adiv(num, zmax(den, eps)));
-  } else if (delta < -eps) {
-    T num = dneg * dneg + ev2 + T(2) * delta * dneg;
-    T den = dneg * dneg + T(2) * delta * delta + delta * dneg + ev2;
-    return clip01(adiv(-num, zmin(den, -eps)));
-  }
-  return T(1);
+  // selects, as phi_clipmin (two branches: 1000 x 1100, four steps, float32 529 us, now
+  // 393, float64 1676, now 1327)
+  const bool pos = delta > eps, neg = delta < -eps;
+  const T d = pos ? dpos : dneg;
+  const T num = d * d + ev2 + T(2) * delta * d;
+  const T den = d * d + T(2) * delta * delta + delta * d + ev2;
+  const T r = clip01(adiv(pos ? num : -num, pos ? zmax(den, eps) : zmin(den, -eps)));
+  return pos || neg ? r : T(1);
 }
 
 template <typename T>
@@ -193,7 +191,8 @@ __device__ __forceinline__ void riemann(const Side<T>& L, const Side<T>& R, T sg
     const T sl = fmn3(unL - cL, unR - cR, T(0));
     const T sr = fmx3(unL + cL, unR + cR, T(0));
     const T den = sr - sl;
-    const T inv = den > T(0) ? adiv(T(1), den) : T(0);
+    const T quo = adiv(T(1), den);   // a select, not a branch
+    const T inv = den > T(0) ? quo : T(0);
     const T slsr = sl * sr;
     Fh = (sr * FLh - sl * FRh + slsr * (hRs - hLs)) * inv;
     Fqx = (sr * FLx - sl * FRx + slsr * (qRx - qLx)) * inv;
@@ -776,29 +775,26 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
     {
       const int m = r - 1;
       const bool bxl = EDGE && m == 0, bxh = EDGE && m == nx - 1, bx = bxl || bxh;   // uniform
-      T phi[4], gxa[4], gya[4];
+      T phi[4], gxa[4], gya[4], dposa[4], dnega[4];
       // x and y scale of the differences
       const T ix = (EDGE && (by || bx)) ? p.inv4dx : p.inv6dx;
       const T iy = (EDGE && (by || bx)) ? p.inv4dy : p.inv6dy;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        if (v == 0 && BED) {
-          gxa[0] = bgx;
-          gya[0] = bgy;
-          phi[0] = bphi;
-          continue;
-        }
+      // gradient and bounds of variable v; BX: a boundary row.  The choice of the row is
+      // made once for the four variables, so that they run side by side (64^2 solve, all
+      // items in this body, 701 -> 679 us; 517 x 389 float32 236 -> 226)
+      auto slope = [&](auto BXT, int v) {
+        constexpr bool BX = decltype(BXT)::value;
         const T u = R1.w(v);
         T wp0 = R2.w(v), wm0 = R0.w(v), w0p = Wp1[v], w0m = Wm1[v];
         T xhi = Sx2[v], xlo = Sx0[v];       // gx = (xhi - xlo) / ..
-        const T tc = (EDGE && bx) ? (bxl ? u + wp0 : wm0 + u) : (wm0 + u) + wp0;
+        const T tc = BX ? (bxl ? u + wp0 : wm0 + u) : (wm0 + u) + wp0;
         T tl = shu(tc), tr = shd(tc);       // gy = (tr - tl) / ..
         T cgx = T(0), cgy = T(0);           // corner cells: the gradient itself
         if (EDGE) {
           // y: the side's ghost
           const T gyv = per_y ? (byl ? w0m : w0p) : ((v == 3 && wall_y) ? -u : u);
           const T cy = gyv + T(2) * u, gg = T(2) * gyv - u;
-          if (bx) {
+          if constexpr (BX) {
             // x: the side's ghost row; the corner cells
             const T gxv = per_x ? (bxl ? wm0 : wp0)
                                 : ((v == 2 && p.bc[bxl ? 0 : 1] == ZB_BC_WALL) ? -u : u);
@@ -834,20 +830,52 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
           dpos = umax - u;
           dneg = umin - u;
         }
-        if (EDGE && bx) {
+        if constexpr (BX) {
           gx = by ? cgx : gx;
           gy = by ? cgy : gy;
         }
         gxa[v] = gx;
         gya[v] = gy;
-        if (PAIR && clipmin) {
-          if constexpr (PAIR) {
-            const float2 ac = mul2(f2(gx, gy), f2(p.half_dx, p.half_dy));
-            phi[v] = phi_clipmin(ac.x, ac.y, dpos, dneg);
-          }
-        } else {
-          phi[v] = limiter_phi<T>(limiter, gx, gy, p.half_dx, p.half_dy, dpos, dneg, p.vk_eps2);
+        dposa[v] = dpos;
+        dnega[v] = dneg;
+      };
+      if (BED) {
+        gxa[0] = bgx;
+        gya[0] = bgy;
+        phi[0] = bphi;
+      }
+      bool plain = true;
+      if constexpr (EDGE) {
+        if (bx) {
+          plain = false;
+#pragma unroll
+          for (int v = 0; v < 4; ++v) slope(std::true_type(), v);
         }
+      }
+      if (plain) {
+#pragma unroll
+        for (int v = BED ? 1 : 0; v < 4; ++v) slope(std::false_type(), v);
+      }
+      // One choice of the limiter for the four variables, so that their quotients run
+      // side by side: a warp waits for dependent instructions most of its time (float64:
+      // issue 55 %), and a branch per variable kept the four chains apart.  2048^2
+      // float64, three steps, 1723 -> 1585 us, float32, six, 1085 -> 1060; 64 instances
+      // 1396 -> 1301.
+      if (clipmin) {
+#pragma unroll
+        for (int v = BED ? 1 : 0; v < 4; ++v) {
+          if constexpr (PAIR) {
+            const float2 ac = mul2(f2(gxa[v], gya[v]), f2(p.half_dx, p.half_dy));
+            phi[v] = phi_clipmin(ac.x, ac.y, dposa[v], dnega[v]);
+          } else {
+            phi[v] = phi_clipmin(gxa[v] * p.half_dx, gya[v] * p.half_dy, dposa[v], dnega[v]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int v = BED ? 1 : 0; v < 4; ++v)
+          phi[v] = limiter_phi<T>(limiter, gxa[v], gya[v], p.half_dx, p.half_dy, dposa[v],
+                                  dnega[v], p.vk_eps2);
       }
       if (RECON == ZB_RECON_ETA) {
         if (p.eps_wet >= T(0) && R1.h < p.eps_wet) {
