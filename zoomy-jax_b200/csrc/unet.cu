@@ -117,9 +117,10 @@ conv3x3_fwd(const float* __restrict__ inA, int cin_a, const float* __restrict__ 
 // the partial sets in order, so the gradients are deterministic.  One thread per
 // weight walking the pixels in shared memory with a float atomic per tile, as
 // before, was bound by its two shared loads per FMA: the six layers of a
-// 64 x 32^2 batch (24, 48) took 1234 us, now 201 and 13 for the reduction (the
-// FMA pipe's floor is 35; the copies of the halo tiles are the rest).
-constexpr int WG_TX = 16, WG_TY = 4, WG_SEG = 8;          // tile, pixels per row segment
+// 64 x 32^2 batch (24, 48) took 1234 us, now 194 and 10 for the reduction (the
+// FMA pipe's floor is 35; the copies of the halo tiles are the rest: tiles of
+// four rows instead of eight, half of them halo, 201 and 13).
+constexpr int WG_TX = 16, WG_TY = 8, WG_SEG = 8;          // tile, pixels per row segment
 constexpr int WG_HX = WG_TX + 2, WG_HY = WG_TY + 2;
 constexpr int WG_PLANE = WG_HX * WG_HY + 1;               // odd: lanes of a warp hit 32 banks
 constexpr int WG_UNITS = WG_TY * (WG_TX / WG_SEG);        // row segments of a tile
@@ -332,7 +333,7 @@ conv3x3_wgrad(const float* __restrict__ in, int cin, const float* __restrict__ d
 // memory; a thread owns one input and four output channels with all nine taps, and per
 // pixel one value and nine 16-byte loads (the same address for most of a warp) feed 36
 // FMAs.  64 x 32^2, 48 + 24 -> 24 channels: all 72 channels at full resolution 116 us,
-// now 30 here and 41 for the other 24.
+// now 30 here and 38 for the other 24.
 __global__ void __launch_bounds__(UG_THREADS, 2)
 conv3x3_wgrad_up(const float* __restrict__ in, int cin, const float* __restrict__ dout, int cout,
                  float* __restrict__ part, int direct, int B, int H, int W, int nsl) {
