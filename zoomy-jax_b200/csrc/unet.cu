@@ -1007,7 +1007,7 @@ static bool cb8_map(CUtensorMap* m, const uint4* base, int nchunks, int B, int H
 }
 
 // conv3x3_cb8 over B images H x W (see conv_tc.cuh); resident CTAs are capped
-// so that their TMEM columns (two M tiles of coutp each) fit in 512
+// so that their TMEM columns (two buffers of two M tiles of coutp each) fit in 512
 static int conv_cb8_launch(const uint4* inA, int chA, int mode_a, const uint4* inB, int chB,
                            int cin, const __nv_bfloat16* w, const float* bias, void* out,
                            uint4* pool, int cout, int out_form, int B, int H, int W, int act,
