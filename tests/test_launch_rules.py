@@ -1,0 +1,63 @@
+"""Host rules that choose launch shapes from sizes (csrc/launch_rules.h), compiled by the
+host compiler and evaluated over their whole range: every rule ends, covers the grid and
+keeps within the slots it is given."""
+import pathlib
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = pathlib.Path(__file__).resolve().parent.parent / "zoomy-jax_b200" / "csrc"
+
+
+@pytest.fixture(scope="module")
+def evaluate(tmp_path_factory):
+    """``evaluate(body, rows)``: a program that reads one line of integers per call of
+    ``body`` (as ``a[]``) and prints what it prints."""
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no C++ compiler")
+
+    def run(body, rows):
+        d = tmp_path_factory.mktemp("rules")
+        n = len(rows[0])
+        (d / "rules.cpp").write_text(
+            '#include <cstdio>\n#include "launch_rules.h"\nusing namespace zb;\n'
+            f"int main() {{\n  long long a[{n}];\n  for (;;) {{\n"
+            f"    for (int i = 0; i < {n}; ++i) if (std::scanf(\"%lld\", &a[i]) != 1) return 0;\n"
+            f"    {body}\n  }}\n}}\n")
+        subprocess.run([gxx, "-std=c++17", "-O2", "-I", str(CSRC), str(d / "rules.cpp"), "-o",
+                        str(d / "rules")], check=True)
+        text = "\n".join(" ".join(str(int(v)) for v in r) for r in rows)
+        out = subprocess.run([str(d / "rules")], input=text, capture_output=True, text=True,
+                             check=True, timeout=60).stdout
+        return [[int(v) for v in line.split()] for line in out.splitlines()]
+
+    return run
+
+
+# (nx, ny) of a level on strips: square, tall, wide; wide ones with more strips than there
+# are slots for partial sums, up to the largest level (2^31 cells)
+LEVELS = [(800, 800), (1024, 1024), (2048, 2048), (46340, 46340), (10242, 64), (80004, 8),
+          (64, 10242), (8, 80004), (8, 851968), (8, 852020), (8, 900000), (8, 1000000),
+          (4, 500000), (6, 3000000), (8, 260000000), (4, 536870910), (536870910, 4)]
+
+
+@pytest.mark.parametrize("nu", [1, 2, 3, 4])
+def test_multigrid_strips(evaluate, nu):
+    cols, parts = 64 - 2 * (2 * nu + 2), 4096
+    got = evaluate("MgStrips s = mg_strips((int)a[0], (int)a[1], (int)a[2], a[3] != 0, (int)a[4]);"
+                   ' std::printf("%d %d %d %d\\n", s.strips, s.rows, s.ctas, (int)s.dot);',
+                   [(nx, ny, cols, dot, parts) for nx, ny in LEVELS for dot in (0, 1)])
+    for k, (nx, ny) in enumerate(LEVELS):
+        plain, with_dot = got[2 * k], got[2 * k + 1]
+        for strips, rows, ctas, dot in (plain, with_dot):
+            assert strips * cols >= ny > (strips - 1) * cols
+            assert rows >= 4 and rows % 2 == 0
+            assert 4 * ctas >= strips * -(-nx // rows) > 4 * (ctas - 1)
+            assert not dot or ctas <= parts
+        assert not plain[3]
+        # the sums are left out only where full-height items do not fit
+        assert with_dot[3] == (-(-with_dot[0] // 4) <= parts)
+        if not with_dot[3] or plain[2] <= parts:
+            assert with_dot[:3] == plain[:3]

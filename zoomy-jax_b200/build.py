@@ -42,7 +42,7 @@ def nvcc():
 
 
 def _newest_header():
-    hs = list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
+    hs = [*CSRC.glob("*.cuh"), *CSRC.glob("*.h"), *INCLUDE.glob("*.h")]
     return max((h.stat().st_mtime for h in hs), default=0.0)
 
 

@@ -29,6 +29,7 @@
 #include <utility>
 
 #include "common.cuh"
+#include "launch_rules.h"
 
 namespace zb {
 namespace pois {
@@ -1025,7 +1026,7 @@ mg_up_kernel(const float* __restrict__ f, const float* __restrict__ cx,
 // Updates two rows apart instead of one (independent half-sweeps in a step) lost:
 // down 14.4, up 15.7 us.
 constexpr int MW = 64;            // columns of a strip
-constexpr int MG_NT = 128;        // four independent warps per CTA
+constexpr int MG_NT = 128;        // four independent warps per CTA (mg_strips counts on it)
 
 // halo rows of an item, halo columns of a strip (each half-sweep, the residual,
 // the restriction and the prolongation's coarse neighbour take one column)
@@ -1807,23 +1808,15 @@ static int fused_level(bool down, int nu, const Level& L, float* fw, float* to, 
 }
 
 // A large level's launch on strips (on level 0 of the flexible CG the way up also
-// leaves the partial sums of z.q).  The rows of an item spread the level over two
-// warps per scheduler (1184), four rows at least, 64 at most; an item marches its
-// rows plus the pipeline's 4 nu + 3 (down) or 4 nu (up).
-// Returns the number of CTAs through *blocks.
+// leaves the partial sums of z.q, their count in *blocks, where the level fits them:
+// mg_strips).  An item marches its rows plus the pipeline's 4 nu + 3 (down) or 4 nu (up).
 static int fused_strip(bool down, int nu, const Level& L, float* fw, float* to, float idx2,
                  cudaStream_t st, const double* q = nullptr, double* part = nullptr,
                  int* blocks = nullptr) {
-  const int strips = (L.ny + mg_cols(nu) - 1) / mg_cols(nu);
-  int rows = std::max(4, (int)((long long)strips * L.nx / 1184 + 1) & ~1);
-  rows = std::min(rows, 64);
-  const int wpb = MG_NT / 32;
-  auto ctas = [&](int rw) {
-    return (int)(((long long)strips * ((L.nx + rw - 1) / rw) + wpb - 1) / wpb);
-  };
-  while (q && ctas(rows) > MG_PARTS) rows *= 2;
-  const int n = ctas(rows);
-  if (blocks) *blocks = n;
+  const MgStrips S = mg_strips(L.nx, L.ny, mg_cols(nu), q != nullptr, MG_PARTS);
+  const int strips = S.strips, rows = S.rows, n = S.ctas;
+  if (!S.dot) q = nullptr;
+  if (blocks) *blocks = S.dot ? n : 0;
   const float *a0 = fw + L.f, *a1 = fw + L.cx, *a2 = fw + L.cy, *a3 = fw + L.idg;
   float *a4 = fw + L.x, *a5 = fw + L.xo;
   cudaError_t e = cudaSuccess;
