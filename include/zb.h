@@ -330,7 +330,10 @@ typedef struct {
   int32_t nx, ny;
   double dx;
   double cmin, cmax;
-  int32_t nu;            /* pre- and post-smoothing red-black sweeps          */
+  int32_t nu;            /* pre- and post-smoothing red-black sweeps, 1..4; 0
+                          * where no level is smoothed (no preconditioner, a
+                          * single level, the learned smoother above one coarsest
+                          * level), else the solves answer ZB_E_UNSUPPORTED    */
   int32_t coarse_sweeps; /* symmetric sweep pairs on the coarsest level       */
   int32_t coarsest;      /* stop coarsening at this side                      */
 } zb_poisson_cfg;

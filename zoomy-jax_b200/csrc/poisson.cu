@@ -916,7 +916,7 @@ mg_down_kernel(const float* __restrict__ f, const float* __restrict__ cx,
   constexpr int nt = fused_threads(TT);
   const int tid = threadIdx.x;
   const Stage<HALO, TT> S = stage_level<HALO, TT>(fsm, i0, j0, nx, ny, f, cx, cy, idg, nullptr, vec);
-  if (NU > 0) S.sweep_from_zero(0);
+  S.sweep_from_zero(0);
   for (int s = 1; s < 2 * NU; ++s) S.sweep(s & 1, s + 1, idx2);
   // residual where the sweeps are final and one ring beyond the tile (one
   // list of cells over all the threads)
@@ -1113,6 +1113,7 @@ __global__ void __launch_bounds__(MG_NT)
 mg_down_strip(const float* __restrict__ f, const float* __restrict__ cx,
                const float* __restrict__ cy, const float* __restrict__ idg, float* __restrict__ x,
                float* __restrict__ fc, int nx, int ny, float idx2, int nstrips, int rows) {
+  static_assert(NU >= 1, "the first half-sweep starts from x = 0");
   constexpr int HALO = mg_halo(true, NU), CH = mg_chalo(NU), WN = 2 * NU + 2, NS = 2 * NU;
   const int item = blockIdx.x * (MG_NT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int strip = item % nstrips, i0 = (item / nstrips) * rows;
@@ -1166,8 +1167,8 @@ mg_down_strip(const float* __restrict__ f, const float* __restrict__ cx,
         // half-sweep 0 starts from x = 0: x = f / d on its colour (even
         // columns of even rows)
         const float e = R.f[s][0] * R.g[s][0], o = R.f[s][1] * R.g[s][1];
-        R.x[s][0] = (NU == 0 || (ph & 1)) ? 0.f : e;
-        R.x[s][1] = (NU == 0 || !(ph & 1)) ? 0.f : o;
+        R.x[s][0] = (ph & 1) ? 0.f : e;
+        R.x[s][1] = (ph & 1) ? o : 0.f;
       }
 #pragma unroll
       for (int k = 1; k < NS; ++k) {
@@ -1178,7 +1179,7 @@ mg_down_strip(const float* __restrict__ f, const float* __restrict__ cx,
           mg_sweep<WN, false>(R, sl(ph, k + 1), sl(ph, k), sl(ph, k - 1), idx2);
       }
       {   // the row of the last half-sweep is final
-        constexpr int FIN = NS > 0 ? NS - 1 : 0;
+        constexpr int FIN = NS - 1;
         const int i = r - FIN, s = sl(ph, FIN);
         if (out && i >= i0 && i < i1)
           *(float2*)(x + (long long)i * ny + j) = make_float2(R.x[s][0], R.x[s][1]);
@@ -1792,14 +1793,16 @@ static int fused_level(bool down, int nu, const Level& L, float* fw, float* to, 
       case 1: ZB_FUSED((mg_down_kernel<1, TT>)); break;
       case 2: ZB_FUSED((mg_down_kernel<2, TT>)); break;
       case 3: ZB_FUSED((mg_down_kernel<3, TT>)); break;
-      default: ZB_FUSED((mg_down_kernel<4, TT>)); break;
+      case 4: ZB_FUSED((mg_down_kernel<4, TT>)); break;
+      default: return ZB_E_UNSUPPORTED;
     }
   } else {
     switch (nu) {
       case 1: ZB_FUSED_UP((mg_up_kernel<1, TT>)); break;
       case 2: ZB_FUSED_UP((mg_up_kernel<2, TT>)); break;
       case 3: ZB_FUSED_UP((mg_up_kernel<3, TT>)); break;
-      default: ZB_FUSED_UP((mg_up_kernel<4, TT>)); break;
+      case 4: ZB_FUSED_UP((mg_up_kernel<4, TT>)); break;
+      default: return ZB_E_UNSUPPORTED;
     }
   }
 #undef ZB_FUSED
@@ -1830,7 +1833,8 @@ static int fused_strip(bool down, int nu, const Level& L, float* fw, float* to, 
     case 1: ZB_STRIP(1); break;
     case 2: ZB_STRIP(2); break;
     case 3: ZB_STRIP(3); break;
-    default: ZB_STRIP(4); break;
+    case 4: ZB_STRIP(4); break;
+    default: return ZB_E_UNSUPPORTED;
   }
 #undef ZB_STRIP
   return e == cudaSuccess ? ZB_OK : ZB_E_CUDA;
@@ -1853,6 +1857,15 @@ static int fused(bool down, int nu, const Level& L, float* fw, float* to, float 
   const bool big = ((L.ny + FT - 1) / FT) * ((L.nx + FT - 1) / FT) >= 148;
   if (big) return fused_level<FT>(down, nu, L, fw, to, idx2, dim3(fused_threads(FT)), st);
   return fused_level<FTS>(down, nu, L, fw, to, idx2, dim3(fused_threads(FTS)), st);
+}
+
+// Whether a preconditioner can run on a plan: a level above the coarsest takes nu >= 1
+// sweeps on the way down and up, unless the learned smoother replaces them (precond 3, on
+// level 0 where that is not in the one-CTA part).  With nu = 0 nothing would set such a
+// level's x.
+static bool smooths(const Plan& P, int precond) {
+  const int first = precond == 3 && P.small0 > 0 ? 1 : 0;
+  return precond == 0 || P.nu >= 1 || first >= P.nlev - 1;
 }
 
 // q, part, nzq (the flexible CG): where level 0's way up forms the partial sums of
@@ -2029,6 +2042,7 @@ int zb_poisson_vcycle(const zb_poisson_cfg* cfg, void* ws, const float* r, float
   if (!valid(cfg) || !ws || !r || !z || precond < 0 || precond > 3) return ZB_E_ARG;
   if (precond >= 2 && !smo) return ZB_E_ARG;
   const Plan P = make_plan(cfg);
+  if (!smooths(P, precond)) return ZB_E_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   float* fw = (float*)((char*)ws + P.fbase);
   const long long n0 = (long long)cfg->nx * cfg->ny;
@@ -2099,6 +2113,7 @@ static int fcg_start_impl(const zb_poisson_cfg* cfg, void* ws, const double* b, 
   if (!valid(cfg) || !ws || !b || !x || precond < 0 || precond > 3) return ZB_E_ARG;
   if (precond >= 2 && !smo) return ZB_E_ARG;
   const Plan P = make_plan(cfg);
+  if (!smooths(P, precond)) return ZB_E_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   double* dw = (double*)ws;
   float* fw = (float*)((char*)ws + P.fbase);
@@ -2124,6 +2139,7 @@ static int fcg_iterate_impl(const zb_poisson_cfg* cfg, void* ws, double* x, int 
   if (!valid(cfg) || !ws || !x || precond < 0 || precond > 3) return ZB_E_ARG;
   if (precond >= 2 && !smo) return ZB_E_ARG;
   const Plan P = make_plan(cfg);
+  if (!smooths(P, precond)) return ZB_E_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   double* dw = (double*)ws;
   float* fw = (float*)((char*)ws + P.fbase);
@@ -2176,6 +2192,7 @@ int zb_fcg_graph_create(const zb_poisson_cfg* cfg, void* ws, const double* b, do
   *out = nullptr;
   (void)stream;   // capture runs on private streams; nothing executes here
   const Plan P = make_plan(cfg);
+  if (!smooths(P, precond)) return ZB_E_UNSUPPORTED;
   cudaStream_t st = nullptr, body = nullptr;
   ZB_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   if (cudaStreamCreateWithFlags(&body, cudaStreamNonBlocking) != cudaSuccess) {
