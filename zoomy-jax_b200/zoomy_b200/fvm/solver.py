@@ -253,7 +253,7 @@ class HyperbolicSolver:
         self._ws_bytes = self.be.workspace_bytes()
         self._ws = torch.empty(self._ws_bytes, dtype=torch.uint8, device=dev)
         self._ctrl = torch.zeros(L.CTRL_BYTES, dtype=torch.uint8, device=dev)
-        self._probe = torch.zeros_like(self._ctrl)    # zero between steps
+        self._probe = torch.zeros_like(self._ctrl)    # zero: a step's own block is its copy
         self._mass_part = torch.zeros(self.be.mass_partials(), dtype=torch.float64, device=dev)
         self._n = 0
         self._bed, self._bed_key = None, None
@@ -322,17 +322,17 @@ class HyperbolicSolver:
             L.ptr(self._ws), C.c_size_t(self._ws_bytes),
             L.ptr(self._ctrl if ctrl is None else ctrl), self._s()), "stage")
 
-    def _probe_troubled(self):
-        """Whether the stage that ran with the probe control block flagged a cell
+    def _probe_troubled(self, probe):
+        """Whether the stage that ran with the control block ``probe`` flagged a cell
         (synchronises).  Its status word replaces a reduction over the mask (18 us
         at 320 x 200, and the fill before it); a set status moves to the solver's
-        block, and the probe is zero again."""
+        block.  The block is the call's own, a copy of the zero one: two threads
+        stepping one solver decide apart."""
         import torch
         i = L.ZbCtrl.status.offset // 4
-        status = int(self._probe.view(torch.int32)[i].item())
+        status = int(probe.view(torch.int32)[i].item())
         if status:
             self._ctrl.view(torch.int32)[i].bitwise_or_(status)
-            self._probe.zero_()
         return bool(status & L.ZB_ST_TROUBLED)
 
     def _advance(self, Q, dt, force_o1=None, trouble=None, ctrl=None):
@@ -364,9 +364,9 @@ class HyperbolicSolver:
             # the last stage writes every byte of the mask; a negative dt is the
             # solver's control block's, so that block goes to the stage
             mask = torch.empty(Q.shape[1], dtype=torch.uint8, device=Q.device)
-            probe = dt >= 0.0
-            Qn = self._advance(Q, dt, trouble=mask, ctrl=self._probe if probe else None)
-            if self._probe_troubled() if probe else bool(mask.any()):
+            probe = self._probe.clone() if dt >= 0.0 else None
+            Qn = self._advance(Q, dt, trouble=mask, ctrl=probe)
+            if bool(mask.any()) if probe is None else self._probe_troubled(probe):
                 Qn = self._advance(Q, dt, force_o1=mask)
         else:
             Qn = self._advance(Q, dt)

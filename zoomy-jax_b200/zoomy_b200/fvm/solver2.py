@@ -109,8 +109,10 @@ class MarchSolver(HyperbolicSolver):
         cfg = self._cfg_o1 if o1 else self.cfg
         hinv = Qaux[6].contiguous() if self.cfg.manning_n != 0.0 else None
         dt = float(dt)
-        probe = dt >= 0.0    # a negative dt is the control block's
-        mask = None if probe else torch.empty(Q0.shape[1], dtype=torch.uint8, device=Q0.device)
+        # a negative dt is the control block's
+        probe = self._probe.clone() if dt >= 0.0 else None
+        mask = (torch.empty(Q0.shape[1], dtype=torch.uint8, device=Q0.device)
+                if probe is None else None)
         Qk = Q0
         last = len(self.tableau) - 1
         for k, (alpha, beta) in enumerate(self.tableau):
@@ -118,9 +120,9 @@ class MarchSolver(HyperbolicSolver):
             if k == last or not self.be.stage_b_from_q0:
                 out[0].copy_(Q0[0])
             self._stage(cfg, Qk, Q0, out, alpha, beta, dt, hinv=hinv, tr=mask,
-                        ctrl=self._probe if probe and k == last else None)
+                        ctrl=probe if k == last else None)
             Qk = out
-        return Qk, self._probe_troubled() if probe else bool(mask.any())
+        return Qk, bool(mask.any()) if probe is None else self._probe_troubled(probe)
 
     def hyperbolic_step(self, S, dt, p=None):
         Q_cand, troubled = self.stage_loop(S.Q, S.Qaux, dt, False)
