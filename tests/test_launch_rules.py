@@ -61,3 +61,17 @@ def test_multigrid_strips(evaluate, nu):
         assert with_dot[3] == (-(-with_dot[0] // 4) <= parts)
         if not with_dot[3] or plain[2] <= parts:
             assert with_dot[:3] == plain[:3]
+
+
+# (16, 16) networks at 512 x 724^2 and 512 x 726^2 lie on both sides of 2^32 elements
+PLANES = [(8, 64 * 32 ** 2), (24, 64 * 32 ** 2), (24, 512 * 256 ** 2), (16, 512 * 724 ** 2),
+          (16, 512 * 726 ** 2), (24, 178956971), (8, 430000000), (16, 279000000)]
+
+
+def test_plane_slices(evaluate):
+    stride = 148 * 16 * 256    # a grid's threads
+    got = evaluate('std::printf("%d\\n", plane_slice((int)a[0], a[1]));', PLANES)
+    for (channels, pixels), (n,) in zip(PLANES, got):
+        assert 1 <= n <= channels
+        assert n * pixels + stride < 2 ** 32
+        assert n == channels or (n + 1) * pixels > 2 ** 31

@@ -37,4 +37,12 @@ inline MgStrips mg_strips(int nx, int ny, int cols, bool dot, int parts) {
   return s;
 }
 
+// Channels that one launch of an elementwise kernel with a 32-bit index takes of
+// [channels][pixels] planes: at most 2^31 elements, so that the index plus a grid's stride
+// stays below 2^32.  (16, 16) networks train on batches of up to 2.8e8 pixels in 180 GB,
+// more than 2^32 elements of 16 channels; every usual batch is one launch.
+inline int plane_slice(int channels, long long pixels) {
+  return (int)std::max(1LL, std::min<long long>(channels, (1LL << 31) / pixels));
+}
+
 }  // namespace zb

@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "conv_tc.cuh"
+#include "launch_rules.h"
 
 namespace zb {
 namespace unet {
@@ -494,7 +495,7 @@ __global__ void flip_weights(const __nv_bfloat16* __restrict__ w, __nv_bfloat16*
 // took 22 us of a 64 x 32^2 batch's step, the upsampling 12.
 
 // gradient of e2: the average pool's (g1 / 4, half resolution) plus the
-// concatenation's, then the derivative
+// concatenation's, then the derivative (C channels of at most 2^31 elements: plane_slice)
 __global__ void pool_add_tanh_back(const float* __restrict__ g1, const float* __restrict__ g2,
                                    const float* __restrict__ y, float* __restrict__ gin, int C,
                                    int B, int H, int W) {
@@ -1429,9 +1430,15 @@ int zb_unet_backward(const zb_unet_trainer* t, const float* r, const float* targ
   if ((rc = data_grad(n, 3, a.wflip, a.d_m2, a.d_m1, B, H1, W1, st, a.m1))) return rc;
   if ((rc = wgrad(a.e2, n.c1, a.d_m1, n.c2, a.wpart[2], B, H1, W1, st, SRC_POOL))) return rc;
   if ((rc = data_grad(n, 2, a.wflip, a.d_m1, a.d_p, B, H1, W1, st))) return rc;
-  ZB_CUDA_TRY(pdl_launch(pool_add_tanh_back, dim3(gridn((size_t)n.c1 * N0)), nt, 0, st,
-                         (const float*)a.d_p, (const float*)(a.d_cat + (size_t)n.c2 * N0),
-                         (const float*)a.e2, a.d_e2, n.c1, B, H, W));
+  const int slice = plane_slice(n.c1, (long long)N0);
+  for (int c = 0; c < n.c1; c += slice) {
+    const int nc = std::min(slice, n.c1 - c);
+    ZB_CUDA_TRY(pdl_launch(pool_add_tanh_back, dim3(gridn((size_t)nc * N0)), nt, 0, st,
+                           (const float*)(a.d_p + (size_t)c * N1),
+                           (const float*)(a.d_cat + (size_t)(n.c2 + c) * N0),
+                           (const float*)(a.e2 + (size_t)c * N0), a.d_e2 + (size_t)c * N0, nc, B,
+                           H, W));
+  }
   if ((rc = wgrad(a.e1, n.c1, a.d_e2, n.c1, a.wpart[1], B, H, W, st))) return rc;
   if ((rc = data_grad(n, 1, a.wflip, a.d_e2, a.d_e1, B, H, W, st, a.e1))) return rc;
   if ((rc = wgrad(a.in, 2, a.d_e1, n.c1, a.wpart[0], B, H, W, st))) return rc;
