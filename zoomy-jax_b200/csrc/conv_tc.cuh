@@ -631,6 +631,16 @@ conv3x3_cb8(const uint4* __restrict__ inA, int chA, int mode_a, const uint4* __r
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       if (pending) signal();
     }
+    // The last regions' commits have arrived at `empty` before the CTA gives its shared
+    // memory back: the epilogue waits for the ones at acc_full alone.
+    if (ok && warp == CB_EPI) {
+      int k = s;
+      uint32_t kpar = par;
+      for (int n = 0; n < stages; ++n) {
+        ok = ok && wait(b_empty + 8 * k, kpar);
+        if (++k == stages) { k = 0; kpar ^= 1u; }
+      }
+    }
     if (!ok) {
       give_up();
       // tensor copies still in flight: the stages issued before this one (a phase
