@@ -75,3 +75,26 @@ def test_plane_slices(evaluate):
         assert 1 <= n <= channels
         assert n * pixels + stride < 2 ** 32
         assert n == channels or (n + 1) * pixels > 2 ** 31
+
+
+# widths on both sides of the first middle strip (58 columns), heights on both sides of the
+# uniform list's limit; the tall narrow grids have boundary strips alone
+GRIDS = [(nx, ny) for ny in (3, 28, 40, 56, 57, 58, 84, 300, 2048)
+         for nx in (3, 5, 64, 500, 2048, 20000, 100000, 300000) if nx * ny < 2 ** 31] + [
+             (700000000, 3), (3, 700000000), (4, 500000000)]
+
+
+@pytest.mark.parametrize("f32", [0, 1])
+def test_strip_rows(evaluate, f32):
+    got = evaluate("StripRows r = strip_rows((int)a[0], (int)a[1], a[2] != 0);"
+                   ' std::printf("%d %d %d %d\\n", r.sx, r.sxc, (int)r.single,'
+                   " full_mid_strips((int)a[1]));", [(nx, ny, f32) for nx, ny in GRIDS])
+    for (nx, ny), (sx, sxc, single, nmid) in zip(GRIDS, got):
+        strips = -(-ny // 28)
+        assert 1 <= sx <= 64 and sxc == 4
+        assert nmid == max(0, (ny - 30) // 28 if ny >= 30 else 0)
+        assert single == (nmid == 0 or strips * nx < 6 * 592)
+        # boundary strips alone: never in shorter chunks than beside middle strips, and
+        # few halo rows on a grid of many waves
+        if nmid == 0 and strips * nx >= 6 * 592:
+            assert sx >= (32 if strips * nx >= 200000 else 4)

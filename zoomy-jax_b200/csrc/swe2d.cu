@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "launch_rules.h"
 
 namespace zb {
 
@@ -434,7 +435,6 @@ swe2d_stage_kernel(const T* __restrict__ bP, const T* __restrict__ hP,
 // the limited slopes of two rows and the last x-face's fluxes in registers; the
 // column neighbours come from warp shuffles.  Every face is evaluated once.
 constexpr int SX = 64;          // output rows per work item at most
-constexpr int SW = 28;          // output columns per strip
 constexpr int STRIP_NT = 128;   // four independent warps per CTA
 constexpr int SXC_MAX = 32;     // output rows of the ensemble's longest boundary-strip item
 
@@ -1080,13 +1080,6 @@ __device__ __forceinline__ void strip_item(const T* __restrict__ bP, const T* __
   }
 }
 
-// The strips of a full-coverage grid whose lanes 28 s - 2 .. 28 s + 29 all lie
-// inside it (strips 1 .. the count).
-__host__ __device__ inline int full_mid_strips(int ny) {
-  const int ns = (ny + SW - 1) / SW, mh = ny >= 30 ? (ny - 30) / SW : 0;
-  return mh > ns - 1 ? ns - 1 : mh;
-}
-
 // Work items of a grid with nx, ny >= 3 (strips of SW columns from column 0).
 // The strips whose lanes reach outside the grid (the first, and the last one
 // or two) go in chunks of sxc rows; every other strip has two items for the
@@ -1096,7 +1089,6 @@ __host__ __device__ inline int full_mid_strips(int ny) {
 // block.  Returns the item count (item = -1), the count of boundary items
 // (item = -2), or with item >= 0 fills its strip, rows and kind (1 boundary, 0
 // interior).
-constexpr int SXC_GRID = 4;
 constexpr int SXC_ENS = 32;
 __host__ __device__ inline int full_items(int nx, int ny, int item, int* strip, int* r0,
                                           int* r1, int* kind, int sxc, int sx) {
@@ -1130,54 +1122,6 @@ __host__ __device__ inline int full_items(int nx, int ny, int item, int* strip, 
   *r1 = b;
   *kind = k;
   return nint + nside;
-}
-
-// Row-chunk heights of a single grid's items.  An item of S rows marches S + 4
-// (two halo rows each side): long chunks save halo rows, short ones spread a
-// small grid over more warps.  A row of a CTA (four items) takes about a + b k,
-// k the CTAs on its SM -- a lone warp is bound by its own dependent
-// instructions, so the first CTA costs most (float32 1 + 0.3 k us for the two
-// stages, k <= 4; float64 2.6 + 0.7 k, k <= 2; fitted to 250 timings of 15 grid
-// sizes, mean error 5 %).  The height is the least modelled time over the
-// candidates: whole waves of interior CTAs, the last wave with the boundary
-// CTAs beside it, and a tail where those do not fit.  Measured on a B200 (us per
-// step, minmod eta / HLL-HR; 64 rows everywhere after it): float32 512^2 25 / 94,
-// 1024^2 59 / 97, 1448^2 93 / 137, 2048^2 174 / 174; float64 512^2 62 / 230,
-// 1024^2 177 / 245, 2048^2 571 / 571; over the 15 sizes within 0.5 % (float64
-// 2 %) of the best of ten fixed heights on average.
-// A grid of fewer than 6 x 592 strip rows (about 300^2) takes the general body
-// everywhere in one uniform list: its two-row boundary items and four-row
-// boundary chunks would outlast the rest (256^2 float32 17.6 against 20.5,
-// 64^2 14 against 20; 400^2 24 against 22.6).
-template <typename T>
-static void strip_rows(int nx, int ny, SweParams<T>* p) {
-  constexpr bool F32 = sizeof(T) == 4;
-  constexpr double A = F32 ? 1.0 : 2.6, B = F32 ? 0.3 : 0.7, CPS = F32 ? 4 : 2;
-  constexpr double EDGE_ROWS = 8.0 * (F32 ? 1.3 : 1.1);   // a boundary item, in interior rows
-  constexpr double SLOTS = 148.0 * CPS, FULL = A + B * CPS;
-  const int ns = (ny + SW - 1) / SW, nmid = full_mid_strips(ny);
-  p->single = (double)ns * nx < 6.0 * 592.0 ? 1 : 0;
-  p->sxc = SXC_GRID;
-  const int strips = p->single ? ns : nmid, rows = p->single ? nx : std::max(nx - 4, 1);
-  const double ne =
-      p->single ? 0.0 : ((ns - nmid) * ((nx + SXC_GRID - 1) / SXC_GRID) + 2.0 * nmid) / 4.0;
-  double best = 1e300;
-  for (int s : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64}) {
-    const int n = (rows + s - 1) / s, h = (rows + n - 1) / n;   // chunks of equal height
-    const double L = h + 4, ctas = strips * (double)n / 4.0;
-    const double q = std::floor(ctas / SLOTS), r = ctas - q * SLOTS, last = r + ne;
-    const double own = r > 0.0 ? L : 0.0;
-    double cost = L * q * FULL;
-    if (last <= SLOTS)
-      cost += std::max(own, ne > 0.0 ? EDGE_ROWS : 0.0) *
-              (A + B * (F32 ? std::max(1.0, last / 148.0) : std::ceil(last / 148.0)));
-    else
-      cost += (own + EDGE_ROWS * std::max(0.5, (last - SLOTS) / SLOTS)) * FULL;
-    if (cost < best) {
-      best = cost;
-      p->sx = h;
-    }
-  }
 }
 
 // One stage of a grid: a warp per item, the interior or the general body by
@@ -1664,7 +1608,10 @@ static int launch_strips(const zb_swe2d_cfg* c, const T* b, const T* h, const T*
                          zb_ctrl* ctrl, int phase, SweParams<T> p, cudaStream_t st,
                          const T* hinv_src = nullptr, const unsigned char* force_o1 = nullptr,
                          unsigned char* trouble_out = nullptr) {
-  strip_rows(c->nx, c->ny, &p);
+  const StripRows rows = strip_rows(c->nx, c->ny, sizeof(T) == 4);
+  p.sx = rows.sx;
+  p.sxc = rows.sxc;
+  p.single = rows.single ? 1 : 0;
   const int n = p.single ? ((c->ny + SW - 1) / SW) * ((c->nx + p.sx - 1) / p.sx)
                          : full_items(c->nx, c->ny, -1, nullptr, nullptr, nullptr, nullptr, p.sxc,
                                       p.sx);
