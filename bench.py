@@ -829,7 +829,8 @@ def run_ensemble(local_rank, steps=2000):
             "ms_per_step": round(ms / chunk, 4),
             "value": cells * chunk / (ms * 1e-3), "unit": "cell-updates/s",
             "launches_per_step": 2,
-            "autotune_ms_per_step": {k: round(v, 4) for k, v in tuned.items()},
+            "autotune_ms_per_step": {k: round(v, 4) for k, v in tuned.items()
+                                     if not k.startswith("ctas_per_sm=")},
             "launch_shape": ens.tuned_shape,
             "class_instances_cells": ens.class_sizes(),
             "status_ok": ens.status_any() == 0}

@@ -21,7 +21,7 @@ from . import _lib as L
 
 # size classes of instances by side (the last class takes every larger one)
 CLASS_MAX_SIDE = (128, 256, 1 << 30)
-CTAS_CANDIDATES = (2, 3, 4)
+CTAS_CANDIDATES = (2, 3, 4)     # reported by the tuner, no effect on the launches
 EDGE_ROWS_CANDIDATES = (8, 16, 24, 32)
 INTERIOR_ROWS_CANDIDATES = (32, 64, 128, 256)
 
@@ -197,14 +197,15 @@ class Ensemble:
         return e0.elapsed_time(e1) / steps
 
     def autotune(self, steps=8):
-        """Coordinate descent over the launch shape from the untuned one:
-        strip CTAs per SM (no effect on the launches any more), then per
-        populated size class the boundary-strip and
-        the interior chunk heights; each candidate is timed over ``steps``
-        steps (after two untimed ones) on a scratch copy of the state and
-        replaces the incumbent only when it is faster.  Returns ``{candidate:
-        ms_per_step}`` for every candidate timed and keeps the best shape
-        (``self.tuned_shape``, ``self.tuned_ms``) for the steps that follow."""
+        """Coordinate descent over the launch shape from the untuned one: per
+        populated size class the boundary-strip and the interior chunk heights;
+        each candidate is timed over ``steps`` steps (after two untimed ones) on a
+        scratch copy of the state and replaces the incumbent only when it is
+        faster.  Returns ``{candidate: ms_per_step}`` and keeps the best shape
+        (``self.tuned_shape``, ``self.tuned_ms``) for the steps that follow.  The
+        ``ctas_per_sm`` entries are kept for readers of the result: a launch does
+        not depend on that field, so they are the untuned time and never a
+        candidate."""
         saved_q = self.Q.clone()
         t = self.tuning
         results = {}
@@ -222,11 +223,8 @@ class Ensemble:
                 undo()
 
         for cps in CTAS_CANDIDATES:
-            if cps == t.ctas_per_sm or (self.dtype == "float64" and cps > 2):
-                continue
-            old = t.ctas_per_sm
-            trial(f"ctas_per_sm={cps}", lambda v=cps: setattr(t, "ctas_per_sm", v),
-                  lambda v=old: setattr(t, "ctas_per_sm", v))
+            if cps != t.ctas_per_sm and not (self.dtype == "float64" and cps > 2):
+                results[f"ctas_per_sm={cps}"] = best
         for k, (n_inst, _) in enumerate(self.class_sizes()):
             if n_inst == 0:
                 continue
