@@ -150,9 +150,12 @@ __device__ __forceinline__ double block_max_double(double v, double* sh) {
 // Programmatic dependent launch: the kernels of a step, of a solve iteration and
 // of the V-cycle are launched with programmatic stream serialisation, so the next
 // kernel's launch overlaps the tail of this one.  Each of them first waits for
-// its predecessor's completion and memory (griddepcontrol.wait, before any
-// global read or write), then lets its own successor launch; launched without
-// the attribute, both instructions are no-ops.
+// its predecessor's completion and memory (griddepcontrol.wait), then lets its own
+// successor launch; launched without the attribute, both instructions are no-ops.
+// Before the wait a kernel may only read what its predecessor does not write.  What
+// an older launch wrote is complete there, since every CTA of the predecessor waited
+// for that launch before it let this one start: the convolutions stage their
+// weights, the ensemble its work list.
 __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

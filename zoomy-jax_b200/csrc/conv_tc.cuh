@@ -280,7 +280,11 @@ conv3x3_tc(const float* __restrict__ inA, int cin_a, const float* __restrict__ i
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  pdl_enter();   // the weights do not come from the preceding launch
+  // The weights were read above, before this wait: the launch directly before this one must
+  // not write them, and each of its CTAs must wait for its own predecessor before it lets
+  // this one start.  Between adam_kernel or flip_weights and the first convolution that
+  // reads their result stand at least the features' or the loss's launches.
+  pdl_enter();
   const uint32_t tmem = *tmem_slot;
   const uint32_t mbar_a = smem_u32(mbar);
   const uint32_t sA_a = smem_u32(sA), sB_a = smem_u32(sB);
@@ -509,7 +513,9 @@ conv3x3_cb8(const uint4* __restrict__ inA, int chA, int mode_a, const uint4* __r
   // cp.async copies: the warps for them, or (the fallback) the tensor-copy warp
   const int ncpt = cp_hi > cp_lo ? (NTH > CB_NTH ? NTH - CB_NTH : 32) : 0;
 
-  // weights and biases do not come from the preceding launch
+  // Weights and biases are read before the wait for the launch before this one, which must
+  // not write them and all of whose CTAs must wait before they let this one start (the
+  // residual and the features' launches stand between a writer and the first convolution)
   for (int st = 0; st < stages; ++st)
     for (int e = tid; e < (nch - chA - chB) * (CB_CHUNK_STRIDE / 16); e += NTH)
       ((uint4*)(sA + st * STAGE + (size_t)(chA + chB) * CB_CHUNK_STRIDE))[e] =

@@ -16,12 +16,12 @@
 // with odd reflection at the Dirichlet boundary, restriction R = P^T / 4,
 // red-black Gauss-Seidel (pre red/black, post black/red), a symmetric V-cycle
 // whose coarsest level (at most 64 cells) is solved exactly with an inverse
-// built at set-up.  Each level larger than 16 x 16 costs two launches per
+// built at set-up.  Each level larger than 32 x 32 costs two launches per
 // V-cycle: a fused pre-smooth + residual + restriction kernel on the way down
-// and a fused prolongation + post-smooth kernel on the way up (32 x 32 tiles
-// with a halo in shared memory).  Levels whose side is <= 16 run in ONE CTA
-// with every array in shared memory (their launches would otherwise be pure
-// latency).  Layout: cell (i, j) at i*ny + j; x-faces (nx+1, ny) at i*ny + j;
+// and a fused prolongation + post-smooth kernel on the way up (strips marched in
+// registers from 800^2 cells, tiles with a halo in shared memory below).  Levels
+// whose sides are <= 32 run in ONE CTA with every array in shared memory (their
+// launches would otherwise be pure latency).  Layout: cell (i, j) at i*ny + j; x-faces (nx+1, ny) at i*ny + j;
 // y-faces (nx, ny+1) at i*(ny+1) + j.
 #include <cstring>
 #include <algorithm>
@@ -1761,9 +1761,6 @@ static bool valid(const zb_poisson_cfg* c) {
          (long long)c->nx * c->ny < (1LL << 31);
 }
 
-// z32 = M r32 on level 0 (f0 already holds r); precond: 0 none, 1 MG, 2 MG
-// followed by one learned smoothing step on level 0 (x += S(f - A x)), 3 MG
-// with the level-0 red-black smoothing replaced by the learned smoother
 // One fused level launch (down: pre-smoothing, residual, restriction into the
 // coarse right-hand side `to`; up: coarse correction from `to`, post-smoothing)
 // with TT x TT tiles.
@@ -1868,6 +1865,9 @@ static bool smooths(const Plan& P, int precond) {
   return precond == 0 || P.nu >= 1 || first >= P.nlev - 1;
 }
 
+// z32 = M r32 on level 0 (f0 already holds r); precond: 0 none, 1 MG, 2 MG
+// followed by one learned smoothing step on level 0 (x += S(f - A x)), 3 MG
+// with the level-0 red-black smoothing replaced by the learned smoother.
 // q, part, nzq (the flexible CG): where level 0's way up forms the partial sums of
 // z.q with q itself, they land in part and *nzq is their count, else 0
 static int vcycle(const Plan& P, void* ws, int precond, const zb_smoother* smo, cudaStream_t st,

@@ -1196,7 +1196,10 @@ __device__ __forceinline__ void ens_item(const volatile SweParams<T>& p, T* q, T
 // {interior items, boundary items}; the lists follow it.  A warp's instance
 // parameters sit in shared memory: read from global memory they were held in
 // registers and spilled (408 bytes a thread with both bodies in one kernel,
-// 222 us a stage of 64 instances).
+// 222 us a stage of 64 instances; now 8 in float32, none in float64).  The work
+// list and the parameters are read before the wait for the launch before this one:
+// zb_ens_prepare writes them with a copy that has landed when it returns, never a
+// launch.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(STRIP_NT, sizeof(T) == 4 ? 4 : 2)
 ens_strip_kernel(const EnsDesc<T>* __restrict__ desc, const int4* __restrict__ items, T* Q,
@@ -1716,8 +1719,6 @@ static size_t ens_desc_bytes(int n_inst) {
   return ((size_t)n_inst * sizeof(EnsDesc<T>) + 255) / 256 * 256;
 }
 
-// strip items of an instance (the single grid's list): {strip, r0, r1, kind,
-// first item}
 // the chunk heights of an instance's size class (zb_ens_tuning)
 static void ens_class_rows(const zb_ens_tuning& t, const zb_ens_instance& in, int* sxc,
                            int* sx) {
@@ -1728,6 +1729,8 @@ static void ens_class_rows(const zb_ens_tuning& t, const zb_ens_instance& in, in
   *sx = t.interior_rows[c];
 }
 
+// strip items of an instance (the single grid's list): {strip, r0, r1, kind,
+// first item}
 template <typename F>
 static void ens_strip_items(const zb_ens_instance& in, const zb_ens_tuning& t, F&& visit) {
   int sxc, sx;
@@ -1752,8 +1755,8 @@ static size_t ens_count(const zb_ens_instance* inst, int n, const zb_ens_tuning&
 }
 
 // the launch shape of the untuned entry points: one size class, 32-row
-// boundary-strip chunks, 64-row interior chunks, 4 (float) or 2 (double) strip
-// CTAs per SM
+// boundary-strip chunks, 64-row interior chunks (the CTAs per SM are a field that
+// no launch reads)
 static zb_ens_tuning ens_default_tuning(const zb_swe2d_cfg* c, int tile_x) {
   zb_ens_tuning t;
   std::memset(&t, 0, sizeof(t));
@@ -2074,8 +2077,8 @@ int zb_ens_prepare_tuned(const zb_swe2d_cfg* common, const zb_ens_instance* inst
         (kind ? estrips : strips).push_back(make_int4(i, st, r0, (lead ? 1 : 0) | (r1 << 1)));
       });
     }
-    // longest items first: the persistent warps take items round-robin, so
-    // each warp's k-th item is about as long as every other warp's k-th
+    // longest items first: the block scheduler hands out CTAs in order, so the
+    // short ones fill the tail of the long ones
     auto longest_first = [](std::vector<int4>& v) {
       std::stable_sort(v.begin(), v.end(), [](const int4& a, const int4& b) {
         return (a.w >> 1) - a.z > (b.w >> 1) - b.z;

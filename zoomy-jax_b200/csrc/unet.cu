@@ -20,10 +20,12 @@
 // with c the cell mean of the four face coefficients.  Activations are
 // channel planes [C][B][H][W] in float32; weights [Cout][Cin][3][3] in bf16
 // (the training keeps a float32 master copy and rounds it to bf16 for every
-// forward, so the gradients are those of the bf16 network).  Convolutions are
-// direct: a 16x16 pixel tile with a 1-pixel halo per 8-channel input chunk in
-// shared memory, one thread per output pixel with all output channels in
-// registers.  Zero padding at image borders.
+// forward, so the gradients are those of the bf16 network).  Convolutions run on
+// the tensor cores (conv_tc.cuh): inference through chunked bf16 activations
+// (conv3x3_cb8), training and its data gradients through the planes (conv3x3_tc);
+// conv3x3_fwd, direct in float32 on the FMA pipe, is the exactness reference
+// (zb_unet_conv_impl 0).  Weight gradients run on the FMA pipe (conv3x3_wgrad,
+// conv3x3_wgrad_up).  Zero padding at image borders.
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 
@@ -47,6 +49,8 @@ enum { ACT_NONE = 0, ACT_TANH = 1, ACT_TANH_SFU = 2 };   // see conv_tc.cuh
 
 
 // out[co][b][y][x] = act(bias[co] + sum_ci sum_tap w[co][ci][tap] in[ci][b][y+dy][x+dx])
+// by a 16 x 16 pixel tile with a 1-pixel halo per 8-channel input chunk in shared memory,
+// a thread per output pixel with all output channels in registers;
 // input channels may come from two planes sets (the concatenation): channels
 // [0, cin_a) from inA, [cin_a, cin) from inB; ytanh (a data gradient): the result
 // times 1 - ytanh^2

@@ -10,7 +10,7 @@ time and the CFL reduction live in a device control block and the host only
 polls it between batches of steps.
 
 Two meshes are served through one backend interface: the Cartesian mesh
-(``create_2d``; fused tile kernels) and the unstructured triangle mesh
+(``create_2d``; fused strip and tile kernels) and the unstructured triangle mesh
 (``trimesh.create_tri``; gradient / face / gather-update kernels).
 """
 from __future__ import annotations
