@@ -51,7 +51,8 @@ def solver(cls):
     s._ws, s._ws_bytes = torch.zeros(8, dtype=torch.uint8), 8
     s._ctrl = torch.zeros(L.CTRL_BYTES, dtype=torch.uint8)
     s._probe = torch.zeros_like(s._ctrl)
-    s._s = lambda: None
+    s._probes, s._probe_blocks = [], []
+    s._s = lambda: C.c_void_p(0)
     return s
 
 
@@ -70,6 +71,24 @@ def test_step(first, second):
     want = [d for d in (second, first) if d < 0.0 for _ in range(2)]
     assert s.be.masked == want
     assert L.ZbCtrl.from_buffer_copy(s._ctrl.numpy().tobytes()).status == L.ZB_ST_TROUBLED
+    # the free blocks are zero, one for each call that ran at once, and serve the next calls
+    blocks = {p.data_ptr() for p, _ in s._probes}
+    assert len(blocks) == len(s._probes) == 2
+    assert not any(p.any() for p, _ in s._probes)
+    s.step(0.1, 0.0, state(2.0), None)
+    assert {p.data_ptr() for p, _ in s._probes} == blocks
+
+
+def test_a_block_waits_for_its_fill_on_another_stream(monkeypatch):
+    s = solver(HyperbolicSolver)
+    waits = []
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: waits.append(device))
+    for stream, depth in ((0, -1.0), (0, 2.0), (8, 2.0), (0, -1.0), (8, 2.0), (8, -1.0), (0, 2.0)):
+        s._s = lambda v=stream: C.c_void_p(v)
+        s.step(0.1, 0.0, state(depth), None)
+    # only a block that a troubled step zeroes on one stream and that another one takes
+    assert len(waits) == 2
+    assert len(s._probe_blocks) == 1
 
 
 @pytest.mark.parametrize("first,second", [(-1.0, 2.0), (2.0, -1.0), (-1.0, -3.0)])

@@ -253,7 +253,8 @@ class HyperbolicSolver:
         self._ws_bytes = self.be.workspace_bytes()
         self._ws = torch.empty(self._ws_bytes, dtype=torch.uint8, device=dev)
         self._ctrl = torch.zeros(L.CTRL_BYTES, dtype=torch.uint8, device=dev)
-        self._probe = torch.zeros_like(self._ctrl)    # zero: a step's own block is its copy
+        self._probe = torch.zeros_like(self._ctrl)    # zero: the blocks of _take_probe are copies
+        self._probes, self._probe_blocks = [], []     # free ones, all of them
         self._mass_part = torch.zeros(self.be.mass_partials(), dtype=torch.float64, device=dev)
         self._n = 0
         self._bed, self._bed_key = None, None
@@ -322,17 +323,34 @@ class HyperbolicSolver:
             L.ptr(self._ws), C.c_size_t(self._ws_bytes),
             L.ptr(self._ctrl if ctrl is None else ctrl), self._s()), "stage")
 
+    def _take_probe(self):
+        """A zero control block for one call's redo decision.  It is the call's until
+        :meth:`_probe_troubled` gives it back, so two threads stepping one solver
+        decide apart; the solver keeps as many as calls ran at once."""
+        import torch
+        try:
+            probe, filled = self._probes.pop()
+        except IndexError:
+            probe, filled = self._probe.clone(), None
+            self._probe_blocks.append(probe)
+        if filled is not None and filled != (self._s().value or 0):
+            torch.cuda.synchronize(probe.device)   # the fill is another stream's
+        return probe
+
     def _probe_troubled(self, probe):
         """Whether the stage that ran with the control block ``probe`` flagged a cell
         (synchronises).  Its status word replaces a reduction over the mask (18 us
         at 320 x 200, and the fill before it); a set status moves to the solver's
-        block.  The block is the call's own, a copy of the zero one: two threads
-        stepping one solver decide apart."""
+        block, and the probe is free again."""
         import torch
         i = L.ZbCtrl.status.offset // 4
         status = int(probe.view(torch.int32)[i].item())
+        filled = None       # the stream that zeroes it again
         if status:
             self._ctrl.view(torch.int32)[i].bitwise_or_(status)
+            probe.zero_()
+            filled = self._s().value or 0
+        self._probes.append((probe, filled))
         return bool(status & L.ZB_ST_TROUBLED)
 
     def _advance(self, Q, dt, force_o1=None, trouble=None, ctrl=None):
@@ -364,7 +382,7 @@ class HyperbolicSolver:
             # the last stage writes every byte of the mask; a negative dt is the
             # solver's control block's, so that block goes to the stage
             mask = torch.empty(Q.shape[1], dtype=torch.uint8, device=Q.device)
-            probe = self._probe.clone() if dt >= 0.0 else None
+            probe = self._take_probe() if dt >= 0.0 else None
             Qn = self._advance(Q, dt, trouble=mask, ctrl=probe)
             if bool(mask.any()) if probe is None else self._probe_troubled(probe):
                 Qn = self._advance(Q, dt, force_o1=mask)

@@ -110,7 +110,7 @@ class MarchSolver(HyperbolicSolver):
         hinv = Qaux[6].contiguous() if self.cfg.manning_n != 0.0 else None
         dt = float(dt)
         # a negative dt is the control block's
-        probe = self._probe.clone() if dt >= 0.0 else None
+        probe = self._take_probe() if dt >= 0.0 else None
         mask = (torch.empty(Q0.shape[1], dtype=torch.uint8, device=Q0.device)
                 if probe is None else None)
         Qk = Q0
