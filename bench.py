@@ -729,7 +729,7 @@ def run_triangles(local_rank, n_side=1415, steps=500, warmup=3, host_prep=True):
                          "unit": "GB/s", "frac": round(achieved / hbm_peak, 4),
                          "bytes_per_cell_update": 208},
             "ms_per_step": round(ms, 4), "value": cells / (ms * 1e-3),
-            "unit": "cell-updates/s", "kernels_per_step": 6, "device_copies_per_step": 1,
+            "unit": "cell-updates/s", "kernels_per_step": 6, "device_copies_per_step": 0,
             "mass_rel_change": abs(m1 - m0) / m0, "status_ok": c.status == 0,
             "dry_fraction_initial": float((state[1] <= 0).mean()),
             "mesh_generation_s": round(t_gen, 1),
